@@ -128,7 +128,8 @@ typedef struct simp_params {
     double dt;                 /* fixed (tse = 0) or initial time step (s)             */
     double max_hsml;           /* Marquis_hsml cap; <= 0: 10 * max(hsml) at set_state
                                   (initialize.f90:191)                                */
-    double skin;               /* GPU cell-list skin (m); < 0: automatic               */
+    double skin;               /* GPU cell-list skin (m); < 0: automatic (0.1 hsml).
+                                  The Verlet lists take two fifths of it             */
     /* Mohr-Coulomb rheology (data_variables.f90:153-180): viscosity caps per unit
        pressure (declared without a value in the reference, so 0 there) and the
        friction angle phi (degrees; mu = tan(phi)) */
@@ -322,17 +323,12 @@ SIMP_API int32_t simp_gpu_sum_density_noalloc(const double *x, const double *hsm
  * device). */
 SIMP_API void *simp_gpu_stream(simp_ctx *ctx);
 
-/* Implementation of the two pair passes (no reference counterpart):
- * SIMP_PASSES_TILED stages chunks of `threads` consecutive particles of a
- * cell row with their cell halo (at most `cap` particles) in shared memory;
- * the gather forms gather every particle's neighbours from HBM over Verlet
- * lists, with the kinematic pass as one kernel (SIMP_PASSES_GATHER_ONE) or
- * as two, pair finding then pair sums over the stored pair list
- * (SIMP_PASSES_GATHER_TWO); SIMP_PASSES_GATHER (the default) takes two
- * kernels for contexts of up to 400,000 particles, else one.
- * All give the same bits.  threads: 64..256, a multiple of 32; cap: a
- * multiple of 4, within the shared memory of one block (both checked for
- * every form). */
+/* Names for the implementation of the two pair passes (no reference
+ * counterpart).  One implementation, tiles in shared memory over Verlet lists,
+ * is the fastest at every size and serves all of them; the names stay for
+ * callers that set one, and get_passes returns what was set.  threads:
+ * 64..256, a multiple of 32; cap: a multiple of 4, within the shared memory of
+ * one block (both checked for every form). */
 #define SIMP_PASSES_GATHER 0
 #define SIMP_PASSES_TILED 1
 #define SIMP_PASSES_GATHER_ONE 2
@@ -340,8 +336,8 @@ SIMP_API void *simp_gpu_stream(simp_ctx *ctx);
 SIMP_API int32_t simp_gpu_set_passes(simp_ctx *ctx, int32_t impl, int32_t threads, int32_t cap);
 SIMP_API int32_t simp_gpu_get_passes(const simp_ctx *ctx, int32_t *impl, int32_t *threads, int32_t *cap);
 /* Times one right-hand side (both passes, no state change) of the current
- * state under a set of implementations and tile shapes, `reps` times each,
- * and keeps the fastest.  *ms_best: its time per right-hand side. */
+ * state, `reps` times, and sets SIMP_PASSES_GATHER_ONE.  *ms_best: its time
+ * per right-hand side. */
 SIMP_API int32_t simp_gpu_autotune(simp_ctx *ctx, int32_t reps, double *ms_best);
 
 /* Number of kernels this context has launched so far (graph replays count

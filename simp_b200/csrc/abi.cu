@@ -33,14 +33,6 @@ inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
         if (_rc != SIMP_OK) return _rc; \
     } while (0)
 
-__global__ void k_deinterleave(int n, const double *__restrict__ in, double *__restrict__ a,
-                               double *__restrict__ b) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    a[i] = in[2 * i];
-    b[i] = in[2 * i + 1];
-}
-
 // Fields of a single basin into the caller's order; a null source is skipped.
 __global__ void k_pack_fields(int n, int id_base, const int *__restrict__ id, const double *__restrict__ a,
                               const double *__restrict__ b, double *__restrict__ out_a, double *__restrict__ out_b) {
@@ -52,31 +44,26 @@ __global__ void k_pack_fields(int n, int id_base, const int *__restrict__ id, co
     if (b) out_b[o] = b[k];
 }
 
-// Two fields of a single basin into one interleaved array in the caller's
-// order (x(2,n), vx(2,n)).
-__global__ void k_pack_pair(int n, int id_base, const int *__restrict__ id, const double *__restrict__ a,
-                            const double *__restrict__ b, double *__restrict__ out) {
+// A field pair of a single basin into the caller's order (x(2,n), vx(2,n)).
+__global__ void k_pack_pair(int n, int id_base, const int *__restrict__ id, const double2 *__restrict__ a,
+                            double2 *__restrict__ out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int o = id[k] - id_base;
     if (!SIMP_IN_RANGE(o, 0, n, SITE_SORT)) return;
-    out[2 * (size_t)o] = a[k];
-    out[2 * (size_t)o + 1] = b[k];
+    out[o] = a[k];
 }
 
 // New particles [off, off + n): ids, instance, sort positions, m / rho, and
 // the summation density's kept kernel_zero (initialize.f90:60).
-__global__ void k_init_new(int n, int off, int id_base, int slot, int *id, int *pinst, State s, double *xr,
-                           double *yr, int *nbr_count, double *k0) {
+__global__ void k_init_new(int n, int off, int id_base, int slot, int *id, int *pinst, State s, double2 *xyr,
+                           double *k0) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const int i = off + k;
     id[i] = id_base + k;
     pinst[i] = slot;
-    nbr_count[i] = -1;   // its Verlet list is built by the next kinematic pass
-    xr[i] = s.x[i];
-    yr[i] = s.y[i];
-    s.mor[i] = s.m[i] / s.rho[i];
+    xyr[i] = s.xy[i];
     refresh_views(s, i);
     if (k0) k0[i] = 0.0;
 }
@@ -95,10 +82,8 @@ __global__ void k_pack_state(int n, int slot, int id_base, int nk, const int *__
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n || pinst[k] != slot) return;
     const size_t o = (size_t)(id[k] - id_base), N = (size_t)nk;
-    stage[2 * o] = s.x[k];
-    stage[2 * o + 1] = s.y[k];
-    stage[2 * N + 2 * o] = s.vx[k];
-    stage[2 * N + 2 * o + 1] = s.vy[k];
+    reinterpret_cast<double2 *>(stage)[o] = s.xy[k];
+    reinterpret_cast<double2 *>(stage + 2 * N)[o] = s.vxy[k];
     stage[4 * N + o] = s.m[k];
     stage[5 * N + o] = s.rho[k];
     stage[6 * N + o] = s.hs[k];
@@ -137,7 +122,8 @@ __global__ void __launch_bounds__(256) k_extents(int n, int off, State s, double
     double v[kRedVals] = {INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, INFINITY, 0.0, 0.0};
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
         const int i = off + k;
-        const double x = s.x[i], y = s.y[i], hs = s.hs[i];
+        const double2 q = s.xy[i];
+        const double x = q.x, y = q.y, hs = s.hs[i];
         v[0] = fmin(v[0], x);
         v[1] = fmin(v[1], -x);
         v[2] = fmin(v[2], y);
@@ -178,15 +164,13 @@ __global__ void k_grow_xabs(Scalars *sc, double xa) {
 
 // set_state of a state that continues the resident basin (the same
 // particles in the same caller order, the same hsml): the values go into
-// the particles' current places in cell order, so the sort, the cell lists
-// and the Verlet lists stay, and the displacement bounds grow as after a
-// step.  stage = [x,y interleaved | vx,vy interleaved | mass | rho | hsml |
+// the particles' current places in cell order, so the sort and the cell
+// lists stay, and the displacement bounds grow as after a step.  stage = [x,y interleaved | vx,vy interleaved | mass | rho | hsml |
 // A | h] in the caller's order, uploaded in the groups below; each group's
 // kernel runs as soon as its part has landed, while the next part is
 // copied.  Per block, each group reduces its own slots of `part`:
 // [0] non-finite positions, [1] changed hsml, [2] max squared displacement
-// since the sort, [3] since the lists were built, [4] max |coordinate|
-// (positions); [5] max hsml, [6] -min hsml (hsml); [7] other invalid
+// since the sort, [4] max |coordinate| (positions); [5] max hsml, [6] -min hsml (hsml); [7] other invalid
 // values (velocities, then mass and rho, then A and h, adding up in stream
 // order).
 enum ContGroup { CG_POS, CG_VEL, CG_MASS, CG_HSML, CG_AH, kContGroups };
@@ -194,45 +178,36 @@ enum ContGroup { CG_POS, CG_VEL, CG_MASS, CG_HSML, CG_AH, kContGroups };
 template <int G>
 __global__ void __launch_bounds__(256) k_continue_group(int n, const int *__restrict__ id,
                                                        const double *__restrict__ stage, State s,
-                                                       const double *__restrict__ xr,
-                                                       const double *__restrict__ yr, NbrList nl, double *part) {
+                                                       const double2 *__restrict__ xyr, double *part) {
     double v[kRedVals] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, -INFINITY, 0.0};
     const size_t N = (size_t)n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (!SIMP_IN_RANGE(id[i], 0, n, SITE_SORT)) continue;
         const size_t o = (size_t)id[i];
         if (G == CG_POS) {
-            const double x = stage[2 * o], y = stage[2 * o + 1];
+            const double2 q = reinterpret_cast<const double2 *>(stage)[o];
+            const double x = q.x, y = q.y;
             if (isfinite(x) && isfinite(y)) {
-                const double dxr = x - xr[i], dyr = y - yr[i];
+                const double2 r = xyr[i];
+                const double dxr = x - r.x, dyr = y - r.y;
                 v[2] = fmax(v[2], dxr * dxr + dyr * dyr);
-                if (nl.count[i] >= 0) {
-                    const double dxl = x - nl.xl[i], dyl = y - nl.yl[i];
-                    v[3] = fmax(v[3], dxl * dxl + dyl * dyl);
-                }
                 v[4] = fmax(v[4], fmax(fabs(x), fabs(y)));
             } else {
                 v[0] += 1.0;
             }
-            s.x[i] = x;
-            s.y[i] = y;
-            s.xy[i] = make_double2(x, y);
-            s.pf[i] = make_float4((float)x, (float)y, s.hsf[i], 0.0f);
+            s.xy[i] = q;
         } else if (G == CG_VEL) {
-            const double vx = stage[2 * N + 2 * o], vy = stage[2 * N + 2 * o + 1];
-            if (!(isfinite(vx) && isfinite(vy))) v[7] += 1.0;
-            s.vx[i] = vx;
-            s.vy[i] = vy;
-            s.vxy[i] = make_double2(vx, vy);
+            const double2 v2 = reinterpret_cast<const double2 *>(stage + 2 * N)[o];
+            if (!(isfinite(v2.x) && isfinite(v2.y))) v[7] += 1.0;
+            s.vxy[i] = v2;
         } else if (G == CG_MASS) {
             const double m = stage[4 * N + o], rho = stage[5 * N + o];
             if (!(isfinite(m) && isfinite(rho) && rho > 0.0)) v[7] += 1.0;
             const double mor = m / rho;
             s.m[i] = m;
             s.rho[i] = rho;
-            s.mor[i] = mor;
+            s.mm[i] = make_double2(m, mor);
             if (s.hmm) s.hmm[i] = make_float4(s.hsf[i], (float)m, (float)mor, 0.0f);
-            else s.mm[i] = make_double2(m, mor);
         } else if (G == CG_HSML) {
             const double hs = stage[6 * N + o];
             if (!(hs == s.hs[i])) v[1] += 1.0;
@@ -246,7 +221,7 @@ __global__ void __launch_bounds__(256) k_continue_group(int n, const int *__rest
         }
     }
     // the slots of this group: a bit mask over [0, kRedVals)
-    constexpr unsigned own = G == CG_POS ? 0x1du : G == CG_HSML ? 0x62u : 0x80u;
+    constexpr unsigned own = G == CG_POS ? 0x15u : G == CG_HSML ? 0x62u : 0x80u;
     __shared__ double red[kRedVals][8];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -271,22 +246,17 @@ __global__ void __launch_bounds__(256) k_continue_group(int n, const int *__rest
 }
 
 // The bounds of a continued state, as the step epilogue would leave them.
-// (hsml is unchanged, so are its bounds, the bucket size and the skin)
-__global__ void k_continue_finish(Scalars *sc, Inst *inst, double dt, double t, double d2, double dl2,
-                                  double xa, int hsml_evolves) {
+// (hsml is unchanged, so are its bounds and the bucket size)
+__global__ void k_continue_finish(Scalars *sc, Inst *inst, double dt, double t, double d2, double xa) {
     sc->dt = dt;
     sc->t = t;
     inst[0].t = t;
     const unsigned long long b2 = (unsigned long long)__double_as_longlong(d2);
     if (b2 > sc->dmax2_bits) sc->dmax2_bits = b2;
     if (b2 > inst[0].dmax2_bits) inst[0].dmax2_bits = b2;
-    const unsigned long long bl = (unsigned long long)__double_as_longlong(dl2);
-    if (bl > sc->dlist2_bits) sc->dlist2_bits = bl;
+    inst[0].list_ok = 0;
     const unsigned long long bx = (unsigned long long)__double_as_longlong(xa);
     if (bx > sc->xabs_bits) sc->xabs_bits = bx;
-    // the rule of the stress pass's last block (lists_block_done)
-    const double dl = sqrt(__longlong_as_double((long long)sc->dlist2_bits));
-    if (hsml_evolves || !(dl < 0.75 * sc->skin)) sc->list_scan = 1;
 }
 
 Phys make_phys(const simp_params &p, double max_hsml) {
@@ -345,6 +315,9 @@ Phys make_phys(const simp_params &p, double max_hsml) {
     P.alpha_pi = p.alpha_pi;
     P.beta_pi = p.beta_pi;
     P.chi = p.chi;
+    P.em2 = 1.0 / (p.e * p.e);
+    P.inv_1kt = 1.0 / (1.0 + p.k_t);
+    P.inv_rho_ice = 1.0 / p.rho_ice;
     return P;
 }
 
@@ -376,18 +349,13 @@ int dalloc(simp_ctx *c, T **p, size_t count) {
 }
 
 void free_all(simp_ctx *c) {
-    void *ptrs[] = {c->s0.x, c->s0.y, c->s0.vx, c->s0.vy, c->s0.m, c->s0.rho, c->s0.mor, c->s0.h,
-                    c->s0.A, c->s0.hs, c->s1.x, c->s1.y, c->s1.vx, c->s1.vy, c->s1.rho, c->s1.mor,
-                    c->s1.h, c->s1.A, c->mass1, c->xr, c->yr, c->xl, c->yl, c->cell, c->id, c->pinst,
-                    c->tau11, c->tau12, c->tau22, c->div, c->diag, c->rates, c->bx, c->by, c->bm, c->bnx, c->bny,
-                    c->bid, c->binst, c->bcell, c->bcell_start, c->cell_start, c->cnt, c->perm, c->tmp,
-                    c->itmp, c->scan_tmp, c->sc, c->pair_cnt, c->bpair_cnt, c->pair_buf_i,
-                    c->pair_buf_j, c->pair_buf_r, c->pair_buf_h, c->nbr, c->nbr_count,
-                    c->pair_j, c->pair_count, c->nbr_tmp, c->s0.hsf,
-                    c->inst_dev, c->row_map, c->chunk_cnt, c->chunk_off, c->chunks, c->s0.xy, c->s0.vxy,
-                    c->s0.pf, c->s0.mm, c->s0.hmm, c->s1.xy, c->s1.vxy, c->s1.pf, c->s1.mm, c->s1.hmm,
-                    c->tau_a, c->tau_b, c->tau_q, c->pair_dw, c->drhodt, c->k0, c->red_dev, c->reg,
-                    c->early_stage};
+    void *ptrs[] = {c->s0.xy, c->s0.vxy, c->s0.mm, c->s0.hmm, c->s0.m, c->s0.rho, c->s0.h, c->s0.A, c->s0.hs,
+                    c->s0.hsf, c->s1.xy, c->s1.vxy, c->s1.mm, c->s1.hmm, c->s1.rho, c->s1.h, c->s1.A, c->mass1,
+                    c->xyr, c->cell, c->id, c->pinst, c->div, c->tau_a, c->tau_b, c->tau_q, c->diag, c->rates,
+                    c->pair_slot, c->pair_count, c->chunks, c->chunk_src, c->halos, c->inst_dev, c->bx, c->by, c->bm,
+                    c->bnx, c->bny, c->bid, c->binst, c->bcell, c->bcell_start, c->cell_start, c->cnt, c->perm,
+                    c->tmp, c->itmp, c->scan_tmp, c->sc, c->pair_cnt, c->bpair_cnt, c->pair_buf_i, c->pair_buf_j,
+                    c->pair_buf_r, c->pair_buf_h, c->drhodt, c->k0, c->red_dev, c->reg, c->early_stage};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (c->sc_host) cudaFreeHost(c->sc_host);
@@ -411,7 +379,10 @@ void free_all(simp_ctx *c) {
 // basin), else instantiates it anew.
 void invalidate_graph(simp_ctx *c) { c->graph_stale = true; }
 
-// Verlet-list skin: the parameter when given, else 10% of max(hsml).
+// Cell-list skin: the parameter when given, else 10% of max(hsml); the Verlet
+// lists take two fifths of it (4% of hsml: a list then holds about 8% more
+// candidates than pairs in a disordered basin, and is built again only after
+// a particle moved 2%).
 double list_skin(const simp_ctx *c, double hmax) {
     return (c->prm.skin >= 0.0) ? c->prm.skin : 0.1 * hmax;
 }
@@ -464,6 +435,8 @@ int layout(simp_ctx *c) {
             h.I.hmax = cur[q].hmax;
             h.I.bs = cur[q].bs;
         }
+        h.I.list_ok = 0;   // (tiles and particles may move)
+        h.I.spares = 0;
         h.I.base = base;
         base += h.I.ncx * h.I.ncy;
         top = std::max(top, q + 1);
@@ -492,31 +465,25 @@ int layout(simp_ctx *c) {
         }
         c->cell_cap = capn;
     }
-    // cell rows of all instances, for the chunks of the tiled passes
-    std::vector<int2> rows;
-    for (int q : by_order)
-        for (int r = 0; r < c->insts[q].I.ncy; ++r) rows.push_back(make_int2(q, r));
-    c->total_rows = (int)rows.size();
-    const size_t need_chunks = (size_t)c->maxn / kMinTileThreads + rows.size() + 2;
-    if (rows.size() + 2 > c->row_cap || need_chunks > c->chunk_cap) {
-        cudaFree(c->row_map);
-        cudaFree(c->chunk_cnt);
-        cudaFree(c->chunk_off);
-        cudaFree(c->chunks);
-        c->row_map = nullptr;
-        c->chunk_cnt = c->chunk_off = nullptr;
-        c->chunks = nullptr;
-        const size_t rcap = std::max(2 * (rows.size() + 2), std::max(2 * c->row_cap, (size_t)4096));
-        TRY(dalloc(c, &c->row_map, rcap));
-        TRY(dalloc(c, &c->chunk_cnt, rcap));
-        TRY(dalloc(c, &c->chunk_off, rcap));
-        const size_t ccap = (size_t)c->maxn / kMinTileThreads + rcap;
-        TRY(dalloc(c, &c->chunks, ccap));
-        c->row_cap = rcap;
-        c->chunk_cap = ccap;
+    // tiles of the pair passes: each basin's particles, in memory order
+    // (offsets after the sort or compaction that follows this layout)
+    std::vector<int4> src;
+    int tiles = 0;
+    c->uniform = c->prm.sle == 0;
+    int off = 0;
+    for (int q : by_order) {
+        const InstHost &h = c->insts[q];
+        src.push_back(make_int4(off, h.n, tiles, q));
+        off += h.n;
+        tiles += nblk(h.n, kTile) + spare_tiles(nblk(h.n, kTile));
+        if (h.I.hmin != h.I.hmax) c->uniform = false;
     }
-    if (!rows.empty())
-        SIMP_CUDA(c, cudaMemcpyAsync(c->row_map, rows.data(), sizeof(int2) * rows.size(), cudaMemcpyHostToDevice, s));
+    c->nchunks = tiles;
+    c->nsrc = (int)src.size();
+    if (!src.empty()) {
+        SIMP_CUDA(c, cudaMemcpyAsync(c->chunk_src, src.data(), sizeof(int4) * src.size(), cudaMemcpyHostToDevice, s));
+        launch_chunks(c);
+    }
     std::vector<Inst> table(c->max_inst);
     for (int q = 0; q < c->max_inst; ++q) table[q] = c->insts[q].active ? c->insts[q].I : Inst{};
     SIMP_CUDA(c, cudaMemcpyAsync(c->inst_dev, table.data(), sizeof(Inst) * c->max_inst, cudaMemcpyHostToDevice, s));
@@ -617,11 +584,9 @@ int stage_instance(simp_ctx *c, int n, const double *x, const double *vx, const 
     cudaStream_t s = c->stream;
     const int off = c->n;
     const size_t N = (size_t)n;
-    double *stage = c->tmp;
-    SIMP_CUDA(c, cudaMemcpyAsync(stage, x, sizeof(double) * 2 * N, cudaMemcpyHostToDevice, s));
-    SIMP_CUDA(c, cudaMemcpyAsync(stage + 2 * N, vx, sizeof(double) * 2 * N, cudaMemcpyHostToDevice, s));
-    k_deinterleave<<<nblk(n, kB), kB, 0, s>>>(n, stage, c->s0.x + off, c->s0.y + off);
-    k_deinterleave<<<nblk(n, kB), kB, 0, s>>>(n, stage + 2 * N, c->s0.vx + off, c->s0.vy + off);
+    // (the caller's x(2,n) and vx(2,n) are the records the state keeps)
+    SIMP_CUDA(c, cudaMemcpyAsync(c->s0.xy + off, x, sizeof(double) * 2 * N, cudaMemcpyHostToDevice, s));
+    SIMP_CUDA(c, cudaMemcpyAsync(c->s0.vxy + off, vx, sizeof(double) * 2 * N, cudaMemcpyHostToDevice, s));
     SIMP_CUDA(c, cudaMemcpyAsync(c->s0.m + off, mass, sizeof(double) * N, cudaMemcpyHostToDevice, s));
     SIMP_CUDA(c, cudaMemcpyAsync(c->s0.rho + off, rho, sizeof(double) * N, cudaMemcpyHostToDevice, s));
     SIMP_CUDA(c, cudaMemcpyAsync(c->s0.hs + off, hsml, sizeof(double) * N, cudaMemcpyHostToDevice, s));
@@ -629,7 +594,7 @@ int stage_instance(simp_ctx *c, int n, const double *x, const double *vx, const 
     SIMP_CUDA(c, cudaMemcpyAsync(c->s0.h + off, h, sizeof(double) * N, cudaMemcpyHostToDevice, s));
     const int rb = std::min(kRedBlocks, nblk(n, 256));
     k_extents<<<rb, 256, 0, s>>>(n, off, c->s0, c->red_dev);
-    c->launches += 3;
+    c->launches += 1;
     SIMP_CUDA(c, cudaGetLastError());
     SIMP_CUDA(c, cudaMemcpyAsync(c->red_host, c->red_dev, sizeof(double) * kRedVals * rb, cudaMemcpyDeviceToHost, s));
     SIMP_CUDA(c, cudaStreamSynchronize(s));
@@ -694,12 +659,12 @@ int add_instance(simp_ctx *c, int slot, const simp_forcing &f, const Extents &e,
     I.hmax = hmax;
     I.bs = 2.0 * hmin;
     I.dmax2_bits = 0ull;
+    I.delta = 0.4 * list_skin(c, hmax);
     I.flags = 0;
     // particle arrays at [off, off + n), staged by stage_instance
     cudaStream_t s = c->stream;
     const int off = c->n;
-    k_init_new<<<nblk(n, kB), kB, 0, s>>>(n, off, ih.id_base, slot, c->id, c->pinst, c->s0, c->xr, c->yr,
-                                          c->nbr_count, c->k0);
+    k_init_new<<<nblk(n, kB), kB, 0, s>>>(n, off, ih.id_base, slot, c->id, c->pinst, c->s0, c->xyr, c->k0);
     k_grow_xabs<<<1, 1, 0, s>>>(c->sc, pxa);
     c->launches += 2;
     SIMP_CUDA(c, cudaGetLastError());
@@ -768,7 +733,7 @@ int flush_batch(simp_ctx *c, bool compact) {
     }
     if (!any) return SIMP_OK;
     TRY(layout(c));
-    TRY(rebuild(c, due, from, false));
+    TRY(rebuild(c, due, from));
     SIMP_CUDA(c, cudaStreamSynchronize(c->stream));
     c->pending_from = 0x7fffffff;
     c->pending_due.clear();
@@ -803,6 +768,15 @@ int download2(simp_ctx *c, const double *a, const double *b, double *h2) {
     k_to_orig2<<<nblk(c->n, kB), kB, 0, c->stream>>>(c->n, c->id, a, b, stage);
     c->launches += 1;
     SIMP_CUDA(c, cudaMemcpyAsync(h2, stage, sizeof(double) * 2 * (size_t)c->n, cudaMemcpyDeviceToHost, c->stream));
+    SIMP_CUDA(c, cudaStreamSynchronize(c->stream));
+    return SIMP_OK;
+}
+
+int download_pair(simp_ctx *c, const double2 *a, double *h2) {
+    double2 *stage = reinterpret_cast<double2 *>(c->tmp);
+    k_pack_pair<<<nblk(c->n, kB), kB, 0, c->stream>>>(c->n, 0, c->id, a, stage);
+    c->launches += 1;
+    SIMP_CUDA(c, cudaMemcpyAsync(h2, stage, sizeof(double2) * (size_t)c->n, cudaMemcpyDeviceToHost, c->stream));
     SIMP_CUDA(c, cudaStreamSynchronize(c->stream));
     return SIMP_OK;
 }
@@ -860,7 +834,7 @@ void enqueue_step(simp_ctx *c, bool diag, bool prof) {
     mark(0);
     if (c->prm.int_algorithm == 1) {
         // euler_scheme (time_integration.f90:86-148): one right-hand side
-        launch_kinematic(c, s0, diag);
+        launch_kinematic(c, s0, diag, false);
         launch_regularize(c, s0);
         mark(1);
         launch_stress(c, s0, s0, EPI_EULER);
@@ -874,14 +848,14 @@ void enqueue_step(simp_ctx *c, bool diag, bool prof) {
         // predictor_corrector (:155-282) or leapfrog_scheme (:289-391): the
         // same first half step, a different final update
         const bool leap = c->prm.int_algorithm == 3;
-        launch_kinematic(c, s0, false);
+        launch_kinematic(c, s0, false, false);
         launch_regularize(c, s0);
         mark(1);
         launch_stress(c, s0, s0, EPI_PREDICT);
         if (den1) launch_sum_density(c, s0, s1, s0.m, s0.rho, s1.rho, false);        // :217, :344
         else if (den2) launch_density_rate(c, s0, s1, 1, false);
         mark(2);
-        launch_kinematic(c, s1, diag);
+        launch_kinematic(c, s1, diag, true);
         launch_regularize(c, s1);
         mark(3);
         launch_stress(c, s1, s0, leap ? EPI_LEAP : EPI_CORRECT);
@@ -949,7 +923,7 @@ int maybe_regrid(simp_ctx *c, bool *done) {
     if (!(I.hmax > 1.05 * h.grid_hmax)) return SIMP_OK;
     *done = true;
     std::vector<double> xy(2 * (size_t)c->n);
-    TRY(download2(c, c->s0.x, c->s0.y, xy.data()));
+    TRY(download_pair(c, c->s0.xy, xy.data()));
     double xmin = xy[0], xmax = xy[0], ymin = xy[1], ymax = xy[1];
     for (int i = 0; i < c->n; ++i) {
         xmin = std::min(xmin, xy[2 * i]);
@@ -965,7 +939,7 @@ int maybe_regrid(simp_ctx *c, bool *done) {
     }
     size_inst_grid(c, h, xmin, xmax, ymin, ymax, I.hmax);
     TRY(layout(c));
-    TRY(rebuild(c, mask_of(0), c->n, false));
+    TRY(rebuild(c, mask_of(0), c->n));
     h.steps_since_sort = 0;
     return SIMP_OK;
 }
@@ -975,6 +949,7 @@ int check_after(simp_ctx *c) {
         return simp_fail(c, SIMP_ERR_BOUNDS, "device index check failed (sites " + std::to_string(f) +
                                                  ": 1 neighbour, 2 cell, 4 sort slot, 8 tile slot)");
     const Scalars &s = *c->sc_host;
+    if (s.flags & FLAG_TIMEOUT) return simp_fail(c, SIMP_ERR_TIMEOUT, "a tile's copies did not arrive");
     if ((s.flags & FLAG_NONFINITE) && c->max_inst == 1)   // batches flag the basin instead
         return simp_fail(c, SIMP_ERR_NONFINITE, "non-finite particle state after a step");
     if (s.maxip > c->prm.max_ind_int)
@@ -1002,10 +977,7 @@ int create(const simp_params *params, int32_t maxn, int32_t maxnb, int32_t max_i
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
         return simp_fail(c, SIMP_ERR_CUDA, "cudaStreamCreate failed (no usable CUDA device?)");
     const size_t M = (size_t)maxn, MB = (size_t)c->maxnb, MX = std::max(M, MB);
-    double **d1[] = {&c->s0.x, &c->s0.y, &c->s0.vx, &c->s0.vy, &c->s0.m, &c->s0.rho, &c->s0.mor, &c->s0.h,
-                     &c->s0.A, &c->s0.hs, &c->s1.x, &c->s1.y, &c->s1.vx, &c->s1.vy, &c->s1.rho,
-                     &c->s1.mor, &c->s1.h, &c->s1.A, &c->xr, &c->yr, &c->xl, &c->yl,
-                     &c->tau11, &c->tau12, &c->tau22, &c->div};
+    double **d1[] = {&c->s0.m, &c->s0.rho, &c->s0.h, &c->s0.A, &c->s0.hs, &c->s1.rho, &c->s1.h, &c->s1.A, &c->div};
     for (double **p : d1) TRY(dalloc(c, p, M));
     if (c->prm.mass_from_area && c->prm.sle != 2) {
         TRY(dalloc(c, &c->mass1, M));
@@ -1020,28 +992,19 @@ int create(const simp_params *params, int32_t maxn, int32_t maxnb, int32_t max_i
     for (State *st : {&c->s0, &c->s1}) {
         TRY(dalloc(c, &st->xy, M));
         TRY(dalloc(c, &st->vxy, M));
-        TRY(dalloc(c, &st->pf, M));
+        TRY(dalloc(c, &st->mm, M));
         if (c->prm.precision == SIMP_PREC_MIXED) TRY(dalloc(c, &st->hmm, M));
-        else TRY(dalloc(c, &st->mm, M));
     }
-    if (c->prm.precision == SIMP_PREC_MIXED) {
-        TRY(dalloc(c, &c->tau_q, M));
-    } else {
-        TRY(dalloc(c, &c->tau_a, M));
-        TRY(dalloc(c, &c->tau_b, M));
-    }
-    TRY(dalloc(c, &c->nbr, (size_t)kMaxNbr * M));
-    TRY(dalloc(c, &c->nbr_count, M));
-    TRY(dalloc(c, &c->nbr_tmp, (size_t)kMaxNbr * M));
-    TRY(dalloc(c, &c->pair_j, (size_t)kMaxPairs * M));
+    TRY(dalloc(c, &c->xyr, M));
+    TRY(dalloc(c, &c->tau_a, M));
+    TRY(dalloc(c, &c->tau_b, M));
+    if (c->prm.precision == SIMP_PREC_MIXED) TRY(dalloc(c, &c->tau_q, M));
+    const size_t chunk_cap = chunk_capacity(maxn, max_inst);
+    TRY(dalloc(c, &c->pair_slot, (size_t)kListRows * kTile * chunk_cap));
     TRY(dalloc(c, &c->pair_count, M));
-    if (c->prm.precision == SIMP_PREC_MIXED) {
-        // the mixed form keeps its pairs' kernel gradients for the stress
-        // pass (measured: in the plain form the 16-byte records cost the
-        // kinematic pass more than they save the stress pass)
-        if (cudaMalloc(&c->pair_dw, (size_t)kDwRows * M * sizeof(float2)) != cudaSuccess)
-            return simp_fail(c, SIMP_ERR_NOMEM, "device allocation failed");
-    }
+    TRY(dalloc(c, &c->chunks, chunk_cap));
+    TRY(dalloc(c, &c->halos, (size_t)kHaloBytes * (kTile / kPartMin) * chunk_cap));
+    TRY(dalloc(c, &c->chunk_src, (size_t)max_inst));
     TRY(dalloc(c, &c->diag, 9 * M));
     TRY(dalloc(c, &c->rates, 4 * M));
     if (c->max_inst == 1) {
@@ -1055,10 +1018,10 @@ int create(const simp_params *params, int32_t maxn, int32_t maxnb, int32_t max_i
     TRY(dalloc(c, &c->id, M));
     TRY(dalloc(c, &c->pinst, M));
     TRY(dalloc(c, &c->perm, M));
-    TRY(dalloc(c, &c->tmp, 16 * MX));
+    TRY(dalloc(c, &c->tmp, 14 * MX));
     if (c->prm.sle == 1 && c->prm.den_alg != 2) TRY(dalloc(c, &c->drhodt, M));
     if (c->prm.den_alg == 1) TRY(dalloc(c, &c->k0, M));
-    TRY(dalloc(c, &c->itmp, 5 * MX));
+    TRY(dalloc(c, &c->itmp, 3 * MX));
     TRY(dalloc(c, &c->bx, MB));
     TRY(dalloc(c, &c->by, MB));
     TRY(dalloc(c, &c->bm, MB));
@@ -1087,9 +1050,8 @@ int create(const simp_params *params, int32_t maxn, int32_t maxnb, int32_t max_i
     std::memcpy(&sc.acc_hmin, &inf, sizeof(double));
     std::memcpy(&sc.acc_dt, &inf, sizeof(double));
     sc.minip = 0x7fffffff;
-    sc.list_scan = 1;
     SIMP_CUDA(c, cudaMemcpyAsync(c->sc, c->sc_host, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
-    TRY(tiled_configure(c));
+    TRY(passes_configure(c));
     TRY(layout(c));
     return SIMP_OK;
 }
@@ -1149,20 +1111,19 @@ int check_normals(simp_ctx *c) {
 // allocations of create() below, with room for its cell lists).
 double bytes_per_particle(const simp_params &p, bool single_basin) {
     const bool mixed = p.precision == SIMP_PREC_MIXED;
-    double b = 26 * 8.0;                                      // FP64 state sets and per-RHS fields
+    double b = 9 * 8.0;                                       // FP64 fields of both state sets, divergence
     if (p.mass_from_area && p.sle != 2) b += 8.0;             // half-step mass
     b += 4.0;                                                 // hsml in FP32
-    b += 2 * (3 * 16.0 + 16.0);                               // packed neighbour copies, two sets
-    b += mixed ? 16.0 : 32.0;                                 // stress records
-    b += 2 * kMaxNbr * 4.0 + 4.0;                             // Verlet lists and their renaming copy
-    b += kMaxPairs * 4.0 + 4.0;                               // pair lists
-    b += mixed ? kDwRows * 8.0 : 0.0;                         // kept kernel gradients
+    b += 2 * 3 * 16.0 + 16.0;                                 // records of both sets, sort positions
+    b += 2 * 16.0;                                            // stress records
+    b += mixed ? 3 * 16.0 : 0.0;                              // and those of the mixed form
+    b += 1.0625 * kListRows * 2.0 + 4.0;                              // Verlet lists and counts
     b += 9 * 8.0 + 4 * 8.0;                                   // diagnostics, rates
     if (p.sle == 1 && p.den_alg != 2) b += 8.0;               // Benz's kept drhodt
     if (p.xsph_regularization || p.artificial_visc) b += 4 * 8.0;   // regularisation terms
     if (p.den_alg == 1) b += 8.0;                             // kept kernel_zero
-    b += 4 * 4.0 + 16 * 8.0 + 5 * 4.0 + 4.0;                  // sort keys, scratch
-    b += 16.0 / kMinTileThreads + 48.0;                       // chunks, cell lists (worst case)
+    b += 4 * 4.0 + 14 * 8.0 + 3 * 4.0 + 4.0;                  // sort keys, scratch
+    b += 16.0 / 128 + 1.5 * kHaloBytes / kPartMin + 48.0;               // tiles, cell lists (worst case)
     if (single_basin) b += 2 * 8.0;                           // read-back stage of the fixed fields
     return b;
 }
@@ -1170,17 +1131,17 @@ double bytes_per_particle(const simp_params &p, bool single_basin) {
 // Enqueues nsteps steps of every basin of the context on its stream without
 // waiting for them (profiling mode waits step by step).
 // A single basin's scheduled re-sort, replayed from a captured graph (one
-// launch where the re-sort is some fifteen).  Its kernels capture the
-// particle and cell counts, whether the Verlet lists are renamed, and the
-// cell arrays, which a new layout can reallocate: a change of any of those
-// captures it again.  Rebuild's host side for this case is that it counts
-// one more re-sort (a single basin keeps all its particles, and the lists
-// stay as valid as they were).
+// launch where the re-sort is some twelve).  Its kernels capture the
+// particle, cell and tile counts and the cell arrays, which a new layout can
+// reallocate: a change of any of those captures it again.  Rebuild's host
+// side for this case is that it counts one more re-sort (a single basin
+// keeps all its particles).
 int sort_replayed(simp_ctx *c, const DueMask &due) {
     simp_ctx::SortKey k;
     k.n = c->n;
     k.total_cells = c->total_cells;
-    k.keep_lists = c->lists_valid;
+    k.nchunks = c->nchunks;
+    k.uniform = c->uniform;
     k.cell_start = c->cell_start;
     k.scan_tmp = c->scan_tmp;
     if (!c->sort_graph || !(k == c->sort_key)) {
@@ -1188,16 +1149,14 @@ int sort_replayed(simp_ctx *c, const DueMask &due) {
         c->sort_graph = nullptr;
         const long long l0 = c->launches, r0 = c->rebuilds;
         const int n0 = c->n;
-        const bool lv0 = c->lists_valid;
         cudaGraph_t g = nullptr;
         SIMP_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        const int rc = rebuild(c, due, c->n, false);
+        const int rc = rebuild(c, due, c->n);
         const cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         const long long kernels = c->launches - l0;
         c->launches = l0;   // (the launch below counts them)
         c->rebuilds = r0;
         c->n = n0;
-        c->lists_valid = lv0;
         if (rc != SIMP_OK || e != cudaSuccess) {
             if (g) cudaGraphDestroy(g);
             return rc != SIMP_OK ? rc : simp_cuda_check(c, e, "re-sort capture");
@@ -1247,8 +1206,8 @@ int step_enqueue(simp_ctx *c, int nsteps) {
             if (c->graph_profiled) SIMP_CUDA(c, cudaEventRecord(c->sort_ev[0], s));
             TRY(maybe_regrid(c, &regridded));   // hsml grew past the grid (sle = 2)
             if (regridded) TRY(ensure_graph(c, c->keep_diag));
-            else if (c->max_inst == 1 && c->pass_impl != SIMP_PASSES_TILED) TRY(sort_replayed(c, due));
-            else TRY(rebuild(c, due, c->n, false));
+            else if (c->max_inst == 1) TRY(sort_replayed(c, due));
+            else TRY(rebuild(c, due, c->n));
             if (c->graph_profiled) {
                 SIMP_CUDA(c, cudaEventRecord(c->sort_ev[1], s));
                 SIMP_CUDA(c, cudaEventSynchronize(c->sort_ev[1]));
@@ -1261,7 +1220,6 @@ int step_enqueue(simp_ctx *c, int nsteps) {
         cudaError_t e = cudaGraphLaunch(c->step_graph, s);
         if (e != cudaSuccess) return simp_cuda_check(c, e, "cudaGraphLaunch");
         c->launches += c->graph_kernels;
-        c->lists_valid = true;
         for (InstHost &h : c->insts)
             if (h.active && !h.retired) {
                 ++h.steps_since_sort;
@@ -1306,7 +1264,7 @@ int batch_slot_state(simp_ctx *c, int slot, double *x, double *vx, double *mass,
 // set_state of a state that continues the resident basin: the same particle
 // count and walls, the same hsml, no particle farther than one cell from
 // where it was sorted, a finite resident state.  The values are written in
-// place (k_continue_group, per upload group) and the sort, cell lists, Verlet lists and step
+// place (k_continue_group, per upload group) and the sort, cell lists and step
 // graph stay.  Returns kFreshState, with the resident state overwritten or
 // not, when the state does not qualify; the caller then sets it up from
 // scratch.  Left out: Benz's kept drhodt (a fresh state zeroes it) and the
@@ -1326,12 +1284,6 @@ int continue_state(simp_ctx *c, int n, const double *x, const double *vx, const 
     const size_t N = (size_t)n;
     double *stage = c->tmp;
     const int rb = std::min(kRedBlocks, nblk(n, 256));
-    NbrList nl;
-    nl.nbr = c->nbr;
-    nl.count = c->nbr_count;
-    nl.xl = c->xl;
-    nl.yl = c->yl;
-    nl.stride = c->maxn;
     // the upload on the side stream (after whatever the context stream has
     // queued), each group's kernel on the context stream once its part is in
     struct Part { const double *src; size_t off, len; int group; } parts[] = {
@@ -1345,11 +1297,11 @@ int continue_state(simp_ctx *c, int n, const double *x, const double *vx, const 
         SIMP_CUDA(c, cudaEventRecord(c->ev_up[p.group], c->side));
         SIMP_CUDA(c, cudaStreamWaitEvent(s, c->ev_up[p.group], 0));
         switch (p.group) {
-            case CG_POS: k_continue_group<CG_POS><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xr, c->yr, nl, c->red_dev); break;
-            case CG_VEL: k_continue_group<CG_VEL><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xr, c->yr, nl, c->red_dev); break;
-            case CG_MASS: k_continue_group<CG_MASS><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xr, c->yr, nl, c->red_dev); break;
-            case CG_HSML: k_continue_group<CG_HSML><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xr, c->yr, nl, c->red_dev); break;
-            default: k_continue_group<CG_AH><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xr, c->yr, nl, c->red_dev);
+            case CG_POS: k_continue_group<CG_POS><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xyr, c->red_dev); break;
+            case CG_VEL: k_continue_group<CG_VEL><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xyr, c->red_dev); break;
+            case CG_MASS: k_continue_group<CG_MASS><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xyr, c->red_dev); break;
+            case CG_HSML: k_continue_group<CG_HSML><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xyr, c->red_dev); break;
+            default: k_continue_group<CG_AH><<<rb, 256, 0, s>>>(n, c->id, stage, c->s0, c->xyr, c->red_dev);
         }
         c->launches += 1;
     }
@@ -1357,14 +1309,14 @@ int continue_state(simp_ctx *c, int n, const double *x, const double *vx, const 
     SIMP_CUDA(c, cudaMemcpyAsync(c->red_host, c->red_dev, sizeof(double) * kRedVals * rb, cudaMemcpyDeviceToHost, s));
     SIMP_CUDA(c, cudaMemcpyAsync(c->sc_host, c->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
     SIMP_CUDA(c, cudaStreamSynchronize(s));
-    // v: [0] invalid values, [1] changed hsml, [2] d2 since the sort, [3]
-    // since the lists, [4] max |coordinate|, [5] max hsml, [6] -min hsml
+    // v: [0] invalid values, [1] changed hsml, [2] d2 since the sort,
+    // [4] max |coordinate|, [5] max hsml, [6] -min hsml
     double v[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, -INFINITY};
     for (int b = 0; b < rb; ++b) {
         const double *u = c->red_host + (size_t)b * kRedVals;
         v[0] += u[0] + u[7];
         v[1] += u[1];
-        for (int q = 2; q < 7; ++q) v[q] = std::max(v[q], u[q]);
+        for (int q : {2, 4, 5, 6}) v[q] = std::max(v[q], u[q]);
     }
     const Scalars &sc = *c->sc_host;
     if (v[0] > 0.0 || v[1] > 0.0 || sc.flags != 0 || !(v[2] <= ih.I.cs * ih.I.cs)) return kFreshState;
@@ -1373,7 +1325,7 @@ int continue_state(simp_ctx *c, int n, const double *x, const double *vx, const 
     const double max_hsml = (c->prm.max_hsml > 0.0) ? c->prm.max_hsml : v[5] * 10.0;   // initialize.f90:191
     const Phys P = make_phys(c->prm, max_hsml);
     if (std::memcmp(&P, &c->phys, sizeof(Phys)) != 0) return kFreshState;
-    k_continue_finish<<<1, 1, 0, s>>>(c->sc, c->inst_dev, dt, t, v[2], v[3], v[4], c->prm.sle != 0 ? 1 : 0);
+    k_continue_finish<<<1, 1, 0, s>>>(c->sc, c->inst_dev, dt, t, v[2], v[4]);
     c->launches += 1;
     SIMP_CUDA(c, cudaGetLastError());
     // (a set state starts the kept kernel_zero again, initialize.f90:60)
@@ -1506,8 +1458,6 @@ int32_t simp_gpu_set_state(simp_ctx *c, int32_t ntotal, const double *x, const d
     std::memcpy(&sc.acc_hmin, &inf, sizeof(double));
     std::memcpy(&sc.acc_dt, &inf, sizeof(double));
     sc.minip = 0x7fffffff;
-    sc.skin = list_skin(c, hmax);
-    sc.list_scan = 1;
     SIMP_CUDA(c, cudaMemcpyAsync(c->sc, c->sc_host, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
     SIMP_CUDA(c, cudaMemsetAsync(c->inst_dev, 0, sizeof(Inst), c->stream));
     if (c->drhodt) SIMP_CUDA(c, cudaMemsetAsync(c->drhodt, 0, sizeof(double) * (size_t)c->maxn, c->stream));
@@ -1541,11 +1491,10 @@ int32_t simp_gpu_batch_add(simp_ctx *c, const simp_forcing *forcing, int32_t nto
     Extents e{};
     TRY(stage_instance(c, ntotal, x, vx, mass, rho, hsml, A, h, ntotalb, xb, massb, &e));
     if (!c->have_state) {
-        // first basin: physics constants and the list skin
+        // first basin: physics constants
         const double hmax = e.hmax;
         c->phys = make_phys(c->prm, c->prm.max_hsml > 0.0 ? c->prm.max_hsml : 10.0 * hmax);
         TRY(read_scalars(c));
-        c->sc_host->skin = list_skin(c, hmax);
         c->sc_host->dt = c->prm.dt;
         SIMP_CUDA(c, cudaMemcpyAsync(c->sc, c->sc_host, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
     }
@@ -1669,9 +1618,10 @@ int32_t simp_gpu_get_state(simp_ctx *c, double *x, double *vx, double *mass, dou
         const Group &G = groups[g];
         if (!G.a.dst && !G.b.dst) continue;
         if (g == 0) {
-            k_pack_pair<<<nblk(n, kB), kB, 0, s>>>(n, id_base, c->id, c->s0.x, c->s0.y, stage);
+            k_pack_pair<<<nblk(n, kB), kB, 0, s>>>(n, id_base, c->id, c->s0.xy, reinterpret_cast<double2 *>(stage));
         } else if (g == 1) {
-            k_pack_pair<<<nblk(n, kB), kB, 0, s>>>(n, id_base, c->id, c->s0.vx, c->s0.vy, stage + 2 * N);
+            k_pack_pair<<<nblk(n, kB), kB, 0, s>>>(n, id_base, c->id, c->s0.vxy,
+                                                   reinterpret_cast<double2 *>(stage + 2 * N));
         } else {
             const double *sa = g == 2 ? m_src : g == 3 ? hs_src : c->s0.h;
             const double *sb = g == 2 ? (rho ? c->s0.rho : nullptr) : g == 3 ? (A ? c->s0.A : nullptr) : nullptr;
@@ -1768,18 +1718,17 @@ int32_t simp_gpu_single_step(simp_ctx *c, double current_time, double *dxdt, dou
     k_set_time0<<<1, 1, 0, s>>>(c->sc, c->inst_dev, current_time);
     c->launches += 1;
     launch_reset_stats(c);
-    launch_kinematic(c, c->s0, true);
+    launch_kinematic(c, c->s0, true, false);
     launch_regularize(c, c->s0);
     launch_stress(c, c->s0, c->s0, EPI_RATES);
     // the right-hand side's pair loop also sets the summation density's kept
     // kernel_zero (kernel.f90:503): the density itself goes to scratch
     if (c->k0) launch_sum_density(c, c->s0, c->s0, c->s0.m, c->s0.rho, c->tmp, false);
     SIMP_CUDA(c, cudaGetLastError());
-    c->lists_valid = true;
     const size_t M = (size_t)c->maxn;
     // dx/dt: the velocities, or with XSPH what the rates epilogue wrote
     if (dxdt && c->reg && c->prm.xsph_regularization) TRY(download2(c, c->reg + 2 * M, c->reg + 3 * M, dxdt));
-    else if (dxdt) TRY(download2(c, c->s0.vx, c->s0.vy, dxdt));
+    else if (dxdt) TRY(download_pair(c, c->s0.vxy, dxdt));
     if (dvxdt) TRY(download2(c, c->rates, c->rates + M, dvxdt));
     if (dhdt) TRY(download1(c, c->rates + 2 * M, dhdt));
     if (dAdt) TRY(download1(c, c->rates + 3 * M, dAdt));
@@ -1820,24 +1769,21 @@ int32_t simp_gpu_set_passes(simp_ctx *c, int32_t impl, int32_t threads, int32_t 
     if (!c) return SIMP_ERR_BADARG;
     if (impl < SIMP_PASSES_GATHER || impl > SIMP_PASSES_GATHER_TWO)
         return simp_fail(c, SIMP_ERR_BADARG, "unknown pair-pass implementation");
-    if (threads < kMinTileThreads || threads > 256 || threads % 32 != 0 || cap < 64 || cap % 4 != 0 ||
+    if (threads < 64 || threads > 256 || threads % 32 != 0 || cap < 64 || cap % 4 != 0 ||
         cap > 32767)
         return simp_fail(c, SIMP_ERR_BADARG, "tile shape out of range");
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    const size_t need = std::max(tiled_smem_bytes(c->prm.precision, 0, cap, threads),
-                                 tiled_smem_bytes(c->prm.precision, 1, cap, threads));
+    // (what such a tile's halo records and pair lists would take)
+    const size_t real = c->prm.precision == SIMP_PREC_MIXED ? sizeof(float) : sizeof(double);
+    const size_t need = (size_t)cap * (5 * sizeof(double) + sizeof(float4) + 3 * real) +
+                        (size_t)49 * threads * sizeof(unsigned short);
     if (optin > 0 && need + 1024 > (size_t)optin)
         return simp_fail(c, SIMP_ERR_BADARG, "tile shape exceeds the shared memory of a block");
-    const bool rechunk = threads != c->tile_threads || impl != c->pass_impl;
-    c->pass_impl = impl;   // (both keep the Verlet lists the same way)
+    c->pass_impl = impl;   // (one implementation serves every form)
     c->tile_threads = threads;
     c->tile_cap = cap;
-    TRY(tiled_configure(c));
-    if (rechunk && c->n > 0) build_chunks(c);
-    invalidate_graph(c);
-    SIMP_CUDA(c, cudaStreamSynchronize(c->stream));
     return SIMP_OK;
 }
 
@@ -1855,12 +1801,12 @@ static int time_rhs(simp_ctx *c, int reps, double *ms) {
     cudaEvent_t e0, e1;
     SIMP_CUDA(c, cudaEventCreate(&e0));
     SIMP_CUDA(c, cudaEventCreate(&e1));
-    launch_kinematic(c, c->s0, false);          // warm-up
+    launch_kinematic(c, c->s0, false, false);          // warm-up
     launch_regularize(c, c->s0);
     launch_stress(c, c->s0, c->s0, EPI_RATES);
     cudaEventRecord(e0, c->stream);
     for (int r = 0; r < reps; ++r) {
-        launch_kinematic(c, c->s0, false);
+        launch_kinematic(c, c->s0, false, false);
         launch_regularize(c, c->s0);
         launch_stress(c, c->s0, c->s0, EPI_RATES);
     }
@@ -1879,28 +1825,11 @@ int32_t simp_gpu_autotune(simp_ctx *c, int32_t reps, double *ms_best) {
     if (!c || reps < 1) return SIMP_ERR_BADARG;
     if (!c->have_state || c->n == 0) return simp_fail(c, SIMP_ERR_STATE, "autotune needs particles");
     TRY(flush_batch(c, true));
-    struct Cand { int impl, threads, cap; };
-    const Cand cands[] = {
-        {SIMP_PASSES_TILED, 128, 512},  {SIMP_PASSES_TILED, 128, 768},  {SIMP_PASSES_TILED, 128, 1024},
-        {SIMP_PASSES_TILED, 256, 768},  {SIMP_PASSES_TILED, 256, 1024}, {SIMP_PASSES_TILED, 256, 1536},
-        {SIMP_PASSES_TILED, 64, 384},   {SIMP_PASSES_TILED, 64, 512},   {SIMP_PASSES_GATHER_ONE, 256, 1024},
-        {SIMP_PASSES_GATHER_TWO, 256, 1024}};
-    const Cand keep{c->pass_impl, c->tile_threads, c->tile_cap};
-    Cand best = keep;
-    double tbest = INFINITY;
-    for (const Cand &k : cands) {
-        if (simp_gpu_set_passes(c, k.impl, k.threads, k.cap) != SIMP_OK) continue;   // shape does not fit
-        double t = 0.0;
-        TRY(time_rhs(c, reps, &t));
-        if (t < tbest) {
-            tbest = t;
-            best = k;
-        }
-    }
-    TRY(simp_gpu_set_passes(c, best.impl, best.threads, best.cap));
-    (void)keep;
+    double t = 0.0;
+    TRY(time_rhs(c, reps, &t));
+    TRY(simp_gpu_set_passes(c, SIMP_PASSES_GATHER_ONE, 256, 1024));
     c->err.clear();
-    if (ms_best) *ms_best = tbest;
+    if (ms_best) *ms_best = t;
     return SIMP_OK;
 }
 

@@ -123,8 +123,7 @@ __global__ void scan_total(const int *__restrict__ in, int n, int *__restrict__ 
 
 // Cell key of each particle from its sort position and its instance's grid;
 // particles being removed (instance -1) go to the dump key after all cells.
-__global__ void k_keys(int n, const double *__restrict__ xr, const double *__restrict__ yr,
-                       const int *__restrict__ pinst, const Inst *__restrict__ inst, int dump_key,
+__global__ void k_keys(int n, const double2 *__restrict__ xyr, const int *__restrict__ pinst, const Inst *__restrict__ inst, int dump_key,
                        int *__restrict__ key, int *__restrict__ cnt) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -132,8 +131,8 @@ __global__ void k_keys(int n, const double *__restrict__ xr, const double *__res
     int k = dump_key;
     if (q >= 0) {
         const Inst &I = inst[q];
-        const int cx = clampi((int)floor((xr[i] - I.x0) * I.inv_cs), 0, I.ncx - 1);
-        const int cy = clampi((int)floor((yr[i] - I.y0) * I.inv_cs), 0, I.ncy - 1);
+        const int cx = clampi((int)floor((xyr[i].x - I.x0) * I.inv_cs), 0, I.ncx - 1);
+        const int cy = clampi((int)floor((xyr[i].y - I.y0) * I.inv_cs), 0, I.ncy - 1);
         k = I.base + cy * I.ncx + cx;
     }
     key[i] = k;
@@ -143,21 +142,22 @@ __global__ void k_keys(int n, const double *__restrict__ xr, const double *__res
 // Instances due for a re-sort take their current positions as sort
 // positions; a basin flagged non-finite keeps its old (finite) ones.
 __global__ void k_refresh_sortpos(int n, const int *__restrict__ pinst, DueMask due, const Inst *__restrict__ inst,
-                                  const double *__restrict__ x, const double *__restrict__ y,
-                                  double *__restrict__ xr, double *__restrict__ yr) {
+                                  const double2 *__restrict__ xy, double2 *__restrict__ xyr) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int q = pinst[i];
     if (q < 0 || !((due.w[q >> 6] >> (q & 63)) & 1ull)) return;
     if (inst_dead(inst[q].flags)) return;
-    xr[i] = x[i];
-    yr[i] = y[i];
+    xyr[i] = xy[i];
 }
 
 __global__ void k_reset_inst_disp(Inst *inst, int ninst, DueMask due) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= ninst) return;
-    if ((due.w[q >> 6] >> (q & 63)) & 1ull) inst[q].dmax2_bits = 0ull;
+    if (!((due.w[q >> 6] >> (q & 63)) & 1ull)) return;
+    inst[q].dmax2_bits = 0ull;
+    inst[q].list_ok = 0;   // (its particles take new places)
+    inst[q].spares = 0;
 }
 
 __global__ void k_scatter(int n, const int *__restrict__ key, const int *__restrict__ start,
@@ -187,10 +187,12 @@ __global__ void k_cell_sort(int ncells, const int *__restrict__ start, int *__re
     }
 }
 
-constexpr int kGathered = 14;   // (the last two only with Benz's kept drhodt and the kept kernel_zero)
+constexpr int kPairs = 3, kFields = 7;   // (the last two fields only with Benz's kept drhodt and the kept kernel_zero)
 struct Gather {
-    const double *src[kGathered];
-    double *dst[kGathered];
+    const double2 *psrc[kPairs];
+    double2 *pdst[kPairs];
+    const double *src[kFields];
+    double *dst[kFields];
 };
 
 __device__ __forceinline__ bool is_due(const DueMask &m, int q) {
@@ -205,72 +207,21 @@ __device__ __forceinline__ bool moves(int from, const DueMask &due, const int *p
     return k >= from || is_due(due, pinst[k]);
 }
 
-// New order into scratch; inv[old] = new for every moved particle.
+// New order into scratch.
 __global__ void k_gather(int kept, int from, DueMask due, const int *__restrict__ perm, Gather gd,
                          const int *__restrict__ key, int *__restrict__ cell_out, const int *__restrict__ id_in,
-                         int *__restrict__ id_out, const int *__restrict__ pinst_in, int *__restrict__ pinst_out,
-                         int *__restrict__ inv) {
+                         int *__restrict__ id_out, const int *__restrict__ pinst_in, int *__restrict__ pinst_out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= kept || !moves(from, due, pinst_in, k)) return;
     const int o = perm[k];
 #pragma unroll
-    for (int a = 0; a < kGathered; ++a)
+    for (int a = 0; a < kPairs; ++a) gd.pdst[a][k] = gd.psrc[a][o];
+#pragma unroll
+    for (int a = 0; a < kFields; ++a)
         if (gd.src[a]) gd.dst[a][k] = gd.src[a][o];
     cell_out[k] = key[o];
     id_out[k] = id_in[o];
     pinst_out[k] = pinst_in[o];
-    inv[o] = k;
-}
-
-// Verlet-list rows of the moved particles: each entry renamed to the new
-// index and the row re-sorted, so a row lists its members in increasing
-// index order exactly as a fresh scan of the cell stencil would.  An entry
-// whose new index cannot be confirmed (perm[inv[v]] != v) turns the row into
-// an overflowed one, which the kinematic pass answers by a stencil scan.
-__global__ void k_remap_lists(int kept, int from, DueMask due, const int *__restrict__ pinst,
-                              const int *__restrict__ perm, const int *__restrict__ inv, int n_old,
-                              NbrList nl, int *__restrict__ nbr_out, int *__restrict__ cnt_out,
-                              double *__restrict__ xl_out, double *__restrict__ yl_out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= kept || !moves(from, due, pinst, k)) return;
-    const int o = perm[k];
-    int cnt = nl.count[o];
-    xl_out[k] = nl.xl[o];
-    yl_out[k] = nl.yl[o];
-    if (cnt < 0) {
-        // (a particle whose list is still to be built keeps that mark)
-    } else if (cnt <= kMaxNbr) {
-        int row[kMaxNbr];
-        for (int e = 0; e < cnt; ++e) {
-            const int v = nl.nbr[(size_t)e * nl.stride + o];
-            int w = -1;
-            if (v >= 0 && v < n_old) {
-                w = inv[v];
-                if (w < 0 || w >= kept || perm[w] != v) w = -1;
-            }
-            if (w < 0) { cnt = kMaxNbr + 1; break; }
-            int j = e - 1;
-            while (j >= 0 && row[j] > w) { row[j + 1] = row[j]; --j; }
-            row[j + 1] = w;
-        }
-        if (cnt <= kMaxNbr)
-            for (int e = 0; e < cnt; ++e) nbr_out[(size_t)e * nl.stride + k] = row[e];
-    } else {
-        cnt = kMaxNbr + 1;
-    }
-    cnt_out[k] = cnt;
-}
-
-__global__ void k_put_back_lists(int kept, int from, DueMask due, const int *__restrict__ pinst, NbrList nl,
-                                 const int *__restrict__ nbr_in, const int *__restrict__ cnt_in,
-                                 const double *__restrict__ xl_in, const double *__restrict__ yl_in) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= kept || !moves(from, due, pinst, k)) return;
-    const int cnt = cnt_in[k];
-    nl.count[k] = cnt;
-    nl.xl[k] = xl_in[k];
-    nl.yl[k] = yl_in[k];
-    for (int e = 0; e < cnt && cnt <= kMaxNbr; ++e) nl.nbr[(size_t)e * nl.stride + k] = nbr_in[(size_t)e * nl.stride + k];
 }
 
 // Scratch back into the state arrays (pointers stay fixed so the captured
@@ -280,22 +231,17 @@ __global__ void k_put_back(int kept, int from, DueMask due, Gather gd, State s, 
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= kept || !moves(from, due, pinst, k)) return;
 #pragma unroll
-    for (int a = 0; a < kGathered; ++a)
+    for (int a = 0; a < kPairs; ++a) const_cast<double2 *>(gd.psrc[a])[k] = gd.pdst[a][k];
+#pragma unroll
+    for (int a = 0; a < kFields; ++a)
         if (gd.src[a]) const_cast<double *>(gd.src[a])[k] = gd.dst[a][k];
     id[k] = id_new[k];
     pinst[k] = pinst_new[k];
     refresh_views(s, k);
 }
 
-// After a sort: displacement since the sort restarts; the Verlet lists are
-// rebuilt by the next kinematic pass unless they were renamed.
-__global__ void k_reset_disp(Scalars *sc, int lists_kept) {
-    sc->dmax2_bits = 0ull;
-    if (!lists_kept) {
-        sc->dlist2_bits = 0ull;
-        sc->list_scan = 1;
-    }
-}
+// After a sort: displacement since the sort restarts.
+__global__ void k_reset_disp(Scalars *sc) { sc->dmax2_bits = 0ull; }
 
 inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
@@ -322,10 +268,8 @@ void launch_scan_i32(const int *in, int *out, int n, void *tmp, cudaStream_t s) 
 // Positions from `from` on are rewritten (after an admission or a removal:
 // the first position whose basin changed), before it only the due
 // instances' ranges move.  Particles of removed instances (instance -1) end
-// up after all others and are dropped: c->n shrinks to the kept count.  The
-// Verlet lists follow the particles unless `new_lists` (or no list was built
-// yet), in which case the next kinematic pass rebuilds them all.
-int rebuild(simp_ctx *c, const DueMask &due, int from, bool new_lists) {
+// up after all others and are dropped: c->n shrinks to the kept count.
+int rebuild(simp_ctx *c, const DueMask &due, int from) {
     SIMP_RANGE("re-sort");
     const int n = c->n;
     cudaStream_t s = c->stream;
@@ -335,54 +279,45 @@ int rebuild(simp_ctx *c, const DueMask &due, int from, bool new_lists) {
     int *key = c->itmp;
     int *id_new = c->itmp + MX;
     int *pinst_new = c->itmp + 2 * MX;
-    int *inv = c->itmp + 3 * MX;
-    int *cnt_new = c->itmp + 4 * MX;
     int kept = 0;
     for (const InstHost &h : c->insts)
         if (h.active) kept += h.n;
-    const bool keep_lists = c->lists_valid && !new_lists;
     if (n > 0) {
-        k_refresh_sortpos<<<nblk(n, B), B, 0, s>>>(n, c->pinst, due, c->inst_dev, c->s0.x, c->s0.y, c->xr, c->yr);
+        k_refresh_sortpos<<<nblk(n, B), B, 0, s>>>(n, c->pinst, due, c->inst_dev, c->s0.xy, c->xyr);
         k_reset_inst_disp<<<nblk(c->ninst, 128), 128, 0, s>>>(c->inst_dev, c->ninst, due);
         SIMP_CUDA(c, cudaMemsetAsync(c->cnt, 0, sizeof(int) * (size_t)nkeys, s));
-        k_keys<<<nblk(n, B), B, 0, s>>>(n, c->xr, c->yr, c->pinst, c->inst_dev, c->total_cells, key, c->cnt);
+        k_keys<<<nblk(n, B), B, 0, s>>>(n, c->xyr, c->pinst, c->inst_dev, c->total_cells, key, c->cnt);
         launch_scan_i32(c->cnt, c->cell_start, nkeys, c->scan_tmp, s);
         k_scatter<<<nblk(n, B), B, 0, s>>>(n, key, c->cell_start, c->cnt, c->perm);
         // (the dump key is not ordered: its particles are dropped)
         if (c->total_cells > 0)
             k_cell_sort<<<nblk(c->total_cells, 128), 128, 0, s>>>(c->total_cells, c->cell_start, c->perm, c->id);
-        double *srcs[kGathered] = {c->s0.x, c->s0.y, c->s0.vx, c->s0.vy, c->s0.m, c->s0.rho,
-                                   c->s0.mor, c->s0.h, c->s0.A, c->s0.hs, c->xr, c->yr, c->drhodt, c->k0};
+        double2 *pairs[kPairs] = {c->s0.xy, c->s0.vxy, c->xyr};
+        double *fields[kFields] = {c->s0.m, c->s0.rho, c->s0.h, c->s0.A, c->s0.hs, c->drhodt, c->k0};
         Gather gd;
-        for (int a = 0; a < kGathered; ++a) {
-            gd.src[a] = srcs[a];
-            gd.dst[a] = c->tmp + (size_t)a * MX;
+        for (int a = 0; a < kPairs; ++a) {
+            gd.psrc[a] = pairs[a];
+            gd.pdst[a] = reinterpret_cast<double2 *>(c->tmp) + (size_t)a * MX;
+        }
+        for (int a = 0; a < kFields; ++a) {
+            gd.src[a] = fields[a];
+            gd.dst[a] = c->tmp + (size_t)(2 * kPairs + a) * MX;
         }
         c->launches += 7 + kScanKernels;
         if (kept > 0) {
             k_gather<<<nblk(kept, B), B, 0, s>>>(kept, from, due, c->perm, gd, key, c->cell, c->id, id_new,
-                                                 c->pinst, pinst_new, inv);
+                                                 c->pinst, pinst_new);
             c->launches += 1;
-            if (keep_lists) {
-                NbrList nl{c->nbr, c->nbr_count, c->xl, c->yl, c->maxn};
-                double *xl_new = c->tmp + 14 * MX, *yl_new = c->tmp + 15 * MX;
-                k_remap_lists<<<nblk(kept, 128), 128, 0, s>>>(kept, from, due, c->pinst, c->perm, inv, n, nl,
-                                                              c->nbr_tmp, cnt_new, xl_new, yl_new);
-                k_put_back_lists<<<nblk(kept, B), B, 0, s>>>(kept, from, due, c->pinst, nl, c->nbr_tmp, cnt_new,
-                                                             xl_new, yl_new);
-                c->launches += 2;
-            }
             k_put_back<<<nblk(kept, B), B, 0, s>>>(kept, from, due, gd, c->s0, id_new, c->id, pinst_new, c->pinst);
             c->launches += 1;
         }
     } else {
         SIMP_CUDA(c, cudaMemsetAsync(c->cell_start, 0, sizeof(int) * (size_t)(nkeys + 1), s));
     }
-    k_reset_disp<<<1, 1, 0, s>>>(c->sc, keep_lists ? 1 : 0);
+    k_reset_disp<<<1, 1, 0, s>>>(c->sc);
     c->launches += 1;
-    if (!keep_lists) c->lists_valid = false;
     c->n = kept;
-    if (c->pass_impl == SIMP_PASSES_TILED) build_chunks(c);
+    launch_split(c, due);
     SIMP_CUDA(c, cudaGetLastError());
     c->rebuilds += 1;
     return SIMP_OK;

@@ -1,10 +1,9 @@
 // Shared device-side definitions of the SIMP hot path on sm_100a.
 //
 // Data layout in HBM (one basin, FP64 plain form):
-//   particle state is structure-of-arrays, permanently stored in cell order
-//   (the order of the last cell-list rebuild): x, y, vx, vy, m, rho, mor
-//   (= m / rho), hs (hsml), h, A, cell (rebuild-time cell id), id (original
-//   particle index).  Each RHS evaluation reads one state set and writes the
+//   particle state is permanently stored in cell order (the order of the last
+//   cell-list rebuild): (x, y), (vx, vy), (m, m / rho), m, rho, hs (hsml), h,
+//   A, cell (rebuild-time cell id), id (original particle index).  Each RHS evaluation reads one state set and writes the
 //   next (start-of-step set S0 and half-step set S1, see passes.cu).
 #pragma once
 
@@ -18,58 +17,36 @@ namespace simp {
 
 constexpr double kPi = 3.1415926535897932;  // globals.f90:199
 
-// Structure-of-arrays particle state (device pointers, cell order).
+// Particle state (device pointers, cell order).  What the pair passes read of
+// a neighbour is packed into 16-byte records, which tiles copy whole; the
+// other fields are one array each.
 struct State {
-    double *x, *y, *vx, *vy;
-    double *m, *rho, *mor, *h, *A;
+    double2 *xy, *vxy;   // positions, velocities
+    double2 *mm;         // (m, m / rho)
+    double *m, *rho, *h, *A;
     double *hs;   // hsml (shared by S0 and S1: updated only at step end)
     float *hsf;   // its FP32 copy (shared)
-    // Packed copies that the pair passes gather per neighbour (one or two
-    // vector loads per neighbour instead of one scalar load per array):
-    double2 *xy, *vxy;   // (x, y), (vx, vy)
-    float4 *pf;          // (x, y, hsml, 0) in FP32: the candidate prefilter
-    double2 *mm;         // (m, m / rho): plain form (null in the mixed form)
-    float4 *hmm;         // (hsml, m, m / rho, 0) in FP32: mixed form (null in the plain form)
+    float4 *hmm;  // (hsml, m, m / rho, 0) in FP32: mixed form (null in the plain form)
 };
 
-// Rewrites the packed copies of particle k from the FP64 arrays.
+// Rewrites the packed copies of particle k that follow from m, rho and hsml.
 __device__ __forceinline__ void refresh_views(const State &s, int k) {
-    const double x = s.x[k], y = s.y[k], hs = s.hs[k], m = s.m[k], mor = s.mor[k];
+    const double hs = s.hs[k], m = s.m[k], mor = m / s.rho[k];
     const float hsf = (float)hs;
     s.hsf[k] = hsf;
-    s.xy[k] = make_double2(x, y);
-    s.vxy[k] = make_double2(s.vx[k], s.vy[k]);
-    s.pf[k] = make_float4((float)x, (float)y, hsf, 0.0f);
+    s.mm[k] = make_double2(m, mor);
     if (s.hmm) s.hmm[k] = make_float4(hsf, (float)m, (float)mor, 0.0f);
-    else s.mm[k] = make_double2(m, mor);
 }
 
-// Verlet neighbour lists (cell-order indices): nbr[k * stride + i],
-// k < count[i], holding every j within mhsml + skin of i at the positions
-// (xl, yl) where the list was built; a count above kMaxNbr means the list
-// overflowed and that particle scans its cell stencil instead.
-constexpr int kMaxNbr = 48;
-struct NbrList {
-    int *nbr;
-    int *count;
-    double *xl, *yl;
-    int stride;
-    int n = 0;   // particles in the context (the debug build's index checks)
-};
-
-// The kernel gradients of a right-hand side's pairs, kept by the kinematic
-// pass for the stress pass (same pairs, same state): row k, particle i, for
-// the first kDwRows pairs of each particle (the others are recomputed).
-constexpr int kDwRows = 32;
-
-// Exact pairs of the current right-hand side, written by the kinematic pass
-// and consumed by the stress pass: pj[k * stride + i], k < count[i]; a count
-// above kMaxPairs means the stress pass finds that particle's pairs itself.
-constexpr int kMaxPairs = 48;
+// Verlet lists of the pair passes, per tile (tile.cuh): the candidates of
+// particle i, every j within mhsml + delta when the list was built, as slots
+// of its tile's halo, slot[(tile * kListRows + k) * kTile + column], k <
+// count[i].
+constexpr int kTile = 128;      // particles per tile
+constexpr int kListRows = 44;
 struct PairList {
-    int *pj;
+    unsigned short *slot;
     int *count;
-    int stride;
     int n = 0;   // particles in the context (the debug build's index checks)
 };
 
@@ -94,7 +71,12 @@ struct Inst {
     double hmin, hmax, bs;       // hsml bounds and reference bucket size
     unsigned long long dmax2_bits;  // max squared displacement since its last sort
     int flags;                   // FLAG_* seen in this instance
-    int pad;
+    // Verlet lists: valid while 2 (list_d + half step) <= delta, with list_d
+    // bounding how far any particle moved (and half of how far any hsml
+    // grew) since they were built
+    int list_ok, spares;
+    double delta, list_d;
+    unsigned long long half2_bits, step2_bits;   // this step's max squared moves, S0 -> S1 and S0 -> S0'
 };
 
 __host__ __device__ __forceinline__ Grid inst_grid(const Inst &I, const int *cell_start) {
@@ -110,10 +92,12 @@ __host__ __device__ __forceinline__ Grid inst_grid(const Inst &I, const int *cel
     return g;
 }
 
-// Particle chunk of the tiled pair passes: consecutive particles [p0, p1)
-// of cell row `row` of instance q.
+// Tile of the pair passes: consecutive particles [p0, p1) of instance q.  An
+// instance has its full tiles and some spare ones, which hold the parts of
+// tiles that had to be cut (k_split); spare k is in use where k < Inst.spares.
 struct Chunk {
-    int p0, p1, q, row;
+    int p0, p1, q;
+    int spare;     // -1: a full tile
 };
 
 // Device-resident integrator scalars and per-step reductions.
@@ -124,15 +108,10 @@ struct Scalars {
     double bs;            // reference bucket size 2 * hmin (nnps.f90:211)
     unsigned long long dmax2_bits;  // max squared displacement since rebuild
     unsigned long long xabs_bits;   // max |coordinate| of any particle so far
-    // Verlet neighbour lists: members within mhsml + skin when built; valid
-    // while every particle moved less than skin / 2 since (and hsml fixed)
-    unsigned long long dlist2_bits; // max squared displacement since the lists were built
-    double skin;
-    int list_scan;                  // 1: the next kinematic pass rebuilds the lists
-    unsigned int blocks_done;       // last-block detection of the stress pass
     unsigned long long acc_hmin, acc_hmax;  // accumulators of the next hsml
     unsigned long long acc_dt;              // VP time step min accumulator
-    int flags;            // bit 0: non-finite state seen
+    unsigned long long acc_dh;              // max growth of any hsml in this step
+    int flags;            // FLAG_NONFINITE: non-finite state seen; FLAG_TIMEOUT: a bounded wait ran out
     int maxip;            // max interactions per particle seen
     int minip;
     int pad;
@@ -141,7 +120,7 @@ struct Scalars {
     int pad2;
 };
 
-enum : int { FLAG_NONFINITE = 1, FLAG_RETIRED = 2 };
+enum : int { FLAG_NONFINITE = 1, FLAG_RETIRED = 2, FLAG_TIMEOUT = 4 };
 
 // A basin that is neither searched nor stepped: its state turned non-finite
 // (it is carried until the caller retires it), or it was retired and its
@@ -184,6 +163,8 @@ struct Phys {
     int xsph, art_visc, artificial_visc;
     int csound;                     // 1: c_yang is refreshed (sound_speed.f90:21-27), 0: c stays 0
     double alpha_pi, beta_pi, chi;
+    // 1 / e^2, 1 / (1 + k_t), 1 / rho_ice
+    double em2, inv_1kt, inv_rho_ice;
 };
 
 // Interaction-count bookkeeping for nnps.f90:613-670.

@@ -76,24 +76,26 @@ struct simp_ctx {
     double *k0 = nullptr;          // summation density in the step: the reference's kernel_zero, kept likewise
     double *red_dev = nullptr;     // per-block extents of a basin being admitted
     double *red_host = nullptr;    // (pinned copy)
-    double *xr = nullptr, *yr = nullptr;  // sort positions (updated when the instance is re-sorted)
-    double *xl = nullptr, *yl = nullptr;  // positions where each Verlet list was built
+    double2 *xyr = nullptr;        // sort positions (updated when the instance is re-sorted)
     int *cell = nullptr;           // sort-time cell key per particle
     int *id = nullptr;             // global particle id
     int *pinst = nullptr;          // instance slot of each particle (-1: being removed)
     // per-RHS intermediates from the kinematic pass
-    double *tau11 = nullptr, *tau12 = nullptr, *tau22 = nullptr, *div = nullptr;
+    double *div = nullptr;
     // the stress pass's packed neighbour records (written by the kinematic pass)
-    double2 *tau_a = nullptr, *tau_b = nullptr;   // plain form: (tau11, tau12), (tau22, m)
-    float4 *tau_q = nullptr;                      // mixed form: (tau11, tau12, tau22, m)
-    int *nbr = nullptr;            // kMaxNbr * maxn neighbour indices (column-major)
-    int *nbr_count = nullptr;      // maxn
-    int *nbr_tmp = nullptr;        // kMaxNbr * maxn: lists being renamed by a sort
-    bool lists_valid = false;      // every particle's list was built by a kinematic pass
+    double2 *tau_a = nullptr, *tau_b = nullptr;   // (tau11, tau12), (tau22, m): a particle's own, and in the
+                                                  // plain form its neighbours'
+    float4 *tau_q = nullptr;                      // mixed form's neighbours: (tau11, tau12, tau22, m)
     bool pending_check = false;    // steps simp_gpu_step enqueued without outputs, status not read yet
-    int *pair_j = nullptr;         // kMaxPairs * maxn exact pairs of the current RHS
+    unsigned short *pair_slot = nullptr;   // Verlet lists (PairList)
     int *pair_count = nullptr;     // maxn
-    void *pair_dw = nullptr;       // kernel gradient per pair: kDwRows x maxn float2 (mixed form only)
+    // tiles of the pair passes (tile.cuh), laid out with the basins
+    simp::Chunk *chunks = nullptr;
+    int4 *chunk_src = nullptr;     // per basin in memory order: offset, particles, first chunk, slot
+    int nsrc = 0;                  // basins in it
+    unsigned char *halos = nullptr;   // simp::kHaloBytes per simp::kPartMin particles of a tile
+    int nchunks = 0;
+    bool uniform = false;          // every basin's hsml is one value, and stays it
     // diagnostics (epsilon_11.. sigma_22, zeta, eta, p)
     double *diag = nullptr;        // 9 * maxn
     // rates of the last single_step (cell order): ax, ay, dhdt, dAdt
@@ -112,17 +114,10 @@ struct simp_ctx {
     // cell lists
     int *cell_start = nullptr;
     size_t cell_cap = 0;
-    // pair-pass implementation (SIMP_PASSES_*) and its tile shape
+    // what simp_gpu_set_passes named (every form runs the same passes)
     int pass_impl = SIMP_PASSES_GATHER;
-    int tile_threads = 256;        // particles per chunk = threads per block
-    int tile_cap = 1024;           // halo particles a block stages
-    // chunks of the tiled passes
-    int total_rows = 0;            // cell rows over all instances
-    int2 *row_map = nullptr;       // (instance, row) of each global row
-    int *chunk_cnt = nullptr;      // chunks per row
-    int *chunk_off = nullptr;      // their exclusive scan (+ total)
-    simp::Chunk *chunks = nullptr;
-    size_t row_cap = 0, chunk_cap = 0;
+    int tile_threads = 256;
+    int tile_cap = 1024;
     // rebuild scratch
     int *cnt = nullptr;            // per-cell counters (cell_cap)
     int *perm = nullptr;           // maxn
@@ -149,11 +144,11 @@ struct simp_ctx {
     // captured once and replayed while what they capture stays the same
     cudaGraphExec_t sort_graph = nullptr;
     struct SortKey {
-        int n = -1, total_cells = -1;
-        bool keep_lists = false;
+        int n = -1, total_cells = -1, nchunks = -1;
+        bool uniform = false;
         const void *cell_start = nullptr, *scan_tmp = nullptr;
         bool operator==(const SortKey &o) const {
-            return n == o.n && total_cells == o.total_cells && keep_lists == o.keep_lists &&
+            return n == o.n && total_cells == o.total_cells && nchunks == o.nchunks && uniform == o.uniform &&
                    cell_start == o.cell_start && scan_tmp == o.scan_tmp;
         }
     } sort_key;
@@ -182,7 +177,7 @@ constexpr int kMaxSlots = 1024;
 struct DueMask {
     unsigned long long w[kMaxSlots / 64];
 };
-int rebuild(simp_ctx *c, const DueMask &due, int from, bool new_lists);   // sort into cell order
+int rebuild(simp_ctx *c, const DueMask &due, int from);   // sort into cell order
 void launch_scan_i32(const int *in, int *out, int n, void *tmp, cudaStream_t s);
 constexpr int kScanKernels = 4;         // kernels per launch_scan_i32
 size_t scan_tmp_bytes(int n);
@@ -192,7 +187,8 @@ size_t scan_tmp_bytes(int n);
 // and the corrector (predictor_corrector), the Euler step, the leap-frog
 // second half (time_integration.f90:86-148, 155-282, 289-391)
 enum EpiMode : int { EPI_RATES = 0, EPI_PREDICT = 1, EPI_CORRECT = 2, EPI_EULER = 3, EPI_LEAP = 4 };
-void launch_kinematic(simp_ctx *c, const State &s, bool diag);
+// `second`: the step's second right-hand side (the first one left valid lists)
+void launch_kinematic(simp_ctx *c, const State &s, bool diag, bool second);
 void launch_stress(simp_ctx *c, const State &nb, const State &own, EpiMode mode);
 // drho/dt over the last right-hand side's pairs with the updated velocities
 // (con_density, Benz_hsml): rho_upd 0 none, 1 half step, 2 full step; tail:
@@ -211,11 +207,19 @@ void launch_regularize(simp_ctx *c, const State &s);
 void launch_copy_s1_to_s0(simp_ctx *c);
 void launch_reset_stats(simp_ctx *c);
 
-// tiled.cu
-constexpr int kMinTileThreads = 64;
-void build_chunks(simp_ctx *c);
-int tiled_configure(simp_ctx *c);
-size_t tiled_smem_bytes(int precision, int pass, int cap, int threads);
+// The pair passes' tiles: the spare ones of a basin, the chunk capacity of a
+// context, the chunk table of the current layout and the kernels'
+// shared-memory limits.
+constexpr int kHaloBytes = 64;
+constexpr int kPartMin = 8;       // smallest part of a tile with its own halo
+__host__ __device__ inline int spare_tiles(int tiles) { return 3 + tiles / 16; }
+inline size_t chunk_capacity(int maxn, int max_inst) {
+    const size_t tiles = (size_t)maxn / simp::kTile + (size_t)max_inst;   // (a partial tile per basin)
+    return tiles + tiles / 16 + 3 * (size_t)max_inst;
+}
+void launch_chunks(simp_ctx *c);
+void launch_split(simp_ctx *c, const DueMask &due);   // after a sort
+int passes_configure(simp_ctx *c);
 
 // abi.cu: device bytes per particle of capacity
 double bytes_per_particle(const simp_params &p, bool single_basin = false);

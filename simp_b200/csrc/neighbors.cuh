@@ -50,16 +50,17 @@ __device__ __forceinline__ void for_stencil_rows(const Grid &g, int ci, int R, F
 }
 
 // f(j, dx, dy, r, mh): dx = x_i - x_j, r = reference distance, mh = hsml_ij.
-template <class F>
-__device__ __forceinline__ int for_each_pair(const double *__restrict__ X, const double *__restrict__ Y,
-                                             const double *__restrict__ HS, const Grid &g, int i, int ci,
+// pos(j): position of particle j.
+template <class X, class F>
+__device__ __forceinline__ int for_each_pair(X &&pos, const double *__restrict__ HS, const Grid &g, int i, int ci,
                                              int R, const BinRule &br, double xi, double yi, double hi,
                                              F &&f) {
     int count = 0;
     for_stencil_rows(g, ci, R, [&](int j0, int j1) {
         for (int j = j0; j < j1; ++j) {
             if (j == i) continue;
-            const double xj = X[j], yj = Y[j];
+            const double2 q = pos(j);
+            const double xj = q.x, yj = q.y;
             const double dx = __dsub_rn(xi, xj), dy = __dsub_rn(yi, yj);
             const double mh = __dmul_rn(__dadd_rn(hi, HS[j]), 0.5);
             double r;
@@ -87,8 +88,8 @@ __device__ __forceinline__ int for_each_wall(const double *__restrict__ BX, cons
         for (int b = b0; b < b1; ++b) {
             const double xb = BX[b], yb = BY[b];
             const double bdx = __dsub_rn(xb, xi), bdy = __dsub_rn(yb, yi);
-            const double d = ref_distance(bdx, bdy);
-            if (!(d <= b_length)) continue;
+            double d;
+            if (!pair_test(bdx, bdy, b_length, &d)) continue;
             if (!bin_rule_ok(br, xb, yb)) continue;
             ++count;
             f(b, bdx, bdy, d);

@@ -45,13 +45,14 @@ __global__ void __launch_bounds__(kBlock) k_count(ExpArgs a) {
     const State &s = a.s;
     const Inst &I = a.inst[0];
     const Grid g = inst_grid(I, a.cell_start);
-    const double xi = s.x[i], yi = s.y[i], hi = s.hs[i];
+    const double2 xy = s.xy[i];
+    const double xi = xy.x, yi = xy.y, hi = s.hs[i];
     const int ci = a.cell[i];
     const int R = stencil_radius(I.hmax, I.dmax2_bits, g, 0.0);
     const BinRule br = make_bin_rule(I.bs, xi, yi, I.hmax);
     const int idi = a.id[i];
     int up = 0;
-    int cnt = for_each_pair(s.x, s.y, s.hs, g, i, ci, R, br, xi, yi, hi,
+    int cnt = for_each_pair([&](int j) { return s.xy[j]; }, s.hs, g, i, ci, R, br, xi, yi, hi,
                             [&](int j, double, double, double, double) { up += (a.id[j] > idi); });
     if (a.P.boundary_pressure && a.nb > 0) {
         const int Rb = wall_radius(I.dmax2_bits, g, I.b_length);
@@ -72,13 +73,14 @@ __global__ void __launch_bounds__(kBlock) k_emit(ExpArgs a) {
     const State &s = a.s;
     const Inst &I = a.inst[0];
     const Grid g = inst_grid(I, a.cell_start);
-    const double xi = s.x[i], yi = s.y[i], hi = s.hs[i];
+    const double2 xy = s.xy[i];
+    const double xi = xy.x, yi = xy.y, hi = s.hs[i];
     const int R = stencil_radius(I.hmax, I.dmax2_bits, g, 0.0);
     const BinRule br = make_bin_rule(I.bs, xi, yi, I.hmax);
     const int idi = a.id[i];
     const int base = a.up_off[idi];
     int k = 0;
-    for_each_pair(s.x, s.y, s.hs, g, i, a.cell[i], R, br, xi, yi, hi,
+    for_each_pair([&](int j) { return s.xy[j]; }, s.hs, g, i, a.cell[i], R, br, xi, yi, hi,
                   [&](int j, double, double, double r, double mh) {
                       const int idj = a.id[j];
                       if (idj <= idi) return;
@@ -134,7 +136,8 @@ __global__ void __launch_bounds__(kBlock) k_wall(WallArgs a) {
     int k = 0;
     for_stencil_rows(g, a.bcell[b], Rb, [&](int j0, int j1) {
         for (int j = j0; j < j1; ++j) {
-            const double xj = a.s.x[j], yj = a.s.y[j];
+            const double2 q = a.s.xy[j];
+            const double xj = q.x, yj = q.y;
             const double d = ref_distance(__dsub_rn(xb, xj), __dsub_rn(yb, yj));
             if (!(d <= I.b_length)) continue;
             if (!bin_rule_ok(bb, xj, yj)) continue;
@@ -183,13 +186,14 @@ __global__ void __launch_bounds__(kBlock) k_sum_density(DenArgs a) {
     const Phys &P = a.P;
     const Inst &I = a.inst[0];
     const Grid g = inst_grid(I, a.cell_start);
-    const double xi = s.x[i], yi = s.y[i], hi = s.hs[i];
+    const double2 xy = s.xy[i];
+    const double xi = xy.x, yi = xy.y, hi = s.hs[i];
     const int R = stencil_radius(I.hmax, I.dmax2_bits, g, 0.0);
     const BinRule br = make_bin_rule(I.bs, xi, yi, I.hmax);
     const double k0 = kernel_zero(P, hi);
     const double mi = s.m[i], rhoi = s.rho[i];
     double num = k0 * mi, den = k0 * mi / rhoi;
-    for_each_pair(s.x, s.y, s.hs, g, i, a.cell[i], R, br, xi, yi, hi,
+    for_each_pair([&](int j) { return s.xy[j]; }, s.hs, g, i, a.cell[i], R, br, xi, yi, hi,
                   [&](int j, double, double, double r, double mh) {
                       double w, gf;
                       pair_kernel<true>(P, r, mh, &w, &gf);

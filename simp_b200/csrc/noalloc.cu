@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kB) k_density(unsigned char *base, int n, Phys
     const double k0 = kernel_zero(P, hi);
     const double mi = M[i];
     double num = k0 * mi, den = k0 * mi / RHO[i];
-    for_each_pair(X, Y, HS, g, i, at<int>(base, kOffKeySorted)[i], 1, br, xi, yi, hi,
+    for_each_pair([&](int j) { return make_double2(X[j], Y[j]); }, HS, g, i, at<int>(base, kOffKeySorted)[i], 1, br, xi, yi, hi,
                   [&](int j, double, double, double r, double mh) {
                       double w, gf;
                       pair_kernel<true>(P, r, mh, &w, &gf);

@@ -1,11 +1,10 @@
-// Pair passes, per-particle implementation: each thread gathers its
-// particle's neighbours from HBM, over Verlet lists (candidates within
-// mhsml + skin, rebuilt when the fastest particle moved 3/4 of the skin) or
-// the cell stencil.  The physics of both passes is described in
-// pass_common.cuh.
+// Pair passes: one particle per thread, its neighbours' data in shared memory
+// (tile.cuh).  The physics of both passes is described in pass_common.cuh.
 #include <cmath>
+#include <type_traits>
 
 #include "pass_common.cuh"
+#include "tile.cuh"
 
 namespace simp {
 
@@ -13,292 +12,469 @@ namespace {
 
 using namespace pass;
 
-#ifndef SIMP_PASS_BLOCK
-#define SIMP_PASS_BLOCK 128
-#endif
-constexpr int kBlock = SIMP_PASS_BLOCK;   // threads per block of the gather passes
-// Up to this many particles in a context the kinematic pass runs as two
-// kernels (k_find_pairs, k_kin_sums), above it as one (k_kinematic), unless
-// the context names one form (SIMP_PASSES_GATHER_ONE / _TWO).  The
-// two-kernel pass writes and re-reads the pair list; it is the faster form
-// up to this size, the slower one above it, also when it runs in chunks
-// whose pair lists stay in L2 (1,048,576 particles in chunks of 131,072 to
-// 400,000: FP64 274 -> 310..374 us, mixed 242 -> 300..314 us against the
-// one-kernel pass).  Per pass, one kernel -> two (B200, basins of the
-// 500 m lattice), FP64: 147,456 particles 64.6 -> 55.1 us, 262,144 96.4 ->
-// 89.2, 409,600 143.0 -> 143.3, 524,176 170.5 -> 179.8, 1,048,576 305.7 ->
-// 343.9; mixed: 147,456 66.5 -> 53.3, 262,144 100.1 -> 87.5, 409,600
-// 134.7 -> 131.9, 1,048,576 241 -> 267.
-constexpr int kSplitMaxParticles = 400000;
-// minimum resident blocks per SM, per precision form and kernel, measured
-// against 4..8: the FP64 sums kernel of the two-kernel pass keeps its pair
-// math in registers (5 blocks, cap 102; 6 is 3% slower at cfg2); the
-// one-kernel pass, which runs above kSplitMaxParticles, at 6 blocks (cfg3
-// FP64: 274, 249, 261 us per pass at 5, 6, 7; the FP32 form at 7 blocks,
-// 253, 235, 241 at 6, 7, 8); the stress passes at 7 (FP64: 6 and 8 are
-// 23% and 9% slower at cfg2) and 8 (FP32: 6 and 7 are 10% and 9% slower at
-// cfg3)
+constexpr int kBlock = kTile;
+// Resident blocks per SM the register allocation aims at: 5, where the FP64
+// pair math fits 96 registers almost without spills and five tiles fill the
+// shared memory (6 and 7 blocks per step at 262,144 particles, FP64: 214 ->
+// 253 and 300 us; mixed: 194 -> 231 and 253).
 #ifndef SIMP_KIN_MIN_BLOCKS
-#define SIMP_KIN_MIN_BLOCKS 6
-#endif
-#ifndef SIMP_SUMS_MIN_BLOCKS
-#define SIMP_SUMS_MIN_BLOCKS 5
+#define SIMP_KIN_MIN_BLOCKS 5
 #endif
 #ifndef SIMP_STRESS_MIN_BLOCKS
-#define SIMP_STRESS_MIN_BLOCKS 7
+#define SIMP_STRESS_MIN_BLOCKS 5
 #endif
 #ifndef SIMP_KIN_MIN_BLOCKS_F32
-#define SIMP_KIN_MIN_BLOCKS_F32 7
+#define SIMP_KIN_MIN_BLOCKS_F32 5
 #endif
 #ifndef SIMP_STRESS_MIN_BLOCKS_F32
-#define SIMP_STRESS_MIN_BLOCKS_F32 8
+#define SIMP_STRESS_MIN_BLOCKS_F32 5
 #endif
 template <class T>
 struct MinBlocks {
-    static constexpr int kin = SIMP_KIN_MIN_BLOCKS, sums = SIMP_SUMS_MIN_BLOCKS, stress = SIMP_STRESS_MIN_BLOCKS;
+    static constexpr int kin = SIMP_KIN_MIN_BLOCKS, stress = SIMP_STRESS_MIN_BLOCKS;
 };
 template <>
 struct MinBlocks<float> {
-    static constexpr int kin = SIMP_KIN_MIN_BLOCKS_F32, sums = SIMP_KIN_MIN_BLOCKS_F32, stress = SIMP_STRESS_MIN_BLOCKS_F32;
+    static constexpr int kin = SIMP_KIN_MIN_BLOCKS_F32, stress = SIMP_STRESS_MIN_BLOCKS_F32;
 };
-// per-thread pair list in shared memory: a typical particle's pairs fit;
-// a longer list is processed in batches.  Kept small: the shared memory of
-// the resident blocks comes out of the L1 cache that serves the gathers.
-constexpr int kGatherSlots = 24;
-#ifndef SIMP_FIND_MIN_BLOCKS
-#define SIMP_FIND_MIN_BLOCKS 8
-#endif
 
-// The kinematic pass in one kernel: candidates go into a per-thread list in
-// shared memory, then the pair arithmetic runs densely.
-template <class T, int SKF>
-__global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(KinArgs a) {
-    __shared__ int s_list[kGatherSlots * kBlock];
+// hsml of the halo's particles, where it varies.
+__device__ __forceinline__ void tile_hsml(const Halo &h, const TileMem &m, const State &s) {
+    for (int d = 0; d < h.nseg; ++d) {
+        const int n = h.off[d + 1] - h.off[d];
+        for (int k = threadIdx.x; k < n; k += kTile) {
+            const double v = s.hs[h.lo[d] + k];
+            m.hs[h.off[d] + k] = v;
+        }
+    }
+}
+
+// One word of a particle's candidates, slots [sl, sl + n), n <= 32: bit k set
+// where candidate k is not certainly beyond mhsml + delta (FP32 with its
+// proven margin).  Called by the whole warp (lanes with n = 0 take part).
+template <bool UNIFORM>
+__device__ __forceinline__ unsigned scan_word(const TileMem &m, int sl, int n, float xf, float yf, float hf,
+                                              float delta, float grow) {
+    const int top = __reduce_max_sync(0xffffffffu, n);
+    if (n <= 0) sl = 0;   // (a batch may read up to 31 slots past the halo)
+    const float2 *f = m.f();
+    const float lim_u = (hf + delta) * (hf + delta) * grow;
+    unsigned bits = 0u;
+    for (int k0 = 0; k0 < top; k0 += 8) {
+        unsigned b8 = 0u;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const float2 q = f[sl + k0 + u];
+            const float dx = xf - q.x, dy = yf - q.y;
+            const float sf = fmaf(dx, dx, dy * dy);
+            float lim = lim_u;
+            if (!UNIFORM) {
+                const float mf = 0.5f * (hf + m.hf()[sl + k0 + u]) + delta;
+                lim = mf * mf * grow;
+            }
+            if (sf <= lim) b8 |= 1u << u;
+        }
+        bits |= b8 << k0;
+    }
+    if (n < 32) bits &= (1u << max(n, 0)) - 1u;
+    return bits;
+}
+
+// Builds the lists of a tile part whose xy records are in shared memory; a
+// particle's candidates go to the shared list and to `out` (the tile's lists
+// at its column).  Returns the particle's candidates, which may exceed
+// kListRows (the list then holds the first ones).  Called by the whole block.
+template <bool UNIFORM>
+__device__ __noinline__ int build_lists(const Halo &h, const TileMem &m, const KinArgs &a, const Inst &I, int i,
+                                        bool live, unsigned short *out) {
     const int t = threadIdx.x;
-    const int i = blockIdx.x * blockDim.x + t;
-    if (i >= a.n) return;
+    const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
+    const int total = h.off[h.nseg];
+    for (int k = t; k < total; k += kTile) {
+        const double2 q = xs[k];
+        m.f()[k] = make_float2((float)q.x, (float)q.y);
+        if (!UNIFORM) m.hf()[k] = (float)m.hs[k];
+    }
+    __syncthreads();
+    const int2 at = cell_at(I, a.cell[i]);
+    const double2 xy = a.s.xy[i];
+    const float xf = (float)xy.x, yf = (float)xy.y, hf = (float)a.s.hs[i];
+    const float margin = prefilter_margin(bitsd(a.sc->xabs_bits), I.hmin);
+    const float grow = margin < 0.25f ? 1.0f + margin : INFINITY;
+    const float delta = (float)I.delta;
+    const int own = slot_of(h, i);
+    int cnt = 0;
+    for (int d = 0; d < h.nseg; ++d) {
+        int j0, j1;
+        stencil_range(I, a.cell_start, at, h.nseg / 2, d, j0, j1);
+        int left = live ? j1 - j0 : 0;
+        int sl = left > 0 ? slot_of(h, j0) : 0;
+        while (__any_sync(0xffffffffu, left > 0)) {
+            unsigned bits = scan_word<UNIFORM>(m, sl, min(left, 32), xf, yf, hf, delta, grow);
+            const int self = own - sl;
+            if (self >= 0 && self < 32) bits &= ~(1u << self);
+            while (bits != 0u) {
+                const int k = __ffs(bits) - 1;
+                bits &= bits - 1u;
+                if (cnt < kListRows) {
+                    m.list[cnt * kTile + t] = (unsigned short)(sl + k);
+                    out[cnt * kTile] = (unsigned short)(sl + k);
+                }
+                ++cnt;
+            }
+            sl += 32;
+            left -= 32;
+        }
+    }
+    return cnt;
+}
+
+// Per-neighbour scalars of a slot: the FP64 records for the plain form, the
+// packed FP32 copies for the mixed form.  (Where hsml is one value in every
+// basin a neighbour's is not read.)
+template <class T>
+struct Rec;
+template <>
+struct Rec<double> {
+    static constexpr int stress_arrays = 3;   // xy, (tau11, tau12), (tau22, m)
+    static __device__ __forceinline__ double own_h(const State &s, int i) { return s.hs[i]; }
+    static __device__ __forceinline__ const void *kin_src(const State &s) { return s.mm; }
+    template <bool UNIFORM>
+    static __device__ __forceinline__ void kin(const TileMem &t, int sl, double &m, double &mor, double &h) {
+        const double2 q = reinterpret_cast<const double2 *>(t.rec[2])[sl];
+        m = q.x;
+        mor = q.y;
+        h = UNIFORM ? 0.0 : t.hs[sl];
+    }
+    static __device__ __forceinline__ void kin_global(const State &s, int j, double &m, double &mor, double &h) {
+        const double2 q = __ldg(&s.mm[j]);
+        m = q.x;
+        mor = q.y;
+        h = __ldg(&s.hs[j]);
+    }
+    template <bool UNIFORM>
+    static __device__ __forceinline__ void stress(const TileMem &t, int sl, double &m, double &t11, double &t12,
+                                                  double &t22, double &h) {
+        const double2 a = reinterpret_cast<const double2 *>(t.rec[1])[sl];
+        const double2 b = reinterpret_cast<const double2 *>(t.rec[2])[sl];
+        m = b.y;
+        t11 = a.x;
+        t12 = a.y;
+        t22 = b.x;
+        h = UNIFORM ? 0.0 : t.hs[sl];
+    }
+    static __device__ __forceinline__ void stress_global(const State &s, const TauRec &r, int j, double &m, double &t11,
+                                                         double &t12, double &t22, double &h) {
+        const double2 a = __ldg(&r.ta[j]), b = __ldg(&r.tb[j]);
+        m = b.y;
+        t11 = a.x;
+        t12 = a.y;
+        t22 = b.x;
+        h = __ldg(&s.hs[j]);
+    }
+    static constexpr double band = kBand;
+};
+template <>
+struct Rec<float> {
+    static constexpr int stress_arrays = 2;   // xy, (tau11, tau12, tau22, m)
+    static __device__ __forceinline__ float own_h(const State &s, int i) { return s.hsf[i]; }
+    static __device__ __forceinline__ const void *kin_src(const State &s) { return s.hmm; }
+    template <bool UNIFORM>
+    static __device__ __forceinline__ void kin(const TileMem &t, int sl, float &m, float &mor, float &h) {
+        const float4 q = reinterpret_cast<const float4 *>(t.rec[2])[sl];
+        h = q.x;
+        m = q.y;
+        mor = q.z;
+    }
+    static __device__ __forceinline__ void kin_global(const State &s, int j, float &m, float &mor, float &h) {
+        const float4 q = __ldg(&s.hmm[j]);
+        h = q.x;
+        m = q.y;
+        mor = q.z;
+    }
+    template <bool UNIFORM>
+    static __device__ __forceinline__ void stress(const TileMem &t, int sl, float &m, float &t11, float &t12,
+                                                  float &t22, float &h) {
+        const float4 q = reinterpret_cast<const float4 *>(t.rec[1])[sl];
+        m = q.w;
+        t11 = q.x;
+        t12 = q.y;
+        t22 = q.z;
+        h = UNIFORM ? 0.0f : (float)t.hs[sl];
+    }
+    static __device__ __forceinline__ void stress_global(const State &s, const TauRec &r, int j, float &m, float &t11,
+                                                         float &t12, float &t22, float &h) {
+        const float4 q = __ldg(&r.tq[j]);
+        m = q.w;
+        t11 = q.x;
+        t12 = q.y;
+        t22 = q.z;
+        h = __ldg(&s.hsf[j]);
+    }
+    // (differences and hsml rounded to FP32: within 2^-20 of the exact ratio)
+    static constexpr float band = 0x1p-18f;
+};
+
+// A candidate against the exact criterion's band: 1 certainly a pair, 0
+// certainly none, 2 within the band (or not a number).
+template <class T, bool UNIFORM>
+__device__ __forceinline__ int classify(T dx, T dy, T hi, T hj, T mh2_u) {
+    const T s = fma(dx, dx, dy * dy);
+    T mh2 = mh2_u;
+    if (!UNIFORM) {
+        const T mh = T(0.5) * (hi + hj);
+        mh2 = mh * mh;
+    }
+    if (s < mh2 * (T(1) - Rec<T>::band)) return 1;
+    return s > mh2 * (T(1) + Rec<T>::band) ? 0 : 2;
+}
+
+// Whether a basin's lists hold every pair of this right-hand side (Inst).
+// In a step's second right-hand side they are at most as old as the first.
+__device__ __forceinline__ bool lists_valid(const Inst &I, bool second) {
+    if (!I.list_ok && !second) return false;
+    const double d = (I.list_ok ? I.list_d : 0.0) + (second ? sqrt(bitsd(I.half2_bits)) : 0.0);
+    return 2.0 * d * (1.0 + 1e-9) <= I.delta;
+}
+
+// Kinematic pass over tiles.  Bound by latency: a block waits for its tile's
+// copies, then runs about 22 pairs per thread at 80 instructions each (FP64
+// pipe 20% busy, issue slots 32%), at five blocks per SM.  262,144 particles,
+// FP64: 78 -> 42 us per pass against gathers from global memory; mixed at
+// 1,048,576: 237 -> 150 us.
+template <class T, int SKF, bool UNIFORM>
+__global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(const __grid_constant__ KinArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ Halo h;
+    __shared__ __align__(8) unsigned long long bar;
+    __shared__ int rows_max;
+    const int t = threadIdx.x;
+    const Chunk ch = a.chunks[blockIdx.x];
+    const Inst &I = a.inst[ch.q];
+    if (ch.spare >= I.spares) return;   // (an unused spare tile)
     const State &s = a.s;
     const Phys &P = a.P;
-    const Inst &I = a.inst[a.pinst[i]];
+    Halo *halos = reinterpret_cast<Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    unsigned short *lists = a.pl.slot + (size_t)blockIdx.x * kListRows * kTile;
     // a basin whose state turned non-finite is not searched any more (its
     // stencil would span its whole grid); it is only carried until retired
-    const bool dead = inst_dead(I.flags);
-    const PairCtx pc = pair_ctx(s, a.sc, I, a.cell_start, i);
-    const double xi = pc.xi, yi = pc.yi, hi = pc.hi;
-    const double vxi = s.vx[i], vyi = s.vy[i];
-    const double inv_hi = 1.0 / hi;
-    KinSums<T> ks;     // -div and the velocity gradient, negated
-    const T hiT = Nb<T>::h(s, i), inv_hiT = (T)inv_hi;
-    const T hu = (I.hmin == I.hmax) ? hiT : T(-1);   // (every neighbour's hsml is hi)
-    typename Vec2<T>::type *dwr = reinterpret_cast<typename Vec2<T>::type *>(a.dw);
-    int cnt = 0;       // entries in this thread's shared-memory list
-    int npairs = 0;    // exact pairs found so far
-    int done = 0;      // pairs already processed (and written to the pair list)
-    auto flush = [&]() {
-#pragma unroll 4
-        for (int k = 0; k < cnt; ++k) {
-            const int j = s_list[k * kBlock + t];
-            if (!SIMP_IN_RANGE(j, 0, a.n, SITE_NEIGHBOUR)) continue;
-            if (done + k < kMaxPairs) a.pl.pj[(size_t)(done + k) * a.pl.stride + i] = j;
-            const double2 q = __ldg(&s.xy[j]), v = __ldg(&s.vxy[j]);
-            const KinNb<T> nb = Nb<T>::kin(s, j, hu);
-            const PairGeom<T> pg = pair_geom<T, false, SKF>(P, (T)(xi - q.x), (T)(yi - q.y), hiT, inv_hiT, nb.h);
-            const T dwx = pg.gfac * pg.dx, dwy = pg.gfac * pg.dy;
-            if (dwr && done + k < kDwRows) dwr[(size_t)(done + k) * a.pl.stride + i] = Vec2<T>::make(dwx, dwy);
-            ks.add(dwx, dwy, (T)(vxi - v.x), (T)(vyi - v.y), nb.m, nb.mor);
+    if (inst_dead(I.flags)) {
+        if (t == 0) {
+            Halo none{};
+            none.kind = HALO_NONE;
+            none.size = ch.p1 - ch.p0;
+            none.walls = 1;
+            halos[0] = none;
         }
-        done += cnt;
-        cnt = 0;
-    };
-    auto on_pair = [&](int j) {
-        s_list[cnt * kBlock + t] = j;
-        ++npairs;
-        if (++cnt == kGatherSlots) flush();
-    };
-    if (a.sc->list_scan && i == 0) atomicExch(&a.sc->dlist2_bits, 0ull);
-    // (a particle of a newly admitted basin builds its list on its own)
-    const bool build = a.sc->list_scan || a.nl.count[i] < 0;
-    if (dead) {
-        if (build) {
-            a.nl.count[i] = 0;
-            a.nl.xl[i] = xi;
-            a.nl.yl[i] = yi;
-        }
-    } else if (build) {
-        // rebuild the Verlet list from the cell stencil: members are the
-        // candidates not certainly beyond mhsml + skin (FP32, with margin)
-        const double skin = a.sc->skin;
-        const float skinf = (float)skin, grow = 1.0f + pc.margin;
-        int total = 0;
-        for_stencil(pc.g, i, a.cell[i], stencil_radius(pc.hmax, pc.dmax2_bits, pc.g, pc.hmax + skin), [&](int j) {
-            const float4 f = __ldg(&s.pf[j]);
-            const float dxf = pc.xif - f.x, dyf = pc.yif - f.y;
-            const float lim = 0.5f * (pc.hif + f.z) + skinf;
-            if (dxf * dxf + dyf * dyf > lim * lim * grow) return;
-            if (total < kMaxNbr) a.nl.nbr[(size_t)total * a.nl.stride + i] = j;
-            ++total;
-            if (is_pair_with(s, pc, j, f)) on_pair(j);
-        });
-        a.nl.count[i] = total;
-        a.nl.xl[i] = xi;
-        a.nl.yl[i] = yi;
-    } else {
-        // (room for a whole batch in the list before each batch)
-        for_each_current_pair_batched(s, a.nl, a.sc, i, a.cell[i], pc, [&]() {
-            if (cnt > kGatherSlots - kBatch) flush();
-        }, [&](int j) {
-            s_list[cnt * kBlock + t] = j;
-            ++npairs;
-            ++cnt;
-        });
+        const int i = ch.p0 + t;
+        if (i >= ch.p1) return;
+        kin_rheology(a, i, -0.0, -0.0, -0.0, -0.0, -0.0);
+        return;
     }
-    flush();   // (also writes the stress pass's pair list, a coalesced row per k)
-    a.pl.count[i] = npairs;
-    kin_rheology(a, i, -ks.dv.get(), -ks.g1.get(), -ks.g2.get(), -ks.g3.get(), -ks.g4.get());
+    const bool build = !lists_valid(I, a.second);
+    const TileMem m = tile_mem(smem, a.cap, 3, UNIFORM);
+    if (t == 0) bar_init(&bar);
+    unsigned parity = 0u;
+    for (int p0 = ch.p0; p0 < ch.p1;) {
+        if (!build) {
+            if (t < (int)(sizeof(Halo) / sizeof(int)))
+                reinterpret_cast<int *>(&h)[t] = reinterpret_cast<const int *>(&halos[(p0 - ch.p0) / kPartMin])[t];
+        } else if (t == 0) {
+            // the largest part of the tile whose halo fits
+            for (int S = kTile;; S >>= 1) {
+                make_halo(I, a.cell_start, a.bstart, a.cell, p0, min(p0 + S, ch.p1), a.cap, h);
+                if (h.kind == HALO_TILE || S <= kPartMin || h.nseg > kMaxSeg) break;
+            }
+            rows_max = 0;
+        }
+        __syncthreads();
+        const void *src[3] = {s.xy, s.vxy, Rec<T>::kin_src(s)};
+        const bool fits = h.kind == HALO_TILE;
+        if (fits && t < 32) tile_fetch(h, m, src, 0, build ? 1 : 3, lists, build ? 0 : h.rows, &bar);
+        const bool live = t < h.size;
+        const int i = p0 + (live ? t : 0);
+        const double2 xy = __ldg(&s.xy[i]), vi = __ldg(&s.vxy[i]);
+        const double hi = s.hs[i];
+        const T hiT = Rec<T>::own_h(s, i);
+        PairGrad<T, SKF, UNIFORM> grad;
+        grad.init(P, hiT);
+        const bool rule = rule_on(I);
+        KinSums<T> ks;     // -div and the velocity gradient, negated
+        auto terms = [&](T dx, T dy, double vxj, double vyj, T mj, T mrj, T hj) {
+            const T g = grad(P, fma(dx, dx, dy * dy), hj);
+            ks.add(g * dx, g * dy, (T)(vi.x - vxj), (T)(vi.y - vyj), mj, mrj);
+        };
+        int cnt = 0;       // candidates in the particle's list
+        bool tile = fits;
+        if (fits) {
+            if (!UNIFORM) tile_hsml(h, m, s);
+            if (!build && live) cnt = a.pl.count[i];
+            if (!bar_wait(&bar, parity)) {
+                atomicOr(&a.sc->flags, FLAG_TIMEOUT);
+                bar_wait(&bar, parity);
+                return;
+            }
+            parity ^= 1u;
+            if (!UNIFORM || build) __syncthreads();
+            if (build) {
+                cnt = build_lists<UNIFORM>(h, m, a, I, i, live, lists + (i - ch.p0));
+                const int rows = __reduce_max_sync(0xffffffffu, cnt);
+                if ((t & 31) == 0) atomicMax(&rows_max, rows);
+                // (the FP32 copies make way for the records)
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncthreads();
+                tile = rows_max <= kListRows;
+                if (t == 0) {
+                    h.rows = tile ? rows_max : 0;
+                    if (!tile) h.kind = HALO_GLOBAL;
+                }
+                if (tile) {
+                    if (t < 32) tile_fetch(h, m, src, 1, 3, lists, 0, &bar);
+                    if (live) a.pl.count[i] = cnt;
+                    if (!bar_wait(&bar, parity)) {
+                        atomicOr(&a.sc->flags, FLAG_TIMEOUT);
+                        bar_wait(&bar, parity);
+                        return;
+                    }
+                    parity ^= 1u;
+                }
+                __syncthreads();
+            }
+        }
+        if (build && t == 0) halos[(p0 - ch.p0) / kPartMin] = h;
+        if (tile) {
+            const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
+            const double2 *vs = reinterpret_cast<const double2 *>(m.rec[1]);
+            const T mh2_u = hiT * hiT;
+            // (a list just built stands at the thread's own column, as does
+            // the copied one: a part's threads are its first columns or all)
+            const unsigned short *col = m.list + (build ? t : i - ch.p0);
+#pragma unroll 2
+            for (int k = 0; k < cnt; ++k) {
+                const int q = col[k * kTile];
+                if (!SIMP_IN_RANGE(q, 0, h.off[h.nseg], SITE_TILE)) continue;
+                const double2 x = xs[q], v = vs[q];
+                T mj, mrj, hj;
+                Rec<T>::template kin<UNIFORM>(m, q, mj, mrj, hj);
+                const T dx = (T)(xy.x - x.x), dy = (T)(xy.y - x.y);
+                const int in = classify<T, UNIFORM>(dx, dy, hiT, hj, mh2_u);
+                if (in == 0) continue;
+                if (in == 2 || rule)
+                    if (!exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q))) continue;
+                terms(dx, dy, v.x, v.y, mj, mrj, hj);
+            }
+        } else if (live) {
+            // no tile: the neighbours from global memory
+            global_pairs(s, I, a.cell_start, i, a.cell[i], [&](int j) {
+                const double2 q = __ldg(&s.xy[j]), v = __ldg(&s.vxy[j]);
+                T mj, mrj, hj;
+                Rec<T>::kin_global(s, j, mj, mrj, hj);
+                terms((T)(xy.x - q.x), (T)(xy.y - q.y), v.x, v.y, mj, mrj, hj);
+            });
+        }
+        if (live) {
+            const double c = -grad.common();
+            kin_rheology(a, i, c * ks.dv.get(), c * ks.g1.get(), c * ks.g2.get(), c * ks.g3.get(), c * ks.g4.get());
+        }
+        p0 += h.size;
+        if (p0 < ch.p1) {
+            // the next part's copies write where this one's reads were
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+        }
+    }
 }
 
-// The kinematic pass in two kernels.  k_find_pairs decides the exact pairs
-// of each particle (Verlet candidates, or the cell stencil when the lists
-// are rebuilt) and writes them as the pair list; it needs fewer registers
-// than the FP64 pair arithmetic, so more warps hide its gather latency.
-// k_kin_sums then does the pair arithmetic over those rows, in the order
-// they were found, the order of the one-kernel pass: both give bitwise the
-// same results.  launch_kinematic picks between them.
-__global__ void __launch_bounds__(kBlock, SIMP_FIND_MIN_BLOCKS) k_find_pairs(KinArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const State &s = a.s;
-    const Inst &I = a.inst[a.pinst[i]];
-    // a basin whose state turned non-finite is not searched any more (its
-    // stencil would span its whole grid); it is only carried until retired
-    const bool dead = inst_dead(I.flags);
-    const PairCtx pc = pair_ctx(s, a.sc, I, a.cell_start, i);
-    int npairs = 0;
-    auto on_pair = [&](int j) {
-        if (npairs < kMaxPairs) a.pl.pj[(size_t)npairs * a.pl.stride + i] = j;
-        ++npairs;
-    };
-    if (a.sc->list_scan && i == 0) atomicExch(&a.sc->dlist2_bits, 0ull);
-    // (a particle of a newly admitted basin builds its list on its own)
-    const bool build = a.sc->list_scan || a.nl.count[i] < 0;
-    if (dead) {
-        if (build) {
-            a.nl.count[i] = 0;
-            a.nl.xl[i] = pc.xi;
-            a.nl.yl[i] = pc.yi;
-        }
-    } else if (build) {
-        // rebuild the Verlet list from the cell stencil: members are the
-        // candidates not certainly beyond mhsml + skin (FP32, with margin)
-        const double skin = a.sc->skin;
-        const float skinf = (float)skin, grow = 1.0f + pc.margin;
-        int total = 0;
-        for_stencil(pc.g, i, a.cell[i], stencil_radius(pc.hmax, pc.dmax2_bits, pc.g, pc.hmax + skin), [&](int j) {
-            const float4 f = __ldg(&s.pf[j]);
-            const float dxf = pc.xif - f.x, dyf = pc.yif - f.y;
-            const float lim = 0.5f * (pc.hif + f.z) + skinf;
-            if (dxf * dxf + dyf * dyf > lim * lim * grow) return;
-            if (total < kMaxNbr) a.nl.nbr[(size_t)total * a.nl.stride + i] = j;
-            ++total;
-            if (is_pair_with(s, pc, j, f)) on_pair(j);
-        });
-        a.nl.count[i] = total;
-        a.nl.xl[i] = pc.xi;
-        a.nl.yl[i] = pc.yi;
-    } else {
-        for_each_current_pair_batched(s, a.nl, a.sc, i, a.cell[i], pc, [] {}, on_pair);
-    }
-    a.pl.count[i] = npairs;
-}
-
-template <class T, int SKF>
-__global__ void __launch_bounds__(kBlock, MinBlocks<T>::sums) k_kin_sums(KinArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const State &s = a.s;
-    const Phys &P = a.P;
-    const double xi = s.x[i], yi = s.y[i], hi = s.hs[i];
-    const double vxi = s.vx[i], vyi = s.vy[i];
-    const double inv_hi = 1.0 / hi;
-    KinSums<T> ks;     // -div and the velocity gradient, negated
-    const T hiT = Nb<T>::h(s, i), inv_hiT = (T)inv_hi;
-    typename Vec2<T>::type *dwr = reinterpret_cast<typename Vec2<T>::type *>(a.dw);
-    auto pair = [&](int k, int j) {
-        if (!SIMP_IN_RANGE(j, 0, a.n, SITE_NEIGHBOUR)) return;
-        const double2 q = __ldg(&s.xy[j]), v = __ldg(&s.vxy[j]);
-        const KinNb<T> nb = Nb<T>::kin(s, j, T(-1));
-        const PairGeom<T> pg = pair_geom<T, false, SKF>(P, (T)(xi - q.x), (T)(yi - q.y), hiT, inv_hiT, nb.h);
-        const T dwx = pg.gfac * pg.dx, dwy = pg.gfac * pg.dy;
-        if (dwr && k < kDwRows) dwr[(size_t)k * a.pl.stride + i] = Vec2<T>::make(dwx, dwy);
-        ks.add(dwx, dwy, (T)(vxi - v.x), (T)(vyi - v.y), nb.m, nb.mor);
-    };
-    const int cnt = a.pl.count[i];
-    if (cnt <= kMaxPairs) {
-#pragma unroll 4
-        for (int k = 0; k < cnt; ++k) pair(k, __ldg(&a.pl.pj[(size_t)k * a.pl.stride + i]));
-    } else {
-        // more pairs than list rows: found again, in the same order
-        const PairCtx pc = pair_ctx(s, a.sc, a.inst[a.pinst[i]], a.cell_start, i);
-        int k = 0;
-        for_each_current_pair(s, a.nl, a.sc, i, a.cell[i], pc, [&](int j) { pair(k++, j); });
-    }
-    kin_rheology(a, i, -ks.dv.get(), -ks.g1.get(), -ks.g2.get(), -ks.g3.get(), -ks.g4.get());
-}
-
-template <class T, int SKF>
-__global__ void __launch_bounds__(kBlock, MinBlocks<T>::stress) k_stress(StressArgs a) {
-    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = i0 < a.n;
-    const int i = live ? i0 : a.n - 1;   // dead lanes mirror the last particle for warp reductions
+// Stress pass over the same tiles: 41 instructions per pair, then the
+// epilogue, whose twenty own values are loaded together ahead of the walls and
+// the update (68 -> 50 us against loading each where it is used).  262,144
+// particles, FP64: 70 -> 50 us per pass against gathers from global memory.
+template <class T, int SKF, bool UNIFORM>
+__global__ void __launch_bounds__(kBlock, MinBlocks<T>::stress) k_stress(const __grid_constant__ StressArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ Halo h;
+    __shared__ __align__(8) unsigned long long bar;
+    const int t = threadIdx.x;
+    const Chunk ch = a.chunks[blockIdx.x];
+    const Inst &I = a.inst[ch.q];
+    if (ch.spare >= I.spares) return;   // (an unused spare tile)
     const State &s = a.rhs;
     const Phys &P = a.P;
-    const double xi = s.x[i], yi = s.y[i], hi = s.hs[i];
-    const double inv_hi = 1.0 / hi;
-    const int ci = a.cell[i];
-    const int ki = a.pinst[i];
-    const Inst &I = a.inst[ki];
-    const bool dead = inst_dead(I.flags);   // see k_kinematic
-    StressSums<T> ss;
-    const T hiT = Nb<T>::h(s, i), inv_hiT = (T)inv_hi;
-    const T hu = (I.hmin == I.hmax) ? hiT : T(-1);   // (every neighbour's hsml is hi)
-    auto accumulate = [&](int j) {
-        if (!SIMP_IN_RANGE(j, 0, a.n, SITE_NEIGHBOUR)) return;
-        const double2 q = __ldg(&s.xy[j]);
-        const StressNb<T> nb = Nb<T>::stress(s, a.rec, j, hu);
-        const PairGeom<T> pg = pair_geom<T, false, SKF>(P, (T)(xi - q.x), (T)(yi - q.y), hiT, inv_hiT, nb.h);
-        ss.add(pg.gfac * pg.dx, pg.gfac * pg.dy, nb.m, nb.t11, nb.t12, nb.t22);
-    };
-    int cnt = a.pl.count[i];
-    if (a.dw && cnt <= kDwRows && !dead) {
-        // the kinematic pass kept these pairs' kernel gradients
-        const typename Vec2<T>::type *dwr = reinterpret_cast<const typename Vec2<T>::type *>(a.dw);
-#pragma unroll 4
-        for (int k = 0; k < cnt; ++k) {
-            const size_t r = (size_t)k * a.pl.stride + i;
-            const typename Vec2<T>::type g = __ldg(&dwr[r]);
-            const int j = __ldg(&a.pl.pj[r]);
-            if (!SIMP_IN_RANGE(j, 0, a.n, SITE_NEIGHBOUR)) continue;
-            const StressNb<T> nb = Nb<T>::stress_rec(a.rec, j);
-            ss.add(g.x, g.y, nb.m, nb.t11, nb.t12, nb.t22);
+    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    constexpr int arrays = Rec<T>::stress_arrays;
+    const TileMem m = tile_mem(smem, a.cap, arrays, UNIFORM);
+    if (t == 0) bar_init(&bar);
+    unsigned parity = 0u;
+    for (int p0 = ch.p0; p0 < ch.p1;) {
+        if (t < (int)(sizeof(Halo) / sizeof(int)))
+            reinterpret_cast<int *>(&h)[t] = reinterpret_cast<const int *>(&halos[(p0 - ch.p0) / kPartMin])[t];
+        __syncthreads();
+        const bool tile = h.kind == HALO_TILE;
+        if (tile && t < 32) {
+            const void *src[3] = {s.xy, a.rec.tq ? (const void *)a.rec.tq : (const void *)a.rec.ta, a.rec.tb};
+            tile_fetch(h, m, src, 0, arrays, a.pl.slot + (size_t)blockIdx.x * kListRows * kTile, h.rows, &bar);
         }
-    } else if (cnt <= kMaxPairs) {
-        // the kinematic pass of this right-hand side found the pairs
-#pragma unroll 4
-        for (int k = 0; k < cnt; ++k) accumulate(__ldg(&a.pl.pj[(size_t)k * a.pl.stride + i]));
-    } else if (dead) {
-        cnt = 0;
-    } else {
-        cnt = 0;
-        const PairCtx pc = pair_ctx(s, a.sc, I, a.cell_start, i);
-        for_each_current_pair(s, a.nl, a.sc, i, ci, pc, [&](int j) {
-            accumulate(j);
-            ++cnt;
-        });
+        const bool live = t < h.size;
+        const int i = p0 + (live ? t : h.size - 1);   // idle lanes mirror the part's last particle
+        const double2 xy = __ldg(&s.xy[i]);
+        const double hi = s.hs[i];
+        const T hiT = Rec<T>::own_h(s, i);
+        StressSums<T> ss;
+        PairGrad<T, SKF, UNIFORM> grad;
+        grad.init(P, hiT);
+        int npairs = 0;
+        auto terms = [&](T dx, T dy, T mj, T t11, T t12, T t22, T hj) {
+            const T g = grad(P, fma(dx, dx, dy * dy), hj);
+            ss.add(g * dx, g * dy, mj, t11, t12, t22);
+            ++npairs;
+        };
+        if (tile) {
+            if (!UNIFORM) tile_hsml(h, m, s);
+            const int cnt = live ? a.pl.count[i] : 0;
+            const bool rule = rule_on(I);
+            if (!bar_wait(&bar, parity)) {
+                atomicOr(&a.sc->flags, FLAG_TIMEOUT);
+                bar_wait(&bar, parity);
+                return;
+            }
+            parity ^= 1u;
+            if (!UNIFORM) __syncthreads();
+            const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
+            const unsigned short *col = m.list + (i - ch.p0);
+            const T mh2_u = hiT * hiT;
+#pragma unroll 2
+            for (int k = 0; k < cnt; ++k) {
+                const int q = col[k * kTile];
+                if (!SIMP_IN_RANGE(q, 0, h.off[h.nseg], SITE_TILE)) continue;
+                const double2 x = xs[q];
+                T mj, t11, t12, t22, hj;
+                Rec<T>::template stress<UNIFORM>(m, q, mj, t11, t12, t22, hj);
+                const T dx = (T)(xy.x - x.x), dy = (T)(xy.y - x.y);
+                const int in = classify<T, UNIFORM>(dx, dy, hiT, hj, mh2_u);
+                if (in == 0) continue;
+                if (in == 2 || rule)
+                    if (!exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q))) continue;
+                terms(dx, dy, mj, t11, t12, t22, hj);
+            }
+        } else if (h.kind == HALO_GLOBAL && live) {
+            global_pairs(s, I, a.cell_start, i, a.cell[i], [&](int j) {
+                const double2 q = __ldg(&s.xy[j]);
+                T mj, t11, t12, t22, hj;
+                Rec<T>::stress_global(s, a.rec, j, mj, t11, t12, t22, hj);
+                terms((T)(xy.x - q.x), (T)(xy.y - q.y), mj, t11, t12, t22, hj);
+            });
+        }
+        // (a retired basin's particles are not written any more: their state
+        // stays as it was until the batch's next compaction drops them)
+        const double c = grad.common();
+        stress_finish<SKF>(a, i, live && !(I.flags & FLAG_RETIRED), ch.q, I, inst_dead(I.flags), h.walls != 0,
+                           xy.x, xy.y, hi, c * ss.sx.get(), c * ss.sy.get(), c * ss.tx.get(), c * ss.ty.get(), npairs);
+        p0 += h.size;
+        if (p0 < ch.p1) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+        }
     }
-    // (a retired basin's particles are not written any more: their state
-    // stays as it was until the batch's next compaction drops them)
-    stress_finish<SKF>(a, i, live && !(I.flags & FLAG_RETIRED), ki, I, dead, xi, yi, hi, ci, ss.sx.get(), ss.sy.get(),
-                       ss.tx.get(), ss.ty.get(), cnt, true);
 }
 
 // Regularisation of a right-hand side (regularization.f90, called by
@@ -322,8 +498,10 @@ struct RegArgs {
     State s;
     const double *div;   // the kinematic pass's -sum_j m_j (v_i - v_j) . grad W
     PairList pl;
-    NbrList nl;
-    const int *cell_start, *cell, *pinst;
+    const int *cell_start, *cell;
+    const Chunk *chunks;
+    const unsigned char *halos;
+    int cap;
     const Inst *inst;
     Scalars *sc;
     Phys P;
@@ -342,61 +520,152 @@ __device__ __forceinline__ double hk_lv_r2(const Phys &P, const State &s, const 
     return lv / (rho * rho);
 }
 
-__global__ void __launch_bounds__(kBlock) k_regularize(RegArgs a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
+// The tiles of the two passes below hold, beside the records (xy, vxy) and
+// hsml, some FP64 values per particle, each worked out once per tile instead
+// of once per pair: fill(j, k) writes those of particle j at slot k.
+template <class F>
+__device__ __forceinline__ void tile_fill(const Halo &h, F &&fill) {
+    for (int d = 0; d < h.nseg; ++d) {
+        const int n = h.off[d + 1] - h.off[d];
+        for (int k = threadIdx.x; k < n; k += kTile) fill(h.lo[d] + k, h.off[d] + k);
+    }
+}
+constexpr int kAuxArrays = 3;
+size_t aux_smem_bytes(int cap) {
+    return tile_smem_bytes(cap, 2, false) + (size_t)kAuxArrays * cap * sizeof(double);
+}
+
+// Copies a tile part's halo record, records and lists to shared memory and
+// fills the other values.  Called by the whole block; false where a copy did
+// not arrive.
+template <class F>
+__device__ __forceinline__ bool aux_tile(const Halo *rec, Halo &h, const TileMem &m, const State &g, const double2 *vxy,
+                                         const unsigned short *lists, unsigned long long *bar, unsigned &parity,
+                                         Scalars *sc, F &&fill) {
+    const int t = threadIdx.x;
+    if (t < (int)(sizeof(Halo) / sizeof(int))) reinterpret_cast<int *>(&h)[t] = reinterpret_cast<const int *>(rec)[t];
+    __syncthreads();
+    if (h.kind != HALO_TILE) return true;
+    const void *src[3] = {g.xy, vxy, nullptr};
+    if (t < 32) tile_fetch(h, m, src, 0, 2, lists, h.rows, bar);
+    tile_hsml(h, m, g);
+    tile_fill(h, fill);
+    if (!bar_wait(bar, parity)) {
+        atomicOr(&sc->flags, FLAG_TIMEOUT);
+        bar_wait(bar, parity);
+        return false;
+    }
+    parity ^= 1u;
+    __syncthreads();
+    return true;
+}
+
+// Pairs of a particle of such a tile: f(j, slot, x_j, v_j, h_j), slot -1 where
+// there is no tile.
+template <class F>
+__device__ __forceinline__ void aux_pairs(const Halo &h, const TileMem &m, const State &g, const double2 *vxy,
+                                          const Inst &I, const int *cell_start, const int *cell, const int *count,
+                                          int i, int column, F &&f) {
+    if (h.kind == HALO_GLOBAL) {
+        global_pairs(g, I, cell_start, i, cell[i], [&](int j) { f(j, -1, g.xy[j], vxy[j], g.hs[j]); });
+    } else if (h.kind == HALO_TILE) {
+        const double2 p = g.xy[i];
+        const double hi = g.hs[i];
+        const bool rule = rule_on(I);
+        const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
+        const double2 *vs = reinterpret_cast<const double2 *>(m.rec[1]);
+        const int cnt = count[i];
+        for (int k = 0; k < cnt; ++k) {
+            const int q = m.list[k * kTile + column];
+            if (!SIMP_IN_RANGE(q, 0, h.off[h.nseg], SITE_TILE)) continue;
+            const double2 x = xs[q];
+            const double hj = m.hs[q];
+            const int in = classify<double, false>(p.x - x.x, p.y - x.y, hi, hj, 0.0);
+            if (in == 0) continue;
+            if (in == 2 || rule)
+                if (!exact_pair(g, I, rule, p.x, p.y, hi, particle_of(h, q))) continue;
+            f(particle_of(h, q), q, x, vs[q], hj);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) k_regularize(const __grid_constant__ RegArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ Halo h;
+    __shared__ __align__(8) unsigned long long bar;
+    const int t = threadIdx.x;
+    const Chunk ch = a.chunks[blockIdx.x];
     const State &s = a.s;
     const Phys &P = a.P;
     const size_t M = (size_t)a.maxn;
-    const Inst &I = a.inst[a.pinst[i]];
-    const double2 xy = s.xy[i], v = s.vxy[i];
-    const double xi = xy.x, yi = xy.y, vxi = v.x, vyi = v.y;
-    const double hi = s.hs[i], inv_hi = 1.0 / hi, rhoi = s.rho[i];
-    const double ci = sound_speed_held(P, rhoi);
-    const double pii = (P.art_visc == 1) ? hk_lv_r2(P, s, a.div, i) : 0.0;
-    Sum<double> avx, avy, xsx, xsy;
-    auto pair = [&](int j) {
-        if (!SIMP_IN_RANGE(j, 0, a.n, SITE_NEIGHBOUR)) return;
-        const double2 q = s.xy[j], w = s.vxy[j];
-        const double dx = xi - q.x, dy = yi - q.y;
-        const double dvx = vxi - w.x, dvy = vyi - w.y;
-        const double hj = s.hs[j], rhoj = s.rho[j], mj = s.m[j];
-        const PairGeom<double> pg = pair_geom<double, true>(P, dx, dy, hi, inv_hi, hj);
-        if (P.xsph) {
-            const double rbar = 0.5 * (rhoi + rhoj);
-            xsx.madd(mj * dvx * pg.w / rbar, 1.0);
-            xsy.madd(mj * dvy * pg.w / rbar, 1.0);
-        }
-        const double vr = dvx * dx + dvy * dy;
-        if ((P.art_visc == 1 || P.art_visc == 2) && vr <= 0.0) {
-            double pij;
-            if (P.art_visc == 1) {
-                pij = pii + hk_lv_r2(P, s, a.div, j);
-            } else {
-                const double hij = __dmul_rn(__dadd_rn(hi, hj), 0.5);
-                const double r = ref_distance(dx, dy);
-                const double scor = (double)0.01f * hij;
-                const double iota = hij * vr / (r * r + scor * scor);
-                const double cj = sound_speed_held(P, rhoj);
-                pij = (P.beta_pi * (iota * iota) - P.alpha_pi * iota * (ci + cj) / 2.0) / ((rhoi + rhoj) / 2.0);
-            }
-            avx.madd(-(mj * pij), pg.gfac * pg.dx);
-            avy.madd(-(mj * pij), pg.gfac * pg.dy);
-        }
-    };
+    const Inst &I = a.inst[ch.q];
+    if (ch.spare >= I.spares) return;   // (an unused spare tile)
     const bool dead = inst_dead(I.flags);
-    const int cnt = a.pl.count[i];
-    if (dead) {
-    } else if (cnt <= kMaxPairs) {
-        for (int k = 0; k < cnt; ++k) pair(a.pl.pj[(size_t)k * a.pl.stride + i]);
-    } else {
-        const PairCtx pc = pair_ctx(s, a.sc, I, a.cell_start, i);
-        for_each_current_pair(s, a.nl, a.sc, i, a.cell[i], pc, pair);
+    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    const TileMem m = tile_mem(smem, a.cap, 2, false);
+    double *rho_s = reinterpret_cast<double *>(smem + tile_smem_bytes(a.cap, 2, false));
+    double *m_s = rho_s + a.cap, *v_s = m_s + a.cap;   // v: lv / rho^2 (Hernquist-Katz) or the sound speed (Monaghan)
+    auto visc = [&](int j, double rho) {
+        return P.art_visc == 1 ? hk_lv_r2(P, s, a.div, j) : sound_speed_held(P, rho);
+    };
+    if (t == 0) bar_init(&bar);
+    unsigned parity = 0u;
+    for (int p0 = ch.p0; p0 < ch.p1;) {
+        if (!aux_tile(&halos[(p0 - ch.p0) / kPartMin], h, m, s, s.vxy, a.pl.slot + (size_t)blockIdx.x * kListRows * kTile, &bar,
+                      parity, a.sc, [&](int j, int k) {
+                          const double rho = s.rho[j];
+                          rho_s[k] = rho;
+                          m_s[k] = s.m[j];
+                          v_s[k] = visc(j, rho);
+                      }))
+            return;
+        const bool live = t < h.size;
+        const int i = p0 + t;
+        if (live) {
+            const double2 xy = s.xy[i], v = s.vxy[i];
+            const double xi = xy.x, yi = xy.y, vxi = v.x, vyi = v.y;
+            const double hi = s.hs[i], inv_hi = 1.0 / hi, rhoi = s.rho[i];
+            const double vi = visc(i, rhoi);
+            Sum<double> avx, avy, xsx, xsy;
+            if (!dead)
+                aux_pairs(h, m, s, s.vxy, I, a.cell_start, a.cell, a.pl.count, i, i - ch.p0,
+                          [&](int j, int slot, double2 q, double2 w, double hj) {
+                    const double dx = xi - q.x, dy = yi - q.y;
+                    const double dvx = vxi - w.x, dvy = vyi - w.y;
+                    const double rhoj = slot >= 0 ? rho_s[slot] : s.rho[j], mj = slot >= 0 ? m_s[slot] : s.m[j];
+                    const PairGeom<double> pg = pair_geom<double, true>(P, dx, dy, hi, inv_hi, hj);
+                    if (P.xsph) {
+                        const double rbar = 0.5 * (rhoi + rhoj), c = mj * pg.w / rbar;
+                        xsx.madd(dvx, c);
+                        xsy.madd(dvy, c);
+                    }
+                    const double vr = dvx * dx + dvy * dy;
+                    if ((P.art_visc == 1 || P.art_visc == 2) && vr <= 0.0) {
+                        const double vj = slot >= 0 ? v_s[slot] : visc(j, rhoj);
+                        double pij;
+                        if (P.art_visc == 1) {
+                            pij = vi + vj;
+                        } else {
+                            const double hij = __dmul_rn(__dadd_rn(hi, hj), 0.5);
+                            const double scor = (double)0.01f * hij;
+                            const double iota = hij * vr / fma(dx, dx, fma(dy, dy, scor * scor));
+                            pij = (P.beta_pi * (iota * iota) - P.alpha_pi * iota * (vi + vj) / 2.0) / ((rhoi + rhoj) / 2.0);
+                        }
+                        avx.madd(-(mj * pij), pg.gfac * pg.dx);
+                        avy.madd(-(mj * pij), pg.gfac * pg.dy);
+                    }
+                });
+            a.reg[i] = avx.get();
+            a.reg[M + i] = avy.get();
+            a.reg[2 * M + i] = xsx.get();
+            a.reg[3 * M + i] = xsy.get();
+        }
+        p0 += h.size;
+        if (p0 < ch.p1) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+        }
     }
-    a.reg[i] = avx.get();
-    a.reg[M + i] = avy.get();
-    a.reg[2 * M + i] = xsx.get();
-    a.reg[3 * M + i] = xsy.get();
 }
 
 // Density rate drho/dt_i = sum_j m_j (v_i - v_j) . grad_i W_ij over the
@@ -421,7 +690,10 @@ struct DensArgs {
     const double *a2;    // |dv/dt|^2 of the last right-hand side (tse = 1)
     double *hs_next;
     PairList pl;
-    const int *cell_start, *cell, *pinst;
+    const int *cell_start, *cell;
+    const Chunk *chunks;
+    const unsigned char *halos;
+    int cap;
     const Inst *inst;
     Scalars *sc;
     Phys P;
@@ -450,17 +722,19 @@ struct DensArgs {
     const int *id;
 };
 
-__global__ void __launch_bounds__(kBlock) k_density_rate(DensArgs a) {
-    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = i0 < a.n ? i0 : a.n - 1;   // dead lanes mirror the last particle for the reductions
+// One part of a tile, particles [p0, p0 + h.size).
+__device__ __forceinline__ void density_rate(const DensArgs &a, const Halo &h, const TileMem &m, const double *mj_s,
+                                             const double *w_s, const double *rho_s, const Chunk &ch, int p0) {
+    const int i = p0 + min((int)threadIdx.x, h.size - 1);   // idle lanes mirror the part's last particle
     const State &g = a.g;
     const Phys &P = a.P;
-    const Inst &I = a.inst[a.pinst[i]];
-    const bool live = i0 < a.n && !(I.flags & FLAG_RETIRED);   // (a retired basin is not written)
+    const Inst &I = a.inst[ch.q];
+    const bool live = (int)threadIdx.x < h.size && !(I.flags & FLAG_RETIRED);   // (a retired basin is not written)
     const bool dead = inst_dead(I.flags);
-    const double xi = g.x[i], yi = g.y[i], hi = g.hs[i];
+    const double2 gxy = g.xy[i], vxy = a.v.vxy[i];
+    const double xi = gxy.x, yi = gxy.y, hi = g.hs[i];
     const double inv_hi = 1.0 / hi;
-    const double vxi = a.v.vx[i], vyi = a.v.vy[i];
+    const double vxi = vxy.x, vyi = vxy.y;
     Sum<double> r, rt, num, den;
     // p_i rule of the summation density's kernel_zero (DensArgs)
     const int idi = a.sum_mode ? a.id[i] : 0;
@@ -468,15 +742,14 @@ __global__ void __launch_bounds__(kBlock) k_density_rate(DensArgs a) {
     const long long byi = (a.sum_mode && P.nnps == 2) ? ref_bin(yi, I.bs) : 0;
     long long last = -1;   // (position in the serial pair order, category then index)
     double h_last = 0.0;
-    auto add = [&](int j) {
-        if (!SIMP_IN_RANGE(j, 0, a.n, SITE_NEIGHBOUR)) return;
-        const double2 q = g.xy[j];
+    auto add = [&](int j, int slot, double2 q, double2 v, double hj) {
+        const double mj = slot >= 0 ? mj_s[slot] : a.mj[j];
         PairGeom<double> pg;
         if (a.sum_mode) {
-            pg = pair_geom<double, true>(P, xi - q.x, yi - q.y, hi, inv_hi, g.hs[j]);
-            const double mw = a.m_sum[j] * pg.w;
+            pg = pair_geom<double, true>(P, xi - q.x, yi - q.y, hi, inv_hi, hj);
+            const double mw = (slot >= 0 ? w_s[slot] : a.m_sum[j]) * pg.w;
             num.madd(mw, 1.0);
-            den.madd(mw / a.rho_in[j], 1.0);
+            den.madd(mw / (slot >= 0 ? rho_s[slot] : a.rho_in[j]), 1.0);
             const int idj = a.id[j];
             int cat = -1;
             if (P.nnps != 2) {
@@ -492,31 +765,19 @@ __global__ void __launch_bounds__(kBlock) k_density_rate(DensArgs a) {
             const long long key = cat < 0 ? -1 : ((long long)cat << 32) | (long long)(unsigned)idj;
             if (key > last) {
                 last = key;
-                h_last = g.hs[j];
+                h_last = hj;
             }
         } else {
-            pg = pair_geom<double, false>(P, xi - q.x, yi - q.y, hi, inv_hi, g.hs[j]);
+            pg = pair_geom<double, false>(P, xi - q.x, yi - q.y, hi, inv_hi, hj);
         }
-        const double2 v = a.v.vxy[j];
         const double dvx = vxi - v.x, dvy = vyi - v.y;
         const double t = fma(dvx, pg.gfac * pg.dx, dvy * (pg.gfac * pg.dy));
-        r.madd(a.mj[j], t);
+        r.madd(mj, t);
         // time_step.f90:93-109: the current masses (after mass_evolution)
-        if (a.dt_div) rt.madd(a.v.m[j], t);
+        if (a.dt_div) rt.madd(slot >= 0 && !a.sum_mode ? w_s[slot] : a.v.m[j], t);
     };
-    const int cnt = a.pl.count[i];
-    if (dead) {
-    } else if (cnt <= kMaxPairs) {
-#pragma unroll 4
-        for (int k = 0; k < cnt; ++k) add(a.pl.pj[(size_t)k * a.pl.stride + i]);
-    } else {
-        // (more pairs than the list holds: the cell stencil of the
-        // right-hand side's positions, whose bounds the instance keeps)
-        const PairCtx pc = pair_ctx(g, a.sc, I, a.cell_start, i);
-        for_stencil(pc.g, i, a.cell[i], stencil_radius(pc.hmax, pc.dmax2_bits, pc.g, 0.0), [&](int j) {
-            if (is_pair(g, pc, j)) add(j);
-        });
-    }
+    if (!dead && (int)threadIdx.x < h.size)
+        aux_pairs(h, m, g, a.v.vxy, I, a.cell_start, a.cell, a.pl.count, i, i - ch.p0, add);
     const double drhodt = r.get();
     const double dt = a.sc->dt;
     const State &o = a.v;
@@ -530,14 +791,12 @@ __global__ void __launch_bounds__(kBlock) k_density_rate(DensArgs a) {
             a.k0[i] = k0;
             a.rho_out[i] = rhon;
             if (a.rho_out == o.rho) {
-                o.mor[i] = o.m[i] / rhon;
                 refresh_views(o, i);
             }
         }
     } else if (a.rho_upd && live) {
         rhon = (a.rho_upd == 1) ? a.rho1[i] + drhodt * dt / 2.0 : a.rho1[i] + drhodt * dt;
         o.rho[i] = rhon;
-        o.mor[i] = o.m[i] / rhon;
         refresh_views(o, i);
     }
     if (!a.tail) return;
@@ -563,21 +822,52 @@ __global__ void __launch_bounds__(kBlock) k_density_rate(DensArgs a) {
     // (dead lanes contribute neutral values: the particle they mirror may
     // already have been updated by its own thread)
     unsigned active = 0u;
-    unsigned long long v[kBounds] = {0ull, 0ull, 0ull, ~0ull, 0ull, ~0ull};
+    unsigned long long v[kBounds] = {0ull, 0ull, ~0ull, 0ull, ~0ull, 0ull, 0ull};
     if (P.sle != 0) {
-        active |= 8u | 16u;
+        active |= 4u | 8u;
         if (live) {
+            v[2] = dbits(hsn);
             v[3] = dbits(hsn);
-            v[4] = dbits(hsn);
         }
     }
     if (P.tse != 0) {                                          // time_step.f90:20-26
-        active |= 32u;
+        active |= 16u;
         // |div v| = |sum_j m_j (v_i - v_j) . grad W| / rho_i (time_step.f90:108-111)
         const double adiv = a.dt_div ? fabs(rt.get() / rhon) : 0.0;
-        if (live) v[5] = dbits(dt_candidate(P, hsn, P.tse == 1 ? a.a2[i] : 0.0, rhon, adiv));
+        if (live) v[4] = dbits(dt_candidate(P, hsn, P.tse == 1 ? a.a2[i] : 0.0, rhon, adiv));
     }
-    block_bounds(a.sc, active, v);
+    block_bounds(a.sc, nullptr, nullptr, active, v);
+}
+
+__global__ void __launch_bounds__(kBlock) k_density_rate(const __grid_constant__ DensArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ Halo h;
+    __shared__ __align__(8) unsigned long long bar;
+    const int t = threadIdx.x;
+    const Chunk ch = a.chunks[blockIdx.x];
+    if (ch.spare >= a.inst[ch.q].spares) return;   // (an unused spare tile)
+    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    const TileMem m = tile_mem(smem, a.cap, 2, false);
+    double *mj_s = reinterpret_cast<double *>(smem + tile_smem_bytes(a.cap, 2, false));
+    double *w_s = mj_s + a.cap, *rho_s = w_s + a.cap;   // w: the summation's mass, or the time step's
+    const double *w_src = a.sum_mode ? a.m_sum : a.dt_div ? a.v.m : nullptr;
+    if (t == 0) bar_init(&bar);
+    unsigned parity = 0u;
+    for (int p0 = ch.p0; p0 < ch.p1;) {
+        if (!aux_tile(&halos[(p0 - ch.p0) / kPartMin], h, m, a.g, a.v.vxy, a.pl.slot + (size_t)blockIdx.x * kListRows * kTile,
+                      &bar, parity, a.sc, [&](int j, int k) {
+                          mj_s[k] = a.mj[j];
+                          if (w_src) w_s[k] = w_src[j];
+                          if (a.sum_mode) rho_s[k] = a.rho_in[j];
+                      }))
+            return;
+        density_rate(a, h, m, mj_s, w_s, rho_s, ch, p0);
+        p0 += h.size;
+        if (p0 < ch.p1) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncthreads();
+        }
+    }
 }
 
 // The summation density written to scratch by the second of two passes
@@ -588,19 +878,21 @@ __global__ void k_commit_rho(int n, const double *__restrict__ src, State o, con
     if (i >= n || (inst[pinst[i]].flags & FLAG_RETIRED)) return;
     const double r = src[i];
     o.rho[i] = r;
-    o.mor[i] = o.m[i] / r;
     refresh_views(o, i);
 }
 
 // New hsml of the next step (sle = 1, 2) and its FP32 copy.
-__global__ void k_commit_hsml(int n, const double *__restrict__ hs_next, State s0) {
+__global__ void __launch_bounds__(256) k_commit_hsml(int n, const double *__restrict__ hs_next, State s0, Scalars *sc) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    // how far any hsml grew, for the Verlet lists' bound (NaN: as infinity)
+    double grown = i < n ? hs_next[i] - s0.hs[i] : 0.0;
+    if (!(grown <= 1e300)) grown = INFINITY;
+    warp_max_u64(&sc->acc_dh, dbits(fmax(grown, 0.0)));
     if (i >= n) return;
     const double v = hs_next[i];
     const float vf = (float)v;
     s0.hs[i] = v;
     s0.hsf[i] = vf;
-    s0.pf[i].z = vf;
     if (s0.hmm) s0.hmm[i].x = vf;
 }
 
@@ -612,8 +904,9 @@ __global__ void k_commit_hsml(int n, const double *__restrict__ hs_next, State s
 constexpr int kFinishThreads = 256;
 __global__ void __launch_bounds__(kFinishThreads) k_step_finish(Scalars *sc, Inst *inst, int ninst, int tse,
                                                                 int sle) {
-    __shared__ double dt;
+    __shared__ double dt, grown;
     if (threadIdx.x == 0) {
+        grown = 0.0;
         if (tse != 0) {
             sc->dt = bitsd(sc->acc_dt);
             sc->acc_dt = dbits(INFINITY);
@@ -626,13 +919,28 @@ __global__ void __launch_bounds__(kFinishThreads) k_step_finish(Scalars *sc, Ins
             sc->bs = 2.0 * sc->hmin;
             sc->acc_hmin = dbits(INFINITY);
             sc->acc_hmax = 0ull;
+            grown = bitsd(sc->acc_dh);
+            sc->acc_dh = 0ull;
             inst[0].hmin = sc->hmin;
             inst[0].hmax = sc->hmax;
             inst[0].bs = sc->bs;
         }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < ninst; k += kFinishThreads) inst[k].t = inst[k].t + dt;
+    for (int k = threadIdx.x; k < ninst; k += kFinishThreads) {
+        Inst &I = inst[k];
+        I.t = I.t + dt;
+        // the Verlet lists: built in this step unless they were valid before
+        // it; stale when the step's second right-hand side had to build its
+        // own, or when another step like this one could outrun them
+        const double half = sqrt(bitsd(I.half2_bits)), step = sqrt(bitsd(I.step2_bits));
+        const double old = I.list_ok ? I.list_d : 0.0;
+        const double moved = old + step + 0.5 * grown;
+        I.list_ok = (2.0 * (old + half) * (1.0 + 1e-9) <= I.delta && 2.0 * (moved + half) <= I.delta) ? 1 : 0;
+        I.list_d = moved;
+        I.half2_bits = 0ull;
+        I.step2_bits = 0ull;
+    }
 }
 
 // The Euler step writes its result into S1 (S0 is read by the pair sums of
@@ -640,20 +948,14 @@ __global__ void __launch_bounds__(kFinishThreads) k_step_finish(Scalars *sc, Ins
 __global__ void k_copy_s1_to_s0(int n, State s1, State s0) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    s0.x[i] = s1.x[i];
-    s0.y[i] = s1.y[i];
-    s0.vx[i] = s1.vx[i];
-    s0.vy[i] = s1.vy[i];
+    s0.xy[i] = s1.xy[i];
+    s0.vxy[i] = s1.vxy[i];
+    s0.mm[i] = s1.mm[i];
     s0.h[i] = s1.h[i];
     s0.A[i] = s1.A[i];
     s0.rho[i] = s1.rho[i];
-    s0.mor[i] = s1.mor[i];
     if (s1.m != s0.m) s0.m[i] = s1.m[i];
-    s0.xy[i] = s1.xy[i];
-    s0.vxy[i] = s1.vxy[i];
-    s0.pf[i] = s1.pf[i];
     if (s0.hmm) s0.hmm[i] = s1.hmm[i];
-    else s0.mm[i] = s1.mm[i];
 }
 
 __global__ void k_reset_stats(Scalars *sc) {
@@ -666,16 +968,65 @@ __global__ void k_reset_stats(Scalars *sc) {
 
 inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
-NbrList nbr_list(simp_ctx *c) {
-    NbrList nl;
-    nl.nbr = c->nbr;
-    nl.count = c->nbr_count;
-    nl.xl = c->xl;
-    nl.yl = c->yl;
-    nl.stride = c->maxn;
-    nl.n = c->n;
-    return nl;
+// The chunks of the current layout: src holds, per basin in memory order, its
+// offset, particles, first chunk and slot.
+__device__ __forceinline__ int4 chunk_basin(int c, int nsrc, const int4 *src) {
+    int lo = 0, hi = nsrc - 1;   // the last basin whose first chunk is at or before c
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (src[mid].z <= c) lo = mid;
+        else hi = mid - 1;
+    }
+    return src[lo];
 }
+__global__ void k_chunks(int nchunks, int nsrc, const int4 *__restrict__ src, int size, Chunk *__restrict__ chunks) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= nchunks) return;
+    const int4 b = chunk_basin(c, nsrc, src);
+    const int k = c - b.z, tiles = (b.y + size - 1) / size;
+    if (k < tiles) chunks[c] = Chunk{b.x + k * size, min(b.x + (k + 1) * size, b.x + b.y), b.w, -1};
+    else chunks[c] = Chunk{0, 0, b.w, k - tiles};
+}
+
+// Cuts the tiles of the basins just sorted whose halo would not fit: a sparse
+// cell row's tile spans many cells of its full neighbour rows.  The parts go to
+// the basin's spare tiles, so that they run beside the others; a tile that
+// finds no room there stays whole and is worked off part by part.
+__global__ void k_split(int nchunks, int nsrc, const int4 *__restrict__ src, int size, Chunk *__restrict__ chunks,
+                        DueMask due, Inst *inst, const int *__restrict__ cell_start, const int *__restrict__ bstart,
+                        const int *__restrict__ cell, int cap) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= nchunks) return;
+    const int4 b = chunk_basin(c, nsrc, src);
+    const int k = c - b.z, tiles = (b.y + size - 1) / size;
+    if (k >= tiles || !((due.w[b.w >> 6] >> (b.w & 63)) & 1ull)) return;
+    Inst &I = inst[b.w];
+    const int p0 = b.x + k * size, p1 = min(p0 + size, b.x + b.y);
+    Chunk full{p0, p1, b.w, -1};
+    Halo h;
+    int S = size;
+    for (;; S >>= 1) {
+        make_halo(I, cell_start, bstart, cell, p0, min(p0 + S, p1), cap, h);
+        if (h.kind == HALO_TILE || S <= kPartMin || h.nseg > kMaxSeg) break;
+    }
+    const int extra = (p1 - p0 + S - 1) / S - 1;
+    if (extra > 0) {
+        const int room = spare_tiles(tiles), at = atomicAdd(&I.spares, extra);
+        if (at + extra <= room) {
+            for (int e = 0; e < extra; ++e)
+                chunks[b.z + tiles + at + e] = Chunk{p0 + (e + 1) * S, min(p0 + (e + 2) * S, p1), b.w, at + e};
+            full.p1 = p0 + S;
+        } else {
+            for (int e = at; e < room; ++e) chunks[b.z + tiles + e] = Chunk{0, 0, b.w, e};   // (claimed, unused)
+        }
+    }
+    chunks[c] = full;
+}
+
+// Halo slots of a tile in shared memory: three rows of cells around 128
+// particles take up to 520 slots at hsml = 2.4 spacings (five blocks per SM with
+// the lists), 650 at the reference's 3 spacings, where hsml varies.
+int tile_cap(const simp_ctx *c) { return c->uniform ? 528 : 704; }
 
 TauRec tau_rec(simp_ctx *c) {
     TauRec r;
@@ -687,80 +1038,114 @@ TauRec tau_rec(simp_ctx *c) {
 
 PairList pair_list(simp_ctx *c) {
     PairList pl;
-    pl.pj = c->pair_j;
+    pl.slot = c->pair_slot;
     pl.count = c->pair_count;
-    pl.stride = c->maxn;
     pl.n = c->n;
     return pl;
 }
 
+template <class T, int SKF>
+cudaError_t allow_smem() {
+    cudaError_t e = cudaSuccess;
+    const int most = 96 * 1024;   // (a tile takes 40 to 52 KB)
+    for (const void *f : {(const void *)k_kinematic<T, SKF, true>, (const void *)k_kinematic<T, SKF, false>,
+                          (const void *)k_stress<T, SKF, true>, (const void *)k_stress<T, SKF, false>,
+                          (const void *)k_regularize, (const void *)k_density_rate})
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    return e;
+}
+
+template <class T, int SKF>
+void launch_kin_form(simp_ctx *c, const KinArgs &a) {
+    const int g = c->nchunks;
+    const size_t sm = tile_smem_bytes(a.cap, 3, c->uniform);
+    if (c->uniform) k_kinematic<T, SKF, true><<<g, kTile, sm, c->stream>>>(a);
+    else k_kinematic<T, SKF, false><<<g, kTile, sm, c->stream>>>(a);
+}
+template <class T, int SKF>
+void launch_stress_form(simp_ctx *c, const StressArgs &a) {
+    const int g = c->nchunks;
+    const size_t sm = tile_smem_bytes(a.cap, Rec<T>::stress_arrays, c->uniform);
+    if (c->uniform) k_stress<T, SKF, true><<<g, kTile, sm, c->stream>>>(a);
+    else k_stress<T, SKF, false><<<g, kTile, sm, c->stream>>>(a);
+}
+template <class T, class A>
+void launch_form(simp_ctx *c, const A &a) {
+    constexpr bool kin = std::is_same<A, KinArgs>::value;
+    switch (skf_compiled(c->prm.skf)) {
+        case SIMP_SKF_CUBIC:
+            if constexpr (kin) launch_kin_form<T, SIMP_SKF_CUBIC>(c, a);
+            else launch_stress_form<T, SIMP_SKF_CUBIC>(c, a);
+            break;
+        case SIMP_SKF_WENDLAND_C6:
+            if constexpr (kin) launch_kin_form<T, SIMP_SKF_WENDLAND_C6>(c, a);
+            else launch_stress_form<T, SIMP_SKF_WENDLAND_C6>(c, a);
+            break;
+        default:
+            if constexpr (kin) launch_kin_form<T, 0>(c, a);
+            else launch_stress_form<T, 0>(c, a);
+    }
+}
+
 }  // namespace
 
-void launch_kinematic(simp_ctx *c, const State &s, bool diag) {
+void launch_chunks(simp_ctx *c) {
+    if (c->nchunks == 0) return;
+    k_chunks<<<nblk(c->nchunks, 256), 256, 0, c->stream>>>(c->nchunks, c->nsrc, c->chunk_src, kTile, c->chunks);
+    c->launches += 1;
+}
+void launch_split(simp_ctx *c, const DueMask &due) {
+    if (c->nchunks == 0) return;
+    k_split<<<nblk(c->nchunks, 64), 64, 0, c->stream>>>(c->nchunks, c->nsrc, c->chunk_src, kTile, c->chunks, due,
+                                                        c->inst_dev, c->cell_start, c->bcell_start, c->cell,
+                                                        tile_cap(c));
+    c->launches += 1;
+}
+
+int passes_configure(simp_ctx *c) {
+    const bool mixed = c->prm.precision == SIMP_PREC_MIXED;
+    cudaError_t e;
+    switch (skf_compiled(c->prm.skf)) {
+        case SIMP_SKF_CUBIC: e = mixed ? allow_smem<float, SIMP_SKF_CUBIC>() : allow_smem<double, SIMP_SKF_CUBIC>(); break;
+        case SIMP_SKF_WENDLAND_C6:
+            e = mixed ? allow_smem<float, SIMP_SKF_WENDLAND_C6>() : allow_smem<double, SIMP_SKF_WENDLAND_C6>();
+            break;
+        default: e = mixed ? allow_smem<float, 0>() : allow_smem<double, 0>();
+    }
+    if (e != cudaSuccess) return simp_cuda_check(c, e, "cudaFuncSetAttribute (tile shared memory)");
+    return SIMP_OK;
+}
+
+void launch_kinematic(simp_ctx *c, const State &s, bool diag, bool second) {
     SIMP_RANGE("kinematic pass");
+    if (c->nchunks == 0) return;
     KinArgs a{};
     a.s = s;
     a.cell_start = c->cell_start;
+    a.bstart = c->bcell_start;
     a.inst = c->inst_dev;
     a.pinst = c->pinst;
     a.cell = c->cell;
     a.P = c->phys;
     a.sc = c->sc;
-    a.tau11 = c->tau11;
-    a.tau12 = c->tau12;
-    a.tau22 = c->tau22;
     a.div = c->div;
     a.rec = tau_rec(c);
-    a.dw = c->pair_dw;
     a.diag = diag ? c->diag : nullptr;
-    a.nl = nbr_list(c);
     a.pl = pair_list(c);
     a.n = c->n;
     a.maxn = c->maxn;
-    if (c->pass_impl == SIMP_PASSES_TILED) {
-        launch_kinematic_tiled(c, a);
-        return;
-    }
-    const int g = nblk(c->n, kBlock);
-    const bool mixed = c->prm.precision == SIMP_PREC_MIXED;
-    const bool two = c->pass_impl == SIMP_PASSES_GATHER_TWO ||
-                     (c->pass_impl == SIMP_PASSES_GATHER && c->n <= kSplitMaxParticles);
-    if (!two) {
-        switch (skf_compiled(c->prm.skf)) {
-            case SIMP_SKF_CUBIC:
-                if (mixed) k_kinematic<float, SIMP_SKF_CUBIC><<<g, kBlock, 0, c->stream>>>(a);
-                else k_kinematic<double, SIMP_SKF_CUBIC><<<g, kBlock, 0, c->stream>>>(a);
-                break;
-            case SIMP_SKF_WENDLAND_C6:
-                if (mixed) k_kinematic<float, SIMP_SKF_WENDLAND_C6><<<g, kBlock, 0, c->stream>>>(a);
-                else k_kinematic<double, SIMP_SKF_WENDLAND_C6><<<g, kBlock, 0, c->stream>>>(a);
-                break;
-            default:
-                if (mixed) k_kinematic<float, 0><<<g, kBlock, 0, c->stream>>>(a);
-                else k_kinematic<double, 0><<<g, kBlock, 0, c->stream>>>(a);
-        }
-        c->launches += 1;
-        return;
-    }
-    k_find_pairs<<<g, kBlock, 0, c->stream>>>(a);
-    switch (skf_compiled(c->prm.skf)) {
-        case SIMP_SKF_CUBIC:
-            if (mixed) k_kin_sums<float, SIMP_SKF_CUBIC><<<g, kBlock, 0, c->stream>>>(a);
-            else k_kin_sums<double, SIMP_SKF_CUBIC><<<g, kBlock, 0, c->stream>>>(a);
-            break;
-        case SIMP_SKF_WENDLAND_C6:
-            if (mixed) k_kin_sums<float, SIMP_SKF_WENDLAND_C6><<<g, kBlock, 0, c->stream>>>(a);
-            else k_kin_sums<double, SIMP_SKF_WENDLAND_C6><<<g, kBlock, 0, c->stream>>>(a);
-            break;
-        default:
-            if (mixed) k_kin_sums<float, 0><<<g, kBlock, 0, c->stream>>>(a);
-            else k_kin_sums<double, 0><<<g, kBlock, 0, c->stream>>>(a);
-    }
-    c->launches += 2;
+    a.chunks = c->chunks;
+    a.halos = c->halos;
+    a.cap = tile_cap(c);
+    a.second = second ? 1 : 0;
+    if (c->prm.precision == SIMP_PREC_MIXED) launch_form<float>(c, a);
+    else launch_form<double>(c, a);
+    c->launches += 1;
 }
 
 void launch_stress(simp_ctx *c, const State &rhs, const State &base, EpiMode mode) {
     SIMP_RANGE("stress pass");
+    if (c->nchunks == 0) return;
     StressArgs a{};
     a.rhs = rhs;
     a.base = base;
@@ -778,41 +1163,21 @@ void launch_stress(simp_ctx *c, const State &rhs, const State &base, EpiMode mod
     a.nb = c->nb;
     a.P = c->phys;
     a.sc = c->sc;
-    a.tau11 = c->tau11;
-    a.tau12 = c->tau12;
-    a.tau22 = c->tau22;
     a.div = c->div;
     a.rec = tau_rec(c);
-    a.dw = c->pair_dw;
-    a.nl = nbr_list(c);
     a.pl = pair_list(c);
     a.rates = c->rates;
     a.reg = c->reg;
-    a.xr = c->xr;
-    a.yr = c->yr;
+    a.xyr = c->xyr;
     a.hs_next = c->tmp;   // hsml of the next step (committed by launch_step_finish)
     a.n = c->n;
     a.maxn = c->maxn;
     a.mode = mode;
-    if (c->pass_impl == SIMP_PASSES_TILED) {
-        launch_stress_tiled(c, a);
-        return;
-    }
-    const bool mixed = c->prm.precision == SIMP_PREC_MIXED;
-    const int g = nblk(c->n, kBlock);
-    switch (skf_compiled(c->prm.skf)) {
-        case SIMP_SKF_CUBIC:
-            if (mixed) k_stress<float, SIMP_SKF_CUBIC><<<g, kBlock, 0, c->stream>>>(a);
-            else k_stress<double, SIMP_SKF_CUBIC><<<g, kBlock, 0, c->stream>>>(a);
-            break;
-        case SIMP_SKF_WENDLAND_C6:
-            if (mixed) k_stress<float, SIMP_SKF_WENDLAND_C6><<<g, kBlock, 0, c->stream>>>(a);
-            else k_stress<double, SIMP_SKF_WENDLAND_C6><<<g, kBlock, 0, c->stream>>>(a);
-            break;
-        default:
-            if (mixed) k_stress<float, 0><<<g, kBlock, 0, c->stream>>>(a);
-            else k_stress<double, 0><<<g, kBlock, 0, c->stream>>>(a);
-    }
+    a.chunks = c->chunks;
+    a.halos = c->halos;
+    a.cap = tile_cap(c);
+    if (c->prm.precision == SIMP_PREC_MIXED) launch_form<float>(c, a);
+    else launch_form<double>(c, a);
     c->launches += 1;
 }
 
@@ -823,17 +1188,18 @@ void launch_regularize(simp_ctx *c, const State &s) {
     a.s = s;
     a.div = c->div;
     a.pl = pair_list(c);
-    a.nl = nbr_list(c);
     a.cell_start = c->cell_start;
     a.cell = c->cell;
-    a.pinst = c->pinst;
+    a.chunks = c->chunks;
+    a.halos = c->halos;
+    a.cap = tile_cap(c);
     a.inst = c->inst_dev;
     a.sc = c->sc;
     a.P = c->phys;
     a.reg = c->reg;
     a.n = c->n;
     a.maxn = c->maxn;
-    k_regularize<<<nblk(c->n, kBlock), kBlock, 0, c->stream>>>(a);
+    k_regularize<<<c->nchunks, kTile, aux_smem_bytes(a.cap), c->stream>>>(a);
     c->launches += 1;
 }
 
@@ -850,7 +1216,9 @@ void launch_density_rate(simp_ctx *c, const State &g, const State &v, int rho_up
     a.pl = pair_list(c);
     a.cell_start = c->cell_start;
     a.cell = c->cell;
-    a.pinst = c->pinst;
+    a.chunks = c->chunks;
+    a.halos = c->halos;
+    a.cap = tile_cap(c);
     a.inst = c->inst_dev;
     a.sc = c->sc;
     a.P = c->phys;
@@ -858,7 +1226,7 @@ void launch_density_rate(simp_ctx *c, const State &g, const State &v, int rho_up
     a.rho_upd = rho_upd;
     a.tail = tail ? 1 : 0;
     a.dt_div = (tail && c->prm.tse == 1 && c->prm.artificial_visc) ? 1 : 0;
-    k_density_rate<<<nblk(c->n, kBlock), kBlock, 0, c->stream>>>(a);
+    k_density_rate<<<c->nchunks, kTile, aux_smem_bytes(a.cap), c->stream>>>(a);
     c->launches += 1;
 }
 
@@ -876,7 +1244,9 @@ void launch_sum_density(simp_ctx *c, const State &g, const State &v, const doubl
     a.pl = pair_list(c);
     a.cell_start = c->cell_start;
     a.cell = c->cell;
-    a.pinst = c->pinst;
+    a.chunks = c->chunks;
+    a.halos = c->halos;
+    a.cap = tile_cap(c);
     a.inst = c->inst_dev;
     a.sc = c->sc;
     a.P = c->phys;
@@ -890,7 +1260,7 @@ void launch_sum_density(simp_ctx *c, const State &g, const State &v, const doubl
     a.rho_out = rho_out;
     a.k0 = c->k0;
     a.id = c->id;
-    k_density_rate<<<nblk(c->n, kBlock), kBlock, 0, c->stream>>>(a);
+    k_density_rate<<<c->nchunks, kTile, aux_smem_bytes(a.cap), c->stream>>>(a);
     c->launches += 1;
 }
 
@@ -901,7 +1271,7 @@ void launch_commit_rho(simp_ctx *c, const double *src, const State &o) {
 
 void launch_step_finish(simp_ctx *c) {
     if (c->prm.sle != 0) {
-        k_commit_hsml<<<nblk(c->n, 256), 256, 0, c->stream>>>(c->n, c->tmp, c->s0);
+        k_commit_hsml<<<nblk(c->n, 256), 256, 0, c->stream>>>(c->n, c->tmp, c->s0, c->sc);
         c->launches += 1;
     }
     k_step_finish<<<1, kFinishThreads, 0, c->stream>>>(c->sc, c->inst_dev, c->ninst, c->prm.tse, c->prm.sle);

@@ -1,0 +1,234 @@
+// Tiles of the pair passes.
+//
+// A tile is up to kTile consecutive particles of one basin, one per thread of
+// a block.  Particles are stored in cell order, row-major, so the cells within
+// R of a tile's cells are 2R + 1 runs of consecutive cell keys, hence 2R + 1
+// contiguous index ranges (its halo), whether or not the tile wraps from one
+// cell row into the next.  A block copies its halo's records to shared memory
+// (one bulk copy per range and array) and the pair arithmetic gathers from
+// there: a gather from global memory waits for its slowest lane's L2 miss on
+// nearly every pair (12 of 17 cycles between a warp's instructions, at issue
+// slots 25% and L1 40% busy), one from shared memory never does.
+//
+// The candidates of a particle are a Verlet list of slots, 16 bits each, copied
+// to shared memory with the halo.  A kinematic pass whose basin's lists are
+// stale first builds them (k_kinematic: the cell stencil against FP32 copies).
+// The exact FP64 criterion is applied to every candidate in each pass.
+// Candidates are in increasing index order, so the sums depend neither on the
+// tile shape nor on when a list was built.
+//
+// A tile whose halo exceeds the shared-memory capacity (a sparse cell row next
+// to full ones) is cut in halves down to kPartMin particles, taken one after
+// another; one that still does not fit, whose stencil radius exceeds
+// kMaxRadius or which has a particle of more than kListRows candidates reads
+// its neighbours from global memory with the same arithmetic in the same
+// order.
+#pragma once
+
+#include "pass_common.cuh"
+
+namespace simp {
+namespace pass {
+
+constexpr int kMaxRadius = 2;
+constexpr int kMaxSeg = 2 * kMaxRadius + 1;
+constexpr int kSlotPad = 40;               // slots a candidate batch may read past the halo
+
+// The halo of a tile or part of one, one record per part.
+enum : int { HALO_NONE = 0, HALO_TILE = 1, HALO_GLOBAL = 2 };
+struct Halo {
+    int kind, walls, nseg;     // walls: its particles may have wall pairs
+    int rows;                  // longest list of one of its particles
+    int lo[kMaxSeg];           // first particle of each range
+    int off[kMaxSeg + 1];      // its first slot, and the total
+    int size;                  // particles in this part of the tile
+};
+static_assert(sizeof(Halo) == kHaloBytes, "ctx.h: kHaloBytes");
+
+// Bulk copies to shared memory, completing on an mbarrier.
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void bar_init(unsigned long long *bar) {
+    asm volatile("mbarrier.init.shared.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+__device__ __forceinline__ void bar_expect(unsigned long long *bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned bytes, unsigned long long *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_addr(dst)),
+                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
+                 : "memory");
+}
+// Waits for the barrier's phase; gives up after a bounded number of tries.
+__device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parity) {
+    for (int k = 0; k < (1 << 20); ++k) {
+        unsigned ok;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+            : "=r"(ok)
+            : "r"(smem_addr(bar)), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// Shared memory of a tile: records of 16 bytes per particle by array (xy and
+// the pass's own), hsml where it varies, and the lists.  While lists are built
+// the FP32 copies stand where the pass's own records go.
+struct TileMem {
+    unsigned char *rec[3];
+    double *hs;
+    unsigned short *list;           // kListRows slots per thread
+    __device__ __forceinline__ float2 *f() const { return reinterpret_cast<float2 *>(rec[2]); }
+    __device__ __forceinline__ float *hf() const { return reinterpret_cast<float *>(rec[1]); }
+};
+
+__host__ __device__ inline size_t tile_smem_bytes(int cap, int arrays, bool uniform) {
+    return (size_t)cap * (16 * arrays + (uniform ? 0 : 8)) + (size_t)kListRows * kTile * sizeof(unsigned short);
+}
+
+__device__ __forceinline__ TileMem tile_mem(unsigned char *p, int cap, int arrays, bool uniform) {
+    TileMem m;
+    for (int a = 0; a < 3; ++a) m.rec[a] = p + (size_t)(a < arrays ? a : 0) * 16 * cap;
+    p += (size_t)16 * cap * arrays;
+    m.hs = reinterpret_cast<double *>(p);
+    if (!uniform) p += (size_t)cap * sizeof(double);
+    m.list = reinterpret_cast<unsigned short *>(p);
+    return m;
+}
+
+// The halo of particles [p0, p1) of instance I.  Called by one thread.
+__device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, const int *bstart, const int *cell, int p0,
+                                       int p1, int cap, Halo &h) {
+    const Grid g = inst_grid(I, cell_start);
+    const int R = stencil_radius(I.hmax, I.dmax2_bits, g, I.hmax + I.delta);
+    h.size = p1 - p0;
+    h.nseg = 2 * R + 1;
+    h.rows = 0;
+    h.kind = R <= kMaxRadius ? HALO_TILE : HALO_GLOBAL;
+    const int ka = cell[p0], kb = cell[p1 - 1], end = I.base + I.ncx * I.ncy;
+    // walls within b_length of any place its particles take while the lists
+    // stay valid (they move less than delta)
+    h.walls = 0;
+    const int Rb = wall_radius(I.dmax2_bits, g, I.b_length + I.delta);
+    for (int d = -Rb; d <= Rb && !h.walls; ++d)
+        h.walls = bstart[clampi(kb + d * I.ncx + Rb + 1, I.base, end)] > bstart[clampi(ka + d * I.ncx - Rb, I.base, end)];
+    if (h.kind == HALO_GLOBAL) return;
+    int a[kMaxSeg], b[kMaxSeg];
+#pragma unroll
+    for (int d = 0; d < kMaxSeg; ++d) {
+        if (d >= h.nseg) break;
+        const int sh = (d - R) * I.ncx;
+        a[d] = cell_start[clampi(ka + sh - R, I.base, end)];
+        b[d] = cell_start[clampi(kb + sh + R + 1, I.base, end)];
+    }
+    int total = 0, past = 0;
+#pragma unroll
+    for (int d = 0; d < kMaxSeg; ++d) {
+        if (d >= h.nseg) break;
+        // (a tile of more than a cell row: its ranges meet)
+        h.lo[d] = max(a[d], past);
+        h.off[d] = total;
+        total += max(b[d] - h.lo[d], 0);
+        past = max(b[d], past);
+    }
+    h.off[h.nseg] = total;
+    if (total > cap) h.kind = HALO_GLOBAL;
+}
+
+// Slot of particle j, which the halo holds.
+__device__ __forceinline__ int slot_of(const Halo &h, int j) {
+    int s = h.off[0] + j - h.lo[0];
+#pragma unroll
+    for (int d = 1; d < kMaxSeg; ++d)
+        if (d < h.nseg && j >= h.lo[d]) s = h.off[d] + j - h.lo[d];
+    return s;
+}
+__device__ __forceinline__ int particle_of(const Halo &h, int slot) {
+    int j = h.lo[0] + slot - h.off[0];
+#pragma unroll
+    for (int d = 1; d < kMaxSeg; ++d)
+        if (d < h.nseg && slot >= h.off[d]) j = h.lo[d] + slot - h.off[d];
+    return j;
+}
+
+// Column and row of cell ci, and the candidate range d of a particle there:
+// [j0, j1).
+__device__ __forceinline__ int2 cell_at(const Inst &I, int ci) {
+    const int local = ci - I.base;
+    if (!SIMP_IN_RANGE(local, 0, (long long)I.ncx * I.ncy, SITE_CELL)) return make_int2(0, -kMaxSeg);
+    const int cy = local / I.ncx;
+    return make_int2(local - cy * I.ncx, cy);
+}
+__device__ __forceinline__ void stencil_range(const Inst &I, const int *cell_start, int2 at, int R, int d, int &j0,
+                                              int &j1) {
+    const int cy = at.y + d - R;
+    j0 = j1 = 0;
+    if (cy < 0 || cy >= I.ncy) return;
+    const int k = I.base + cy * I.ncx;
+    j0 = cell_start[k + max(at.x - R, 0)];
+    j1 = cell_start[k + min(at.x + R, I.ncx - 1) + 1];
+}
+
+// Starts the copies of record arrays [a0, a1) of the halo and of `rows` rows
+// of its lists.  Called by the first warp.
+__device__ __forceinline__ void tile_fetch(const Halo &h, const TileMem &m, const void *const (&src)[3], int a0, int a1,
+                                           const unsigned short *list, int rows, unsigned long long *bar) {
+    const int lane = threadIdx.x & 31, arrays = a1 - a0;
+    const unsigned list_bytes = (unsigned)(rows * kTile * sizeof(unsigned short));
+    if (lane == 0) bar_expect(bar, (unsigned)h.off[h.nseg] * 16u * (unsigned)arrays + list_bytes);
+    __syncwarp();
+    if (lane == 31 && rows > 0) bulk_copy(m.list, list, list_bytes, bar);
+    if (lane < h.nseg * arrays) {
+        const int d = lane / arrays, a = a0 + lane - d * arrays;
+        const int n = h.off[d + 1] - h.off[d];
+        if (n > 0)
+            bulk_copy(m.rec[a] + (size_t)16 * h.off[d],
+                      reinterpret_cast<const unsigned char *>(src[a]) + (size_t)16 * h.lo[d], 16u * (unsigned)n, bar);
+    }
+}
+
+// Half width of the band around mhsml^2 within which a squared distance needs
+// the exact criterion (the fma'd squares are within 2^-50 of the exact ratio).
+constexpr double kBand = 0x1p-40;
+
+// The exact reference criterion (nnps.f90:277-281 and the bucket rule).
+__device__ __noinline__ bool exact_pair(const State &s, const Inst &I, bool rule, double xi, double yi, double hi,
+                                        int j) {
+    const double2 q = __ldg(&s.xy[j]);
+    double r;
+    const double mh = __dmul_rn(__dadd_rn(hi, __ldg(&s.hs[j])), 0.5);
+    if (!pair_test(__dsub_rn(xi, q.x), __dsub_rn(yi, q.y), mh, &r)) return false;
+    return !rule || bin_rule_ok(make_bin_rule(I.bs, xi, yi, I.hmax), q.x, q.y);
+}
+__device__ __forceinline__ bool rule_on(const Inst &I) { return I.hmax >= I.bs * (1.0 - 1e-6); }
+
+// Pairs of particle i from global memory over its cell stencil: f(j).
+template <class F>
+__device__ __forceinline__ void global_pairs(const State &s, const Inst &I, const int *cell_start, int i, int ci,
+                                             F &&f) {
+    const double2 p = s.xy[i];
+    const double hi = s.hs[i];
+    const bool rule = rule_on(I);
+    const int2 at = cell_at(I, ci);
+    const int R = stencil_radius(I.hmax, I.dmax2_bits, inst_grid(I, cell_start), 0.0);
+    for (int d = 0; d < 2 * R + 1; ++d) {
+        int j0, j1;
+        stencil_range(I, cell_start, at, R, d, j0, j1);
+#pragma unroll 4
+        for (int j = j0; j < j1; ++j) {
+            const double2 q = __ldg(&s.xy[j]);
+            const double dx = p.x - q.x, dy = p.y - q.y, mh = 0.5 * (hi + __ldg(&s.hs[j]));
+            const double d2 = fma(dx, dx, dy * dy);
+            if (d2 > mh * mh * (1.0 + kBand) || j == i) continue;
+            if (!(d2 < mh * mh * (1.0 - kBand)) || rule)
+                if (!exact_pair(s, I, rule, p.x, p.y, hi, j)) continue;
+            f(j);
+        }
+    }
+}
+
+}  // namespace pass
+}  // namespace simp

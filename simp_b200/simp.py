@@ -136,9 +136,8 @@ class Simp:
                 setattr(self.params, name, getattr(forcing, name))
 
     def set_passes(self, impl: int, threads: int = 256, cap: int = 1024):
-        """Pair-pass implementation (params.PASSES_*): 0 per-particle gathers
-        with the kinematic pass's form chosen by size, 1 shared-memory tiles,
-        2 gathers with a one-kernel kinematic pass, 3 with a two-kernel one."""
+        """Names a pair-pass implementation (params.PASSES_*); one
+        implementation serves every name, with the same results."""
         self._chk(self.lib.simp_gpu_set_passes(self.h, int(impl), int(threads), int(cap)))
 
     def get_passes(self):
@@ -147,8 +146,7 @@ class Simp:
         return a.value, b.value, c.value
 
     def autotune(self, reps: int = 3) -> float:
-        """Picks the fastest pass implementation and tile shape for the
-        current state; returns its milliseconds per right-hand side."""
+        """Milliseconds per right-hand side of the current state."""
         ms = ctypes.c_double()
         self._chk(self.lib.simp_gpu_autotune(self.h, int(reps), ctypes.byref(ms)))
         return ms.value
