@@ -251,9 +251,7 @@ __global__ void k_continue_finish(Scalars *sc, Inst *inst, double dt, double t, 
     sc->dt = dt;
     sc->t = t;
     inst[0].t = t;
-    const unsigned long long b2 = (unsigned long long)__double_as_longlong(d2);
-    if (b2 > sc->dmax2_bits) sc->dmax2_bits = b2;
-    if (b2 > inst[0].dmax2_bits) inst[0].dmax2_bits = b2;
+    inst[0].disp = fmax(inst[0].disp, sqrt(d2));
     inst[0].list_ok = 0;
     const unsigned long long bx = (unsigned long long)__double_as_longlong(xa);
     if (bx > sc->xabs_bits) sc->xabs_bits = bx;
@@ -318,6 +316,7 @@ Phys make_phys(const simp_params &p, double max_hsml) {
     P.em2 = 1.0 / (p.e * p.e);
     P.inv_1kt = 1.0 / (1.0 + p.k_t);
     P.inv_rho_ice = 1.0 / p.rho_ice;
+    P.inv_b_length = 1.0 / p.b_length;
     return P;
 }
 
@@ -429,7 +428,7 @@ int layout(simp_ctx *c) {
         InstHost &h = c->insts[q];
         if (h.I.base >= 0) {   // already on the device: keep its evolving fields
             h.I.t = cur[q].t;
-            h.I.dmax2_bits = cur[q].dmax2_bits;
+            h.I.disp = cur[q].disp;
             h.I.flags = cur[q].flags;
             h.I.hmin = cur[q].hmin;
             h.I.hmax = cur[q].hmax;
@@ -658,7 +657,7 @@ int add_instance(simp_ctx *c, int slot, const simp_forcing &f, const Extents &e,
     I.hmin = hmin;
     I.hmax = hmax;
     I.bs = 2.0 * hmin;
-    I.dmax2_bits = 0ull;
+    I.disp = 0.0;
     I.delta = 0.4 * list_skin(c, hmax);
     I.flags = 0;
     // particle arrays at [off, off + n), staged by stage_instance
@@ -887,7 +886,9 @@ int ensure_graph(simp_ctx *c, bool diag) {
     cudaGraph_t g = nullptr;
     const long long before = c->launches;
     SIMP_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    c->overlap_launches = !prof;   // (the events between the kernels end each one)
     enqueue_step(c, diag, prof);
+    c->overlap_launches = false;
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
     c->graph_kernels = c->launches - before;   // captured, not yet launched
     c->launches = before;

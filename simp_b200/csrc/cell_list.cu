@@ -155,7 +155,7 @@ __global__ void k_reset_inst_disp(Inst *inst, int ninst, DueMask due) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= ninst) return;
     if (!((due.w[q >> 6] >> (q & 63)) & 1ull)) return;
-    inst[q].dmax2_bits = 0ull;
+    inst[q].disp = 0.0;
     inst[q].list_ok = 0;   // (its particles take new places)
     inst[q].spares = 0;
 }
@@ -240,9 +240,6 @@ __global__ void k_put_back(int kept, int from, DueMask due, Gather gd, State s, 
     refresh_views(s, k);
 }
 
-// After a sort: displacement since the sort restarts.
-__global__ void k_reset_disp(Scalars *sc) { sc->dmax2_bits = 0ull; }
-
 inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
 }  // namespace
@@ -314,8 +311,6 @@ int rebuild(simp_ctx *c, const DueMask &due, int from) {
     } else {
         SIMP_CUDA(c, cudaMemsetAsync(c->cell_start, 0, sizeof(int) * (size_t)(nkeys + 1), s));
     }
-    k_reset_disp<<<1, 1, 0, s>>>(c->sc);
-    c->launches += 1;
     c->n = kept;
     launch_split(c, due);
     SIMP_CUDA(c, cudaGetLastError());

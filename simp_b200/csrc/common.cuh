@@ -40,10 +40,10 @@ __device__ __forceinline__ void refresh_views(const State &s, int k) {
 
 // Verlet lists of the pair passes, per tile (tile.cuh): the candidates of
 // particle i, every j within mhsml + delta when the list was built, as slots
-// of its tile's halo, slot[(tile * kListRows + k) * kTile + column], k <
+// of its tile's halo, slot[tile * kListRows * kTile + list_at(k, column)], k <
 // count[i].
 constexpr int kTile = 128;      // particles per tile
-constexpr int kListRows = 44;
+constexpr int kListRows = 44;   // (even)
 struct PairList {
     unsigned short *slot;
     int *count;
@@ -69,7 +69,7 @@ struct Inst {
     double b_length;
     double t;                    // this instance's current_time
     double hmin, hmax, bs;       // hsml bounds and reference bucket size
-    unsigned long long dmax2_bits;  // max squared displacement since its last sort
+    double disp;                 // bound on any displacement since its last sort, at the step's start
     int flags;                   // FLAG_* seen in this instance
     // Verlet lists: valid while 2 (list_d + half step) <= delta, with list_d
     // bounding how far any particle moved (and half of how far any hsml
@@ -106,8 +106,7 @@ struct Scalars {
     double t;             // current_time
     double hmin, hmax;    // exact min / max of the current hsml
     double bs;            // reference bucket size 2 * hmin (nnps.f90:211)
-    unsigned long long dmax2_bits;  // max squared displacement since rebuild
-    unsigned long long xabs_bits;   // max |coordinate| of any particle so far
+    unsigned long long xabs_bits;   // bound on any particle's |coordinate|, at the step's start
     unsigned long long acc_hmin, acc_hmax;  // accumulators of the next hsml
     unsigned long long acc_dt;              // VP time step min accumulator
     unsigned long long acc_dh;              // max growth of any hsml in this step
@@ -163,8 +162,8 @@ struct Phys {
     int xsph, art_visc, artificial_visc;
     int csound;                     // 1: c_yang is refreshed (sound_speed.f90:21-27), 0: c stays 0
     double alpha_pi, beta_pi, chi;
-    // 1 / e^2, 1 / (1 + k_t), 1 / rho_ice
-    double em2, inv_1kt, inv_rho_ice;
+    // 1 / e^2, 1 / (1 + k_t), 1 / rho_ice, 1 / b_length
+    double em2, inv_1kt, inv_rho_ice, inv_b_length;
 };
 
 // Interaction-count bookkeeping for nnps.f90:613-670.
@@ -369,8 +368,8 @@ __device__ __forceinline__ double kernel_zero(const Phys &P, double hij) {
 template <int SKF = 0>
 __device__ __forceinline__ double boundary_w(const Phys &P, double br, double hs_i) {
     const double sh = (double)P.scale_h;
-    const double q = br / P.b_length * sh;
-    const double shb = sh / P.b_length, s2 = shb * shb;
+    const double shb = sh * P.inv_b_length, s2 = shb * shb;
+    const double q = br * shb;
     switch (skf_of<SKF>(P.skf)) {
         case SIMP_SKF_QUADRATIC:
             return (2.0 / kPi) * s2 * (0.1875 * q * q - 0.75 * q + 0.75);
@@ -516,7 +515,7 @@ __device__ __forceinline__ void wind_at(const Inst &I, double x, double y, doubl
 
 // Stencil radius in cells that is guaranteed to contain every pair at the
 // current positions: pairs are at most hmax apart now, each particle moved at
-// most sqrt(dmax2) since it was binned.
+// most dm since it was binned.
 // The result is clamped to [1, max(ncx, ncy)] (a non-finite bound, which the
 // step reports as an error, then scans the whole grid instead of overflowing).
 __device__ __forceinline__ int clamp_radius(double Rd, const Grid &g) {
@@ -526,9 +525,10 @@ __device__ __forceinline__ int clamp_radius(double Rd, const Grid &g) {
     return (int)Rd;
 }
 
-__device__ __forceinline__ int stencil_radius(double hmax, unsigned long long dmax2_bits, const Grid &g,
-                                              double extra) {
-    const double dm = sqrt(bitsd(dmax2_bits));
+// Bound on how far any particle of an instance is from where it was sorted
+// (also in the half-step state).
+__device__ __forceinline__ double inst_disp(const Inst &I) { return I.disp + sqrt(bitsd(I.half2_bits)); }
+__device__ __forceinline__ int stencil_radius(double hmax, double dm, const Grid &g, double extra) {
     const double reach = fmax(hmax, extra) + 2.0 * dm;
     return clamp_radius(ceil(reach * g.inv_cs * (1.0 + 1e-12) + 1e-9), g);
 }

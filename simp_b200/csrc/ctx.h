@@ -139,6 +139,7 @@ struct simp_ctx {
     bool graph_stale = false;      // captured arguments changed since the last capture
     bool graph_diag = false;
     bool graph_profiled = false;
+    bool overlap_launches = false; // while a step is captured: programmatic dependent launches
     long long graph_kernels = 0;   // kernels per replay
     // re-sort graph of a single basin: the kernels of one scheduled re-sort,
     // captured once and replayed while what they capture stays the same

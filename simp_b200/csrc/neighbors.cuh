@@ -119,9 +119,8 @@ __device__ __forceinline__ int prefilter(float dxf, float dyf, float mf, float m
 }
 
 // Stencil radius for wall pairs: walls are static, the particle moved at
-// most sqrt(dmax2) since it was binned.
-__device__ __forceinline__ int wall_radius(unsigned long long dmax2_bits, const Grid &g, double b_length) {
-    const double dm = sqrt(bitsd(dmax2_bits));
+// most dm since it was binned.
+__device__ __forceinline__ int wall_radius(double dm, const Grid &g, double b_length) {
     return clamp_radius(ceil((b_length + dm) * g.inv_cs * (1.0 + 1e-12) + 1e-9), g);
 }
 

@@ -48,14 +48,14 @@ __global__ void __launch_bounds__(kBlock) k_count(ExpArgs a) {
     const double2 xy = s.xy[i];
     const double xi = xy.x, yi = xy.y, hi = s.hs[i];
     const int ci = a.cell[i];
-    const int R = stencil_radius(I.hmax, I.dmax2_bits, g, 0.0);
+    const int R = stencil_radius(I.hmax, inst_disp(I), g, 0.0);
     const BinRule br = make_bin_rule(I.bs, xi, yi, I.hmax);
     const int idi = a.id[i];
     int up = 0;
     int cnt = for_each_pair([&](int j) { return s.xy[j]; }, s.hs, g, i, ci, R, br, xi, yi, hi,
                             [&](int j, double, double, double, double) { up += (a.id[j] > idi); });
     if (a.P.boundary_pressure && a.nb > 0) {
-        const int Rb = wall_radius(I.dmax2_bits, g, I.b_length);
+        const int Rb = wall_radius(inst_disp(I), g, I.b_length);
         const BinRule bb = make_bin_rule(I.bs, xi, yi, I.b_length);
         cnt += for_each_wall(a.bx, a.by, a.bstart, g, ci, Rb, bb, xi, yi, I.b_length,
                              [&](int, double, double, double) {});
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kBlock) k_emit(ExpArgs a) {
     const Grid g = inst_grid(I, a.cell_start);
     const double2 xy = s.xy[i];
     const double xi = xy.x, yi = xy.y, hi = s.hs[i];
-    const int R = stencil_radius(I.hmax, I.dmax2_bits, g, 0.0);
+    const int R = stencil_radius(I.hmax, inst_disp(I), g, 0.0);
     const BinRule br = make_bin_rule(I.bs, xi, yi, I.hmax);
     const int idi = a.id[i];
     const int base = a.up_off[idi];
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(kBlock) k_wall(WallArgs a) {
     const Inst &I = a.inst[0];
     const Grid g = inst_grid(I, a.cell_start);
     const double xb = a.bx[b], yb = a.by[b];
-    const int Rb = wall_radius(I.dmax2_bits, g, I.b_length);
+    const int Rb = wall_radius(inst_disp(I), g, I.b_length);
     const BinRule bb = make_bin_rule(I.bs, xb, yb, I.b_length);
     const int idb = a.bid[b];
     const int base = a.emit ? a.off[idb] : 0;
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kBlock) k_sum_density(DenArgs a) {
     const Grid g = inst_grid(I, a.cell_start);
     const double2 xy = s.xy[i];
     const double xi = xy.x, yi = xy.y, hi = s.hs[i];
-    const int R = stencil_radius(I.hmax, I.dmax2_bits, g, 0.0);
+    const int R = stencil_radius(I.hmax, inst_disp(I), g, 0.0);
     const BinRule br = make_bin_rule(I.bs, xi, yi, I.hmax);
     const double k0 = kernel_zero(P, hi);
     const double mi = s.m[i], rhoi = s.rho[i];

@@ -170,7 +170,6 @@ __global__ void k_grid(unsigned char *base) {
     s.hmin = hmin;
     s.hmax = hmax;
     s.bs = 2.0 * hmin;
-    s.dmax2_bits = 0ull;
     h->sc = s;
 }
 

@@ -97,11 +97,39 @@ __device__ __forceinline__ PairGeom<T> pair_geom(const Phys &P, T dx, T dy, T hi
     return g;
 }
 
+// sqrt(u) and 1 / (2 sqrt(u)).  FP64, from the hardware's approximate
+// reciprocal root (relative error 2^-20): a round of Goldschmidt's coupled
+// iteration (g -> sqrt(u), h -> 1 / (2 sqrt(u)), r = 1/2 - g h) to 2^-39, then
+// one correction of both: with d = u - g^2, sqrt(u) = g + d h, and the deviation
+// of 2 h sqrt(u) from 1 is 2 (d h^2 - r).  What is left is the last rounding
+// (largest error over 3 million arguments: 1.00 of 2^-53; u * rsqrt(u)
+// and rsqrt(u) have 1.49 and 1.00).  Unlike rsqrt() it has no branch for subnormal
+// arguments, which a squared distance is not, so that two pairs' roots
+// interleave.  u = 0 gives NaN, as rsqrt(0) * 0 does.
+__device__ __forceinline__ void root_pair(double u, double &g, double &h) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(u));
+    g = u * y;
+    h = 0.5 * y;
+    double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    const double e = fma(-g, g, u) * h;
+    r = fma(-e, h, fma(-g, h, 0.5));
+    g += e;
+    h = fma(h + h, r, h);
+}
+__device__ __forceinline__ void root_pair(float u, float &g, float &h) {
+    const float y = rsqrtf(u);
+    g = u * y;
+    h = 0.5f * y;
+}
+
 // grad W_ij = g (x_i - x_j) of the compiled kernels, split so that a uniform
 // hsml costs nothing per pair: g = scale * shape, where the shape depends on
-// q^2 alone and the scale on hsml_ij.  With H = hsml_ij and y = 1 / (r H):
-// q / scale_h = r / H = r^2 y, 1 / H^2 = r^2 y^2, so one reciprocal root
-// gives both without a division.
+// q^2 alone and the scale on hsml_ij.  With H = hsml_ij, R = sqrt(r^2 H^2) = r H
+// and n = 1 / (2 R): q / scale_h = r / H = 2 r^2 n and 1 / H^2 = 4 r^2 n^2, so
+// one root gives both without a division.
 //   cubic (kernel.f90:324-340), q = 2 r / H: dW/dq / q is 1.5 q - 2 up to
 //     q = 1 and -(2 - q)^2 / (2 q) beyond, scale 15/(7 pi) (2 / H)^4;
 //   Wendland C6 (kernel.f90:499-508), q = r / H: -22 (1 - q)^7 (16 q^2 +
@@ -111,25 +139,25 @@ struct Grad;
 template <class T>
 struct Grad<T, SIMP_SKF_CUBIC> {
     static constexpr double factor = 15.0 / (7.0 * kPi) * 16.0;
-    // k = 4 / H^2, inv_q = 1 / q
-    static __device__ __forceinline__ T shape(T q, T inv_q) {
-        const T u = T(2) - q;
-        return q <= T(1) ? fma(T(1.5), q, T(-2)) : (u * u) * (T(-0.5) * inv_q);
-    }
     static constexpr double qscale = 2.0;
+    // h = 1 / (2 q)
+    static __device__ __forceinline__ T shape(T q, T h) {
+        const T u = T(2) - q;
+        return q <= T(1) ? fma(T(1.5), q, T(-2)) : -(u * u) * h;
+    }
 };
 template <class T>
 struct Grad<T, SIMP_SKF_WENDLAND_C6> {
     static constexpr double factor = 78.0 / (7.0 * kPi);
+    static constexpr double qscale = 1.0;
     static __device__ __forceinline__ T shape(T q, T) {
         const T om = T(1) - q, om2 = om * om;
         return (T(-22) * (om2 * om2) * (om2 * om)) * fma(fma(T(16), q, T(7)), q, T(1));
     }
-    static constexpr double qscale = 1.0;
 };
 
-// The pair's gradient factor without the constant part of a particle's sums:
-// s = r^2 (with dx, dy in T).  Own: what the particle's side contributes.
+// The pair's gradient factor without the constant part of a particle's sums,
+// from s = r^2.
 template <class T, int SKF, bool UNIFORM>
 struct PairGrad {
     T hi, k;   // hsml_i; uniform: (qscale / hsml)^2
@@ -159,13 +187,16 @@ struct PairGrad {
             kernel_wg<T, false, 0>(P.skf, r * shh, shh, inv_h, &w, &gq);
             return gq * shh * rs;
         } else if constexpr (UNIFORM) {
-            const T u = s * k, y = rsq(u);
-            return Grad<T, SKF>::shape(u * y, y);
+            T q, h;
+            root_pair(s * k, q, h);
+            return Grad<T, SKF>::shape(q, h);
         } else {
-            const T H = T(0.5) * (hi + hj), H2 = H * H;
-            const T y = rsq(s * H2), q = s * y, ih2 = q * y;
             constexpr T c = (T)Grad<T, SKF>::qscale;
-            return (ih2 * ih2) * Grad<T, SKF>::shape(c * q, H2 * y * (T(1) / c));
+            const T H = T(0.5) * (hi + hj), H2 = H * H;
+            T R, n;
+            root_pair(s * H2, R, n);
+            const T q = T(2) * s * n, ih2 = T(2) * q * n;   // r / H, 1 / H^2
+            return (ih2 * ih2) * Grad<T, SKF>::shape(c * q, (H2 / c) * n);
         }
     }
 };
@@ -179,19 +210,21 @@ struct TauRec {
 };
 
 // Kinematic-pass pair terms (kernel.f90:515-518, vector_divergence.f90:27,
-// vector_gradient.f90:56-69): sums of -div and of the velocity gradient.
+// vector_gradient.f90:56-69): sums of -div and of the velocity gradient, whose
+// off-diagonal parts are only needed added (the shear strain rate).
 template <class T>
 struct KinSums {
-    Sum<T> dv, g1, g2, g3, g4;
-    // grad W_ij = (dwx, dwy)
-    __device__ __forceinline__ void add(T dwx, T dwy, T dvx, T dvy, T mj, T mrj) {
-        const T w2 = dvy * dwx, w3 = dvx * dwy, w4 = dvy * dwy;
-        const T w1 = dvx * dwx;
-        dv.madd(mj, fma(dvx, dwx, w4));
-        g1.madd(mrj, w1);
-        g2.madd(mrj, w2);
-        g3.madd(mrj, w3);
-        g4.madd(mrj, w4);
+    Sum<T> dv, g1, g23, g4;
+    // grad W_ij = (dwx, dwy); nothing is added where `in` is false
+    __device__ __forceinline__ void add(bool in, T dwx, T dwy, T dvx, T dvy, T mj, T mrj) {
+        const T w1 = dvx * dwx, w4 = dvy * dwy;
+        const T w23 = fma(dvy, dwx, dvx * dwy);
+        if (in) {
+            dv.madd(mj, w1 + w4);
+            g1.madd(mrj, w1);
+            g23.madd(mrj, w23);
+            g4.madd(mrj, w4);
+        }
     }
 };
 
@@ -200,11 +233,15 @@ struct KinSums {
 template <class T>
 struct StressSums {
     Sum<T> sx, sy, tx, ty;
-    __device__ __forceinline__ void add(T dwx, T dwy, T mj, T t11, T t12, T t22) {
-        sx.madd(mj, dwx);
-        sy.madd(mj, dwy);
-        tx.madd(mj, fma(t11, dwx, t12 * dwy));
-        ty.madd(mj, fma(t12, dwx, t22 * dwy));
+    // (nothing is added where `in` is false)
+    __device__ __forceinline__ void add(bool in, T dwx, T dwy, T mj, T t11, T t12, T t22) {
+        const T fx = fma(t11, dwx, t12 * dwy), fy = fma(t12, dwx, t22 * dwy);
+        if (in) {
+            sx.madd(mj, dwx);
+            sy.madd(mj, dwy);
+            tx.madd(mj, fx);
+            ty.madd(mj, fy);
+        }
     }
 };
 
@@ -225,18 +262,19 @@ struct KinArgs {
     unsigned char *halos;  // their halos (written here)
     int cap;               // halo particles that fit in shared memory
     int second;            // the step's second right-hand side
+    int single;            // instance 0 owns every particle
+    int prefetch;          // fetch the epilogue's values ahead
 };
 
 // Strain rates, rheology and stress of particle i from its velocity
-// divergence dv and velocity gradient g (single_step.f90:80-84,
+// divergence dv and velocity gradient (g1, g23 / 2, g4) (single_step.f90:80-84,
 // internal_stress.f90:20-42): writes tau = sigma / rho^2, div and the
 // optional diagnostics.
-__device__ __forceinline__ void kin_rheology(const KinArgs &a, int i, double dv, double g1, double g2,
-                                             double g3, double g4) {
+__device__ __forceinline__ void kin_rheology(const KinArgs &a, int i, double dv, double g1, double g23, double g4) {
     const State &s = a.s;
     const Phys &P = a.P;
     // strain rates, single_step.f90:80-84
-    const double e11 = g1, e22 = g4, e12 = 0.5 * (g2 + g3);
+    const double e11 = g1, e22 = g4, e12 = 0.5 * g23;
     // rheology, internal_stress.f90:20-42
     const double hh = s.h[i], AA = s.A[i];
     const double rho = s.rho[i];
@@ -329,9 +367,8 @@ struct StressArgs {
     // the artificial-viscosity acceleration (x, y) and the XSPH sum (x, y),
     // which a rates epilogue replaces by dx/dt; null when both are off
     double *reg;
-    const double2 *xyr;
     double *hs_next;
-    int n, maxn, mode;
+    int n, maxn, mode, single, prefetch;
     const Chunk *chunks;
     const unsigned char *halos;
     int cap;
@@ -382,40 +419,40 @@ __device__ __forceinline__ void warp_max_i32(int *dst, int v) {
 }
 
 // The per-step bounds of the stress pass in one block-wide reduction (two
-// warp reductions per value, one barrier, one atomic per value and block):
-// of the run, maxip (max), max |coordinate| (max), the next hsml minimum and
-// maximum and the VP time step (min); of the block's instance, the squared
-// displacement since the sort and the squared move of this update (into
-// `move`).  Values whose bit in `active` is clear are skipped.  Every thread
-// of the block calls it.
-constexpr int kBounds = 7;
-__device__ __forceinline__ void block_bounds(Scalars *sc, Inst *I, unsigned long long *move, unsigned active,
+// warp reductions per value, one barrier, one atomic per value and block): of
+// the run, maxip (max), the next hsml minimum and maximum and the VP time step
+// (min); of the block's instance, the squared move of this update (max, into
+// `move`), from which the step's end keeps the bounds on displacements and
+// coordinates.  Values whose bit in `active` is clear are skipped.  Every
+// thread of the block calls it.
+constexpr int kBounds = 5;
+__device__ __forceinline__ void block_bounds(Scalars *sc, unsigned long long *move, unsigned active,
                                              unsigned long long (&v)[kBounds]) {
-    __shared__ unsigned long long part[8][kBounds];
+    __shared__ unsigned long long part[kTile / 32][kBounds];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int q = 0; q < kBounds; ++q) {
         if (!((active >> q) & 1u)) continue;
-        const bool mn = (q == 2 || q == 4);
-        const unsigned long long r = mn ? warp_least(v[q]) : warp_top(v[q]);
+        const bool mn = (q == 1 || q == 3);
+        const unsigned long long r = q == 0 ? (unsigned long long)__reduce_max_sync(0xffffffffu, (unsigned)v[0])
+                                            : mn ? warp_least(v[q]) : warp_top(v[q]);
         if (lane == 0) part[w][q] = r;
     }
     __syncthreads();
     const int q = threadIdx.x;
     if (q < kBounds && ((active >> q) & 1u)) {
-        const bool mn = (q == 2 || q == 4);
+        const bool mn = (q == 1 || q == 3);
         unsigned long long r = part[0][q];
-        for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
+#pragma unroll
+        for (int k = 1; k < kTile / 32; ++k) {
             const unsigned long long t = part[k][q];
             r = mn ? (t < r ? t : r) : (t > r ? t : r);
         }
         switch (q) {
             case 0: atomicMax(&sc->maxip, (int)r); break;
-            case 1: atomicMax(&sc->xabs_bits, r); break;
-            case 2: atomicMin(&sc->acc_hmin, r); break;
-            case 3: atomicMax(&sc->acc_hmax, r); break;
-            case 4: atomicMin(&sc->acc_dt, r); break;
-            case 5: atomicMax(&I->dmax2_bits, r); break;
+            case 1: atomicMin(&sc->acc_hmin, r); break;
+            case 2: atomicMax(&sc->acc_hmax, r); break;
+            case 3: atomicMin(&sc->acc_dt, r); break;
             default: atomicMax(move, r); break;
         }
     }
@@ -429,75 +466,140 @@ struct WallSums {
     double fx = 0.0, fy = 0.0, gx = 0.0, gy = 0.0;
     int cnt = 0;
 };
+// The walls a tile may have pairs with, in their order, in shared memory: a
+// particle then runs past them without the dependent loads of a cell walk
+// (with the whole walk per particle, the tiles at a wall held a small basin's
+// stress pass up by 6 us).
+constexpr int kWallCap = 128;
+struct WallTile {
+    int n;                         // walls, -1: too many, or none looked up
+    int id[kWallCap];
+    double x[kWallCap], y[kWallCap], m[kWallCap];
+};
+// Fills it for a part of a tile with cells ka .. kb, from the cells within Rb
+// of them (Halo.walls).  Called by the whole block, which synchronises before
+// the walls are read.
+__device__ __forceinline__ void wall_tile(const StressArgs &a, const Inst &I, int Rb, int ka, int kb, WallTile &w) {
+    const int end = I.base + I.ncx * I.ncy;
+    int n = 0, past = 0;
+    for (int d = -Rb; d <= Rb; ++d) {
+        const int b0 = max(a.bstart[clampi(ka + d * I.ncx - Rb, I.base, end)], past);
+        const int b1 = a.bstart[clampi(kb + d * I.ncx + Rb + 1, I.base, end)];
+        for (int k = threadIdx.x; k < b1 - b0 && n + k < kWallCap; k += kTile) {
+            w.id[n + k] = b0 + k;
+            w.x[n + k] = a.bx[b0 + k];
+            w.y[n + k] = a.by[b0 + k];
+            w.m[n + k] = a.bm[b0 + k];
+        }
+        n += max(b1 - b0, 0);
+        past = max(b1, past);
+    }
+    if (threadIdx.x == 0) w.n = n <= kWallCap ? n : -1;
+}
 template <int SKF>
-__device__ __noinline__ WallSums wall_sums(const StressArgs &a, int i, const Inst &I, double xi, double yi, double hi) {
+__device__ __noinline__ WallSums wall_sums(const StressArgs &a, const WallTile &wt, int i, const Inst &I, double xi,
+                                           double yi, double hi) {
     const Phys &P = a.P;
     const double rho = a.rhs.rho[i];
     const double2 v = a.rhs.vxy[i];
     const double vxi = v.x, vyi = v.y;
-    const int ci = a.cell[i];
     const double mi = a.rhs.m[i], dt = a.sc->dt;
-    const Grid g = inst_grid(I, a.cell_start);
     const double bl = I.b_length;
-    const int Rb = wall_radius(I.dmax2_bits, g, bl);
     const BinRule bb = make_bin_rule(I.bs, xi, yi, bl);
     const double sh = (double)P.scale_h;
     const double csnd = P.boundary_friction ? sound_speed(P, rho) : 0.0;
     WallSums w;
-    w.cnt = for_each_wall(a.bx, a.by, a.bstart, g, ci, Rb, bb, xi, yi, bl,
-                         [&](int b, double bdx, double bdy, double d) {
-                             if (P.bfa == 1) {
-                                 const double mb = a.bm[b];
-                                 if (P.boundary_pressure) {
-                                     const double bw = boundary_w<SKF>(P, d, hi);
-                                     const double coef = P.kappa_n * bw * 2.0 * mb / ((mi + mb) * (d * d));
-                                     w.fx += coef * bdx;
-                                     w.fy += coef * bdy;
-                                 }
-                                 if (P.boundary_friction) {   // :85-100
-                                     const double t = boundary_fdwdq<SKF>(P, d, hi) / bl;
-                                     const double bwx = -(t * (bdx / d) * sh), bwy = -(t * (bdy / d) * sh);
-                                     const double v_r = vxi * bdx + vyi * bdy;
-                                     const double pi_aj = P.kappa_t * csnd * v_r / d / rho;
-                                     w.gx += (-1.0 * mb * pi_aj * bwx) / rho;
-                                     w.gy += (-1.0 * mb * pi_aj * bwy) / rho;
-                                 }
-                             } else if (P.bfa == 2) {
-                                 if (P.boundary_pressure) {   // :146-172
-                                     const double nx = a.bnx[b], ny = a.bny[b];
-                                     const double v1 = nx * vxi + ny * vyi;
-                                     double v2 = sqrt(vxi * vxi + vyi * vyi) - v1;
-                                     const double F1 = mi * v1 / dt;
-                                     double F2 = mi * v2 / dt;
-                                     if (P.boundary_friction && fabs(v2) > fabs(P.xi * v1)) {
-                                         v2 = v2 * P.xi * fabs(F1 / F2);
-                                         F2 = mi * v2 / dt;
-                                     }
-                                     w.gx += F1 * nx + F2 * ny;
-                                     w.gy += F1 * ny - F2 * nx;
-                                 }
-                             } else if (!P.boundary_pressure && P.boundary_friction) {   // :212-222
-                                 w.gx -= vxi * (1.0 - d / bl);
-                                 w.gy -= vyi * (1.0 - d / bl);
-                             }
-                         });
+    auto wall = [&](int b, double mb, double bdx, double bdy, double d) {
+        if (P.bfa == 1) {
+            if (P.boundary_pressure) {
+                const double bw = boundary_w<SKF>(P, d, hi);
+                const double coef = P.kappa_n * bw * 2.0 * mb / ((mi + mb) * (d * d));
+                w.fx += coef * bdx;
+                w.fy += coef * bdy;
+            }
+            if (P.boundary_friction) {   // :85-100
+                const double t = boundary_fdwdq<SKF>(P, d, hi) / bl;
+                const double bwx = -(t * (bdx / d) * sh), bwy = -(t * (bdy / d) * sh);
+                const double v_r = vxi * bdx + vyi * bdy;
+                const double pi_aj = P.kappa_t * csnd * v_r / d / rho;
+                w.gx += (-1.0 * mb * pi_aj * bwx) / rho;
+                w.gy += (-1.0 * mb * pi_aj * bwy) / rho;
+            }
+        } else if (P.bfa == 2) {
+            if (P.boundary_pressure) {   // :146-172
+                const double nx = a.bnx[b], ny = a.bny[b];
+                const double v1 = nx * vxi + ny * vyi;
+                double v2 = sqrt(vxi * vxi + vyi * vyi) - v1;
+                const double F1 = mi * v1 / dt;
+                double F2 = mi * v2 / dt;
+                if (P.boundary_friction && fabs(v2) > fabs(P.xi * v1)) {
+                    v2 = v2 * P.xi * fabs(F1 / F2);
+                    F2 = mi * v2 / dt;
+                }
+                w.gx += F1 * nx + F2 * ny;
+                w.gy += F1 * ny - F2 * nx;
+            }
+        } else if (!P.boundary_pressure && P.boundary_friction) {   // :212-222
+            w.gx -= vxi * (1.0 - d / bl);
+            w.gy -= vyi * (1.0 - d / bl);
+        }
+    };
+    if (wt.n >= 0) {
+        for (int k = 0; k < wt.n; ++k) {
+            const double xb = wt.x[k], yb = wt.y[k];
+            const double bdx = __dsub_rn(xb, xi), bdy = __dsub_rn(yb, yi);
+            double d;
+            if (!pair_test(bdx, bdy, bl, &d)) continue;
+            if (!bin_rule_ok(bb, xb, yb)) continue;
+            ++w.cnt;
+            wall(wt.id[k], wt.m[k], bdx, bdy, d);
+        }
+    } else {
+        const Grid g = inst_grid(I, a.cell_start);
+        const int Rb = wall_radius(inst_disp(I), g, bl);
+        w.cnt = for_each_wall(a.bx, a.by, a.bstart, g, a.cell[i], Rb, bb, xi, yi, bl,
+                              [&](int b, double bdx, double bdy, double d) { wall(b, a.bm[b], bdx, bdy, d); });
+    }
     return w;
+}
+
+// What stress_finish will read of particle i, brought to the L1 cache while the
+// pairs are summed.
+template <class P>
+__device__ __forceinline__ void prefetch_l1(const P *p) {
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+__device__ __forceinline__ void stress_prefetch(const StressArgs &a, int i) {
+    const State &s = a.rhs, &b = a.base;
+    prefetch_l1(&s.rho[i]);
+    prefetch_l1(&s.h[i]);
+    prefetch_l1(&s.A[i]);
+    prefetch_l1(&a.div[i]);
+    prefetch_l1(&a.rec.ta[i]);
+    prefetch_l1(&a.rec.tb[i]);
+    prefetch_l1(&s.vxy[i]);
+    prefetch_l1(&b.m[i]);
+    if (a.mode == EPI_CORRECT || a.mode == EPI_LEAP) {
+        prefetch_l1(&b.xy[i]);
+        prefetch_l1(&b.vxy[i]);
+        prefetch_l1(&b.h[i]);
+        prefetch_l1(&b.A[i]);
+    }
 }
 
 // Everything of the stress pass after the pair sums S = sum_j m_j grad W_ij
 // and T = sum_j m_j tau_j . grad W_ij of particle i: internal force, walls,
 // drag, rates and the integrator epilogue with the bounds reductions.
 // Called by every thread of the block (dead lanes with live = false).
-// `walls`: whether the tile may have wall pairs.
+// `walls`: the tile's walls, null where it has none.
 template <int SKF>
 __device__ __forceinline__ void stress_finish(const StressArgs &a, int i, bool live, int ki, const Inst &I,
-                                              bool dead, bool walls, double xi, double yi, double hi, double Sx,
+                                              const WallTile *walls, double xi, double yi, double hi, double Sx,
                                               double Sy, double Tx, double Ty, int cnt) {
     const State &s = a.rhs;
     const Phys &P = a.P;
     WallSums wl;
-    if (walls && (P.boundary_pressure || P.boundary_friction) && a.nb > 0 && !dead)
-        wl = wall_sums<SKF>(a, i, I, xi, yi, hi);
+    if (walls) wl = wall_sums<SKF>(a, *walls, i, I, xi, yi, hi);
     // everything else the epilogue reads, before anything that could hold it up
     const State &b = a.base;
     const bool own = a.mode == EPI_PREDICT || a.mode == EPI_EULER || a.mode == EPI_RATES;   // (base is the rhs state)
@@ -511,7 +613,6 @@ __device__ __forceinline__ void stress_finish(const StressArgs &a, int i, bool l
         h0 = b.h[i];
         A0 = b.A[i];
     }
-    const double2 xyr = a.xyr[i];
     double mn = b.m[i];
     const double dt = a.sc->dt;
     const double ih = 1.0 / hh, irho = 1.0 / rho;
@@ -646,19 +747,10 @@ __device__ __forceinline__ void stress_finish(const StressArgs &a, int i, bool l
         hsn = sqrt(mn / rhon) * (double)P.hsml_multiplicity;
         if (hsn > P.max_hsml) hsn = P.max_hsml;
     }
-    // displacement since the instance's last sort, max per instance
-    const double dxr = xn - xyr.x, dyr = yn - xyr.y;
-    // (non-finite values stay out of these bounds: the basin is flagged below)
-    double d2 = dxr * dxr + dyr * dyr;
-    if (!live || !isfinite(d2)) d2 = 0.0;
-    // and in this update, for the Verlet lists' bound (a non-finite one
-    // flags its basin below; an idle lane may see its particle updated)
+    // how far this update moves the particle (a non-finite move flags its
+    // basin below; an idle lane may see its particle updated)
     double m2 = (xn - x0) * (xn - x0) + (yn - y0) * (yn - y0);
     if (!live || !isfinite(m2)) m2 = 0.0;
-    // (dead lanes contribute neutral bounds: in place updates, the particle
-    // they mirror may already have been written by its own thread)
-    double xa = fmax(fabs(xn), fabs(yn));
-    if (!live || !isfinite(xa)) xa = 0.0;
     const bool bad = !(isfinite(xn) && isfinite(yn) && isfinite(vxn) && isfinite(vyn) &&
                        isfinite(hn) && isfinite(An));
     if (live && bad) {
@@ -680,23 +772,22 @@ __device__ __forceinline__ void stress_finish(const StressArgs &a, int i, bool l
     }
     // this step's bounds, one block-wide reduction
     const bool corr = final_update && !tail_later;
-    unsigned active = 1u | 2u | 32u | 64u;
-    unsigned long long v[kBounds] = {(unsigned long long)(live ? cnt : 0), dbits(xa), ~0ull, 0ull, ~0ull, dbits(d2),
-                                     dbits(m2)};
+    unsigned active = 1u | 16u;
+    unsigned long long v[kBounds] = {(unsigned long long)(live ? cnt : 0), ~0ull, 0ull, ~0ull, dbits(m2)};
     if (corr && P.sle == 2) {                                   // smoothing_length.f90:136-142
-        active |= 4u | 8u;
+        active |= 2u | 4u;
         if (live) {
+            v[1] = dbits(hsn);
             v[2] = dbits(hsn);
-            v[3] = dbits(hsn);
         }
     }
     if (corr && P.tse != 0) {                                   // time_step.f90:20-26
-        active |= 16u;
-        if (live) v[4] = dbits(dt_candidate(P, hsn, ax * ax + ay * ay, rhon, 0.0));
+        active |= 8u;
+        if (live) v[3] = dbits(dt_candidate(P, hsn, ax * ax + ay * ay, rhon, 0.0));
     }
     if (tail_later && P.tse == 1 && live) a.rates[i] = ax * ax + ay * ay;   // for k_density_rate
     Inst *Iw = a.inst + ki;
-    block_bounds(a.sc, Iw, a.mode == EPI_PREDICT ? &Iw->half2_bits : &Iw->step2_bits, active, v);
+    block_bounds(a.sc, a.mode == EPI_PREDICT ? &Iw->half2_bits : &Iw->step2_bits, active, v);
 }
 
 }  // namespace pass

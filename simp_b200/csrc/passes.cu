@@ -13,30 +13,13 @@ namespace {
 using namespace pass;
 
 constexpr int kBlock = kTile;
-// Resident blocks per SM the register allocation aims at: 5, where the FP64
-// pair math fits 96 registers almost without spills and five tiles fill the
-// shared memory (6 and 7 blocks per step at 262,144 particles, FP64: 214 ->
-// 253 and 300 us; mixed: 194 -> 231 and 253).
-#ifndef SIMP_KIN_MIN_BLOCKS
-#define SIMP_KIN_MIN_BLOCKS 5
-#endif
-#ifndef SIMP_STRESS_MIN_BLOCKS
-#define SIMP_STRESS_MIN_BLOCKS 5
-#endif
-#ifndef SIMP_KIN_MIN_BLOCKS_F32
-#define SIMP_KIN_MIN_BLOCKS_F32 5
-#endif
-#ifndef SIMP_STRESS_MIN_BLOCKS_F32
-#define SIMP_STRESS_MIN_BLOCKS_F32 5
-#endif
-template <class T>
-struct MinBlocks {
-    static constexpr int kin = SIMP_KIN_MIN_BLOCKS, stress = SIMP_STRESS_MIN_BLOCKS;
-};
-template <>
-struct MinBlocks<float> {
-    static constexpr int kin = SIMP_KIN_MIN_BLOCKS_F32, stress = SIMP_STRESS_MIN_BLOCKS_F32;
-};
+// Resident blocks per SM the register allocation aims at.  4 (128 registers)
+// holds the pair math of two candidates without spills: FP64 always (5 and 6
+// blocks per step at 262,144 particles: 160 -> 168 and 234 us; the reference's
+// switches at 90,007: 131 -> 154 and 197), and the mixed form where all tiles
+// are resident at once anyway (24,649 particles: 54 -> 49 us).  Above that the
+// mixed form takes 5 (1,048,576: 597 against 617 and 609 us at 4 and 6).
+constexpr int kResidentTiles = 1024;
 
 // hsml of the halo's particles, where it varies.
 __device__ __forceinline__ void tile_hsml(const Halo &h, const TileMem &m, const State &s) {
@@ -81,12 +64,12 @@ __device__ __forceinline__ unsigned scan_word(const TileMem &m, int sl, int n, f
 }
 
 // Builds the lists of a tile part whose xy records are in shared memory; a
-// particle's candidates go to the shared list and to `out` (the tile's lists
-// at its column).  Returns the particle's candidates, which may exceed
+// particle's candidates go to the shared list and to the tile's lists `out`,
+// at its column.  Returns the particle's candidates, which may exceed
 // kListRows (the list then holds the first ones).  Called by the whole block.
 template <bool UNIFORM>
 __device__ __noinline__ int build_lists(const Halo &h, const TileMem &m, const KinArgs &a, const Inst &I, int i,
-                                        bool live, unsigned short *out) {
+                                        bool live, unsigned short *out, int column) {
     const int t = threadIdx.x;
     const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
     const int total = h.off[h.nseg];
@@ -99,7 +82,7 @@ __device__ __noinline__ int build_lists(const Halo &h, const TileMem &m, const K
     const int2 at = cell_at(I, a.cell[i]);
     const double2 xy = a.s.xy[i];
     const float xf = (float)xy.x, yf = (float)xy.y, hf = (float)a.s.hs[i];
-    const float margin = prefilter_margin(bitsd(a.sc->xabs_bits), I.hmin);
+    const float margin = prefilter_margin(bitsd(a.sc->xabs_bits) + sqrt(bitsd(I.half2_bits)), I.hmin);
     const float grow = margin < 0.25f ? 1.0f + margin : INFINITY;
     const float delta = (float)I.delta;
     const int own = slot_of(h, i);
@@ -117,8 +100,8 @@ __device__ __noinline__ int build_lists(const Halo &h, const TileMem &m, const K
                 const int k = __ffs(bits) - 1;
                 bits &= bits - 1u;
                 if (cnt < kListRows) {
-                    m.list[cnt * kTile + t] = (unsigned short)(sl + k);
-                    out[cnt * kTile] = (unsigned short)(sl + k);
+                    m.list[list_at(cnt, t)] = (unsigned short)(sl + k);
+                    out[list_at(cnt, column)] = (unsigned short)(sl + k);
                 }
                 ++cnt;
             }
@@ -127,6 +110,15 @@ __device__ __noinline__ int build_lists(const Halo &h, const TileMem &m, const K
         }
     }
     return cnt;
+}
+
+// Programmatic dependent launch: a pass's blocks may start while the last
+// blocks of the kernel before still run, and wait here before they read what
+// it wrote.  The kernels after it may follow once every block is this far (so
+// that everything before the previous kernel has ended).
+__device__ __forceinline__ void pass_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Per-neighbour scalars of a slot: the FP64 records for the plain form, the
@@ -229,32 +221,39 @@ __device__ __forceinline__ int classify(T dx, T dy, T hi, T hj, T mh2_u) {
     return s > mh2 * (T(1) + Rec<T>::band) ? 0 : 2;
 }
 
+constexpr int kHaloWords = sizeof(Halo) / sizeof(int);
+__device__ __forceinline__ int halo_word(const Halo *h, int k) { return reinterpret_cast<const int *>(h)[k]; }
+
 // Whether a basin's lists hold every pair of this right-hand side (Inst).
 // In a step's second right-hand side they are at most as old as the first.
 __device__ __forceinline__ bool lists_valid(const Inst &I, bool second) {
     if (!I.list_ok && !second) return false;
-    const double d = (I.list_ok ? I.list_d : 0.0) + (second ? sqrt(bitsd(I.half2_bits)) : 0.0);
-    return 2.0 * d * (1.0 + 1e-9) <= I.delta;
+    const double room = 0.5 * I.delta * (1.0 - 1e-9) - (I.list_ok ? I.list_d : 0.0);
+    return room >= 0.0 && (!second || bitsd(I.half2_bits) <= room * room);
 }
 
-// Kinematic pass over tiles.  Bound by latency: a block waits for its tile's
-// copies, then runs about 22 pairs per thread at 80 instructions each (FP64
-// pipe 20% busy, issue slots 32%), at five blocks per SM.  262,144 particles,
-// FP64: 78 -> 42 us per pass against gathers from global memory; mixed at
-// 1,048,576: 237 -> 150 us.
-template <class T, int SKF, bool UNIFORM>
-__global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(const __grid_constant__ KinArgs a) {
+// Kinematic pass over tiles.  Bound by shared memory and latency: a block waits
+// for its tile's copies, then reads three 16-byte records per pair at slots that
+// have no order, so that their banks collide (L1 55% busy in FP64, 70% mixed;
+// issue slots 31% and 51%).  Two candidates at a time put six such reads in
+// flight.  262,144 particles, FP64: 79 -> 40 us per pass against gathers from
+// global memory; mixed at 1,048,576: 237 -> 132 us.
+template <class T, int SKF, bool UNIFORM, int BLOCKS>
+__global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_constant__ KinArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Halo h;
     __shared__ __align__(8) unsigned long long bar;
     __shared__ int rows_max;
     const int t = threadIdx.x;
-    const Chunk ch = a.chunks[blockIdx.x];
-    const Inst &I = a.inst[ch.q];
-    if (ch.spare >= I.spares) return;   // (an unused spare tile)
+    const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
+    if (t == 0) bar_init(&bar);
+    pass_begin();
+    const Inst &I = a.inst[a.single ? 0 : ch.q];
     const State &s = a.s;
     const Phys &P = a.P;
     Halo *halos = reinterpret_cast<Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    const int first = t < kHaloWords ? halo_word(halos, t) : 0;   // (read along with the instance)
+    if (ch.spare >= I.spares) return;   // (an unused spare tile)
     unsigned short *lists = a.pl.slot + (size_t)blockIdx.x * kListRows * kTile;
     // a basin whose state turned non-finite is not searched any more (its
     // stencil would span its whole grid); it is only carried until retired
@@ -263,22 +262,20 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(const _
             Halo none{};
             none.kind = HALO_NONE;
             none.size = ch.p1 - ch.p0;
-            none.walls = 1;
             halos[0] = none;
         }
         const int i = ch.p0 + t;
         if (i >= ch.p1) return;
-        kin_rheology(a, i, -0.0, -0.0, -0.0, -0.0, -0.0);
+        kin_rheology(a, i, -0.0, -0.0, -0.0, -0.0);
         return;
     }
     const bool build = !lists_valid(I, a.second);
     const TileMem m = tile_mem(smem, a.cap, 3, UNIFORM);
-    if (t == 0) bar_init(&bar);
     unsigned parity = 0u;
     for (int p0 = ch.p0; p0 < ch.p1;) {
         if (!build) {
-            if (t < (int)(sizeof(Halo) / sizeof(int)))
-                reinterpret_cast<int *>(&h)[t] = reinterpret_cast<const int *>(&halos[(p0 - ch.p0) / kPartMin])[t];
+            if (t < kHaloWords)
+                reinterpret_cast<int *>(&h)[t] = p0 == ch.p0 ? first : halo_word(&halos[(p0 - ch.p0) / kPartMin], t);
         } else if (t == 0) {
             // the largest part of the tile whose halo fits
             for (int S = kTile;; S >>= 1) {
@@ -295,14 +292,20 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(const _
         const int i = p0 + (live ? t : 0);
         const double2 xy = __ldg(&s.xy[i]), vi = __ldg(&s.vxy[i]);
         const double hi = s.hs[i];
+        if (sizeof(T) == sizeof(float) && a.prefetch) {   // (the plain form has no register to spare)
+            prefetch_l1(&s.h[i]);
+            prefetch_l1(&s.A[i]);
+            prefetch_l1(&s.rho[i]);
+            prefetch_l1(&s.mm[i]);
+        }
         const T hiT = Rec<T>::own_h(s, i);
         PairGrad<T, SKF, UNIFORM> grad;
         grad.init(P, hiT);
         const bool rule = rule_on(I);
         KinSums<T> ks;     // -div and the velocity gradient, negated
-        auto terms = [&](T dx, T dy, double vxj, double vyj, T mj, T mrj, T hj) {
+        auto terms = [&](bool in, T dx, T dy, double2 v, T mj, T mrj, T hj) {
             const T g = grad(P, fma(dx, dx, dy * dy), hj);
-            ks.add(g * dx, g * dy, (T)(vi.x - vxj), (T)(vi.y - vyj), mj, mrj);
+            ks.add(in, g * dx, g * dy, (T)(vi.x - v.x), (T)(vi.y - v.y), mj, mrj);
         };
         int cnt = 0;       // candidates in the particle's list
         bool tile = fits;
@@ -317,7 +320,7 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(const _
             parity ^= 1u;
             if (!UNIFORM || build) __syncthreads();
             if (build) {
-                cnt = build_lists<UNIFORM>(h, m, a, I, i, live, lists + (i - ch.p0));
+                cnt = build_lists<UNIFORM>(h, m, a, I, i, live, lists, i - ch.p0);
                 const int rows = __reduce_max_sync(0xffffffffu, cnt);
                 if ((t & 31) == 0) atomicMax(&rows_max, rows);
                 // (the FP32 copies make way for the records)
@@ -346,22 +349,29 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(const _
             const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
             const double2 *vs = reinterpret_cast<const double2 *>(m.rec[1]);
             const T mh2_u = hiT * hiT;
-            // (a list just built stands at the thread's own column, as does
-            // the copied one: a part's threads are its first columns or all)
-            const unsigned short *col = m.list + (build ? t : i - ch.p0);
-#pragma unroll 2
-            for (int k = 0; k < cnt; ++k) {
-                const int q = col[k * kTile];
-                if (!SIMP_IN_RANGE(q, 0, h.off[h.nseg], SITE_TILE)) continue;
-                const double2 x = xs[q], v = vs[q];
-                T mj, mrj, hj;
-                Rec<T>::template kin<UNIFORM>(m, q, mj, mrj, hj);
-                const T dx = (T)(xy.x - x.x), dy = (T)(xy.y - x.y);
-                const int in = classify<T, UNIFORM>(dx, dy, hiT, hj, mh2_u);
-                if (in == 0) continue;
-                if (in == 2 || rule)
-                    if (!exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q))) continue;
-                terms(dx, dy, v.x, v.y, mj, mrj, hj);
+            // (a list just built stands at the thread's own column, a copied
+            // one at the particle's)
+            const ushort2 *col = reinterpret_cast<const ushort2 *>(m.list) + (build ? t : i - ch.p0);
+            // two candidates at a time, so that their chains overlap
+            for (int k = 0; k < cnt; k += 2) {
+                const ushort2 w = col[(k >> 1) * kTile];
+                const int q0 = w.x, q1 = k + 1 < cnt ? w.y : w.x;
+                if (!SIMP_IN_RANGE(q0, 0, h.off[h.nseg], SITE_TILE) || !SIMP_IN_RANGE(q1, 0, h.off[h.nseg], SITE_TILE))
+                    continue;
+                const double2 x0 = xs[q0], x1 = xs[q1], v0 = vs[q0], v1 = vs[q1];
+                T m0, r0, h0, m1, r1, h1;
+                Rec<T>::template kin<UNIFORM>(m, q0, m0, r0, h0);
+                Rec<T>::template kin<UNIFORM>(m, q1, m1, r1, h1);
+                const T dx0 = (T)(xy.x - x0.x), dy0 = (T)(xy.y - x0.y);
+                const T dx1 = (T)(xy.x - x1.x), dy1 = (T)(xy.y - x1.y);
+                int in0 = classify<T, UNIFORM>(dx0, dy0, hiT, h0, mh2_u);
+                int in1 = k + 1 < cnt ? classify<T, UNIFORM>(dx1, dy1, hiT, h1, mh2_u) : 0;
+                if (((in0 | in1) & 2) || rule) {
+                    if (in0) in0 = in0 == 1 && !rule ? 1 : exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q0));
+                    if (in1) in1 = in1 == 1 && !rule ? 1 : exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q1));
+                }
+                terms(in0 != 0, dx0, dy0, v0, m0, r0, h0);
+                terms(in1 != 0, dx1, dy1, v1, m1, r1, h1);
             }
         } else if (live) {
             // no tile: the neighbours from global memory
@@ -369,12 +379,12 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(const _
                 const double2 q = __ldg(&s.xy[j]), v = __ldg(&s.vxy[j]);
                 T mj, mrj, hj;
                 Rec<T>::kin_global(s, j, mj, mrj, hj);
-                terms((T)(xy.x - q.x), (T)(xy.y - q.y), v.x, v.y, mj, mrj, hj);
+                terms(true, (T)(xy.x - q.x), (T)(xy.y - q.y), v, mj, mrj, hj);
             });
         }
         if (live) {
             const double c = -grad.common();
-            kin_rheology(a, i, c * ks.dv.get(), c * ks.g1.get(), c * ks.g2.get(), c * ks.g3.get(), c * ks.g4.get());
+            kin_rheology(a, i, c * ks.dv.get(), c * ks.g1.get(), c * ks.g23.get(), c * ks.g4.get());
         }
         p0 += h.size;
         if (p0 < ch.p1) {
@@ -385,29 +395,35 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::kin) k_kinematic(const _
     }
 }
 
-// Stress pass over the same tiles: 41 instructions per pair, then the
-// epilogue, whose twenty own values are loaded together ahead of the walls and
-// the update (68 -> 50 us against loading each where it is used).  262,144
-// particles, FP64: 70 -> 50 us per pass against gathers from global memory.
-template <class T, int SKF, bool UNIFORM>
-__global__ void __launch_bounds__(kBlock, MinBlocks<T>::stress) k_stress(const __grid_constant__ StressArgs a) {
+// Stress pass over the same tiles, then the epilogue, whose twenty own values
+// are loaded together ahead of the walls and the update (68 -> 50 us against
+// loading each where it is used).  Half of a block's time is the latency of its
+// copies and of that epilogue (issue slots 29%, L1 50%).  262,144 particles,
+// FP64: 71 -> 46 us per pass against gathers from global memory; mixed at
+// 1,048,576: 192 -> 155 us.
+template <class T, int SKF, bool UNIFORM, int BLOCKS>
+__global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant__ StressArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Halo h;
+    __shared__ WallTile wt;
     __shared__ __align__(8) unsigned long long bar;
     const int t = threadIdx.x;
-    const Chunk ch = a.chunks[blockIdx.x];
-    const Inst &I = a.inst[ch.q];
+    const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
+    if (t == 0) bar_init(&bar);
+    pass_begin();
+    const Inst &I = a.inst[a.single ? 0 : ch.q];
+    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    const int first = t < kHaloWords ? halo_word(halos, t) : 0;   // (read along with the instance)
     if (ch.spare >= I.spares) return;   // (an unused spare tile)
     const State &s = a.rhs;
     const Phys &P = a.P;
-    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    const bool have_walls = (P.boundary_pressure || P.boundary_friction) && a.nb > 0 && !inst_dead(I.flags);
     constexpr int arrays = Rec<T>::stress_arrays;
     const TileMem m = tile_mem(smem, a.cap, arrays, UNIFORM);
-    if (t == 0) bar_init(&bar);
     unsigned parity = 0u;
     for (int p0 = ch.p0; p0 < ch.p1;) {
-        if (t < (int)(sizeof(Halo) / sizeof(int)))
-            reinterpret_cast<int *>(&h)[t] = reinterpret_cast<const int *>(&halos[(p0 - ch.p0) / kPartMin])[t];
+        if (t < kHaloWords)
+            reinterpret_cast<int *>(&h)[t] = p0 == ch.p0 ? first : halo_word(&halos[(p0 - ch.p0) / kPartMin], t);
         __syncthreads();
         const bool tile = h.kind == HALO_TILE;
         if (tile && t < 32) {
@@ -416,6 +432,12 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::stress) k_stress(const _
         }
         const bool live = t < h.size;
         const int i = p0 + (live ? t : h.size - 1);   // idle lanes mirror the part's last particle
+        if (a.prefetch) stress_prefetch(a, i);
+        const bool walls = have_walls && h.walls;
+        if (walls) {
+            wall_tile(a, I, h.walls, a.cell[p0], a.cell[p0 + h.size - 1], wt);
+            __syncthreads();
+        }
         const double2 xy = __ldg(&s.xy[i]);
         const double hi = s.hs[i];
         const T hiT = Rec<T>::own_h(s, i);
@@ -423,10 +445,10 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::stress) k_stress(const _
         PairGrad<T, SKF, UNIFORM> grad;
         grad.init(P, hiT);
         int npairs = 0;
-        auto terms = [&](T dx, T dy, T mj, T t11, T t12, T t22, T hj) {
+        auto terms = [&](bool in, T dx, T dy, T mj, T t11, T t12, T t22, T hj) {
             const T g = grad(P, fma(dx, dx, dy * dy), hj);
-            ss.add(g * dx, g * dy, mj, t11, t12, t22);
-            ++npairs;
+            ss.add(in, g * dx, g * dy, mj, t11, t12, t22);
+            npairs += in;
         };
         if (tile) {
             if (!UNIFORM) tile_hsml(h, m, s);
@@ -440,35 +462,42 @@ __global__ void __launch_bounds__(kBlock, MinBlocks<T>::stress) k_stress(const _
             parity ^= 1u;
             if (!UNIFORM) __syncthreads();
             const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
-            const unsigned short *col = m.list + (i - ch.p0);
+            const ushort2 *col = reinterpret_cast<const ushort2 *>(m.list) + (i - ch.p0);
             const T mh2_u = hiT * hiT;
-#pragma unroll 2
-            for (int k = 0; k < cnt; ++k) {
-                const int q = col[k * kTile];
-                if (!SIMP_IN_RANGE(q, 0, h.off[h.nseg], SITE_TILE)) continue;
-                const double2 x = xs[q];
-                T mj, t11, t12, t22, hj;
-                Rec<T>::template stress<UNIFORM>(m, q, mj, t11, t12, t22, hj);
-                const T dx = (T)(xy.x - x.x), dy = (T)(xy.y - x.y);
-                const int in = classify<T, UNIFORM>(dx, dy, hiT, hj, mh2_u);
-                if (in == 0) continue;
-                if (in == 2 || rule)
-                    if (!exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q))) continue;
-                terms(dx, dy, mj, t11, t12, t22, hj);
+            // two candidates at a time, so that their chains overlap
+            for (int k = 0; k < cnt; k += 2) {
+                const ushort2 w = col[(k >> 1) * kTile];
+                const int q0 = w.x, q1 = k + 1 < cnt ? w.y : w.x;
+                if (!SIMP_IN_RANGE(q0, 0, h.off[h.nseg], SITE_TILE) || !SIMP_IN_RANGE(q1, 0, h.off[h.nseg], SITE_TILE))
+                    continue;
+                const double2 x0 = xs[q0], x1 = xs[q1];
+                T m0, a0, b0, c0, h0, m1, a1, b1, c1, h1;
+                Rec<T>::template stress<UNIFORM>(m, q0, m0, a0, b0, c0, h0);
+                Rec<T>::template stress<UNIFORM>(m, q1, m1, a1, b1, c1, h1);
+                const T dx0 = (T)(xy.x - x0.x), dy0 = (T)(xy.y - x0.y);
+                const T dx1 = (T)(xy.x - x1.x), dy1 = (T)(xy.y - x1.y);
+                int in0 = classify<T, UNIFORM>(dx0, dy0, hiT, h0, mh2_u);
+                int in1 = k + 1 < cnt ? classify<T, UNIFORM>(dx1, dy1, hiT, h1, mh2_u) : 0;
+                if (((in0 | in1) & 2) || rule) {
+                    if (in0) in0 = in0 == 1 && !rule ? 1 : exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q0));
+                    if (in1) in1 = in1 == 1 && !rule ? 1 : exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q1));
+                }
+                terms(in0 != 0, dx0, dy0, m0, a0, b0, c0, h0);
+                terms(in1 != 0, dx1, dy1, m1, a1, b1, c1, h1);
             }
         } else if (h.kind == HALO_GLOBAL && live) {
             global_pairs(s, I, a.cell_start, i, a.cell[i], [&](int j) {
                 const double2 q = __ldg(&s.xy[j]);
                 T mj, t11, t12, t22, hj;
                 Rec<T>::stress_global(s, a.rec, j, mj, t11, t12, t22, hj);
-                terms((T)(xy.x - q.x), (T)(xy.y - q.y), mj, t11, t12, t22, hj);
+                terms(true, (T)(xy.x - q.x), (T)(xy.y - q.y), mj, t11, t12, t22, hj);
             });
         }
         // (a retired basin's particles are not written any more: their state
         // stays as it was until the batch's next compaction drops them)
         const double c = grad.common();
-        stress_finish<SKF>(a, i, live && !(I.flags & FLAG_RETIRED), ch.q, I, inst_dead(I.flags), h.walls != 0,
-                           xy.x, xy.y, hi, c * ss.sx.get(), c * ss.sy.get(), c * ss.tx.get(), c * ss.ty.get(), npairs);
+        stress_finish<SKF>(a, i, live && !(I.flags & FLAG_RETIRED), ch.q, I, walls ? &wt : nullptr, xy.x,
+                           xy.y, hi, c * ss.sx.get(), c * ss.sy.get(), c * ss.tx.get(), c * ss.ty.get(), npairs);
         p0 += h.size;
         if (p0 < ch.p1) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -576,7 +605,7 @@ __device__ __forceinline__ void aux_pairs(const Halo &h, const TileMem &m, const
         const double2 *vs = reinterpret_cast<const double2 *>(m.rec[1]);
         const int cnt = count[i];
         for (int k = 0; k < cnt; ++k) {
-            const int q = m.list[k * kTile + column];
+            const int q = m.list[list_at(k, column)];
             if (!SIMP_IN_RANGE(q, 0, h.off[h.nseg], SITE_TILE)) continue;
             const double2 x = xs[q];
             const double hj = m.hs[q];
@@ -822,21 +851,21 @@ __device__ __forceinline__ void density_rate(const DensArgs &a, const Halo &h, c
     // (dead lanes contribute neutral values: the particle they mirror may
     // already have been updated by its own thread)
     unsigned active = 0u;
-    unsigned long long v[kBounds] = {0ull, 0ull, ~0ull, 0ull, ~0ull, 0ull, 0ull};
+    unsigned long long v[kBounds] = {0ull, ~0ull, 0ull, ~0ull, 0ull};
     if (P.sle != 0) {
-        active |= 4u | 8u;
+        active |= 2u | 4u;
         if (live) {
+            v[1] = dbits(hsn);
             v[2] = dbits(hsn);
-            v[3] = dbits(hsn);
         }
     }
     if (P.tse != 0) {                                          // time_step.f90:20-26
-        active |= 16u;
+        active |= 8u;
         // |div v| = |sum_j m_j (v_i - v_j) . grad W| / rho_i (time_step.f90:108-111)
         const double adiv = a.dt_div ? fabs(rt.get() / rhon) : 0.0;
-        if (live) v[4] = dbits(dt_candidate(P, hsn, P.tse == 1 ? a.a2[i] : 0.0, rhon, adiv));
+        if (live) v[3] = dbits(dt_candidate(P, hsn, P.tse == 1 ? a.a2[i] : 0.0, rhon, adiv));
     }
-    block_bounds(a.sc, nullptr, nullptr, active, v);
+    block_bounds(a.sc, nullptr, active, v);
 }
 
 __global__ void __launch_bounds__(kBlock) k_density_rate(const __grid_constant__ DensArgs a) {
@@ -904,9 +933,12 @@ __global__ void __launch_bounds__(256) k_commit_hsml(int n, const double *__rest
 constexpr int kFinishThreads = 256;
 __global__ void __launch_bounds__(kFinishThreads) k_step_finish(Scalars *sc, Inst *inst, int ninst, int tse,
                                                                 int sle) {
+    pass_begin();
     __shared__ double dt, grown;
+    __shared__ unsigned long long farthest;
     if (threadIdx.x == 0) {
         grown = 0.0;
+        farthest = 0ull;
         if (tse != 0) {
             sc->dt = bitsd(sc->acc_dt);
             sc->acc_dt = dbits(INFINITY);
@@ -936,11 +968,18 @@ __global__ void __launch_bounds__(kFinishThreads) k_step_finish(Scalars *sc, Ins
         const double half = sqrt(bitsd(I.half2_bits)), step = sqrt(bitsd(I.step2_bits));
         const double old = I.list_ok ? I.list_d : 0.0;
         const double moved = old + step + 0.5 * grown;
-        I.list_ok = (2.0 * (old + half) * (1.0 + 1e-9) <= I.delta && 2.0 * (moved + half) <= I.delta) ? 1 : 0;
+        const double room = 0.5 * I.delta * (1.0 - 1e-9) - old;   // (as lists_valid)
+        I.list_ok = (room >= 0.0 && bitsd(I.half2_bits) <= room * room && 2.0 * (moved + half) <= I.delta) ? 1 : 0;
         I.list_d = moved;
+        // displacement since the sort and largest coordinate: each step adds
+        // the farthest any particle moved in it
+        I.disp += step;
+        atomicMax(&farthest, I.step2_bits);
         I.half2_bits = 0ull;
         I.step2_bits = 0ull;
     }
+    __syncthreads();
+    if (threadIdx.x == 0) sc->xabs_bits = dbits(bitsd(sc->xabs_bits) + sqrt(bitsd(farthest)));
 }
 
 // The Euler step writes its result into S1 (S0 is read by the pair sums of
@@ -1023,10 +1062,22 @@ __global__ void k_split(int nchunks, int nsrc, const int4 *__restrict__ src, int
     chunks[c] = full;
 }
 
-// Halo slots of a tile in shared memory: three rows of cells around 128
-// particles take up to 520 slots at hsml = 2.4 spacings (five blocks per SM with
-// the lists), 650 at the reference's 3 spacings, where hsml varies.
-int tile_cap(const simp_ctx *c) { return c->uniform ? 528 : 704; }
+// Halo slots of a tile in shared memory.  Three rows of cells around 128
+// particles take up to 520 slots at hsml = 2.4 spacings and 650 at the
+// reference's 3 spacings; five rows (after more motion), or a sparse row's tile
+// among full ones, about 850.  A context whose tiles are resident all at once
+// has room for the latter (40,401 particles with the density passes: 158 -> 137
+// us per step); a larger one is faster with what shared memory then leaves to
+// the L1 cache (1,048,576 particles FP64: 598 us against 632 with room for 832).
+int tile_cap(const simp_ctx *c) {
+    if (c->nchunks <= kResidentTiles) return 832;
+    return c->uniform ? 528 : 704;
+}
+
+// Whether a pass fetches its epilogue's values ahead of its pairs: where they
+// come from DRAM (1,048,576 particles: 597 -> 588 us FP64, 583 -> 570 mixed;
+// 600,011: 376 -> 370), not where L2 holds the state (262,144: 158 -> 161).
+bool prefetch_own(const simp_ctx *c) { return c->n > 400000; }
 
 TauRec tau_rec(simp_ctx *c) {
     TauRec r;
@@ -1044,46 +1095,75 @@ PairList pair_list(simp_ctx *c) {
     return pl;
 }
 
+// (calls f with every kernel of a form)
+template <class T, int SKF, class F>
+void each_kernel(F &&f) {
+    f(k_kinematic<T, SKF, true, 4>);
+    f(k_kinematic<T, SKF, false, 4>);
+    f(k_stress<T, SKF, true, 4>);
+    f(k_stress<T, SKF, false, 4>);
+    if (sizeof(T) == sizeof(float)) {
+        f(k_kinematic<float, SKF, true, 5>);
+        f(k_kinematic<float, SKF, false, 5>);
+        f(k_stress<float, SKF, true, 5>);
+        f(k_stress<float, SKF, false, 5>);
+    }
+    f(k_regularize);
+    f(k_density_rate);
+}
 template <class T, int SKF>
 cudaError_t allow_smem() {
     cudaError_t e = cudaSuccess;
-    const int most = 96 * 1024;   // (a tile takes 40 to 52 KB)
-    for (const void *f : {(const void *)k_kinematic<T, SKF, true>, (const void *)k_kinematic<T, SKF, false>,
-                          (const void *)k_stress<T, SKF, true>, (const void *)k_stress<T, SKF, false>,
-                          (const void *)k_regularize, (const void *)k_density_rate})
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    const int most = 96 * 1024;   // (a tile takes 40 to 64 KB)
+    each_kernel<T, SKF>([&](auto *k) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    });
     return e;
 }
 
-template <class T, int SKF>
-void launch_kin_form(simp_ctx *c, const KinArgs &a) {
-    const int g = c->nchunks;
-    const size_t sm = tile_smem_bytes(a.cap, 3, c->uniform);
-    if (c->uniform) k_kinematic<T, SKF, true><<<g, kTile, sm, c->stream>>>(a);
-    else k_kinematic<T, SKF, false><<<g, kTile, sm, c->stream>>>(a);
+// Launches a kernel that calls pass_begin, overlapping the one before it where
+// the context says so (within a step graph: after the kernel before it, which
+// may be any).
+template <class... P, class... A>
+void launch_pass(simp_ctx *c, void (*k)(P...), int grid, int block, size_t smem, const A &...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = c->overlap_launches ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, k, args...);   // (an error is found by the caller's next check)
 }
-template <class T, int SKF>
-void launch_stress_form(simp_ctx *c, const StressArgs &a) {
+
+template <class T, int SKF, int BLOCKS, class A>
+void launch_tiles(simp_ctx *c, const A &a) {
     const int g = c->nchunks;
-    const size_t sm = tile_smem_bytes(a.cap, Rec<T>::stress_arrays, c->uniform);
-    if (c->uniform) k_stress<T, SKF, true><<<g, kTile, sm, c->stream>>>(a);
-    else k_stress<T, SKF, false><<<g, kTile, sm, c->stream>>>(a);
+    if constexpr (std::is_same<A, KinArgs>::value) {
+        const size_t sm = tile_smem_bytes(a.cap, 3, c->uniform);
+        if (c->uniform) launch_pass(c, k_kinematic<T, SKF, true, BLOCKS>, g, kTile, sm, a);
+        else launch_pass(c, k_kinematic<T, SKF, false, BLOCKS>, g, kTile, sm, a);
+    } else {
+        const size_t sm = tile_smem_bytes(a.cap, Rec<T>::stress_arrays, c->uniform);
+        if (c->uniform) launch_pass(c, k_stress<T, SKF, true, BLOCKS>, g, kTile, sm, a);
+        else launch_pass(c, k_stress<T, SKF, false, BLOCKS>, g, kTile, sm, a);
+    }
 }
-template <class T, class A>
+template <int SKF, class A>
+void launch_kernel_form(simp_ctx *c, const A &a) {
+    if (c->prm.precision != SIMP_PREC_MIXED) launch_tiles<double, SKF, 4>(c, a);
+    else if (c->nchunks <= kResidentTiles) launch_tiles<float, SKF, 4>(c, a);
+    else launch_tiles<float, SKF, 5>(c, a);
+}
+template <class A>
 void launch_form(simp_ctx *c, const A &a) {
-    constexpr bool kin = std::is_same<A, KinArgs>::value;
     switch (skf_compiled(c->prm.skf)) {
-        case SIMP_SKF_CUBIC:
-            if constexpr (kin) launch_kin_form<T, SIMP_SKF_CUBIC>(c, a);
-            else launch_stress_form<T, SIMP_SKF_CUBIC>(c, a);
-            break;
-        case SIMP_SKF_WENDLAND_C6:
-            if constexpr (kin) launch_kin_form<T, SIMP_SKF_WENDLAND_C6>(c, a);
-            else launch_stress_form<T, SIMP_SKF_WENDLAND_C6>(c, a);
-            break;
-        default:
-            if constexpr (kin) launch_kin_form<T, 0>(c, a);
-            else launch_stress_form<T, 0>(c, a);
+        case SIMP_SKF_CUBIC: launch_kernel_form<SIMP_SKF_CUBIC>(c, a); break;
+        case SIMP_SKF_WENDLAND_C6: launch_kernel_form<SIMP_SKF_WENDLAND_C6>(c, a); break;
+        default: launch_kernel_form<0>(c, a);
     }
 }
 
@@ -1134,12 +1214,13 @@ void launch_kinematic(simp_ctx *c, const State &s, bool diag, bool second) {
     a.pl = pair_list(c);
     a.n = c->n;
     a.maxn = c->maxn;
+    a.single = c->max_inst == 1;
+    a.prefetch = prefetch_own(c);
     a.chunks = c->chunks;
     a.halos = c->halos;
     a.cap = tile_cap(c);
     a.second = second ? 1 : 0;
-    if (c->prm.precision == SIMP_PREC_MIXED) launch_form<float>(c, a);
-    else launch_form<double>(c, a);
+    launch_form(c, a);
     c->launches += 1;
 }
 
@@ -1168,16 +1249,16 @@ void launch_stress(simp_ctx *c, const State &rhs, const State &base, EpiMode mod
     a.pl = pair_list(c);
     a.rates = c->rates;
     a.reg = c->reg;
-    a.xyr = c->xyr;
     a.hs_next = c->tmp;   // hsml of the next step (committed by launch_step_finish)
     a.n = c->n;
     a.maxn = c->maxn;
     a.mode = mode;
+    a.single = c->max_inst == 1;
+    a.prefetch = prefetch_own(c);
     a.chunks = c->chunks;
     a.halos = c->halos;
     a.cap = tile_cap(c);
-    if (c->prm.precision == SIMP_PREC_MIXED) launch_form<float>(c, a);
-    else launch_form<double>(c, a);
+    launch_form(c, a);
     c->launches += 1;
 }
 
@@ -1274,7 +1355,7 @@ void launch_step_finish(simp_ctx *c) {
         k_commit_hsml<<<nblk(c->n, 256), 256, 0, c->stream>>>(c->n, c->tmp, c->s0, c->sc);
         c->launches += 1;
     }
-    k_step_finish<<<1, kFinishThreads, 0, c->stream>>>(c->sc, c->inst_dev, c->ninst, c->prm.tse, c->prm.sle);
+    launch_pass(c, k_step_finish, 1, kFinishThreads, 0, c->sc, c->inst_dev, c->ninst, (int)c->prm.tse, (int)c->prm.sle);
     c->launches += 1;
 }
 

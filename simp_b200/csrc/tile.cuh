@@ -37,13 +37,18 @@ constexpr int kSlotPad = 40;               // slots a candidate batch may read p
 // The halo of a tile or part of one, one record per part.
 enum : int { HALO_NONE = 0, HALO_TILE = 1, HALO_GLOBAL = 2 };
 struct Halo {
-    int kind, walls, nseg;     // walls: its particles may have wall pairs
+    int kind, nseg;
+    int walls;                 // cells around its own that hold every wall pair, 0: none
     int rows;                  // longest list of one of its particles
     int lo[kMaxSeg];           // first particle of each range
     int off[kMaxSeg + 1];      // its first slot, and the total
     int size;                  // particles in this part of the tile
 };
 static_assert(sizeof(Halo) == kHaloBytes, "ctx.h: kHaloBytes");
+
+// Place of candidate k in a particle's list (PairList): consecutive candidates
+// of a thread share a 32-bit word.
+__host__ __device__ __forceinline__ int list_at(int k, int column) { return ((k >> 1) * kTile + column) * 2 + (k & 1); }
 
 // Bulk copies to shared memory, completing on an mbarrier.
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -103,7 +108,7 @@ __device__ __forceinline__ TileMem tile_mem(unsigned char *p, int cap, int array
 __device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, const int *bstart, const int *cell, int p0,
                                        int p1, int cap, Halo &h) {
     const Grid g = inst_grid(I, cell_start);
-    const int R = stencil_radius(I.hmax, I.dmax2_bits, g, I.hmax + I.delta);
+    const int R = stencil_radius(I.hmax, inst_disp(I), g, I.hmax + I.delta);
     h.size = p1 - p0;
     h.nseg = 2 * R + 1;
     h.rows = 0;
@@ -112,9 +117,10 @@ __device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, con
     // walls within b_length of any place its particles take while the lists
     // stay valid (they move less than delta)
     h.walls = 0;
-    const int Rb = wall_radius(I.dmax2_bits, g, I.b_length + I.delta);
+    const int Rb = wall_radius(inst_disp(I), g, I.b_length + I.delta);
     for (int d = -Rb; d <= Rb && !h.walls; ++d)
-        h.walls = bstart[clampi(kb + d * I.ncx + Rb + 1, I.base, end)] > bstart[clampi(ka + d * I.ncx - Rb, I.base, end)];
+        if (bstart[clampi(kb + d * I.ncx + Rb + 1, I.base, end)] > bstart[clampi(ka + d * I.ncx - Rb, I.base, end)])
+            h.walls = Rb;
     if (h.kind == HALO_GLOBAL) return;
     int a[kMaxSeg], b[kMaxSeg];
 #pragma unroll
@@ -177,7 +183,7 @@ __device__ __forceinline__ void stencil_range(const Inst &I, const int *cell_sta
 __device__ __forceinline__ void tile_fetch(const Halo &h, const TileMem &m, const void *const (&src)[3], int a0, int a1,
                                            const unsigned short *list, int rows, unsigned long long *bar) {
     const int lane = threadIdx.x & 31, arrays = a1 - a0;
-    const unsigned list_bytes = (unsigned)(rows * kTile * sizeof(unsigned short));
+    const unsigned list_bytes = (unsigned)(((rows + 1) & ~1) * kTile * sizeof(unsigned short));
     if (lane == 0) bar_expect(bar, (unsigned)h.off[h.nseg] * 16u * (unsigned)arrays + list_bytes);
     __syncwarp();
     if (lane == 31 && rows > 0) bulk_copy(m.list, list, list_bytes, bar);
@@ -213,7 +219,7 @@ __device__ __forceinline__ void global_pairs(const State &s, const Inst &I, cons
     const double hi = s.hs[i];
     const bool rule = rule_on(I);
     const int2 at = cell_at(I, ci);
-    const int R = stencil_radius(I.hmax, I.dmax2_bits, inst_grid(I, cell_start), 0.0);
+    const int R = stencil_radius(I.hmax, inst_disp(I), inst_grid(I, cell_start), 0.0);
     for (int d = 0; d < 2 * R + 1; ++d) {
         int j0, j1;
         stencil_range(I, cell_start, at, R, d, j0, j1);

@@ -8,13 +8,16 @@ One right-hand side at the state reached, against the oracle at that state.
 The bars are those of the other right-hand-side tests: 1e-11 relative L2 in
 FP64, where only the order of the sums differs, 2e-6 in mixed precision.
 """
+import ctypes
+import subprocess
+
 import numpy as np
 import pytest
 
 from helpers import assert_same_pairs, rel_l2, smooth_velocity
-from simp_b200 import basins
+from simp_b200 import basins, build
 from simp_b200.params import PREC_FP64, PREC_MIXED
-from simp_b200.simp import Simp
+from simp_b200.simp import Batch, Simp
 
 pytestmark = pytest.mark.gpu
 
@@ -75,3 +78,60 @@ def test_tile_right_hand_side(gpu_lib, oracle_mod, name, precision):
     ro = o.single_step(600.0)
     for k in ("dvxdt", "dhdt", "dAdt"):
         assert rel_l2(r[k], ro[k]) < TOL[precision], (name, k)
+
+
+_ROOTS = """
+#include "pass_common.cuh"
+__global__ void roots(int n, const double *u, double *g, double *h) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) simp::pass::root_pair(u[i], g[i], h[i]);
+}
+extern "C" int run(int n, const double *u, double *g, double *h) {
+    double *d;
+    const size_t b = n * sizeof(double);
+    if (cudaMalloc(&d, 3 * b) != cudaSuccess) return 1;
+    cudaMemcpy(d, u, b, cudaMemcpyHostToDevice);
+    roots<<<(n + 127) / 128, 128>>>(n, d, d + n, d + 2 * n);
+    cudaMemcpy(g, d + n, b, cudaMemcpyDeviceToHost);
+    cudaMemcpy(h, d + 2 * n, b, cudaMemcpyDeviceToHost);
+    return cudaFree(d) != cudaSuccess;
+}
+"""
+
+
+def test_root_pair(gpu_lib, tmp_path):
+    """sqrt(u) and 1 / (2 sqrt(u)) of the pair passes in FP64, in 80-bit arithmetic.
+
+    The corrections leave errors of second order (2^-78) and one rounding each,
+    2^-53 at most, plus that of the correction itself (2^-39 of it): 1.001 * 2^-53.
+    """
+    (tmp_path / "roots.cu").write_text(_ROOTS)
+    so = str(tmp_path / "roots.so")
+    subprocess.run([build.nvcc(), "-shared", *build.ARCH, "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-I", build.INCLUDE,
+                    "-I", build.CSRC, *build.host_compiler(), "-o", so, str(tmp_path / "roots.cu")], check=True)
+    rng = np.random.default_rng(7)
+    u = np.concatenate([2.0 ** rng.uniform(-120.0, 120.0, 200000), rng.uniform(1.0, 4.0, 200000),
+                        [1.0, 4.0, 2.0, np.nextafter(1.0, 0.0), np.nextafter(4.0, 5.0)]])
+    g, h = np.empty_like(u), np.empty_like(u)
+    p = [a.ctypes.data_as(ctypes.c_void_p) for a in (u, g, h)]
+    assert ctypes.CDLL(so).run(len(u), *p) == 0
+    root = np.sqrt(u.astype(np.longdouble))
+    assert np.finfo(np.longdouble).nmant >= 63
+    assert np.max(np.abs(g / root - 1)) < 1.001 * 2.0 ** -53
+    assert np.max(np.abs(2 * h * root - 1)) < 1.001 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED])
+def test_alone_and_among_many(gpu_lib, precision):
+    """A basin gives the same bits in its own context and in a batch of so many
+    tiles that the passes take their other launch form."""
+    bs = [basins.make_basin(n, 1000.0, 3 + n, walls="+x-x+y-y", precision=precision) for n in (40, 370)]
+    batch = Batch(bs[0].params, sum(b.n for b in bs), sum(b.nb for b in bs), len(bs))
+    slots = [batch.add(b) for b in bs]
+    batch.step(12)
+    got = batch.get_state(slots[0])
+    alone = Simp.from_basin(bs[0])
+    alone.time_integration(12)
+    want = alone.get_state()
+    for k in ("x", "vx", "mass", "rho", "hsml", "A", "h"):
+        assert np.array_equal(got[k], want[k]), k
