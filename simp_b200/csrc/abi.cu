@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "host_pages.h"
 
 using namespace simp;
 
@@ -762,15 +763,6 @@ int read_inst(simp_ctx *c, int slot, Inst *out) {
     return SIMP_OK;
 }
 
-int download2(simp_ctx *c, const double *a, const double *b, double *h2) {
-    double *stage = c->tmp;
-    k_to_orig2<<<nblk(c->n, kB), kB, 0, c->stream>>>(c->n, c->id, a, b, stage);
-    c->launches += 1;
-    SIMP_CUDA(c, cudaMemcpyAsync(h2, stage, sizeof(double) * 2 * (size_t)c->n, cudaMemcpyDeviceToHost, c->stream));
-    SIMP_CUDA(c, cudaStreamSynchronize(c->stream));
-    return SIMP_OK;
-}
-
 int download_pair(simp_ctx *c, const double2 *a, double *h2) {
     double2 *stage = reinterpret_cast<double2 *>(c->tmp);
     k_pack_pair<<<nblk(c->n, kB), kB, 0, c->stream>>>(c->n, 0, c->id, a, stage);
@@ -799,12 +791,12 @@ int get_instance_state(simp_ctx *c, int slot, double *x, double *vx, double *mas
     k_pack_state<<<nblk(c->n, kB), kB, 0, s>>>(c->n, slot, ih.id_base, nk, c->pinst, c->id, c->s0, stage);
     c->launches += 1;
     SIMP_CUDA(c, cudaGetLastError());
-    struct Out { double *dst; size_t off, len; } outs[] = {
-        {x, 0, 2 * N}, {vx, 2 * N, 2 * N}, {mass, 4 * N, N}, {rho, 5 * N, N},
-        {hsml, 6 * N, N}, {A, 7 * N, N}, {h, 8 * N, N}};
-    for (const Out &o : outs)
-        if (o.dst)
-            SIMP_CUDA(c, cudaMemcpyAsync(o.dst, stage + o.off, sizeof(double) * o.len, cudaMemcpyDeviceToHost, s));
+    const size_t B = N * sizeof(double);
+    const HostCopy outs[] = {{x, stage, 2 * B, nullptr}, {vx, stage + 2 * N, 2 * B, nullptr},
+                             {mass, stage + 4 * N, B, nullptr}, {rho, stage + 5 * N, B, nullptr},
+                             {hsml, stage + 6 * N, B, nullptr}, {A, stage + 7 * N, B, nullptr},
+                             {h, stage + 8 * N, B, nullptr}};
+    TRY(read_back(c, s, outs, 7));
     Inst I{};
     SIMP_CUDA(c, cudaMemcpyAsync(&I, c->inst_dev + slot, sizeof(Inst), cudaMemcpyDeviceToHost, s));
     SIMP_CUDA(c, cudaStreamSynchronize(s));
@@ -1072,6 +1064,25 @@ simp_forcing forcing_of(const simp_params &p) {
 }  // namespace
 
 namespace simp {
+
+// The arrays get their pages while the stream finishes what it has to.
+int read_back(simp_ctx *c, cudaStream_t s, const HostCopy *v, int n) {
+    HostRange pages[kMaxHostCopies];
+    int m = 0;
+    for (int k = 0; k < n && k < kMaxHostCopies; ++k) {
+        cudaPointerAttributes a{};
+        if (!v[k].dst || v[k].bytes < kPagesFrom) continue;
+        if (cudaPointerGetAttributes(&a, v[k].dst) != cudaSuccess) cudaGetLastError();
+        else if (a.type == cudaMemoryTypeUnregistered) pages[m++] = {v[k].dst, v[k].bytes};
+    }
+    make_resident(pages, m);
+    for (int k = 0; k < n; ++k) {
+        if (!v[k].dst) continue;
+        if (v[k].after) SIMP_CUDA(c, cudaStreamWaitEvent(s, v[k].after, 0));
+        SIMP_CUDA(c, cudaMemcpyAsync(v[k].dst, v[k].src, v[k].bytes, cudaMemcpyDeviceToHost, s));
+    }
+    return SIMP_OK;
+}
 
 int complete_pending(simp_ctx *c) {
     if (!c->pending_check) return SIMP_OK;
@@ -1595,14 +1606,12 @@ int32_t simp_gpu_get_state(simp_ctx *c, double *x, double *vx, double *mass, dou
                                                         c->early_stage + N);
         c->launches += 1;
         SIMP_CUDA(c, cudaGetLastError());
-        if (early_m)
-            SIMP_CUDA(c, cudaMemcpyAsync(early_m, c->early_stage, sizeof(double) * N, cudaMemcpyDeviceToHost, c->side));
-        if (early_h)
-            SIMP_CUDA(c, cudaMemcpyAsync(early_h, c->early_stage + N, sizeof(double) * N, cudaMemcpyDeviceToHost,
-                                         c->side));
+        const HostCopy early[] = {{early_m, c->early_stage, sizeof(double) * N, nullptr},
+                                  {early_h, c->early_stage + N, sizeof(double) * N, nullptr}};
+        TRY(read_back(c, c->side, early, 2));
     }
     // the rest in groups: each group's reorder on the context stream, its
-    // copy on the side stream while the next group is reordered
+    // copy on the side stream while the following groups are reordered
     const int n = c->n, id_base = c->insts[0].id_base;
     const size_t N = (size_t)n;
     cudaStream_t s = c->stream;
@@ -1615,6 +1624,8 @@ int32_t simp_gpu_get_state(simp_ctx *c, double *x, double *vx, double *mass, dou
         {{m_src ? mass : nullptr, 4 * N, N}, {rho, 5 * N, N}},
         {{hs_src ? hsml : nullptr, 6 * N, N}, {A, 7 * N, N}},
         {{h, 8 * N, N}, {nullptr, 0, 0}}};
+    HostCopy outs[kMaxHostCopies];
+    int nout = 0;
     for (int g = 0; g < 5; ++g) {
         const Group &G = groups[g];
         if (!G.a.dst && !G.b.dst) continue;
@@ -1631,12 +1642,10 @@ int32_t simp_gpu_get_state(simp_ctx *c, double *x, double *vx, double *mass, dou
         c->launches += 1;
         SIMP_CUDA(c, cudaGetLastError());
         SIMP_CUDA(c, cudaEventRecord(c->ev_up[g], s));
-        SIMP_CUDA(c, cudaStreamWaitEvent(c->side, c->ev_up[g], 0));
         for (const Out &o : {G.a, G.b})
-            if (o.dst)
-                SIMP_CUDA(c, cudaMemcpyAsync(o.dst, stage + o.off, sizeof(double) * o.len, cudaMemcpyDeviceToHost,
-                                             c->side));
+            if (o.dst) outs[nout++] = {o.dst, stage + o.off, sizeof(double) * o.len, c->ev_up[g]};
     }
+    TRY(read_back(c, c->side, outs, nout));
     SIMP_CUDA(c, cudaMemcpyAsync(c->sc_host, c->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
     SIMP_CUDA(c, cudaStreamSynchronize(s));
     SIMP_CUDA(c, cudaStreamSynchronize(c->side));
@@ -1727,12 +1736,23 @@ int32_t simp_gpu_single_step(simp_ctx *c, double current_time, double *dxdt, dou
     if (c->k0) launch_sum_density(c, c->s0, c->s0, c->s0.m, c->s0.rho, c->tmp, false);
     SIMP_CUDA(c, cudaGetLastError());
     const size_t M = (size_t)c->maxn;
-    // dx/dt: the velocities, or with XSPH what the rates epilogue wrote
-    if (dxdt && c->reg && c->prm.xsph_regularization) TRY(download2(c, c->reg + 2 * M, c->reg + 3 * M, dxdt));
-    else if (dxdt) TRY(download_pair(c, c->s0.vxy, dxdt));
-    if (dvxdt) TRY(download2(c, c->rates, c->rates + M, dvxdt));
-    if (dhdt) TRY(download1(c, c->rates + 2 * M, dhdt));
-    if (dAdt) TRY(download1(c, c->rates + 3 * M, dAdt));
+    // dx/dt (the velocities, or with XSPH what the rates epilogue wrote), dv/dt,
+    // dh/dt and dA/dt in the caller's order
+    const bool xsph = c->reg && c->prm.xsph_regularization;
+    const int n = c->n;
+    const size_t N = (size_t)n, B = N * sizeof(double);
+    double *stage = c->tmp;
+    if (dxdt && !xsph) k_pack_pair<<<nblk(n, kB), kB, 0, s>>>(n, 0, c->id, c->s0.vxy, reinterpret_cast<double2 *>(stage));
+    if (dxdt && xsph) k_to_orig2<<<nblk(n, kB), kB, 0, s>>>(n, c->id, c->reg + 2 * M, c->reg + 3 * M, stage);
+    if (dvxdt) k_to_orig2<<<nblk(n, kB), kB, 0, s>>>(n, c->id, c->rates, c->rates + M, stage + 2 * N);
+    if (dhdt || dAdt)
+        k_pack_fields<<<nblk(n, kB), kB, 0, s>>>(n, 0, c->id, dhdt ? c->rates + 2 * M : nullptr,
+                                                 dAdt ? c->rates + 3 * M : nullptr, stage + 4 * N, stage + 5 * N);
+    c->launches += (dxdt != nullptr) + (dvxdt != nullptr) + (dhdt || dAdt);
+    SIMP_CUDA(c, cudaGetLastError());
+    const HostCopy outs[] = {{dxdt, stage, 2 * B, nullptr}, {dvxdt, stage + 2 * N, 2 * B, nullptr},
+                             {dhdt, stage + 4 * N, B, nullptr}, {dAdt, stage + 5 * N, B, nullptr}};
+    TRY(read_back(c, s, outs, 4));
     TRY(read_scalars(c));
     return check_after(c);
 }

@@ -230,6 +230,11 @@ int step_enqueue(simp_ctx *c, int nsteps);
 int step_complete(simp_ctx *c, double *current_time, double *dt);
 // the status of steps enqueued without outputs (waits for them); SIMP_OK when none
 int complete_pending(simp_ctx *c);
+// Copies device arrays to the caller's (nullptr: not wanted), each after its
+// event, if any, on stream s.
+constexpr int kMaxHostCopies = 7;
+struct HostCopy { void *dst; const void *src; size_t bytes; cudaEvent_t after; };
+int read_back(simp_ctx *c, cudaStream_t s, const HostCopy *v, int n);
 int batch_slot_state(simp_ctx *c, int slot, double *x, double *vx, double *mass, double *rho, double *hsml,
                      double *A, double *h, double *t);
 

@@ -283,10 +283,10 @@ int export_pairs(simp_ctx *c, int32_t *nip, int32_t *p_i, int32_t *p_j, double *
     if (nip) *nip = total;
     const int m = std::min(total, (int)std::max(cap, 0));
     if (m > 0) {
-        if (p_i) SIMP_CUDA(c, cudaMemcpyAsync(p_i, c->pair_buf_i, sizeof(int) * m, cudaMemcpyDeviceToHost, st));
-        if (p_j) SIMP_CUDA(c, cudaMemcpyAsync(p_j, c->pair_buf_j, sizeof(int) * m, cudaMemcpyDeviceToHost, st));
-        if (r_ij) SIMP_CUDA(c, cudaMemcpyAsync(r_ij, c->pair_buf_r, sizeof(double) * m, cudaMemcpyDeviceToHost, st));
-        if (hsml_ij) SIMP_CUDA(c, cudaMemcpyAsync(hsml_ij, c->pair_buf_h, sizeof(double) * m, cudaMemcpyDeviceToHost, st));
+        const HostCopy out[] = {{p_i, c->pair_buf_i, sizeof(int) * m, nullptr}, {p_j, c->pair_buf_j, sizeof(int) * m, nullptr},
+                                {r_ij, c->pair_buf_r, sizeof(double) * m, nullptr},
+                                {hsml_ij, c->pair_buf_h, sizeof(double) * m, nullptr}};
+        if (const int rc = read_back(c, st, out, 4)) return rc;
     }
     SIMP_CUDA(c, cudaStreamSynchronize(st));
     if (bnip) *bnip = btotal;

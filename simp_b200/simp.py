@@ -109,9 +109,9 @@ class Simp:
 
     def get_state(self) -> dict:
         n = self.ntotal
-        out = {"x": np.zeros((n, 2)), "vx": np.zeros((n, 2))}
+        out = {"x": np.empty((n, 2)), "vx": np.empty((n, 2))}
         for k in ("mass", "rho", "hsml", "A", "h"):
-            out[k] = np.zeros(n)
+            out[k] = np.empty(n)
         dt, t = ctypes.c_double(), ctypes.c_double()
         self._chk(self.lib.simp_gpu_get_state(self.h, *[_lib.dptr(out[k]) for k in
                                                         ("x", "vx", "mass", "rho", "hsml", "A", "h")],
@@ -165,10 +165,10 @@ class Simp:
         cap = 40 * self.ntotal if cap is None else int(cap)
         bcap = 40 * self.ntotal if bcap is None else int(bcap)
         nip, bnip = ctypes.c_int32(), ctypes.c_int32()
-        pi, pj = np.zeros(max(cap, 1), np.int32), np.zeros(max(cap, 1), np.int32)
-        r, hm = np.zeros(max(cap, 1)), np.zeros(max(cap, 1))
-        bpi, bpj = np.zeros(max(bcap, 1), np.int32), np.zeros(max(bcap, 1), np.int32)
-        br = np.zeros(max(bcap, 1))
+        pi, pj = np.empty(max(cap, 1), np.int32), np.empty(max(cap, 1), np.int32)
+        r, hm = np.empty(max(cap, 1)), np.empty(max(cap, 1))
+        bpi, bpj = np.empty(max(bcap, 1), np.int32), np.empty(max(bcap, 1), np.int32)
+        br = np.empty(max(bcap, 1))
         rc = self.lib.simp_gpu_nnps(self.h, ctypes.byref(nip), _lib.iptr(pi), _lib.iptr(pj), _lib.dptr(r),
                                     _lib.dptr(hm), cap, ctypes.byref(bnip), _lib.iptr(bpi), _lib.iptr(bpj),
                                     _lib.dptr(br), bcap)
@@ -187,14 +187,14 @@ class Simp:
 
     def single_step(self, current_time: float) -> dict:
         n = self.ntotal
-        out = dict(dxdt=np.zeros((n, 2)), dvxdt=np.zeros((n, 2)), dhdt=np.zeros(n), dAdt=np.zeros(n))
+        out = dict(dxdt=np.empty((n, 2)), dvxdt=np.empty((n, 2)), dhdt=np.empty(n), dAdt=np.empty(n))
         self._chk(self.lib.simp_gpu_single_step(self.h, float(current_time), _lib.dptr(out["dxdt"]),
                                                 _lib.dptr(out["dvxdt"]), _lib.dptr(out["dhdt"]),
                                                 _lib.dptr(out["dAdt"])))
         return out
 
     def sum_density(self) -> np.ndarray:
-        out = np.zeros(self.ntotal)
+        out = np.empty(self.ntotal)
         self._chk(self.lib.simp_gpu_sum_density(self.h, _lib.dptr(out)))
         return out
 
@@ -279,9 +279,9 @@ class Batch:
 
     def get_state(self, slot: int) -> dict:
         n = self.sizes[int(slot)]
-        out = {"x": np.zeros((n, 2)), "vx": np.zeros((n, 2))}
+        out = {"x": np.empty((n, 2)), "vx": np.empty((n, 2))}
         for k in ("mass", "rho", "hsml", "A", "h"):
-            out[k] = np.zeros(n)
+            out[k] = np.empty(n)
         t = ctypes.c_double()
         self._chk(self.lib.simp_gpu_batch_get_state(self.h, int(slot), *[_lib.dptr(out[k]) for k in
                                                                         ("x", "vx", "mass", "rho", "hsml",
