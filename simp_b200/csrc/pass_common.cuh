@@ -459,109 +459,12 @@ __device__ __forceinline__ void block_bounds(Scalars *sc, unsigned long long *mo
 }
 
 // Wall pairs of a particle (boundary_kernel.f90:5-45 calling boundary_force.f90
-// once per pair; bfa 1 bf_Monaghan :38-102, 2 bf_Wang :109-176, 3 bf_Marquis
-// :183-225): the sum of F_b, applied as -F_b / rho, and the acceleration terms
-// added as they are.  Few tiles have any, so this stays out of their registers.
+// once per pair): the sum of F_b, applied as -F_b / rho, and the acceleration
+// terms added as they are.
 struct WallSums {
     double fx = 0.0, fy = 0.0, gx = 0.0, gy = 0.0;
     int cnt = 0;
 };
-// The walls a tile may have pairs with, in their order, in shared memory: a
-// particle then runs past them without the dependent loads of a cell walk
-// (with the whole walk per particle, the tiles at a wall held a small basin's
-// stress pass up by 6 us).
-constexpr int kWallCap = 128;
-struct WallTile {
-    int n;                         // walls, -1: too many, or none looked up
-    int id[kWallCap];
-    double x[kWallCap], y[kWallCap], m[kWallCap];
-};
-// Fills it for a part of a tile with cells ka .. kb, from the cells within Rb
-// of them (Halo.walls).  Called by the whole block, which synchronises before
-// the walls are read.
-__device__ __forceinline__ void wall_tile(const StressArgs &a, const Inst &I, int Rb, int ka, int kb, WallTile &w) {
-    const int end = I.base + I.ncx * I.ncy;
-    int n = 0, past = 0;
-    for (int d = -Rb; d <= Rb; ++d) {
-        const int b0 = max(a.bstart[clampi(ka + d * I.ncx - Rb, I.base, end)], past);
-        const int b1 = a.bstart[clampi(kb + d * I.ncx + Rb + 1, I.base, end)];
-        for (int k = threadIdx.x; k < b1 - b0 && n + k < kWallCap; k += kTile) {
-            w.id[n + k] = b0 + k;
-            w.x[n + k] = a.bx[b0 + k];
-            w.y[n + k] = a.by[b0 + k];
-            w.m[n + k] = a.bm[b0 + k];
-        }
-        n += max(b1 - b0, 0);
-        past = max(b1, past);
-    }
-    if (threadIdx.x == 0) w.n = n <= kWallCap ? n : -1;
-}
-template <int SKF>
-__device__ __noinline__ WallSums wall_sums(const StressArgs &a, const WallTile &wt, int i, const Inst &I, double xi,
-                                           double yi, double hi) {
-    const Phys &P = a.P;
-    const double rho = a.rhs.rho[i];
-    const double2 v = a.rhs.vxy[i];
-    const double vxi = v.x, vyi = v.y;
-    const double mi = a.rhs.m[i], dt = a.sc->dt;
-    const double bl = I.b_length;
-    const BinRule bb = make_bin_rule(I.bs, xi, yi, bl);
-    const double sh = (double)P.scale_h;
-    const double csnd = P.boundary_friction ? sound_speed(P, rho) : 0.0;
-    WallSums w;
-    auto wall = [&](int b, double mb, double bdx, double bdy, double d) {
-        if (P.bfa == 1) {
-            if (P.boundary_pressure) {
-                const double bw = boundary_w<SKF>(P, d, hi);
-                const double coef = P.kappa_n * bw * 2.0 * mb / ((mi + mb) * (d * d));
-                w.fx += coef * bdx;
-                w.fy += coef * bdy;
-            }
-            if (P.boundary_friction) {   // :85-100
-                const double t = boundary_fdwdq<SKF>(P, d, hi) / bl;
-                const double bwx = -(t * (bdx / d) * sh), bwy = -(t * (bdy / d) * sh);
-                const double v_r = vxi * bdx + vyi * bdy;
-                const double pi_aj = P.kappa_t * csnd * v_r / d / rho;
-                w.gx += (-1.0 * mb * pi_aj * bwx) / rho;
-                w.gy += (-1.0 * mb * pi_aj * bwy) / rho;
-            }
-        } else if (P.bfa == 2) {
-            if (P.boundary_pressure) {   // :146-172
-                const double nx = a.bnx[b], ny = a.bny[b];
-                const double v1 = nx * vxi + ny * vyi;
-                double v2 = sqrt(vxi * vxi + vyi * vyi) - v1;
-                const double F1 = mi * v1 / dt;
-                double F2 = mi * v2 / dt;
-                if (P.boundary_friction && fabs(v2) > fabs(P.xi * v1)) {
-                    v2 = v2 * P.xi * fabs(F1 / F2);
-                    F2 = mi * v2 / dt;
-                }
-                w.gx += F1 * nx + F2 * ny;
-                w.gy += F1 * ny - F2 * nx;
-            }
-        } else if (!P.boundary_pressure && P.boundary_friction) {   // :212-222
-            w.gx -= vxi * (1.0 - d / bl);
-            w.gy -= vyi * (1.0 - d / bl);
-        }
-    };
-    if (wt.n >= 0) {
-        for (int k = 0; k < wt.n; ++k) {
-            const double xb = wt.x[k], yb = wt.y[k];
-            const double bdx = __dsub_rn(xb, xi), bdy = __dsub_rn(yb, yi);
-            double d;
-            if (!pair_test(bdx, bdy, bl, &d)) continue;
-            if (!bin_rule_ok(bb, xb, yb)) continue;
-            ++w.cnt;
-            wall(wt.id[k], wt.m[k], bdx, bdy, d);
-        }
-    } else {
-        const Grid g = inst_grid(I, a.cell_start);
-        const int Rb = wall_radius(inst_disp(I), g, bl);
-        w.cnt = for_each_wall(a.bx, a.by, a.bstart, g, a.cell[i], Rb, bb, xi, yi, bl,
-                              [&](int b, double bdx, double bdy, double d) { wall(b, a.bm[b], bdx, bdy, d); });
-    }
-    return w;
-}
 
 // What stress_finish will read of particle i, brought to the L1 cache while the
 // pairs are summed.
@@ -591,15 +494,13 @@ __device__ __forceinline__ void stress_prefetch(const StressArgs &a, int i) {
 // and T = sum_j m_j tau_j . grad W_ij of particle i: internal force, walls,
 // drag, rates and the integrator epilogue with the bounds reductions.
 // Called by every thread of the block (dead lanes with live = false).
-// `walls`: the tile's walls, null where it has none.
-template <int SKF>
+// `walls`: its wall sums.
+template <class W>
 __device__ __forceinline__ void stress_finish(const StressArgs &a, int i, bool live, int ki, const Inst &I,
-                                              const WallTile *walls, double xi, double yi, double hi, double Sx,
+                                              const W &walls, double xi, double yi, double hi, double Sx,
                                               double Sy, double Tx, double Ty, int cnt) {
     const State &s = a.rhs;
     const Phys &P = a.P;
-    WallSums wl;
-    if (walls) wl = wall_sums<SKF>(a, *walls, i, I, xi, yi, hi);
     // everything else the epilogue reads, before anything that could hold it up
     const State &b = a.base;
     const bool own = a.mode == EPI_PREDICT || a.mode == EPI_EULER || a.mode == EPI_RATES;   // (base is the rhs state)
@@ -620,9 +521,7 @@ __device__ __forceinline__ void stress_finish(const StressArgs &a, int i, bool l
     double ax = fi * fma(ta.x, Sx, fma(ta.y, Sy, Tx));
     double ay = fi * fma(ta.y, Sx, fma(tb.x, Sy, Ty));
     const double vxi = vi.x, vyi = vi.y;
-    ax = ax - wl.fx * irho + wl.gx;
-    ay = ay - wl.fy * irho + wl.gy;
-    cnt += wl.cnt;
+    walls.add(irho, ax, ay, cnt);
     // drag, wind_forcing.f90:35-51 and water_drag.f90:35-53 (off at t <= 0)
     const double tnow = I.t;
     if (P.wind_force && tnow > 0.0) {

@@ -4,7 +4,7 @@
 #include <type_traits>
 
 #include "pass_common.cuh"
-#include "tile.cuh"
+#include "walls.cuh"
 
 namespace simp {
 
@@ -400,12 +400,11 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
 // loading each where it is used).  Half of a block's time is the latency of its
 // copies and of that epilogue (issue slots 29%, L1 50%).  262,144 particles,
 // FP64: 71 -> 46 us per pass against gathers from global memory; mixed at
-// 1,048,576: 192 -> 155 us.
+// 1,048,576: 192 -> 148 us.
 template <class T, int SKF, bool UNIFORM, int BLOCKS>
 __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant__ StressArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Halo h;
-    __shared__ WallTile wt;
     __shared__ __align__(8) unsigned long long bar;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
@@ -418,6 +417,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
     const State &s = a.rhs;
     const Phys &P = a.P;
     const bool have_walls = (P.boundary_pressure || P.boundary_friction) && a.nb > 0 && !inst_dead(I.flags);
+    using Walls = typename std::conditional<sizeof(T) == sizeof(float), WallShared, WallRegs>::type;
     constexpr int arrays = Rec<T>::stress_arrays;
     const TileMem m = tile_mem(smem, a.cap, arrays, UNIFORM);
     unsigned parity = 0u;
@@ -433,13 +433,8 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         const bool live = t < h.size;
         const int i = p0 + (live ? t : h.size - 1);   // idle lanes mirror the part's last particle
         if (a.prefetch) stress_prefetch(a, i);
-        const bool walls = have_walls && h.walls;
-        if (walls) {
-            wall_tile(a, I, h.walls, a.cell[p0], a.cell[p0 + h.size - 1], wt);
-            __syncthreads();
-        }
-        const double2 xy = __ldg(&s.xy[i]);
-        const double hi = s.hs[i];
+        double2 xy = __ldg(&s.xy[i]);
+        double hi = s.hs[i];
         const T hiT = Rec<T>::own_h(s, i);
         StressSums<T> ss;
         PairGrad<T, SKF, UNIFORM> grad;
@@ -495,9 +490,37 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         }
         // (a retired basin's particles are not written any more: their state
         // stays as it was until the batch's next compaction drops them)
-        const double c = grad.common();
-        stress_finish<SKF>(a, i, live && !(I.flags & FLAG_RETIRED), ch.q, I, walls ? &wt : nullptr, xy.x,
-                           xy.y, hi, c * ss.sx.get(), c * ss.sy.get(), c * ss.tx.get(), c * ss.ty.get(), npairs);
+        double S[4];
+        auto pair_sums = [&] {
+            const double c = grad.common();
+            S[0] = c * ss.sx.get();
+            S[1] = c * ss.sy.get();
+            S[2] = c * ss.tx.get();
+            S[3] = c * ss.ty.get();
+        };
+        if (Walls::kKeep) pair_sums();
+        Walls wl;
+        if (have_walls && h.walls) {
+            int bytes = (int)tile_smem_bytes(a.cap, arrays, UNIFORM);
+            __syncthreads();
+            double *keep = reinterpret_cast<double *>(smem + bytes) - 4 * kTile + t;
+            if (Walls::kKeep) {
+                bytes -= 4 * kTile * (int)sizeof(double);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) keep[k * kTile] = S[k];
+            }
+            wl.set(reinterpret_cast<WallTile *>(smem),
+                   wall_sums<SKF>(a, I, h.walls, p0, h.size, i, xy, hi, smem, bytes));
+            if (Walls::kKeep) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) S[k] = keep[k * kTile];
+                asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(xy.x), "=d"(xy.y) : "l"(&s.xy[i]));
+                asm volatile("ld.global.f64 %0, [%1];" : "=d"(hi) : "l"(&s.hs[i]));   // (loaded again rather than held)
+            }
+        }
+        if (!Walls::kKeep) pair_sums();
+        stress_finish(a, i, live && !(I.flags & FLAG_RETIRED), ch.q, I, wl, xy.x, xy.y, hi, S[0], S[1], S[2], S[3],
+                      npairs);
         p0 += h.size;
         if (p0 < ch.p1) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

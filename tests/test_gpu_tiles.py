@@ -80,6 +80,29 @@ def test_tile_right_hand_side(gpu_lib, oracle_mod, name, precision):
         assert rel_l2(r[k], ro[k]) < TOL[precision], (name, k)
 
 
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED])
+@pytest.mark.parametrize("bfa, pressure, friction", [(1, 1, 0), (1, 1, 1), (1, 0, 1), (3, 0, 1)])
+@pytest.mark.parametrize("denser", [1, 3, 9])
+def test_tile_walls(gpu_lib, oracle_mod, denser, bfa, pressure, friction, precision):
+    """Wall pairs at the usual spacing, more of them in a tile than its table
+    holds, and more walls than its list holds (corner tiles see all three)."""
+    b = _basin("walls")
+    b.params.bfa, b.params.boundary_pressure, b.params.boundary_friction = bfa, pressure, friction
+    t = np.arange(0.5, denser) / denser
+    along = np.where(np.abs(b.xb[:, :1] - b.xb[:, :1].max()) < 1.0, [[0.0, 1.0]], [[1.0, 0.0]])
+    b.xb = (b.xb[:, None, :] + (t[None, :, None] - 0.5) * along[:, None, :] * b.params.b_length / 3.0).reshape(-1, 2)
+    b.massb = np.full(len(b.xb), b.mass.mean())
+    prm = b.params.copy()
+    prm.precision = precision
+    with Simp.from_basin(b, prm) as g:
+        r = g.single_step(600.0)
+    o = oracle_mod.Oracle(b.params, b.n, b.nb)
+    o.set_state(b.x, b.vx, b.mass, b.rho, b.hsml, b.A, b.h, b.xb, b.massb, 1.0, 600.0)
+    ro = o.single_step(600.0)
+    for k in ("dvxdt", "dhdt", "dAdt"):
+        assert rel_l2(r[k], ro[k]) < TOL[precision], k
+
+
 _ROOTS = """
 #include "pass_common.cuh"
 __global__ void roots(int n, const double *u, double *g, double *h) {
