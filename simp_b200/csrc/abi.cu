@@ -352,7 +352,7 @@ void free_all(simp_ctx *c) {
     void *ptrs[] = {c->s0.xy, c->s0.vxy, c->s0.mm, c->s0.hmm, c->s0.m, c->s0.rho, c->s0.h, c->s0.A, c->s0.hs,
                     c->s0.hsf, c->s1.xy, c->s1.vxy, c->s1.mm, c->s1.hmm, c->s1.rho, c->s1.h, c->s1.A, c->mass1,
                     c->xyr, c->cell, c->id, c->pinst, c->div, c->tau_a, c->tau_b, c->tau_q, c->diag, c->rates,
-                    c->pair_slot, c->pair_count, c->chunks, c->chunk_src, c->halos, c->inst_dev, c->bx, c->by, c->bm,
+                    c->pair_slot, c->pair_count, c->chunks, c->chunk_src, c->halos, c->halo_walls, c->inst_dev, c->bx, c->by, c->bm,
                     c->bnx, c->bny, c->bid, c->binst, c->bcell, c->bcell_start, c->cell_start, c->cnt, c->perm,
                     c->tmp, c->itmp, c->scan_tmp, c->sc, c->pair_cnt, c->bpair_cnt, c->pair_buf_i, c->pair_buf_j,
                     c->pair_buf_r, c->pair_buf_h, c->drhodt, c->k0, c->red_dev, c->reg, c->early_stage};
@@ -997,6 +997,7 @@ int create(const simp_params *params, int32_t maxn, int32_t maxnb, int32_t max_i
     TRY(dalloc(c, &c->pair_count, M));
     TRY(dalloc(c, &c->chunks, chunk_cap));
     TRY(dalloc(c, &c->halos, (size_t)kHaloBytes * (kTile / kPartMin) * chunk_cap));
+    TRY(dalloc(c, &c->halo_walls, (size_t)kHaloWallBytes * (kTile / kPartMin) * chunk_cap));
     TRY(dalloc(c, &c->chunk_src, (size_t)max_inst));
     TRY(dalloc(c, &c->diag, 9 * M));
     TRY(dalloc(c, &c->rates, 4 * M));
@@ -1135,7 +1136,7 @@ double bytes_per_particle(const simp_params &p, bool single_basin) {
     if (p.xsph_regularization || p.artificial_visc) b += 4 * 8.0;   // regularisation terms
     if (p.den_alg == 1) b += 8.0;                             // kept kernel_zero
     b += 4 * 4.0 + 14 * 8.0 + 3 * 4.0 + 4.0;                  // sort keys, scratch
-    b += 16.0 / 128 + 1.5 * kHaloBytes / kPartMin + 48.0;               // tiles, cell lists (worst case)
+    b += 16.0 / 128 + 1.5 * (kHaloBytes + kHaloWallBytes) / kPartMin + 48.0;               // tiles, cell lists (worst case)
     if (single_basin) b += 2 * 8.0;                           // read-back stage of the fixed fields
     return b;
 }

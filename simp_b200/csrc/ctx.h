@@ -94,6 +94,7 @@ struct simp_ctx {
     int4 *chunk_src = nullptr;     // per basin in memory order: offset, particles, first chunk, slot
     int nsrc = 0;                  // basins in it
     unsigned char *halos = nullptr;   // simp::kHaloBytes per simp::kPartMin particles of a tile
+    unsigned char *halo_walls = nullptr;   // likewise, simp::kHaloWallBytes each
     int nchunks = 0;
     bool uniform = false;          // every basin's hsml is one value, and stays it
     // diagnostics (epsilon_11.. sigma_22, zeta, eta, p)
@@ -212,6 +213,7 @@ void launch_reset_stats(simp_ctx *c);
 // context, the chunk table of the current layout and the kernels'
 // shared-memory limits.
 constexpr int kHaloBytes = 64;
+constexpr int kHaloWallBytes = 64;
 constexpr int kPartMin = 8;       // smallest part of a tile with its own halo
 __host__ __device__ inline int spare_tiles(int tiles) { return 3 + tiles / 16; }
 inline size_t chunk_capacity(int maxn, int max_inst) {

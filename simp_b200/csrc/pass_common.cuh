@@ -260,6 +260,7 @@ struct KinArgs {
     int n, maxn;
     const Chunk *chunks;   // tile of each block
     unsigned char *halos;  // their halos (written here)
+    unsigned char *halo_walls;
     int cap;               // halo particles that fit in shared memory
     int second;            // the step's second right-hand side
     int single;            // instance 0 owns every particle
@@ -370,7 +371,7 @@ struct StressArgs {
     double *hs_next;
     int n, maxn, mode, single, prefetch;
     const Chunk *chunks;
-    const unsigned char *halos;
+    const unsigned char *halos, *halo_walls;
     int cap;
 };
 

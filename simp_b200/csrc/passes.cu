@@ -222,7 +222,8 @@ __device__ __forceinline__ int classify(T dx, T dy, T hi, T hj, T mh2_u) {
 }
 
 constexpr int kHaloWords = sizeof(Halo) / sizeof(int);
-__device__ __forceinline__ int halo_word(const Halo *h, int k) { return reinterpret_cast<const int *>(h)[k]; }
+constexpr int kWallWords = 2 * kMaxWallRows;
+__device__ __forceinline__ int halo_word(const void *h, int k) { return reinterpret_cast<const int *>(h)[k]; }
 
 // Whether a basin's lists hold every pair of this right-hand side (Inst).
 // In a step's second right-hand side they are at most as old as the first.
@@ -279,7 +280,9 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
         } else if (t == 0) {
             // the largest part of the tile whose halo fits
             for (int S = kTile;; S >>= 1) {
-                make_halo(I, a.cell_start, a.bstart, a.cell, p0, min(p0 + S, ch.p1), a.cap, h);
+                make_halo(I, a.cell_start, a.bstart, a.cell, p0, min(p0 + S, ch.p1), a.cap, h,
+                          reinterpret_cast<HaloWalls *>(a.halo_walls) + (size_t)blockIdx.x * (kTile / kPartMin) +
+                              (p0 - ch.p0) / kPartMin);
                 if (h.kind == HALO_TILE || S <= kPartMin || h.nseg > kMaxSeg) break;
             }
             rows_max = 0;
@@ -399,12 +402,13 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
 // are loaded together ahead of the walls and the update (68 -> 50 us against
 // loading each where it is used).  Half of a block's time is the latency of its
 // copies and of that epilogue (issue slots 29%, L1 50%).  262,144 particles,
-// FP64: 71 -> 46 us per pass against gathers from global memory; mixed at
-// 1,048,576: 192 -> 148 us.
+// FP64: 71 -> 44 us per pass against gathers from global memory; mixed at
+// 1,048,576: 192 -> 147 us.
 template <class T, int SKF, bool UNIFORM, int BLOCKS>
 __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant__ StressArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Halo h;
+    __shared__ HaloWalls hw;
     __shared__ __align__(8) unsigned long long bar;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
@@ -412,7 +416,10 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
     pass_begin();
     const Inst &I = a.inst[a.single ? 0 : ch.q];
     const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
-    const int first = t < kHaloWords ? halo_word(halos, t) : 0;   // (read along with the instance)
+    const HaloWalls *walls = reinterpret_cast<const HaloWalls *>(a.halo_walls) + (size_t)blockIdx.x * (kTile / kPartMin);
+    // (read along with the instance; the second warp reads the walls)
+    const int first = t < kHaloWords ? halo_word(halos, t)
+                      : BLOCKS == 4 && t >= 32 && t < 32 + kWallWords ? halo_word(walls, t - 32) : 0;
     if (ch.spare >= I.spares) return;   // (an unused spare tile)
     const State &s = a.rhs;
     const Phys &P = a.P;
@@ -422,8 +429,10 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
     const TileMem m = tile_mem(smem, a.cap, arrays, UNIFORM);
     unsigned parity = 0u;
     for (int p0 = ch.p0; p0 < ch.p1;) {
-        if (t < kHaloWords)
-            reinterpret_cast<int *>(&h)[t] = p0 == ch.p0 ? first : halo_word(&halos[(p0 - ch.p0) / kPartMin], t);
+        const int part = (p0 - ch.p0) / kPartMin;
+        if (t < kHaloWords) reinterpret_cast<int *>(&h)[t] = part == 0 ? first : halo_word(&halos[part], t);
+        if (BLOCKS == 4 && t >= 32 && t < 32 + kWallWords)
+            reinterpret_cast<int *>(&hw)[t - 32] = part == 0 ? first : halo_word(&walls[part], t - 32);
         __syncthreads();
         const bool tile = h.kind == HALO_TILE;
         if (tile && t < 32) {
@@ -433,6 +442,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         const bool live = t < h.size;
         const int i = p0 + (live ? t : h.size - 1);   // idle lanes mirror the part's last particle
         if (a.prefetch) stress_prefetch(a, i);
+        if (BLOCKS == 4 && have_walls && h.walls) wall_prefetch(a, hw, a.bstart[I.base], i);
         double2 xy = __ldg(&s.xy[i]);
         double hi = s.hs[i];
         const T hiT = Rec<T>::own_h(s, i);
@@ -510,7 +520,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
                 for (int k = 0; k < 4; ++k) keep[k * kTile] = S[k];
             }
             wl.set(reinterpret_cast<WallTile *>(smem),
-                   wall_sums<SKF>(a, I, h.walls, p0, h.size, i, xy, hi, smem, bytes));
+                   wall_sums<SKF, BLOCKS == 4>(a, I, h.walls, hw, p0, h.size, i, xy, hi, smem, bytes));
             if (Walls::kKeep) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) S[k] = keep[k * kTile];
@@ -1068,7 +1078,7 @@ __global__ void k_split(int nchunks, int nsrc, const int4 *__restrict__ src, int
     Halo h;
     int S = size;
     for (;; S >>= 1) {
-        make_halo(I, cell_start, bstart, cell, p0, min(p0 + S, p1), cap, h);
+        make_halo(I, cell_start, bstart, cell, p0, min(p0 + S, p1), cap, h, nullptr);
         if (h.kind == HALO_TILE || S <= kPartMin || h.nseg > kMaxSeg) break;
     }
     const int extra = (p1 - p0 + S - 1) / S - 1;
@@ -1241,6 +1251,7 @@ void launch_kinematic(simp_ctx *c, const State &s, bool diag, bool second) {
     a.prefetch = prefetch_own(c);
     a.chunks = c->chunks;
     a.halos = c->halos;
+    a.halo_walls = c->halo_walls;
     a.cap = tile_cap(c);
     a.second = second ? 1 : 0;
     launch_form(c, a);
@@ -1280,6 +1291,7 @@ void launch_stress(simp_ctx *c, const State &rhs, const State &base, EpiMode mod
     a.prefetch = prefetch_own(c);
     a.chunks = c->chunks;
     a.halos = c->halos;
+    a.halo_walls = c->halo_walls;
     a.cap = tile_cap(c);
     launch_form(c, a);
     c->launches += 1;

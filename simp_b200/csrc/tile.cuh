@@ -45,6 +45,14 @@ struct Halo {
     int size;                  // particles in this part of the tile
 };
 static_assert(sizeof(Halo) == kHaloBytes, "ctx.h: kHaloBytes");
+// A halo's walls, by cell row: from the basin's first, and how many (-1 in the
+// first row: more rows than there is room for).
+constexpr int kMaxWallRows = 7;
+struct HaloWalls {
+    int lo[kMaxWallRows], n[kMaxWallRows];
+    int spare[2];
+};
+static_assert(sizeof(HaloWalls) == kHaloWallBytes, "ctx.h: kHaloWallBytes");
 
 // Place of candidate k in a particle's list (PairList): consecutive candidates
 // of a thread share a 32-bit word.
@@ -104,9 +112,10 @@ __device__ __forceinline__ TileMem tile_mem(unsigned char *p, int cap, int array
     return m;
 }
 
-// The halo of particles [p0, p1) of instance I.  Called by one thread.
+// The halo of particles [p0, p1) of instance I, and its walls, if it has any
+// and they are asked for.  Called by one thread.
 __device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, const int *bstart, const int *cell, int p0,
-                                       int p1, int cap, Halo &h) {
+                                       int p1, int cap, Halo &h, HaloWalls *hw) {
     const Grid g = inst_grid(I, cell_start);
     const int R = stencil_radius(I.hmax, inst_disp(I), g, I.hmax + I.delta);
     h.size = p1 - p0;
@@ -121,6 +130,21 @@ __device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, con
     for (int d = -Rb; d <= Rb && !h.walls; ++d)
         if (bstart[clampi(kb + d * I.ncx + Rb + 1, I.base, end)] > bstart[clampi(ka + d * I.ncx - Rb, I.base, end)])
             h.walls = Rb;
+    if (h.walls && hw) {
+        const int rows = 2 * Rb + 1, b_first = bstart[I.base];
+        int past = 0;
+        for (int d = 0; d < kMaxWallRows; ++d) {
+            int b0 = past, b1 = past;
+            if (d < rows) {
+                const int sh = (d - Rb) * I.ncx;
+                b0 = max(bstart[clampi(ka + sh - Rb, I.base, end)], past);
+                b1 = bstart[clampi(kb + sh + Rb + 1, I.base, end)];
+            }
+            hw->lo[d] = b0 - b_first;
+            hw->n[d] = d == 0 && rows > kMaxWallRows ? -1 : max(b1 - b0, 0);
+            past = max(past, b1);
+        }
+    }
     if (h.kind == HALO_GLOBAL) return;
     int a[kMaxSeg], b[kMaxSeg];
 #pragma unroll

@@ -6,10 +6,10 @@
 // the block lists the walls near the tile, marks each particle's pairs
 // (comparisons only), takes the pairs one per thread whichever particle they
 // belong to, and each particle sums its own in the walls' order.  Bound by the
-// latency of five such phases, 4 us of a tile's 20.  Per step with walls on four
-// sides, against one thread per particle: FP64 2,500 particles 59 -> 47 us,
-// 65,536 82 -> 67, 262,144 188 -> 165, 1,048,576 585 -> 563; mixed 24,649
-// 67 -> 55, 262,144 189 -> 169, 1,048,576 569 -> 555.
+// latency of five such phases.  Per step with walls on four sides, against one
+// thread per particle: FP64 2,500 particles 59 -> 46 us, 65,536 82 -> 65,
+// 262,144 188 -> 161, 600,011 372 -> 347; mixed 24,649 67 -> 54, 262,144
+// 189 -> 169, 1,048,576 569 -> 554.
 #pragma once
 
 #include "tile.cuh"
@@ -42,10 +42,49 @@ __device__ __forceinline__ int warp_scan(int v, int lane) {   // inclusive
     return v;
 }
 
-// The walls within Rb cells of a part of a tile with cells ka .. kb
-// (Halo.walls), in their order.  Called by the whole block, which synchronises
+// Wall k of the part's, in their order, or -1 behind the last (HaloWalls).
+__device__ __forceinline__ int wall_at(const HaloWalls &h, int b_first, int k) {
+    int b = -1;
+#pragma unroll
+    for (int d = 0; d < kMaxWallRows; ++d) {
+        const int n = h.n[d];
+        if (k >= 0 && k < n) b = b_first + h.lo[d] + k;
+        k -= n;
+    }
+    return b;
+}
+// Brings what wall_sums reads first to the L1 cache, while the pairs are summed.
+__device__ __forceinline__ void wall_prefetch(const StressArgs &a, const HaloWalls &h, int b_first, int i) {
+    const int b = wall_at(h, b_first, threadIdx.x);
+    if (b >= 0) {
+        prefetch_l1(&a.bx[b]);
+        prefetch_l1(&a.by[b]);
+        prefetch_l1(&a.bm[b]);
+    }
+    prefetch_l1(&a.rhs.m[i]);
+}
+// The part's walls.  Called by the whole block, which synchronises before they
+// are read.
+__device__ __forceinline__ void wall_list(const StressArgs &a, const HaloWalls &h, int b_first, WallTile &w) {
+    static_assert(kWallCap <= kTile, "one wall per thread");
+    const int t = threadIdx.x, b = t < kWallCap ? wall_at(h, b_first, t) : -1;
+    if (b >= 0) {
+        w.id[t] = b;
+        w.x[t] = a.bx[b];
+        w.y[t] = a.by[b];
+        w.m[t] = a.bm[b];
+    }
+    if (t == 0) {
+        int n = 0;
+        for (int d = 0; d < kMaxWallRows; ++d) n += h.n[d];
+        w.n = h.n[0] >= 0 && n <= kWallCap ? n : -1;
+    }
+}
+
+// The same from the cell lists, for a part with cells ka .. kb whose walls lie
+// within Rb cells (Halo.walls).  Called by the whole block, which synchronises
 // before they are read.
-__device__ __forceinline__ void wall_list(const StressArgs &a, const Inst &I, int Rb, int ka, int kb, WallTile &w) {
+__device__ __forceinline__ void wall_find(const StressArgs &a, const Inst &I, int Rb, int ka, int kb, WallTile &w) {
     const int end = I.base + I.ncx * I.ncy, rows = 2 * Rb + 1, lane = threadIdx.x & 31;
     // one lane per cell row: its walls, from where the rows before it end
     int b0 = 0, b1 = 0;
@@ -211,12 +250,19 @@ __device__ __noinline__ WallSums wall_serial(const StressArgs &a, const Inst &I,
     return w;
 }
 
+// Whether the walls come with the halo or from the cell lists: in the mixed form
+// of five blocks per SM those hide the cell lists' two more loads in a row, and
+// the halo's cost registers it does not have (1,048,576 particles: 552 us per
+// step from the cell lists, 562 with the halo); everywhere else they come with
+// the halo (FP64 at 262,144: 157 -> 153, at 2,500: 43 -> 40).
+//
 // The wall sums of a part's particles, thread t's particle p0 + t.  Works in
 // `bytes` of shared memory that the block no longer needs.  Called by the whole
 // block.
-template <int SKF>
-__device__ __forceinline__ WallSums wall_sums(const StressArgs &a, const Inst &I, int Rb, int p0, int size, int i,
-                                              double2 p, double hi, unsigned char *smem, int bytes) {
+template <int SKF, bool LISTED>
+__device__ __forceinline__ WallSums wall_sums(const StressArgs &a, const Inst &I, int Rb, const HaloWalls &h, int p0,
+                                              int size, int i, double2 p,
+                                              double hi, unsigned char *smem, int bytes) {
     WallTile &w = *reinterpret_cast<WallTile *>(smem);
     double *res = reinterpret_cast<double *>(smem + sizeof(WallTile));
     const int t = threadIdx.x;
@@ -224,7 +270,8 @@ __device__ __forceinline__ WallSums wall_sums(const StressArgs &a, const Inst &I
     // which sums the parameters give terms to
     const bool f = a.P.bfa == 1 && a.P.boundary_pressure, g = a.P.bfa != 1 || a.P.boundary_friction;
     const int room = (bytes - (int)sizeof(WallTile)) / (16 * max(1, (int)f + (int)g));
-    wall_list(a, I, Rb, a.cell[p0], a.cell[p0 + size - 1], w);
+    if (LISTED) wall_list(a, h, a.bstart[I.base], w);
+    else wall_find(a, I, Rb, a.cell[p0], a.cell[p0 + size - 1], w);
     __syncthreads();
     wall_pairs(a, I, live, i, p, hi, min(kWallPairs, room), w);
     __syncthreads();
