@@ -247,6 +247,7 @@ struct StressSums {
 
 struct KinArgs {
     State s;
+    const double2 *xyr;    // sort positions
     const int *cell_start, *bstart;
     const Inst *inst;
     const int *pinst;      // instance of each particle

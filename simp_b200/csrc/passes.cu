@@ -225,6 +225,24 @@ constexpr int kHaloWords = sizeof(Halo) / sizeof(int);
 constexpr int kWallWords = 2 * kMaxWallRows;
 __device__ __forceinline__ int halo_word(const void *h, int k) { return reinterpret_cast<const int *>(h)[k]; }
 
+// The largest squared distance of the tile's particles from where they were
+// sorted, rounded up, as a float's bits.  Called by the whole block.
+__device__ __noinline__ void tile_moved(const State &s, const double2 *xyr, int p0, int p1, unsigned &out) {
+    const int t = threadIdx.x, i = p0 + t;
+    if (t == 0) out = 0u;
+    __syncthreads();
+    float d2 = 0.0f;
+    if (i < p1) {
+        const double2 a = s.xy[i], b = xyr[i];
+        const double dx = a.x - b.x, dy = a.y - b.y;
+        d2 = __double2float_ru(fma(dx, dx, dy * dy));
+        if (!(d2 >= 0.0f)) d2 = INFINITY;
+    }
+    const unsigned most = __reduce_max_sync(0xffffffffu, __float_as_uint(d2));
+    if ((t & 31) == 0) atomicMax(&out, most);
+    __syncthreads();
+}
+
 // Whether a basin's lists hold every pair of this right-hand side (Inst).
 // In a step's second right-hand side they are at most as old as the first.
 __device__ __forceinline__ bool lists_valid(const Inst &I, bool second) {
@@ -245,6 +263,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
     __shared__ Halo h;
     __shared__ __align__(8) unsigned long long bar;
     __shared__ int rows_max;
+    __shared__ unsigned moved2;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
     if (t == 0) bar_init(&bar);
@@ -273,6 +292,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
     const bool build = !lists_valid(I, a.second);
     const TileMem m = tile_mem(smem, a.cap, 3, UNIFORM);
     unsigned parity = 0u;
+    if (build) tile_moved(s, a.xyr, ch.p0, ch.p1, moved2);
     for (int p0 = ch.p0; p0 < ch.p1;) {
         if (!build) {
             if (t < kHaloWords)
@@ -280,7 +300,8 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
         } else if (t == 0) {
             // the largest part of the tile whose halo fits
             for (int S = kTile;; S >>= 1) {
-                make_halo(I, a.cell_start, a.bstart, a.cell, p0, min(p0 + S, ch.p1), a.cap, h,
+                make_halo(I, a.cell_start, a.bstart, a.cell, p0, min(p0 + S, ch.p1), a.cap,
+                          sqrt((double)__uint_as_float(moved2)) * (1.0 + 1e-6), h,
                           reinterpret_cast<HaloWalls *>(a.halo_walls) + (size_t)blockIdx.x * (kTile / kPartMin) +
                               (p0 - ch.p0) / kPartMin);
                 if (h.kind == HALO_TILE || S <= kPartMin || h.nseg > kMaxSeg) break;
@@ -1078,7 +1099,7 @@ __global__ void k_split(int nchunks, int nsrc, const int4 *__restrict__ src, int
     Halo h;
     int S = size;
     for (;; S >>= 1) {
-        make_halo(I, cell_start, bstart, cell, p0, min(p0 + S, p1), cap, h, nullptr);
+        make_halo(I, cell_start, bstart, cell, p0, min(p0 + S, p1), cap, 0.0, h, nullptr);
         if (h.kind == HALO_TILE || S <= kPartMin || h.nseg > kMaxSeg) break;
     }
     const int extra = (p1 - p0 + S - 1) / S - 1;
@@ -1251,6 +1272,7 @@ void launch_kinematic(simp_ctx *c, const State &s, bool diag, bool second) {
     a.prefetch = prefetch_own(c);
     a.chunks = c->chunks;
     a.halos = c->halos;
+    a.xyr = c->xyr;
     a.halo_walls = c->halo_walls;
     a.cap = tile_cap(c);
     a.second = second ? 1 : 0;

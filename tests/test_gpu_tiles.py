@@ -52,6 +52,10 @@ def _basin(name):
         b.hsml = b.hsml * rng.uniform(1.0, 1.3, size=b.n)
     elif name == "bucket rule":
         b.hsml = b.hsml * rng.uniform(0.6, 1.4, size=b.n)
+    elif name == "drift of few":  # most tiles stay near their cells, a few particles do not
+        b.vx[::97] += [60.0, 30.0]
+        b.xb, b.massb = b.xb[:0], b.massb[:0]
+        b.params.wind_force = b.params.water_force = 0
     elif name.startswith("drift="):
         b.vx = b.vx + np.array([float(name[6:]), 0.5 * float(name[6:])])
         b.xb, b.massb = b.xb[:0], b.massb[:0]
@@ -61,7 +65,7 @@ def _basin(name):
 
 @pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED])
 @pytest.mark.parametrize("name", ["n=1", "n=2", "n=127", "n=128", "n=129", "n=257", "narrow", "sparse", "dense",
-                                  "varied", "bucket rule", "drift=60", "drift=250", "drift=900"])
+                                  "varied", "bucket rule", "drift of few", "drift=60", "drift=250", "drift=900"])
 def test_tile_right_hand_side(gpu_lib, oracle_mod, name, precision):
     b = _basin(name)
     prm = b.params.copy()
