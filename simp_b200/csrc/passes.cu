@@ -444,7 +444,10 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
     if (ch.spare >= I.spares) return;   // (an unused spare tile)
     const State &s = a.rhs;
     const Phys &P = a.P;
-    const bool have_walls = (P.boundary_pressure || P.boundary_friction) && a.nb > 0 && !inst_dead(I.flags);
+    // (of a dead basin the kinematic pass wrote records without walls; its flags
+    // are not asked here, because other blocks set them while this one runs and
+    // the walls' barriers need every thread to decide alike)
+    const bool have_walls = (P.boundary_pressure || P.boundary_friction) && a.nb > 0;
     using Walls = typename std::conditional<sizeof(T) == sizeof(float), WallShared, WallRegs>::type;
     constexpr int arrays = Rec<T>::stress_arrays;
     const TileMem m = tile_mem(smem, a.cap, arrays, UNIFORM);
