@@ -114,8 +114,10 @@ __device__ __noinline__ int build_lists(const Halo &h, const TileMem &m, const K
 
 // Programmatic dependent launch: a pass's blocks may start while the last
 // blocks of the kernel before still run, and wait here before they read what
-// it wrote.  The kernels after it may follow once every block is this far (so
-// that everything before the previous kernel has ended).
+// it wrote (with ordinary loads: the wait does not order those of the read-only
+// path, which are for data that nothing writes while a kernel runs).  The
+// kernels after it may follow once every block is this far (so that everything
+// before the previous kernel has ended).
 __device__ __forceinline__ void pass_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -139,10 +141,10 @@ struct Rec<double> {
         h = UNIFORM ? 0.0 : t.hs[sl];
     }
     static __device__ __forceinline__ void kin_global(const State &s, int j, double &m, double &mor, double &h) {
-        const double2 q = __ldg(&s.mm[j]);
+        const double2 q = s.mm[j];
         m = q.x;
         mor = q.y;
-        h = __ldg(&s.hs[j]);
+        h = s.hs[j];
     }
     template <bool UNIFORM>
     static __device__ __forceinline__ void stress(const TileMem &t, int sl, double &m, double &t11, double &t12,
@@ -157,12 +159,12 @@ struct Rec<double> {
     }
     static __device__ __forceinline__ void stress_global(const State &s, const TauRec &r, int j, double &m, double &t11,
                                                          double &t12, double &t22, double &h) {
-        const double2 a = __ldg(&r.ta[j]), b = __ldg(&r.tb[j]);
+        const double2 a = r.ta[j], b = r.tb[j];
         m = b.y;
         t11 = a.x;
         t12 = a.y;
         t22 = b.x;
-        h = __ldg(&s.hs[j]);
+        h = s.hs[j];
     }
     static constexpr double band = kBand;
 };
@@ -179,7 +181,7 @@ struct Rec<float> {
         mor = q.z;
     }
     static __device__ __forceinline__ void kin_global(const State &s, int j, float &m, float &mor, float &h) {
-        const float4 q = __ldg(&s.hmm[j]);
+        const float4 q = s.hmm[j];
         h = q.x;
         m = q.y;
         mor = q.z;
@@ -196,12 +198,12 @@ struct Rec<float> {
     }
     static __device__ __forceinline__ void stress_global(const State &s, const TauRec &r, int j, float &m, float &t11,
                                                          float &t12, float &t22, float &h) {
-        const float4 q = __ldg(&r.tq[j]);
+        const float4 q = r.tq[j];
         m = q.w;
         t11 = q.x;
         t12 = q.y;
         t22 = q.z;
-        h = __ldg(&s.hsf[j]);
+        h = s.hsf[j];
     }
     // (differences and hsml rounded to FP32: within 2^-20 of the exact ratio)
     static constexpr float band = 0x1p-18f;
@@ -314,8 +316,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
         if (fits && t < 32) tile_fetch(h, m, src, 0, build ? 1 : 3, lists, build ? 0 : h.rows, &bar);
         const bool live = t < h.size;
         const int i = p0 + (live ? t : 0);
-        const double2 xy = __ldg(&s.xy[i]), vi = __ldg(&s.vxy[i]);
-        const double hi = s.hs[i];
+        double2 xy = s.xy[i], vi = s.vxy[i];
         if (sizeof(T) == sizeof(float) && a.prefetch) {   // (the plain form has no register to spare)
             prefetch_l1(&s.h[i]);
             prefetch_l1(&s.A[i]);
@@ -391,8 +392,11 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
                 int in0 = classify<T, UNIFORM>(dx0, dy0, hiT, h0, mh2_u);
                 int in1 = k + 1 < cnt ? classify<T, UNIFORM>(dx1, dy1, hiT, h1, mh2_u) : 0;
                 if (((in0 | in1) & 2) || rule) {
-                    if (in0) in0 = in0 == 1 && !rule ? 1 : exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q0));
-                    if (in1) in1 = in1 == 1 && !rule ? 1 : exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q1));
+                    const int in = exact_two(s, I, rule, i, h, q0, q1, in0, in1);
+                    in0 = in & 1;
+                    in1 = in >> 1;
+                    reload(xy, &s.xy[i]);
+                    reload(vi, &s.vxy[i]);
                 }
                 terms(in0 != 0, dx0, dy0, v0, m0, r0, h0);
                 terms(in1 != 0, dx1, dy1, v1, m1, r1, h1);
@@ -400,7 +404,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
         } else if (live) {
             // no tile: the neighbours from global memory
             global_pairs(s, I, a.cell_start, i, a.cell[i], [&](int j) {
-                const double2 q = __ldg(&s.xy[j]), v = __ldg(&s.vxy[j]);
+                const double2 q = s.xy[j], v = s.vxy[j];
                 T mj, mrj, hj;
                 Rec<T>::kin_global(s, j, mj, mrj, hj);
                 terms(true, (T)(xy.x - q.x), (T)(xy.y - q.y), v, mj, mrj, hj);
@@ -467,7 +471,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         const int i = p0 + (live ? t : h.size - 1);   // idle lanes mirror the part's last particle
         if (a.prefetch) stress_prefetch(a, i);
         if (BLOCKS == 4 && have_walls && h.walls) wall_prefetch(a, hw, a.bstart[I.base], i);
-        double2 xy = __ldg(&s.xy[i]);
+        double2 xy = s.xy[i];
         double hi = s.hs[i];
         const T hiT = Rec<T>::own_h(s, i);
         StressSums<T> ss;
@@ -508,15 +512,17 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
                 int in0 = classify<T, UNIFORM>(dx0, dy0, hiT, h0, mh2_u);
                 int in1 = k + 1 < cnt ? classify<T, UNIFORM>(dx1, dy1, hiT, h1, mh2_u) : 0;
                 if (((in0 | in1) & 2) || rule) {
-                    if (in0) in0 = in0 == 1 && !rule ? 1 : exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q0));
-                    if (in1) in1 = in1 == 1 && !rule ? 1 : exact_pair(s, I, rule, xy.x, xy.y, hi, particle_of(h, q1));
+                    const int in = exact_two(s, I, rule, i, h, q0, q1, in0, in1);
+                    in0 = in & 1;
+                    in1 = in >> 1;
+                    reload(xy, &s.xy[i]);
                 }
                 terms(in0 != 0, dx0, dy0, m0, a0, b0, c0, h0);
                 terms(in1 != 0, dx1, dy1, m1, a1, b1, c1, h1);
             }
         } else if (h.kind == HALO_GLOBAL && live) {
             global_pairs(s, I, a.cell_start, i, a.cell[i], [&](int j) {
-                const double2 q = __ldg(&s.xy[j]);
+                const double2 q = s.xy[j];
                 T mj, t11, t12, t22, hj;
                 Rec<T>::stress_global(s, a.rec, j, mj, t11, t12, t22, hj);
                 terms(true, (T)(xy.x - q.x), (T)(xy.y - q.y), mj, t11, t12, t22, hj);
@@ -548,8 +554,8 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
             if (Walls::kKeep) {
 #pragma unroll
                 for (int k = 0; k < 4; ++k) S[k] = keep[k * kTile];
-                asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(xy.x), "=d"(xy.y) : "l"(&s.xy[i]));
-                asm volatile("ld.global.f64 %0, [%1];" : "=d"(hi) : "l"(&s.hs[i]));   // (loaded again rather than held)
+                reload(xy, &s.xy[i]);
+                reload(hi, &s.hs[i]);
             }
         }
         if (!Walls::kKeep) pair_sums();
@@ -669,7 +675,7 @@ __device__ __forceinline__ void aux_pairs(const Halo &h, const TileMem &m, const
             const int in = classify<double, false>(p.x - x.x, p.y - x.y, hi, hj, 0.0);
             if (in == 0) continue;
             if (in == 2 || rule)
-                if (!exact_pair(g, I, rule, p.x, p.y, hi, particle_of(h, q))) continue;
+                if (!exact_pair(g, I, rule, i, particle_of(h, q))) continue;
             f(particle_of(h, q), q, x, vs[q], hj);
         }
     }

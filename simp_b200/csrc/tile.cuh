@@ -230,13 +230,28 @@ __device__ __forceinline__ void tile_fetch(const Halo &h, const TileMem &m, cons
 constexpr double kBand = 0x1p-40;
 
 // The exact reference criterion (nnps.f90:277-281 and the bucket rule).
-__device__ __noinline__ bool exact_pair(const State &s, const Inst &I, bool rule, double xi, double yi, double hi,
-                                        int j) {
-    const double2 q = __ldg(&s.xy[j]);
+__device__ __noinline__ bool exact_pair(const State &s, const Inst &I, bool rule, int i, int j) {
+    const double2 p = s.xy[i], q = s.xy[j];
     double r;
-    const double mh = __dmul_rn(__dadd_rn(hi, __ldg(&s.hs[j])), 0.5);
-    if (!pair_test(__dsub_rn(xi, q.x), __dsub_rn(yi, q.y), mh, &r)) return false;
-    return !rule || bin_rule_ok(make_bin_rule(I.bs, xi, yi, I.hmax), q.x, q.y);
+    const double mh = __dmul_rn(__dadd_rn(s.hs[i], s.hs[j]), 0.5);
+    if (!pair_test(__dsub_rn(p.x, q.x), __dsub_rn(p.y, q.y), mh, &r)) return false;
+    return !rule || bin_rule_ok(make_bin_rule(I.bs, p.x, p.y, I.hmax), q.x, q.y);
+}
+// The same for two candidates at slots q0 and q1, as classified: bit 0 and bit 1
+// set where they are pairs.
+__device__ __noinline__ int exact_two(const State &s, const Inst &I, bool rule, int i, const Halo &h, int q0, int q1,
+                                      int in0, int in1) {
+    if (in0) in0 = in0 == 1 && !rule ? 1 : exact_pair(s, I, rule, i, particle_of(h, q0));
+    if (in1) in1 = in1 == 1 && !rule ? 1 : exact_pair(s, I, rule, i, particle_of(h, q1));
+    return in0 | in1 << 1;
+}
+// A particle's own value loaded again after a call, so that no register (nor a
+// store to local memory) holds it over the call.
+__device__ __forceinline__ void reload(double2 &v, const double2 *p) {
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+}
+__device__ __forceinline__ void reload(double &v, const double *p) {
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
 }
 __device__ __forceinline__ bool rule_on(const Inst &I) { return I.hmax >= I.bs * (1.0 - 1e-6); }
 
@@ -254,12 +269,12 @@ __device__ __forceinline__ void global_pairs(const State &s, const Inst &I, cons
         stencil_range(I, cell_start, at, R, d, j0, j1);
 #pragma unroll 4
         for (int j = j0; j < j1; ++j) {
-            const double2 q = __ldg(&s.xy[j]);
-            const double dx = p.x - q.x, dy = p.y - q.y, mh = 0.5 * (hi + __ldg(&s.hs[j]));
+            const double2 q = s.xy[j];
+            const double dx = p.x - q.x, dy = p.y - q.y, mh = 0.5 * (hi + s.hs[j]);
             const double d2 = fma(dx, dx, dy * dy);
             if (d2 > mh * mh * (1.0 + kBand) || j == i) continue;
             if (!(d2 < mh * mh * (1.0 - kBand)) || rule)
-                if (!exact_pair(s, I, rule, p.x, p.y, hi, j)) continue;
+                if (!exact_pair(s, I, rule, i, j)) continue;
             f(j);
         }
     }
