@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Halo h;
     __shared__ __align__(8) unsigned long long bar;
-    __shared__ int rows_max;
+    __shared__ int rows_max, failed;
     __shared__ unsigned moved2;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
@@ -275,6 +275,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
     const Phys &P = a.P;
     Halo *halos = reinterpret_cast<Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
     const int first = t < kHaloWords ? halo_word(halos, t) : 0;   // (read along with the instance)
+    if (t == kTile - 1) failed = failed_before(a.sc);
     if (ch.spare >= I.spares) return;   // (an unused spare tile)
     unsigned short *lists = a.pl.slot + (size_t)blockIdx.x * kListRows * kTile;
     // a basin whose state turned non-finite is not searched any more (its
@@ -311,6 +312,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
             rows_max = 0;
         }
         __syncthreads();
+        if (failed < 2 * p0) return;
         const void *src[3] = {s.xy, s.vxy, Rec<T>::kin_src(s)};
         const bool fits = h.kind == HALO_TILE;
         if (fits && t < 32) tile_fetch(h, m, src, 0, build ? 1 : 3, lists, build ? 0 : h.rows, &bar);
@@ -337,11 +339,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
         if (fits) {
             if (!UNIFORM) tile_hsml(h, m, s);
             if (!build && live) cnt = a.pl.count[i];
-            if (!bar_wait(&bar, parity)) {
-                atomicOr(&a.sc->flags, FLAG_TIMEOUT);
-                bar_wait(&bar, parity);
-                return;
-            }
+            if (!copies_arrive(&bar, parity, 2 * p0, &failed, &a.sc->flags)) cnt = 0;
             parity ^= 1u;
             if (!UNIFORM || build) __syncthreads();
             if (build) {
@@ -351,6 +349,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
                 // (the FP32 copies make way for the records)
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncthreads();
+                if (failed <= 2 * p0) return;
                 tile = rows_max <= kListRows;
                 if (t == 0) {
                     h.rows = tile ? rows_max : 0;
@@ -359,11 +358,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
                 if (tile) {
                     if (t < 32) tile_fetch(h, m, src, 1, 3, lists, 0, &bar);
                     if (live) a.pl.count[i] = cnt;
-                    if (!bar_wait(&bar, parity)) {
-                        atomicOr(&a.sc->flags, FLAG_TIMEOUT);
-                        bar_wait(&bar, parity);
-                        return;
-                    }
+                    if (!copies_arrive(&bar, parity, 2 * p0 + 1, &failed, &a.sc->flags)) cnt = 0;
                     parity ^= 1u;
                 }
                 __syncthreads();
@@ -434,6 +429,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Halo h;
     __shared__ HaloWalls hw;
+    __shared__ int failed;
     __shared__ __align__(8) unsigned long long bar;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
@@ -445,6 +441,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
     // (read along with the instance; the second warp reads the walls)
     const int first = t < kHaloWords ? halo_word(halos, t)
                       : BLOCKS == 4 && t >= 32 && t < 32 + kWallWords ? halo_word(walls, t - 32) : 0;
+    if (t == kTile - 1) failed = failed_before(a.sc);
     if (ch.spare >= I.spares) return;   // (an unused spare tile)
     const State &s = a.rhs;
     const Phys &P = a.P;
@@ -462,6 +459,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         if (BLOCKS == 4 && t >= 32 && t < 32 + kWallWords)
             reinterpret_cast<int *>(&hw)[t - 32] = part == 0 ? first : halo_word(&walls[part], t - 32);
         __syncthreads();
+        if (failed < 2 * p0) return;
         const bool tile = h.kind == HALO_TILE;
         if (tile && t < 32) {
             const void *src[3] = {s.xy, a.rec.tq ? (const void *)a.rec.tq : (const void *)a.rec.ta, a.rec.tb};
@@ -485,13 +483,9 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         };
         if (tile) {
             if (!UNIFORM) tile_hsml(h, m, s);
-            const int cnt = live ? a.pl.count[i] : 0;
+            int cnt = live ? a.pl.count[i] : 0;
             const bool rule = rule_on(I);
-            if (!bar_wait(&bar, parity)) {
-                atomicOr(&a.sc->flags, FLAG_TIMEOUT);
-                bar_wait(&bar, parity);
-                return;
-            }
+            if (!copies_arrive(&bar, parity, 2 * p0, &failed, &a.sc->flags)) cnt = 0;
             parity ^= 1u;
             if (!UNIFORM) __syncthreads();
             const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
@@ -628,28 +622,27 @@ size_t aux_smem_bytes(int cap) {
 }
 
 // Copies a tile part's halo record, records and lists to shared memory and
-// fills the other values.  Called by the whole block; false where a copy did
-// not arrive.
+// fills the other values.  Called by the whole block; false, for all of it,
+// where a copy did not arrive, now or in an earlier pass.
 template <class F>
 __device__ __forceinline__ bool aux_tile(const Halo *rec, Halo &h, const TileMem &m, const State &g, const double2 *vxy,
                                          const unsigned short *lists, unsigned long long *bar, unsigned &parity,
                                          Scalars *sc, F &&fill) {
+    __shared__ int failed;
     const int t = threadIdx.x;
     if (t < (int)(sizeof(Halo) / sizeof(int))) reinterpret_cast<int *>(&h)[t] = reinterpret_cast<const int *>(rec)[t];
+    if (t == kTile - 1) failed = failed_before(sc);
     __syncthreads();
+    if (failed < 0) return false;
     if (h.kind != HALO_TILE) return true;
     const void *src[3] = {g.xy, vxy, nullptr};
     if (t < 32) tile_fetch(h, m, src, 0, 2, lists, h.rows, bar);
     tile_hsml(h, m, g);
     tile_fill(h, fill);
-    if (!bar_wait(bar, parity)) {
-        atomicOr(&sc->flags, FLAG_TIMEOUT);
-        bar_wait(bar, parity);
-        return false;
-    }
+    copies_arrive(bar, parity, 0, &failed, &sc->flags);
     parity ^= 1u;
     __syncthreads();
-    return true;
+    return failed == kNoneFailed;
 }
 
 // Pairs of a particle of such a tile: f(j, slot, x_j, v_j, h_j), slot -1 where
@@ -1060,12 +1053,14 @@ __global__ void k_copy_s1_to_s0(int n, State s1, State s0) {
     if (s0.hmm) s0.hmm[i] = s1.hmm[i];
 }
 
+// (FLAG_TIMEOUT stays until the state is set anew: what the passes keep from one
+// step to the next may be incomplete)
 __global__ void k_reset_stats(Scalars *sc) {
     sc->maxip = 0;
     sc->minip = 0x7fffffff;
     sc->sumip = 0ull;
     sc->noip = 0;
-    sc->flags = 0;
+    sc->flags &= FLAG_TIMEOUT;
 }
 
 inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }

@@ -73,9 +73,11 @@ __device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned b
                  "l"(src), "r"(bytes), "r"(smem_addr(bar))
                  : "memory");
 }
-// Waits for the barrier's phase; gives up after a bounded number of tries.
+// Waits for the barrier's phase; gives up after a bounded number of tries, which
+// take 4 us each: about a second.
+constexpr int kWaitTries = 1 << 18;
 __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parity) {
-    for (int k = 0; k < (1 << 20); ++k) {
+    for (int k = 0; k < kWaitTries; ++k) {
         unsigned ok;
         asm volatile(
             "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
@@ -85,6 +87,29 @@ __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parit
         if (ok) return true;
     }
     return false;
+}
+// The wait for a tile's copies.  Where they do not arrive, the step reports it,
+// and the thread gives them as long again to end, marks its block and goes on
+// without pairs, so that the block's barriers still meet.  The block leaves as a
+// whole where it next looks at the mark, behind a barrier: the mark is the least
+// `at` of a wait that failed, so that a thread that looks late does not see one
+// of a wait that others have reached since.
+constexpr int kNoneFailed = 0x7fffffff;
+__device__ __noinline__ void copies_failed(unsigned long long *bar, unsigned parity, int at, int *failed, int *flags) {
+    atomicOr(flags, FLAG_TIMEOUT);
+    bar_wait(bar, parity);
+    atomicMin(failed, at);
+}
+__device__ __forceinline__ bool copies_arrive(unsigned long long *bar, unsigned parity, int at, int *failed, int *flags) {
+    if (bar_wait(bar, parity)) return true;
+    copies_failed(bar, parity, at, failed, flags);
+    return false;
+}
+// A block's mark at its start: where copies of an earlier pass did not arrive its
+// records may be missing, and there is nothing to do.  Asked by one thread, since
+// other blocks may set the flag meanwhile.
+__device__ __forceinline__ int failed_before(const Scalars *sc) {
+    return (*(const volatile int *)&sc->flags & FLAG_TIMEOUT) ? -1 : kNoneFailed;
 }
 
 // Shared memory of a tile: records of 16 bytes per particle by array (xy and
