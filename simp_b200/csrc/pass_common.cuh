@@ -156,17 +156,28 @@ struct Grad<T, SIMP_SKF_WENDLAND_C6> {
     }
 };
 
+// What a launch knows of its basins' hsml: one value in each of them; not so (a
+// single basin, or one whose hsml evolves); or so in some of a batch's, each of
+// which then gets the very operations of the first form, so that its sums do not
+// depend on which basins it is batched with.  (The last form selects operand by
+// operand: a branch would part the chains of a particle's two candidates.  As a
+// form for single basins too it costs the reference's switches at 90,007
+// particles 122 -> 127 us per step.)
+enum Hsml : int { HSML_ONE, HSML_VARIED, HSML_EITHER };
+
 // The pair's gradient factor without the constant part of a particle's sums,
 // from s = r^2.
-template <class T, int SKF, bool UNIFORM>
+template <class T, int SKF, int HS>
 struct PairGrad {
-    T hi, k;   // hsml_i; uniform: (qscale / hsml)^2
+    T hi, k;   // hsml_i; where hsml is one value: (qscale / hsml)^2
     T inv_hi;  // (generic kernels)
-    __device__ __forceinline__ void init(const Phys &P, T h) {
+    bool one;
+    __device__ __forceinline__ void init(const Phys &P, const Inst &I, T h) {
         hi = h;
+        one = HS == HSML_ONE || (HS == HSML_EITHER && I.hmin == I.hmax);
         if (SKF == 0) {
             inv_hi = T(1) / h;
-        } else if (UNIFORM) {
+        } else if (HS != HSML_VARIED) {
             const T r = (T)Grad<T, SKF ? SKF : SIMP_SKF_CUBIC>::qscale / h;
             k = r * r;
         }
@@ -174,19 +185,20 @@ struct PairGrad {
     // factor common to all pairs of the particle
     __device__ __forceinline__ double common() const {
         if (SKF == 0) return 1.0;
-        if (!UNIFORM) return Grad<T, SKF ? SKF : SIMP_SKF_CUBIC>::factor;
+        const double f = Grad<T, SKF ? SKF : SIMP_SKF_CUBIC>::factor;
+        if (HS == HSML_VARIED || !one) return f;
         const double ih = 1.0 / (double)hi;
-        return Grad<T, SKF ? SKF : SIMP_SKF_CUBIC>::factor * ((ih * ih) * (ih * ih));
+        return f * ((ih * ih) * (ih * ih));
     }
     __device__ __forceinline__ T operator()(const Phys &P, T s, T hj) const {
         if constexpr (SKF == 0) {
             const T rs = rsq(s), r = s * rs;
-            const T inv_h = (UNIFORM || hj == hi) ? inv_hi : T(2) / (hi + hj);
+            const T inv_h = (HS == HSML_ONE || hj == hi) ? inv_hi : T(2) / (hi + hj);
             const T shh = (T)P.scale_h * inv_h;
             T w = 0, gq;
             kernel_wg<T, false, 0>(P.skf, r * shh, shh, inv_h, &w, &gq);
             return gq * shh * rs;
-        } else if constexpr (UNIFORM) {
+        } else if constexpr (HS == HSML_ONE) {
             T q, h;
             root_pair(s * k, q, h);
             return Grad<T, SKF>::shape(q, h);
@@ -194,9 +206,10 @@ struct PairGrad {
             constexpr T c = (T)Grad<T, SKF>::qscale;
             const T H = T(0.5) * (hi + hj), H2 = H * H;
             T R, n;
-            root_pair(s * H2, R, n);
+            const bool o = HS == HSML_EITHER && one;
+            root_pair(s * (o ? k : H2), R, n);
             const T q = T(2) * s * n, ih2 = T(2) * q * n;   // r / H, 1 / H^2
-            return (ih2 * ih2) * Grad<T, SKF>::shape(c * q, (H2 / c) * n);
+            return (o ? T(1) : ih2 * ih2) * Grad<T, SKF>::shape(o ? R : c * q, (o ? T(1) : H2 / c) * n);
         }
     }
 };

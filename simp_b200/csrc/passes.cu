@@ -259,8 +259,9 @@ __device__ __forceinline__ bool lists_valid(const Inst &I, bool second) {
 // issue slots 31% and 51%).  Two candidates at a time put six such reads in
 // flight.  262,144 particles, FP64: 79 -> 40 us per pass against gathers from
 // global memory; mixed at 1,048,576: 237 -> 132 us.
-template <class T, int SKF, bool UNIFORM, int BLOCKS>
+template <class T, int SKF, int HS, int BLOCKS>
 __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_constant__ KinArgs a) {
+    constexpr bool UNIFORM = HS == HSML_ONE;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Halo h;
     __shared__ __align__(8) unsigned long long bar;
@@ -326,8 +327,8 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
             prefetch_l1(&s.mm[i]);
         }
         const T hiT = Rec<T>::own_h(s, i);
-        PairGrad<T, SKF, UNIFORM> grad;
-        grad.init(P, hiT);
+        PairGrad<T, SKF, HS> grad;
+        grad.init(P, I, hiT);
         const bool rule = rule_on(I);
         KinSums<T> ks;     // -div and the velocity gradient, negated
         auto terms = [&](bool in, T dx, T dy, double2 v, T mj, T mrj, T hj) {
@@ -424,8 +425,9 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
 // copies and of that epilogue (issue slots 29%, L1 50%).  262,144 particles,
 // FP64: 71 -> 44 us per pass against gathers from global memory; mixed at
 // 1,048,576: 192 -> 147 us.
-template <class T, int SKF, bool UNIFORM, int BLOCKS>
+template <class T, int SKF, int HS, int BLOCKS>
 __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant__ StressArgs a) {
+    constexpr bool UNIFORM = HS == HSML_ONE;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Halo h;
     __shared__ HaloWalls hw;
@@ -473,8 +475,8 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         double hi = s.hs[i];
         const T hiT = Rec<T>::own_h(s, i);
         StressSums<T> ss;
-        PairGrad<T, SKF, UNIFORM> grad;
-        grad.init(P, hiT);
+        PairGrad<T, SKF, HS> grad;
+        grad.init(P, I, hiT);
         int npairs = 0;
         auto terms = [&](bool in, T dx, T dy, T mj, T t11, T t12, T t22, T hj) {
             const T g = grad(P, fma(dx, dx, dy * dy), hj);
@@ -1154,18 +1156,20 @@ PairList pair_list(simp_ctx *c) {
 }
 
 // (calls f with every kernel of a form)
+template <class T, int SKF, int HS, class F>
+void each_pass(F &&f) {
+    f(k_kinematic<T, SKF, HS, 4>);
+    f(k_stress<T, SKF, HS, 4>);
+    if (sizeof(T) == sizeof(float)) {
+        f(k_kinematic<float, SKF, HS, 5>);
+        f(k_stress<float, SKF, HS, 5>);
+    }
+}
 template <class T, int SKF, class F>
 void each_kernel(F &&f) {
-    f(k_kinematic<T, SKF, true, 4>);
-    f(k_kinematic<T, SKF, false, 4>);
-    f(k_stress<T, SKF, true, 4>);
-    f(k_stress<T, SKF, false, 4>);
-    if (sizeof(T) == sizeof(float)) {
-        f(k_kinematic<float, SKF, true, 5>);
-        f(k_kinematic<float, SKF, false, 5>);
-        f(k_stress<float, SKF, true, 5>);
-        f(k_stress<float, SKF, false, 5>);
-    }
+    each_pass<T, SKF, HSML_ONE>(f);
+    each_pass<T, SKF, HSML_VARIED>(f);
+    if (SKF != 0) each_pass<T, SKF, SKF ? HSML_EITHER : HSML_VARIED>(f);   // (the generic kernels' arithmetic is one)
     f(k_regularize);
     f(k_density_rate);
 }
@@ -1197,24 +1201,25 @@ void launch_pass(simp_ctx *c, void (*k)(P...), int grid, int block, size_t smem,
     cudaLaunchKernelEx(&cfg, k, args...);   // (an error is found by the caller's next check)
 }
 
-template <class T, int SKF, int BLOCKS, class A>
+template <class T, int SKF, int HS, int BLOCKS, class A>
 void launch_tiles(simp_ctx *c, const A &a) {
     const int g = c->nchunks;
-    if constexpr (std::is_same<A, KinArgs>::value) {
-        const size_t sm = tile_smem_bytes(a.cap, 3, c->uniform);
-        if (c->uniform) launch_pass(c, k_kinematic<T, SKF, true, BLOCKS>, g, kTile, sm, a);
-        else launch_pass(c, k_kinematic<T, SKF, false, BLOCKS>, g, kTile, sm, a);
-    } else {
-        const size_t sm = tile_smem_bytes(a.cap, Rec<T>::stress_arrays, c->uniform);
-        if (c->uniform) launch_pass(c, k_stress<T, SKF, true, BLOCKS>, g, kTile, sm, a);
-        else launch_pass(c, k_stress<T, SKF, false, BLOCKS>, g, kTile, sm, a);
-    }
+    if constexpr (std::is_same<A, KinArgs>::value)
+        launch_pass(c, k_kinematic<T, SKF, HS, BLOCKS>, g, kTile, tile_smem_bytes(a.cap, 3, c->uniform), a);
+    else
+        launch_pass(c, k_stress<T, SKF, HS, BLOCKS>, g, kTile, tile_smem_bytes(a.cap, Rec<T>::stress_arrays, c->uniform), a);
+}
+template <class T, int SKF, int BLOCKS, class A>
+void launch_hsml_form(simp_ctx *c, const A &a) {
+    if (c->uniform) launch_tiles<T, SKF, HSML_ONE, BLOCKS>(c, a);
+    else if (c->max_inst == 1 || SKF == 0) launch_tiles<T, SKF, HSML_VARIED, BLOCKS>(c, a);
+    else launch_tiles<T, SKF, SKF ? HSML_EITHER : HSML_VARIED, BLOCKS>(c, a);
 }
 template <int SKF, class A>
 void launch_kernel_form(simp_ctx *c, const A &a) {
-    if (c->prm.precision != SIMP_PREC_MIXED) launch_tiles<double, SKF, 4>(c, a);
-    else if (c->nchunks <= kResidentTiles) launch_tiles<float, SKF, 4>(c, a);
-    else launch_tiles<float, SKF, 5>(c, a);
+    if (c->prm.precision != SIMP_PREC_MIXED) launch_hsml_form<double, SKF, 4>(c, a);
+    else if (c->nchunks <= kResidentTiles) launch_hsml_form<float, SKF, 4>(c, a);
+    else launch_hsml_form<float, SKF, 5>(c, a);
 }
 template <class A>
 void launch_form(simp_ctx *c, const A &a) {
