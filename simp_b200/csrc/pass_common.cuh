@@ -246,6 +246,7 @@ struct KinSums {
 template <class T>
 struct StressSums {
     Sum<T> sx, sy, tx, ty;
+    int pairs = 0;
     // (nothing is added where `in` is false)
     __device__ __forceinline__ void add(bool in, T dwx, T dwy, T mj, T t11, T t12, T t22) {
         const T fx = fma(t11, dwx, t12 * dwy), fy = fma(t12, dwx, t22 * dwy);

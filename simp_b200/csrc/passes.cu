@@ -140,12 +140,6 @@ struct Rec<double> {
         mor = q.y;
         h = UNIFORM ? 0.0 : t.hs[sl];
     }
-    static __device__ __forceinline__ void kin_global(const State &s, int j, double &m, double &mor, double &h) {
-        const double2 q = s.mm[j];
-        m = q.x;
-        mor = q.y;
-        h = s.hs[j];
-    }
     template <bool UNIFORM>
     static __device__ __forceinline__ void stress(const TileMem &t, int sl, double &m, double &t11, double &t12,
                                                   double &t22, double &h) {
@@ -156,15 +150,6 @@ struct Rec<double> {
         t12 = a.y;
         t22 = b.x;
         h = UNIFORM ? 0.0 : t.hs[sl];
-    }
-    static __device__ __forceinline__ void stress_global(const State &s, const TauRec &r, int j, double &m, double &t11,
-                                                         double &t12, double &t22, double &h) {
-        const double2 a = r.ta[j], b = r.tb[j];
-        m = b.y;
-        t11 = a.x;
-        t12 = a.y;
-        t22 = b.x;
-        h = s.hs[j];
     }
     static constexpr double band = kBand;
 };
@@ -180,12 +165,6 @@ struct Rec<float> {
         m = q.y;
         mor = q.z;
     }
-    static __device__ __forceinline__ void kin_global(const State &s, int j, float &m, float &mor, float &h) {
-        const float4 q = s.hmm[j];
-        h = q.x;
-        m = q.y;
-        mor = q.z;
-    }
     template <bool UNIFORM>
     static __device__ __forceinline__ void stress(const TileMem &t, int sl, float &m, float &t11, float &t12,
                                                   float &t22, float &h) {
@@ -195,15 +174,6 @@ struct Rec<float> {
         t12 = q.y;
         t22 = q.z;
         h = UNIFORM ? 0.0f : (float)t.hs[sl];
-    }
-    static __device__ __forceinline__ void stress_global(const State &s, const TauRec &r, int j, float &m, float &t11,
-                                                         float &t12, float &t22, float &h) {
-        const float4 q = r.tq[j];
-        m = q.w;
-        t11 = q.x;
-        t12 = q.y;
-        t22 = q.z;
-        h = s.hsf[j];
     }
     // (differences and hsml rounded to FP32: within 2^-20 of the exact ratio)
     static constexpr float band = 0x1p-18f;
@@ -251,6 +221,37 @@ __device__ __forceinline__ bool lists_valid(const Inst &I, bool second) {
     if (!I.list_ok && !second) return false;
     const double room = 0.5 * I.delta * (1.0 - 1e-9) - (I.list_ok ? I.list_d : 0.0);
     return room >= 0.0 && (!second || bitsd(I.half2_bits) <= room * room);
+}
+
+// The sums of a particle without a list, from its stencil.  A call in FP64,
+// inlined in the mixed form, whose five blocks per SM leave no registers for one
+// (us per step, called and inlined: FP64 262,144 particles 157 and 160, 1,048,576
+// 568 and 582; mixed 262,144 178 and 158, 1,048,576 613 and 556).
+template <class T, int SKF, int HS>
+__device__ __forceinline__ KinSums<T> kin_stencil(const KinArgs &a, const Inst &I, const Halo &h, int i) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr bool UNIFORM = HS == HSML_ONE;
+    const State &s = a.s;
+    const void *src[3] = {s.xy, s.vxy, Rec<T>::kin_src(s)};
+    const Around w(h, tile_mem(smem, a.cap, 3, UNIFORM), src, s);
+    const double2 xy = s.xy[i], vi = s.vxy[i];
+    PairGrad<T, SKF, HS> grad;
+    grad.init(a.P, I, Rec<T>::own_h(s, i));
+    KinSums<T> ks;
+    stencil_pairs<UNIFORM>(w, s, I, a.cell_start, i, a.cell[i], [&](int q, int) {
+        const double2 x = reinterpret_cast<const double2 *>(w.m.rec[0])[q];
+        const double2 v = reinterpret_cast<const double2 *>(w.m.rec[1])[q];
+        T mj, mrj, hj;
+        Rec<T>::template kin<UNIFORM>(w.m, q, mj, mrj, hj);
+        const T dx = (T)(xy.x - x.x), dy = (T)(xy.y - x.y);
+        const T g = grad(a.P, fma(dx, dx, dy * dy), hj);
+        ks.add(true, g * dx, g * dy, (T)(vi.x - v.x), (T)(vi.y - v.y), mj, mrj);
+    });
+    return ks;
+}
+template <class T, int SKF, int HS>
+__device__ __noinline__ KinSums<T> kin_stencil_call(const KinArgs &a, const Inst &I, const Halo &h, int i) {
+    return kin_stencil<T, SKF, HS>(a, I, h, i);
 }
 
 // Kinematic pass over tiles.  Bound by shared memory and latency: a block waits
@@ -336,7 +337,6 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
             ks.add(in, g * dx, g * dy, (T)(vi.x - v.x), (T)(vi.y - v.y), mj, mrj);
         };
         int cnt = 0;       // candidates in the particle's list
-        bool tile = fits;
         if (fits) {
             if (!UNIFORM) tile_hsml(h, m, s);
             if (!build && live) cnt = a.pl.count[i];
@@ -351,22 +351,16 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncthreads();
                 if (failed <= 2 * p0) return;
-                tile = rows_max <= kListRows;
-                if (t == 0) {
-                    h.rows = tile ? rows_max : 0;
-                    if (!tile) h.kind = HALO_GLOBAL;
-                }
-                if (tile) {
-                    if (t < 32) tile_fetch(h, m, src, 1, 3, lists, 0, &bar);
-                    if (live) a.pl.count[i] = cnt;
-                    if (!copies_arrive(&bar, parity, 2 * p0 + 1, &failed, &a.sc->flags)) cnt = 0;
-                    parity ^= 1u;
-                }
+                if (t == 0) h.rows = min(rows_max, kListRows);
+                if (t < 32) tile_fetch(h, m, src, 1, 3, lists, 0, &bar);
+                if (live) a.pl.count[i] = cnt;
+                if (!copies_arrive(&bar, parity, 2 * p0 + 1, &failed, &a.sc->flags)) cnt = 0;
+                parity ^= 1u;
                 __syncthreads();
             }
         }
         if (build && t == 0) halos[(p0 - ch.p0) / kPartMin] = h;
-        if (tile) {
+        if (fits && cnt <= kListRows) {
             const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
             const double2 *vs = reinterpret_cast<const double2 *>(m.rec[1]);
             const T mh2_u = hiT * hiT;
@@ -398,13 +392,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
                 terms(in1 != 0, dx1, dy1, v1, m1, r1, h1);
             }
         } else if (live) {
-            // no tile: the neighbours from global memory
-            global_pairs(s, I, a.cell_start, i, a.cell[i], [&](int j) {
-                const double2 q = s.xy[j], v = s.vxy[j];
-                T mj, mrj, hj;
-                Rec<T>::kin_global(s, j, mj, mrj, hj);
-                terms(true, (T)(xy.x - q.x), (T)(xy.y - q.y), v, mj, mrj, hj);
-            });
+            ks = sizeof(T) == sizeof(double) ? kin_stencil_call<T, SKF, HS>(a, I, h, i) : kin_stencil<T, SKF, HS>(a, I, h, i);
         }
         if (live) {
             const double c = -grad.common();
@@ -417,6 +405,35 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
             __syncthreads();
         }
     }
+}
+
+// The stress pass's, and how many pairs it has.
+template <class T, int SKF, int HS>
+__device__ __forceinline__ StressSums<T> stress_stencil(const StressArgs &a, const Inst &I, const Halo &h, int i) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr bool UNIFORM = HS == HSML_ONE;
+    const State &s = a.rhs;
+    const void *src[3] = {s.xy, a.rec.tq ? (const void *)a.rec.tq : (const void *)a.rec.ta, a.rec.tb};
+    const Around w(h, tile_mem(smem, a.cap, Rec<T>::stress_arrays, UNIFORM), src, s);
+    const double2 xy = s.xy[i];
+    PairGrad<T, SKF, HS> grad;
+    grad.init(a.P, I, Rec<T>::own_h(s, i));
+    StressSums<T> ss;
+    stencil_pairs<UNIFORM>(w, s, I, a.cell_start, i, a.cell[i], [&](int q, int) {
+        const double2 x = reinterpret_cast<const double2 *>(w.m.rec[0])[q];
+        T mj, t11, t12, t22, hj;
+        Rec<T>::template stress<UNIFORM>(w.m, q, mj, t11, t12, t22, hj);
+        const T dx = (T)(xy.x - x.x), dy = (T)(xy.y - x.y);
+        const T g = grad(a.P, fma(dx, dx, dy * dy), hj);
+        ss.add(true, g * dx, g * dy, mj, t11, t12, t22);
+        ++ss.pairs;
+    });
+    return ss;
+}
+
+template <class T, int SKF, int HS>
+__device__ __noinline__ StressSums<T> stress_stencil_call(const StressArgs &a, const Inst &I, const Halo &h, int i) {
+    return stress_stencil<T, SKF, HS>(a, I, h, i);
 }
 
 // Stress pass over the same tiles, then the epilogue, whose twenty own values
@@ -463,8 +480,8 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         __syncthreads();
         if (failed < 2 * p0) return;
         const bool tile = h.kind == HALO_TILE;
+        const void *src[3] = {s.xy, a.rec.tq ? (const void *)a.rec.tq : (const void *)a.rec.ta, a.rec.tb};
         if (tile && t < 32) {
-            const void *src[3] = {s.xy, a.rec.tq ? (const void *)a.rec.tq : (const void *)a.rec.ta, a.rec.tb};
             tile_fetch(h, m, src, 0, arrays, a.pl.slot + (size_t)blockIdx.x * kListRows * kTile, h.rows, &bar);
         }
         const bool live = t < h.size;
@@ -477,19 +494,21 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         StressSums<T> ss;
         PairGrad<T, SKF, HS> grad;
         grad.init(P, I, hiT);
-        int npairs = 0;
         auto terms = [&](bool in, T dx, T dy, T mj, T t11, T t12, T t22, T hj) {
             const T g = grad(P, fma(dx, dx, dy * dy), hj);
             ss.add(in, g * dx, g * dy, mj, t11, t12, t22);
-            npairs += in;
+            ss.pairs += in;
         };
+        int cnt = live && h.kind != HALO_NONE ? kListRows + 1 : 0;   // candidates in its list
         if (tile) {
             if (!UNIFORM) tile_hsml(h, m, s);
-            int cnt = live ? a.pl.count[i] : 0;
-            const bool rule = rule_on(I);
+            if (live) cnt = a.pl.count[i];
             if (!copies_arrive(&bar, parity, 2 * p0, &failed, &a.sc->flags)) cnt = 0;
             parity ^= 1u;
             if (!UNIFORM) __syncthreads();
+        }
+        if (cnt <= kListRows) {
+            const bool rule = rule_on(I);
             const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
             const ushort2 *col = reinterpret_cast<const ushort2 *>(m.list) + (i - ch.p0);
             const T mh2_u = hiT * hiT;
@@ -516,13 +535,9 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
                 terms(in0 != 0, dx0, dy0, m0, a0, b0, c0, h0);
                 terms(in1 != 0, dx1, dy1, m1, a1, b1, c1, h1);
             }
-        } else if (h.kind == HALO_GLOBAL && live) {
-            global_pairs(s, I, a.cell_start, i, a.cell[i], [&](int j) {
-                const double2 q = s.xy[j];
-                T mj, t11, t12, t22, hj;
-                Rec<T>::stress_global(s, a.rec, j, mj, t11, t12, t22, hj);
-                terms(true, (T)(xy.x - q.x), (T)(xy.y - q.y), mj, t11, t12, t22, hj);
-            });
+        } else {
+            ss = sizeof(T) == sizeof(double) ? stress_stencil_call<T, SKF, HS>(a, I, h, i)
+                                             : stress_stencil<T, SKF, HS>(a, I, h, i);
         }
         // (a retired basin's particles are not written any more: their state
         // stays as it was until the batch's next compaction drops them)
@@ -556,7 +571,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         }
         if (!Walls::kKeep) pair_sums();
         stress_finish(a, i, live && !(I.flags & FLAG_RETIRED), ch.q, I, wl, xy.x, xy.y, hi, S[0], S[1], S[2], S[3],
-                      npairs);
+                      ss.pairs);
         p0 += h.size;
         if (p0 < ch.p1) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -653,15 +668,20 @@ template <class F>
 __device__ __forceinline__ void aux_pairs(const Halo &h, const TileMem &m, const State &g, const double2 *vxy,
                                           const Inst &I, const int *cell_start, const int *cell, const int *count,
                                           int i, int column, F &&f) {
-    if (h.kind == HALO_GLOBAL) {
-        global_pairs(g, I, cell_start, i, cell[i], [&](int j) { f(j, -1, g.xy[j], vxy[j], g.hs[j]); });
+    const int cnt = h.kind == HALO_TILE ? count[i] : kListRows + 1;
+    if (h.kind != HALO_NONE && cnt > kListRows) {
+        const void *src[3] = {g.xy, vxy, nullptr};
+        const Around w(h, m, src, g);
+        stencil_pairs<false>(w, g, I, cell_start, i, cell[i], [&](int q, int j) {
+            f(j, w.h ? q : -1, reinterpret_cast<const double2 *>(w.m.rec[0])[q],
+              reinterpret_cast<const double2 *>(w.m.rec[1])[q], w.m.hs[q]);
+        });
     } else if (h.kind == HALO_TILE) {
         const double2 p = g.xy[i];
         const double hi = g.hs[i];
         const bool rule = rule_on(I);
         const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
         const double2 *vs = reinterpret_cast<const double2 *>(m.rec[1]);
-        const int cnt = count[i];
         for (int k = 0; k < cnt; ++k) {
             const int q = m.list[list_at(k, column)];
             if (!SIMP_IN_RANGE(q, 0, h.off[h.nseg], SITE_TILE)) continue;

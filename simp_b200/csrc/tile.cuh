@@ -17,12 +17,15 @@
 // Candidates are in increasing index order, so the sums depend neither on the
 // tile shape nor on when a list was built.
 //
-// A tile whose halo exceeds the shared-memory capacity (a sparse cell row next
-// to full ones) is cut in halves down to kPartMin particles, taken one after
-// another; one that still does not fit, whose stencil radius exceeds
-// kMaxRadius or which has a particle of more than kListRows candidates reads
-// its neighbours from global memory with the same arithmetic in the same
-// order.
+// A particle of more than kListRows candidates finds its pairs in the halo's cell
+// stencil, whatever the others of its tile do (65,536 particles, FP64, with 48
+// neighbours each: 221 us per step, 341 when such a particle sent its tile to
+// global memory and 254 with lists per particle in global memory).  A tile whose
+// halo exceeds the shared-memory capacity (a sparse cell row next to full ones) is
+// cut in halves down to kPartMin particles, taken one after another; one that
+// still does not fit or whose stencil radius exceeds kMaxRadius reads its
+// neighbours from global memory.  The arithmetic and its order are the same
+// everywhere.
 #pragma once
 
 #include "pass_common.cuh"
@@ -32,14 +35,13 @@ namespace pass {
 
 constexpr int kMaxRadius = 2;
 constexpr int kMaxSeg = 2 * kMaxRadius + 1;
-constexpr int kSlotPad = 40;               // slots a candidate batch may read past the halo
 
 // The halo of a tile or part of one, one record per part.
 enum : int { HALO_NONE = 0, HALO_TILE = 1, HALO_GLOBAL = 2 };
 struct Halo {
     int kind, nseg;
     int walls;                 // cells around its own that hold every wall pair, 0: none
-    int rows;                  // longest list of one of its particles
+    int rows;                  // longest list of one of its particles, kListRows at most
     int lo[kMaxSeg];           // first particle of each range
     int off[kMaxSeg + 1];      // its first slot, and the total
     int size;                  // particles in this part of the tile
@@ -280,27 +282,44 @@ __device__ __forceinline__ void reload(double &v, const double *p) {
 }
 __device__ __forceinline__ bool rule_on(const Inst &I) { return I.hmax >= I.bs * (1.0 - 1e-6); }
 
-// Pairs of particle i from global memory over its cell stencil: f(j).
-template <class F>
-__device__ __forceinline__ void global_pairs(const State &s, const Inst &I, const int *cell_start, int i, int ci,
-                                             F &&f) {
+// Where a particle without a list finds its candidates: its tile's halo, or for
+// a tile without one (h null) global memory, whose arrays then stand in `m`.
+struct Around {
+    const Halo *h;
+    TileMem m;
+    __device__ __forceinline__ Around(const Halo &halo, const TileMem &tile, const void *const (&src)[3], const State &s)
+        : h(halo.kind == HALO_TILE ? &halo : nullptr), m(tile) {
+        if (h) return;
+        for (int a = 0; a < 3; ++a) m.rec[a] = (unsigned char *)src[a];
+        m.hs = (double *)s.hs;
+    }
+};
+
+// Pairs of particle i over its cell stencil, in increasing index order: f(q, j),
+// q its place in `w`.  The halo covers the stencil it was made with, which holds
+// every pair as long as lists built then would.
+template <bool UNIFORM, class F>
+__device__ __forceinline__ void stencil_pairs(const Around &w, const State &s, const Inst &I, const int *cell_start,
+                                              int i, int ci, F &&f) {
     const double2 p = s.xy[i];
     const double hi = s.hs[i];
     const bool rule = rule_on(I);
     const int2 at = cell_at(I, ci);
-    const int R = stencil_radius(I.hmax, inst_disp(I), inst_grid(I, cell_start), 0.0);
+    const int R = w.h ? w.h->nseg / 2 : stencil_radius(I.hmax, inst_disp(I), inst_grid(I, cell_start), 0.0);
+    const double2 *xs = reinterpret_cast<const double2 *>(w.m.rec[0]);
     for (int d = 0; d < 2 * R + 1; ++d) {
         int j0, j1;
         stencil_range(I, cell_start, at, R, d, j0, j1);
+        const int shift = w.h && j0 < j1 ? slot_of(*w.h, j0) - j0 : 0;
 #pragma unroll 4
         for (int j = j0; j < j1; ++j) {
-            const double2 q = s.xy[j];
-            const double dx = p.x - q.x, dy = p.y - q.y, mh = 0.5 * (hi + s.hs[j]);
+            const double2 q = xs[j + shift];
+            const double dx = p.x - q.x, dy = p.y - q.y, mh = UNIFORM ? hi : 0.5 * (hi + w.m.hs[j + shift]);
             const double d2 = fma(dx, dx, dy * dy);
             if (d2 > mh * mh * (1.0 + kBand) || j == i) continue;
             if (!(d2 < mh * mh * (1.0 - kBand)) || rule)
                 if (!exact_pair(s, I, rule, i, j)) continue;
-            f(j);
+            f(j + shift, j);
         }
     }
 }
