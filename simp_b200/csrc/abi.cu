@@ -159,10 +159,6 @@ __global__ void k_count_walls(int nb, const int *__restrict__ key, int *__restri
     if (k < nb) atomicAdd(&cnt[key[k]], 1);
 }
 
-__global__ void k_grow_xabs(Scalars *sc, double xa) {
-    atomicMax(&sc->xabs_bits, (unsigned long long)__double_as_longlong(xa));
-}
-
 // set_state of a state that continues the resident basin (the same
 // particles in the same caller order, the same hsml): the values go into
 // the particles' current places in cell order, so the sort and the cell
@@ -255,7 +251,7 @@ __global__ void k_continue_finish(Scalars *sc, Inst *inst, double dt, double t, 
     inst[0].disp = fmax(inst[0].disp, sqrt(d2));
     inst[0].list_ok = 0;
     const unsigned long long bx = (unsigned long long)__double_as_longlong(xa);
-    if (bx > sc->xabs_bits) sc->xabs_bits = bx;
+    if (bx > inst[0].xabs_bits) inst[0].xabs_bits = bx;
 }
 
 Phys make_phys(const simp_params &p, double max_hsml) {
@@ -430,6 +426,7 @@ int layout(simp_ctx *c) {
         if (h.I.base >= 0) {   // already on the device: keep its evolving fields
             h.I.t = cur[q].t;
             h.I.disp = cur[q].disp;
+            h.I.xabs_bits = cur[q].xabs_bits;
             h.I.flags = cur[q].flags;
             h.I.hmin = cur[q].hmin;
             h.I.hmax = cur[q].hmax;
@@ -659,14 +656,14 @@ int add_instance(simp_ctx *c, int slot, const simp_forcing &f, const Extents &e,
     I.hmax = hmax;
     I.bs = 2.0 * hmin;
     I.disp = 0.0;
+    std::memcpy(&I.xabs_bits, &pxa, sizeof(double));
     I.delta = 0.4 * list_skin(c, hmax);
     I.flags = 0;
     // particle arrays at [off, off + n), staged by stage_instance
     cudaStream_t s = c->stream;
     const int off = c->n;
     k_init_new<<<nblk(n, kB), kB, 0, s>>>(n, off, ih.id_base, slot, c->id, c->pinst, c->s0, c->xyr, c->k0);
-    k_grow_xabs<<<1, 1, 0, s>>>(c->sc, pxa);
-    c->launches += 2;
+    c->launches += 1;
     SIMP_CUDA(c, cudaGetLastError());
     c->n += n;
     c->nb += nb;

@@ -139,16 +139,30 @@ __global__ void k_keys(int n, const double2 *__restrict__ xyr, const int *__rest
     atomicAdd(&cnt[k], 1);
 }
 
-// Instances due for a re-sort take their current positions as sort
-// positions; a basin flagged non-finite keeps its old (finite) ones.
-__global__ void k_refresh_sortpos(int n, const int *__restrict__ pinst, DueMask due, const Inst *__restrict__ inst,
+// Instances due for a re-sort take their current positions as sort positions and
+// the largest coordinate from them (k_reset_inst_disp has set it to 0); a basin
+// flagged non-finite keeps its old (finite) ones.  Whole warps.
+__global__ void k_refresh_sortpos(int n, const int *__restrict__ pinst, DueMask due, Inst *inst,
                                   const double2 *__restrict__ xy, double2 *__restrict__ xyr) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int q = pinst[i];
-    if (q < 0 || !((due.w[q >> 6] >> (q & 63)) & 1ull)) return;
-    if (inst_dead(inst[q].flags)) return;
-    xyr[i] = xy[i];
+    int q = i < n ? pinst[i] : -1;
+    if (q >= 0 && (!((due.w[q >> 6] >> (q & 63)) & 1ull) || inst_dead(inst[q].flags))) q = -1;
+    unsigned long long far = 0ull;
+    if (q >= 0) {
+        const double2 p = xy[i];
+        xyr[i] = p;
+        far = dbits(fmax(fabs(p.x), fabs(p.y)));
+    }
+    // one atomic per warp where it holds one basin, and none where the bound is
+    // there already
+    const int q0 = __reduce_max_sync(0xffffffffu, q);
+    if (__all_sync(0xffffffffu, q == q0 || q < 0)) {
+        const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(far >> 32));
+        const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(far >> 32) == hi ? (unsigned)far : 0u);
+        far = (unsigned long long)hi << 32 | lo;
+        q = (threadIdx.x & 31) == 0 ? q0 : -1;
+    }
+    if (q >= 0 && *(volatile unsigned long long *)&inst[q].xabs_bits < far) atomicMax(&inst[q].xabs_bits, far);
 }
 
 __global__ void k_reset_inst_disp(Inst *inst, int ninst, DueMask due) {
@@ -158,6 +172,7 @@ __global__ void k_reset_inst_disp(Inst *inst, int ninst, DueMask due) {
     inst[q].disp = 0.0;
     inst[q].list_ok = 0;   // (its particles take new places)
     inst[q].spares = 0;
+    if (!inst_dead(inst[q].flags)) inst[q].xabs_bits = 0ull;
 }
 
 __global__ void k_scatter(int n, const int *__restrict__ key, const int *__restrict__ start,
@@ -280,8 +295,8 @@ int rebuild(simp_ctx *c, const DueMask &due, int from) {
     for (const InstHost &h : c->insts)
         if (h.active) kept += h.n;
     if (n > 0) {
-        k_refresh_sortpos<<<nblk(n, B), B, 0, s>>>(n, c->pinst, due, c->inst_dev, c->s0.xy, c->xyr);
         k_reset_inst_disp<<<nblk(c->ninst, 128), 128, 0, s>>>(c->inst_dev, c->ninst, due);
+        k_refresh_sortpos<<<nblk(n, B), B, 0, s>>>(n, c->pinst, due, c->inst_dev, c->s0.xy, c->xyr);
         SIMP_CUDA(c, cudaMemsetAsync(c->cnt, 0, sizeof(int) * (size_t)nkeys, s));
         k_keys<<<nblk(n, B), B, 0, s>>>(n, c->xyr, c->pinst, c->inst_dev, c->total_cells, key, c->cnt);
         launch_scan_i32(c->cnt, c->cell_start, nkeys, c->scan_tmp, s);

@@ -77,6 +77,8 @@ struct Inst {
     int list_ok, spares;
     double delta, list_d;
     unsigned long long half2_bits, step2_bits;   // this step's max squared moves, S0 -> S1 and S0 -> S0'
+    unsigned long long xabs_bits;   // bound on any particle's |coordinate|, at the step's start: the largest at
+                                    // the last sort and the farthest moves since
 };
 
 __host__ __device__ __forceinline__ Grid inst_grid(const Inst &I, const int *cell_start) {
@@ -106,7 +108,6 @@ struct Scalars {
     double t;             // current_time
     double hmin, hmax;    // exact min / max of the current hsml
     double bs;            // reference bucket size 2 * hmin (nnps.f90:211)
-    unsigned long long xabs_bits;   // bound on any particle's |coordinate|, at the step's start
     unsigned long long acc_hmin, acc_hmax;  // accumulators of the next hsml
     unsigned long long acc_dt;              // VP time step min accumulator
     unsigned long long acc_dh;              // max growth of any hsml in this step

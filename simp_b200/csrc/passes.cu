@@ -82,7 +82,7 @@ __device__ __noinline__ int build_lists(const Halo &h, const TileMem &m, const K
     const int2 at = cell_at(I, a.cell[i]);
     const double2 xy = a.s.xy[i];
     const float xf = (float)xy.x, yf = (float)xy.y, hf = (float)a.s.hs[i];
-    const float margin = prefilter_margin(bitsd(a.sc->xabs_bits) + sqrt(bitsd(I.half2_bits)), I.hmin);
+    const float margin = prefilter_margin(bitsd(I.xabs_bits) + sqrt(bitsd(I.half2_bits)), I.hmin);
     const float grow = margin < 0.25f ? 1.0f + margin : INFINITY;
     const float delta = (float)I.delta;
     const int own = slot_of(h, i);
@@ -1013,10 +1013,8 @@ __global__ void __launch_bounds__(kFinishThreads) k_step_finish(Scalars *sc, Ins
                                                                 int sle) {
     pass_begin();
     __shared__ double dt, grown;
-    __shared__ unsigned long long farthest;
     if (threadIdx.x == 0) {
         grown = 0.0;
-        farthest = 0ull;
         if (tse != 0) {
             sc->dt = bitsd(sc->acc_dt);
             sc->acc_dt = dbits(INFINITY);
@@ -1052,12 +1050,10 @@ __global__ void __launch_bounds__(kFinishThreads) k_step_finish(Scalars *sc, Ins
         // displacement since the sort and largest coordinate: each step adds
         // the farthest any particle moved in it
         I.disp += step;
-        atomicMax(&farthest, I.step2_bits);
+        I.xabs_bits = dbits(bitsd(I.xabs_bits) + step);
         I.half2_bits = 0ull;
         I.step2_bits = 0ull;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) sc->xabs_bits = dbits(bitsd(sc->xabs_bits) + sqrt(bitsd(farthest)));
 }
 
 // The Euler step writes its result into S1 (S0 is read by the pair sums of
