@@ -1138,6 +1138,13 @@ double bytes_per_particle(const simp_params &p, bool single_basin) {
     return b;
 }
 
+// Device bytes of a context per basin it has room for, whatever their sizes: a
+// partial tile and the spare ones (chunk_capacity), with their lists and halos.
+double bytes_per_basin() {
+    constexpr double tile = kListRows * kTile * 2.0 + sizeof(Chunk) + (kHaloBytes + kHaloWallBytes) * (kTile / kPartMin);
+    return (1.0625 + spare_tiles(0)) * tile + sizeof(int4) + sizeof(Inst);
+}
+
 // Enqueues nsteps steps of every basin of the context on its stream without
 // waiting for them (profiling mode waits step by step).
 // A single basin's scheduled re-sort, replayed from a captured graph (one

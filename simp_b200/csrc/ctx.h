@@ -226,6 +226,7 @@ int passes_configure(simp_ctx *c);
 
 // abi.cu: device bytes per particle of capacity
 double bytes_per_particle(const simp_params &p, bool single_basin = false);
+double bytes_per_basin();
 
 // abi.cu: the step driver split for callers that overlap contexts
 int step_enqueue(simp_ctx *c, int nsteps);

@@ -44,6 +44,7 @@ struct simp_server {
     simp_ctx *main = nullptr;
     simp_ctx *spot = nullptr;       // FP64 replicas
     int maxn_main = 0, maxn_spot = 0, maxnb_main = 0, maxnb_spot = 0;
+    int slots_main = 0, slots_spot = 0;   // basins resident at once
     long long res_main = 0, res_spot = 0, resb_main = 0, resb_spot = 0;
     int spot_count = 0;
     std::vector<Request> reqs;
@@ -92,7 +93,7 @@ int admit(simp_server *s, double now) {
             continue;
         }
         if (r.arrival > now) break;
-        if ((int)s->resident.size() >= s->cfg.max_instances) break;
+        if ((int)s->resident.size() >= s->slots_main) break;
         if (s->res_main + r.n > s->maxn_main || s->resb_main + r.nb > s->maxnb_main) {
             if (s->resident.empty())   // could never fit
                 return fail(s, SIMP_ERR_MAXN, "a request exceeds the served batch's capacity");
@@ -106,7 +107,7 @@ int admit(simp_server *s, double now) {
         s->res_main += r.n;
         s->resb_main += r.nb;
         const int id = s->order[s->next];
-        if (s->spot && s->cfg.spot_every > 0 && id % s->cfg.spot_every == 0 && s->spot_count < kSpotSlots &&
+        if (s->spot && s->cfg.spot_every > 0 && id % s->cfg.spot_every == 0 && s->spot_count < s->slots_spot &&
             s->res_spot + r.n <= s->maxn_spot && s->resb_spot + r.nb <= s->maxnb_spot) {
             rc = simp_gpu_batch_add(s->spot, &r.f, r.n, r.x, r.vx, r.mass, r.rho, r.hsml, r.A, r.h, r.nb,
                                     r.xb, r.massb, &slot);
@@ -234,28 +235,37 @@ int32_t simp_server_create(const simp_params *params, const simp_server_config *
     s->cfg = *cfg;
     const double per = simp::bytes_per_particle(s->prm, cfg->max_instances == 1) + kBytesPerWall / kWallsPerParticleDiv;
     double budget = cfg->hbm_budget_bytes;
+    s->slots_main = cfg->max_instances;
     if (cfg->spot_every > 0) {
+        s->slots_spot = std::min(cfg->max_instances, kSpotSlots);
         simp_params p64 = s->prm;
         p64.precision = SIMP_PREC_FP64;
         const double spot_n = 2.0 * cfg->max_request_particles;
         s->maxn_spot = (int)spot_n;
         s->maxnb_spot = std::max(1, s->maxn_spot / kWallsPerParticleDiv);
         // (a batch of one slot is a single-basin context, with its read-back stage)
-        const bool single = std::min(cfg->max_instances, kSpotSlots) == 1;
+        const bool single = s->slots_spot == 1;
         budget -= spot_n * (simp::bytes_per_particle(p64, single) + kBytesPerWall / kWallsPerParticleDiv);
     }
+    // a budget that would hold the largest request but not the tiles of so many
+    // basins holds fewer of them at once
+    const double slot = simp::bytes_per_basin();
+    const double room = std::floor((budget - per * cfg->max_request_particles) / slot);
+    const double share = std::min(1.0, std::max(0.0, room / (s->slots_main + s->slots_spot)));
+    for (int *k : {&s->slots_main, &s->slots_spot}) *k = std::max((int)(*k * share), std::min(*k, 2));
+    budget -= slot * (s->slots_main + s->slots_spot);
     const double cap = std::floor(budget / per);
     if (cap < cfg->max_request_particles)
         return fail(s, SIMP_ERR_NOMEM, "the budget does not hold the largest request");
     s->maxn_main = (int)std::min(cap, 2.0e9);
     s->maxnb_main = std::max(1, s->maxn_main / kWallsPerParticleDiv);
     s->stats.capacity_particles = (double)s->maxn_main;
-    int rc = simp_gpu_create_batch(&s->prm, s->maxn_main, s->maxnb_main, cfg->max_instances, &s->main);
+    int rc = simp_gpu_create_batch(&s->prm, s->maxn_main, s->maxnb_main, s->slots_main, &s->main);
     if (rc != SIMP_OK) return fail(s, rc, s->main ? simp_gpu_last_error(s->main) : "create_batch failed");
     if (cfg->spot_every > 0) {
         simp_params p64 = s->prm;
         p64.precision = SIMP_PREC_FP64;
-        rc = simp_gpu_create_batch(&p64, s->maxn_spot, s->maxnb_spot, std::min(cfg->max_instances, kSpotSlots), &s->spot);
+        rc = simp_gpu_create_batch(&p64, s->maxn_spot, s->maxnb_spot, s->slots_spot, &s->spot);
         if (rc != SIMP_OK) return fail(s, rc, s->spot ? simp_gpu_last_error(s->spot) : "create_batch failed");
     }
     return SIMP_OK;
