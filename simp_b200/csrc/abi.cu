@@ -480,6 +480,7 @@ int layout(simp_ctx *c) {
     if (!src.empty()) {
         SIMP_CUDA(c, cudaMemcpyAsync(c->chunk_src, src.data(), sizeof(int4) * src.size(), cudaMemcpyHostToDevice, s));
         launch_chunks(c);
+        c->chunks_new = true;
     }
     std::vector<Inst> table(c->max_inst);
     for (int q = 0; q < c->max_inst; ++q) table[q] = c->insts[q].active ? c->insts[q].I : Inst{};

@@ -13,6 +13,8 @@
 // Sort: counting sort on cell keys (one radix digit of width log2(ncells)):
 // key histogram, exclusive prefix scan, scatter, then a per-cell sort by
 // original particle index so the order is deterministic.
+#include <cstring>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -327,7 +329,10 @@ int rebuild(simp_ctx *c, const DueMask &due, int from) {
         SIMP_CUDA(c, cudaMemsetAsync(c->cell_start, 0, sizeof(int) * (size_t)(nkeys + 1), s));
     }
     c->n = kept;
-    launch_split(c, due);
+    DueMask cut = due;
+    if (c->chunks_new) std::memset(&cut, 0xff, sizeof(cut));   // (the tiles of every basin)
+    launch_split(c, cut);
+    c->chunks_new = false;
     SIMP_CUDA(c, cudaGetLastError());
     c->rebuilds += 1;
     return SIMP_OK;

@@ -96,6 +96,7 @@ struct simp_ctx {
     unsigned char *halos = nullptr;   // simp::kHaloBytes per simp::kPartMin particles of a tile
     unsigned char *halo_walls = nullptr;   // likewise, simp::kHaloWallBytes each
     int nchunks = 0;
+    bool chunks_new = false;       // laid out anew, none cut yet
     bool uniform = false;          // every basin's hsml is one value, and stays it
     // diagnostics (epsilon_11.. sigma_22, zeta, eta, p)
     double *diag = nullptr;        // 9 * maxn
@@ -214,7 +215,7 @@ void launch_reset_stats(simp_ctx *c);
 // shared-memory limits.
 constexpr int kHaloBytes = 64;
 constexpr int kHaloWallBytes = 64;
-constexpr int kPartMin = 8;       // smallest part of a tile with its own halo
+constexpr int kPartMin = 8;       // smallest part of a whole tile with its own halo (tile.cuh, part_shift)
 __host__ __device__ inline int spare_tiles(int tiles) { return 3 + tiles / 16; }
 inline size_t chunk_capacity(int maxn, int max_inst) {
     const size_t tiles = (size_t)maxn / simp::kTile + (size_t)max_inst;   // (a partial tile per basin)

@@ -270,12 +270,13 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
     __shared__ unsigned moved2;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
+    const int shift = part_shift(ch);
     if (t == 0) bar_init(&bar);
     pass_begin();
     const Inst &I = a.inst[a.single ? 0 : ch.q];
     const State &s = a.s;
     const Phys &P = a.P;
-    Halo *halos = reinterpret_cast<Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    Halo *halos = reinterpret_cast<Halo *>(a.halos) + (size_t)blockIdx.x * kParts;
     const int first = t < kHaloWords ? halo_word(halos, t) : 0;   // (read along with the instance)
     if (t == kTile - 1) failed = failed_before(a.sc);
     if (ch.spare >= I.spares) return;   // (an unused spare tile)
@@ -301,15 +302,15 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
     for (int p0 = ch.p0; p0 < ch.p1;) {
         if (!build) {
             if (t < kHaloWords)
-                reinterpret_cast<int *>(&h)[t] = p0 == ch.p0 ? first : halo_word(&halos[(p0 - ch.p0) / kPartMin], t);
+                reinterpret_cast<int *>(&h)[t] = p0 == ch.p0 ? first : halo_word(&halos[(p0 - ch.p0) >> shift], t);
         } else if (t == 0) {
             // the largest part of the tile whose halo fits
             for (int S = kTile;; S >>= 1) {
                 make_halo(I, a.cell_start, a.bstart, a.cell, p0, min(p0 + S, ch.p1), a.cap,
                           sqrt((double)__uint_as_float(moved2)) * (1.0 + 1e-6), h,
-                          reinterpret_cast<HaloWalls *>(a.halo_walls) + (size_t)blockIdx.x * (kTile / kPartMin) +
-                              (p0 - ch.p0) / kPartMin);
-                if (h.kind == HALO_TILE || S <= kPartMin || h.nseg > kMaxSeg) break;
+                          reinterpret_cast<HaloWalls *>(a.halo_walls) + (size_t)blockIdx.x * kParts +
+                              ((p0 - ch.p0) >> shift));
+                if (h.kind == HALO_TILE || S <= (1 << shift) || h.nseg > kMaxSeg) break;
             }
             rows_max = 0;
         }
@@ -359,7 +360,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
                 __syncthreads();
             }
         }
-        if (build && t == 0) halos[(p0 - ch.p0) / kPartMin] = h;
+        if (build && t == 0) halos[(p0 - ch.p0) >> shift] = h;
         if (fits && cnt <= kListRows) {
             const double2 *xs = reinterpret_cast<const double2 *>(m.rec[0]);
             const double2 *vs = reinterpret_cast<const double2 *>(m.rec[1]);
@@ -452,11 +453,12 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
     __shared__ __align__(8) unsigned long long bar;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];   // (of the last sort)
+    const int shift = part_shift(ch);
     if (t == 0) bar_init(&bar);
     pass_begin();
     const Inst &I = a.inst[a.single ? 0 : ch.q];
-    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
-    const HaloWalls *walls = reinterpret_cast<const HaloWalls *>(a.halo_walls) + (size_t)blockIdx.x * (kTile / kPartMin);
+    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * kParts;
+    const HaloWalls *walls = reinterpret_cast<const HaloWalls *>(a.halo_walls) + (size_t)blockIdx.x * kParts;
     // (read along with the instance; the second warp reads the walls)
     const int first = t < kHaloWords ? halo_word(halos, t)
                       : BLOCKS == 4 && t >= 32 && t < 32 + kWallWords ? halo_word(walls, t - 32) : 0;
@@ -473,7 +475,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
     const TileMem m = tile_mem(smem, a.cap, arrays, UNIFORM);
     unsigned parity = 0u;
     for (int p0 = ch.p0; p0 < ch.p1;) {
-        const int part = (p0 - ch.p0) / kPartMin;
+        const int part = (p0 - ch.p0) >> shift;
         if (t < kHaloWords) reinterpret_cast<int *>(&h)[t] = part == 0 ? first : halo_word(&halos[part], t);
         if (BLOCKS == 4 && t >= 32 && t < 32 + kWallWords)
             reinterpret_cast<int *>(&hw)[t - 32] = part == 0 ? first : halo_word(&walls[part], t - 32);
@@ -702,13 +704,14 @@ __global__ void __launch_bounds__(kBlock) k_regularize(const __grid_constant__ R
     __shared__ __align__(8) unsigned long long bar;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];
+    const int shift = part_shift(ch);
     const State &s = a.s;
     const Phys &P = a.P;
     const size_t M = (size_t)a.maxn;
     const Inst &I = a.inst[ch.q];
     if (ch.spare >= I.spares) return;   // (an unused spare tile)
     const bool dead = inst_dead(I.flags);
-    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * kParts;
     const TileMem m = tile_mem(smem, a.cap, 2, false);
     double *rho_s = reinterpret_cast<double *>(smem + tile_smem_bytes(a.cap, 2, false));
     double *m_s = rho_s + a.cap, *v_s = m_s + a.cap;   // v: lv / rho^2 (Hernquist-Katz) or the sound speed (Monaghan)
@@ -718,7 +721,7 @@ __global__ void __launch_bounds__(kBlock) k_regularize(const __grid_constant__ R
     if (t == 0) bar_init(&bar);
     unsigned parity = 0u;
     for (int p0 = ch.p0; p0 < ch.p1;) {
-        if (!aux_tile(&halos[(p0 - ch.p0) / kPartMin], h, m, s, s.vxy, a.pl.slot + (size_t)blockIdx.x * kListRows * kTile, &bar,
+        if (!aux_tile(&halos[(p0 - ch.p0) >> shift], h, m, s, s.vxy, a.pl.slot + (size_t)blockIdx.x * kListRows * kTile, &bar,
                       parity, a.sc, [&](int j, int k) {
                           const double rho = s.rho[j];
                           rho_s[k] = rho;
@@ -952,8 +955,9 @@ __global__ void __launch_bounds__(kBlock) k_density_rate(const __grid_constant__
     __shared__ __align__(8) unsigned long long bar;
     const int t = threadIdx.x;
     const Chunk ch = a.chunks[blockIdx.x];
+    const int shift = part_shift(ch);
     if (ch.spare >= a.inst[ch.q].spares) return;   // (an unused spare tile)
-    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * (kTile / kPartMin);
+    const Halo *halos = reinterpret_cast<const Halo *>(a.halos) + (size_t)blockIdx.x * kParts;
     const TileMem m = tile_mem(smem, a.cap, 2, false);
     double *mj_s = reinterpret_cast<double *>(smem + tile_smem_bytes(a.cap, 2, false));
     double *w_s = mj_s + a.cap, *rho_s = w_s + a.cap;   // w: the summation's mass, or the time step's
@@ -961,7 +965,7 @@ __global__ void __launch_bounds__(kBlock) k_density_rate(const __grid_constant__
     if (t == 0) bar_init(&bar);
     unsigned parity = 0u;
     for (int p0 = ch.p0; p0 < ch.p1;) {
-        if (!aux_tile(&halos[(p0 - ch.p0) / kPartMin], h, m, a.g, a.v.vxy, a.pl.slot + (size_t)blockIdx.x * kListRows * kTile,
+        if (!aux_tile(&halos[(p0 - ch.p0) >> shift], h, m, a.g, a.v.vxy, a.pl.slot + (size_t)blockIdx.x * kListRows * kTile,
                       &bar, parity, a.sc, [&](int j, int k) {
                           mj_s[k] = a.mj[j];
                           if (w_src) w_s[k] = w_src[j];
@@ -1104,38 +1108,51 @@ __global__ void k_chunks(int nchunks, int nsrc, const int4 *__restrict__ src, in
 }
 
 // Cuts the tiles of the basins just sorted whose halo would not fit: a sparse
-// cell row's tile spans many cells of its full neighbour rows.  The parts go to
-// the basin's spare tiles, so that they run beside the others; a tile that
-// finds no room there stays whole and is worked off part by part.
-__global__ void k_split(int nchunks, int nsrc, const int4 *__restrict__ src, int size, Chunk *__restrict__ chunks,
-                        DueMask due, Inst *inst, const int *__restrict__ cell_start, const int *__restrict__ bstart,
-                        const int *__restrict__ cell, int cap) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// cell row's tile spans many cells of its full neighbour rows.  One warp per tile
+// cuts it from the front, each time the longest power of two of particles that
+// fits, down to single ones (65,536 particles, one of whose cell rows holds a few
+// of them: 57 us per step; 112 when parts of 8 were the shortest, one of which
+// then read its neighbours from global memory).  The parts go to the basin's
+// spare tiles, so that they run beside the others; what finds no room there stays
+// together and is worked off part by part.
+constexpr int kSplitWarps = 4;
+__global__ void __launch_bounds__(32 * kSplitWarps)
+    k_split(int nchunks, int nsrc, const int4 *__restrict__ src, int size, Chunk *__restrict__ chunks, DueMask due,
+            Inst *inst, const int *__restrict__ cell_start, const int *__restrict__ cell, int cap) {
+    static_assert(kTile == 128, "sizes tried");
+    __shared__ unsigned char starts[kSplitWarps][kTile];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.x * kSplitWarps + w;
     if (c >= nchunks) return;
     const int4 b = chunk_basin(c, nsrc, src);
     const int k = c - b.z, tiles = (b.y + size - 1) / size;
     if (k >= tiles || !((due.w[b.w >> 6] >> (b.w & 63)) & 1ull)) return;
     Inst &I = inst[b.w];
     const int p0 = b.x + k * size, p1 = min(p0 + size, b.x + b.y);
-    Chunk full{p0, p1, b.w, -1};
-    Halo h;
-    int S = size;
-    for (;; S >>= 1) {
-        make_halo(I, cell_start, bstart, cell, p0, min(p0 + S, p1), cap, 0.0, h, nullptr);
-        if (h.kind == HALO_TILE || S <= kPartMin || h.nseg > kMaxSeg) break;
-    }
-    const int extra = (p1 - p0 + S - 1) / S - 1;
-    if (extra > 0) {
-        const int room = spare_tiles(tiles), at = atomicAdd(&I.spares, extra);
-        if (at + extra <= room) {
-            for (int e = 0; e < extra; ++e)
-                chunks[b.z + tiles + at + e] = Chunk{p0 + (e + 1) * S, min(p0 + (e + 2) * S, p1), b.w, at + e};
-            full.p1 = p0 + S;
-        } else {
-            for (int e = at; e < room; ++e) chunks[b.z + tiles + e] = Chunk{0, 0, b.w, e};   // (claimed, unused)
+    const int R = stencil_radius(I.hmax, inst_disp(I), inst_grid(I, cell_start), I.hmax + I.delta);
+    int parts = 0;
+    for (int p = p0; p < p1;) {
+        // (lane k tries 128 >> k; nothing fits: the rest stays one part)
+        const int e = min(p + (kTile >> min(lane, 7)), p1);
+        bool fits = false;
+        if (lane < 8 && R <= kMaxRadius) {
+            int lo[kMaxSeg], off[kMaxSeg + 1];
+            fits = halo_ranges(I, cell_start, cell[p], cell[e - 1], R, lo, off) <= cap;
         }
+        const unsigned ok = __ballot_sync(0xffffffffu, fits);
+        if (lane == 0) starts[w][parts] = (unsigned char)(p - p0);
+        ++parts;
+        p = ok ? min(p + (kTile >> (__ffs(ok) - 1)), p1) : p1;
     }
-    chunks[c] = full;
+    __syncwarp();
+    const int extra = parts - 1, room = spare_tiles(tiles);
+    int at = 0;
+    if (lane == 0 && extra > 0) at = atomicAdd(&I.spares, extra);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    const int more = max(min(extra, room - at), 0);   // parts that get a tile of their own
+    auto start = [&](int q) { return q <= more && q < parts ? p0 + starts[w][q] : p1; };
+    for (int q = 1 + lane; q <= more; q += 32)
+        chunks[b.z + tiles + at + q - 1] = Chunk{start(q), start(q + 1), b.w, at + q - 1};
+    if (lane == 0) chunks[c] = Chunk{p0, start(1), b.w, -1};
 }
 
 // Halo slots of a tile in shared memory.  Three rows of cells around 128
@@ -1255,9 +1272,8 @@ void launch_chunks(simp_ctx *c) {
 }
 void launch_split(simp_ctx *c, const DueMask &due) {
     if (c->nchunks == 0) return;
-    k_split<<<nblk(c->nchunks, 64), 64, 0, c->stream>>>(c->nchunks, c->nsrc, c->chunk_src, kTile, c->chunks, due,
-                                                        c->inst_dev, c->cell_start, c->bcell_start, c->cell,
-                                                        tile_cap(c));
+    k_split<<<nblk(c->nchunks, kSplitWarps), 32 * kSplitWarps, 0, c->stream>>>(
+        c->nchunks, c->nsrc, c->chunk_src, kTile, c->chunks, due, c->inst_dev, c->cell_start, c->cell, tile_cap(c));
     c->launches += 1;
 }
 

@@ -22,10 +22,10 @@
 // neighbours each: 221 us per step, 341 when such a particle sent its tile to
 // global memory and 254 with lists per particle in global memory).  A tile whose
 // halo exceeds the shared-memory capacity (a sparse cell row next to full ones) is
-// cut in halves down to kPartMin particles, taken one after another; one that
-// still does not fit or whose stencil radius exceeds kMaxRadius reads its
-// neighbours from global memory.  The arithmetic and its order are the same
-// everywhere.
+// cut (k_split); one that comes to exceed it later, by motion, is taken in parts
+// one after another.  What still does not fit, or has a stencil radius above
+// kMaxRadius, reads its neighbours from global memory.  The arithmetic and its
+// order are the same everywhere.
 #pragma once
 
 #include "pass_common.cuh"
@@ -139,6 +139,38 @@ __device__ __forceinline__ TileMem tile_mem(unsigned char *p, int cap, int array
     return m;
 }
 
+// The ranges of a halo of radius R around cells ka .. kb, and their total.
+__device__ __forceinline__ int halo_ranges(const Inst &I, const int *cell_start, int ka, int kb, int R, int (&lo)[kMaxSeg],
+                                           int (&off)[kMaxSeg + 1]) {
+    const int end = I.base + I.ncx * I.ncy, nseg = 2 * R + 1;
+    int a[kMaxSeg], b[kMaxSeg];
+#pragma unroll
+    for (int d = 0; d < kMaxSeg; ++d) {
+        if (d >= nseg) break;
+        const int sh = (d - R) * I.ncx;
+        a[d] = cell_start[clampi(ka + sh - R, I.base, end)];
+        b[d] = cell_start[clampi(kb + sh + R + 1, I.base, end)];
+    }
+    int total = 0, past = 0;
+#pragma unroll
+    for (int d = 0; d < kMaxSeg; ++d) {
+        if (d >= nseg) break;
+        // (a tile of more than a cell row: its ranges meet)
+        lo[d] = max(a[d], past);
+        off[d] = total;
+        total += max(b[d] - lo[d], 0);
+        past = max(b[d], past);
+    }
+    off[nseg] = total;
+    return total;
+}
+
+// Parts of a tile begin at multiples of 8 particles, or anywhere in a tile of 16
+// or fewer: either way it has at most 16 parts, and records.
+constexpr int kParts = kTile / kPartMin;
+__device__ __forceinline__ int part_shift(const Chunk &ch) { return ch.p1 - ch.p0 <= kParts ? 0 : 3; }
+static_assert(kPartMin == 1 << 3, "part_shift");
+
 // The halo of particles [p0, p1) of instance I, and its walls, if it has any
 // and they are asked for.  `moved`: how far any of the particles is from where
 // it was sorted.  Called by one thread.
@@ -177,27 +209,7 @@ __device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, con
             past = max(past, b1);
         }
     }
-    if (h.kind == HALO_GLOBAL) return;
-    int a[kMaxSeg], b[kMaxSeg];
-#pragma unroll
-    for (int d = 0; d < kMaxSeg; ++d) {
-        if (d >= h.nseg) break;
-        const int sh = (d - R) * I.ncx;
-        a[d] = cell_start[clampi(ka + sh - R, I.base, end)];
-        b[d] = cell_start[clampi(kb + sh + R + 1, I.base, end)];
-    }
-    int total = 0, past = 0;
-#pragma unroll
-    for (int d = 0; d < kMaxSeg; ++d) {
-        if (d >= h.nseg) break;
-        // (a tile of more than a cell row: its ranges meet)
-        h.lo[d] = max(a[d], past);
-        h.off[d] = total;
-        total += max(b[d] - h.lo[d], 0);
-        past = max(b[d], past);
-    }
-    h.off[h.nseg] = total;
-    if (total > cap) h.kind = HALO_GLOBAL;
+    if (h.kind == HALO_TILE && halo_ranges(I, cell_start, ka, kb, R, h.lo, h.off) > cap) h.kind = HALO_GLOBAL;
 }
 
 // Slot of particle j, which the halo holds.

@@ -1,6 +1,7 @@
-"""Particles of more candidates than a list holds, among others of their tile
-that have lists: they find their pairs in the tile's halo, and no tile is sent
-to global memory for them.
+"""What once sent tiles, or parts of them, to global memory: particles of more
+candidates than a list holds, which find their pairs in the tile's halo now,
+among others of their tile that have lists; and sparse cell rows, whose tiles
+are cut as short as their halo needs, also when other basins join the batch.
 
 The bars are those of the other comparisons: 1e-11 of a right-hand side in FP64
 (2e-6 mixed), where only the order of the sums differs, and 1e-9 after ten steps
@@ -15,7 +16,7 @@ import pytest
 from helpers import rel_l2, smooth_velocity
 from simp_b200 import basins, build
 from simp_b200.params import ART_VISC_MON, PREC_FP64, PREC_MIXED
-from simp_b200.simp import Simp
+from simp_b200.simp import Batch, Simp
 
 pytestmark = pytest.mark.gpu
 
@@ -25,22 +26,21 @@ _SRC = """
 using namespace simp;
 using namespace simp::pass;
 // parts of the tiles in use by kind, and the particles whose list is too short
-extern "C" int tiles(void *ctx, int *kinds, int *over) {
+extern "C" int tiles(void *ctx, int slot, int *kinds, int *over) {
     simp_ctx *c = (simp_ctx *)ctx;
-    constexpr int parts = kTile / kPartMin;
     if (cudaStreamSynchronize(c->stream) != cudaSuccess) return 1;
     std::vector<Chunk> ch(c->nchunks);
-    std::vector<Halo> h((size_t)c->nchunks * parts);
+    std::vector<Halo> h((size_t)c->nchunks * kParts);
     std::vector<int> cnt(c->n);
     Inst I;
     cudaMemcpy(ch.data(), c->chunks, ch.size() * sizeof(Chunk), cudaMemcpyDeviceToHost);
     cudaMemcpy(h.data(), c->halos, h.size() * sizeof(Halo), cudaMemcpyDeviceToHost);
     cudaMemcpy(cnt.data(), c->pair_count, cnt.size() * sizeof(int), cudaMemcpyDeviceToHost);
-    if (cudaMemcpy(&I, c->inst_dev, sizeof(I), cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
+    if (cudaMemcpy(&I, c->inst_dev + slot, sizeof(I), cudaMemcpyDeviceToHost) != cudaSuccess) return 2;
     for (int k = 0; k < c->nchunks; ++k) {
-        if (ch[k].spare >= I.spares) continue;
+        if (ch[k].q != slot || ch[k].spare >= I.spares) continue;
         for (int p = ch[k].p0; p < ch[k].p1;) {
-            const Halo &r = h[(size_t)k * parts + (p - ch[k].p0) / kPartMin];
+            const Halo &r = h[(size_t)k * kParts + ((p - ch[k].p0) >> (ch[k].p1 - ch[k].p0 <= kParts ? 0 : 3))];
             if (r.size < 1 || r.kind < 0 || r.kind > 2) return 3;
             ++kinds[r.kind];
             p += r.size;
@@ -60,11 +60,11 @@ def tiles(gpu_lib, tmp_path_factory):
     subprocess.run([build.nvcc(), "-shared", *build.ARCH, "-O2", "-std=c++17", "-Xcompiler", "-fPIC", "-I", build.INCLUDE,
                     "-I", build.CSRC, *build.host_compiler(), "-o", so, str(d / "t.cu")], check=True)
     lib = ctypes.CDLL(so)
-    lib.tiles.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    lib.tiles.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p]
 
-    def look(sim):
+    def look(sim, slot=0):
         kinds, over = (ctypes.c_int * 3)(), ctypes.c_int(0)
-        assert lib.tiles(sim.h, kinds, ctypes.byref(over)) == 0
+        assert lib.tiles(sim.h, slot, kinds, ctypes.byref(over)) == 0
         return list(kinds), over.value
     return look
 
@@ -115,3 +115,47 @@ def test_long_lists(gpu_lib, tiles, oracle_mod, form, precision):
     for k in ("x", "vx", "h", "A", "rho"):
         ref = b.x if k == "x" else 0.0
         assert rel_l2(s[k] - ref, so[k] - ref) < 1e-9, k
+
+
+def _sparse(every, seed=5):
+    """Twelve full rows, one of every `every`-th particle, and full rows again above a gap."""
+    b = basins.make_basin(300, 2000.0, seed, walls="+x-x", dt=0.5)
+    b.vx = smooth_velocity(b.x, b.L, amp=0.3, seed=4)
+    row, col = (np.floor(b.x[:, k] / b.dx).astype(int) for k in (1, 0))
+    keep = (row < 12) | ((row == 14) & (col % every == every // 2)) | ((row >= 17) & (row < 24))
+    for k in ("x", "vx", "mass", "rho", "hsml", "A", "h"):
+        setattr(b, k, np.ascontiguousarray(getattr(b, k)[keep]))
+    return b
+
+
+@pytest.mark.parametrize("precision", [PREC_FP64, PREC_MIXED])
+@pytest.mark.parametrize("every", [3, 25, 140, 290])
+def test_sparse_rows(gpu_lib, tiles, oracle_mod, every, precision):
+    b = _sparse(every)
+    prm = b.params.copy()
+    prm.precision = precision
+    with Simp.from_basin(b, prm) as g:
+        r = g.single_step(600.0)
+        kinds, _ = tiles(g)
+    assert kinds[1] > 0 and kinds[0] == kinds[2] == 0, kinds
+    ro = oracle_mod.Oracle.from_basin(b, b.params).single_step(600.0)
+    for k in ("dvxdt", "dhdt", "dAdt"):
+        assert rel_l2(r[k], ro[k]) < (1e-11 if precision == PREC_FP64 else 2e-6), k
+
+
+def test_sparse_rows_stay_cut_as_others_join(gpu_lib, tiles):
+    b, other = _sparse(25), _sparse(140, seed=6)
+    with Batch(b.params, b.n + other.n, b.nb + other.nb, 2) as g:
+        slot = g.add(b)
+        g.step(2)
+        guest = g.add(other)
+        g.step(2)
+        for s in (slot, guest):
+            kinds, _ = tiles(g, s)
+            assert kinds[1] > 0 and kinds[0] == kinds[2] == 0, (s, kinds)
+        got = g.get_state(slot)
+    with Simp.from_basin(b) as alone:
+        alone.time_integration(4)
+        want = alone.get_state()
+    for k in ("x", "vx", "h", "A"):
+        assert np.array_equal(got[k], want[k]), k
