@@ -324,20 +324,22 @@ SIMP_API int32_t simp_gpu_sum_density_noalloc(const double *x, const double *hsm
 SIMP_API void *simp_gpu_stream(simp_ctx *ctx);
 
 /* Names for the implementation of the two pair passes (no reference
- * counterpart).  One implementation, tiles in shared memory over Verlet lists,
- * is the fastest at every size and serves all of them; the names stay for
- * callers that set one, and get_passes returns what was set.  threads:
- * 64..256, a multiple of 32; cap: a multiple of 4, within the shared memory of
- * one block (both checked for every form). */
+ * counterpart).  One implementation serves all of them: tiles in shared memory
+ * over Verlet lists.  With SIMP_PASSES_TILED a tile's halo holds `cap` particles
+ * (1344 at most); with the other names, the default among them, the library
+ * chooses.  Results are the same bits.  threads: 64..256, a multiple of 32 (a
+ * tile has 128 particles whatever it says); cap: a multiple of 4, within the
+ * shared memory of one block (both checked for every name).  get_passes returns
+ * what was set. */
 #define SIMP_PASSES_GATHER 0
 #define SIMP_PASSES_TILED 1
 #define SIMP_PASSES_GATHER_ONE 2
 #define SIMP_PASSES_GATHER_TWO 3
 SIMP_API int32_t simp_gpu_set_passes(simp_ctx *ctx, int32_t impl, int32_t threads, int32_t cap);
 SIMP_API int32_t simp_gpu_get_passes(const simp_ctx *ctx, int32_t *impl, int32_t *threads, int32_t *cap);
-/* Times one right-hand side (both passes, no state change) of the current
- * state, `reps` times, and sets SIMP_PASSES_GATHER_ONE.  *ms_best: its time
- * per right-hand side. */
+/* Sets SIMP_PASSES_GATHER_ONE and times one right-hand side (both passes, no
+ * state change) of the current state, `reps` times.  *ms_best: its time per
+ * right-hand side. */
 SIMP_API int32_t simp_gpu_autotune(simp_ctx *ctx, int32_t reps, double *ms_best);
 
 /* Number of kernels this context has launched so far (graph replays count

@@ -1159,6 +1159,7 @@ int sort_replayed(simp_ctx *c, const DueMask &due) {
     k.n = c->n;
     k.total_cells = c->total_cells;
     k.nchunks = c->nchunks;
+    k.halo_cap = c->halo_cap;
     k.uniform = c->uniform;
     k.cell_start = c->cell_start;
     k.scan_tmp = c->scan_tmp;
@@ -1802,15 +1803,22 @@ int32_t simp_gpu_set_passes(simp_ctx *c, int32_t impl, int32_t threads, int32_t 
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    // (what such a tile's halo records and pair lists would take)
+    // (what a block of such a tile took when these names were separate kernels:
+    // the shapes that were refused still are)
     const size_t real = c->prm.precision == SIMP_PREC_MIXED ? sizeof(float) : sizeof(double);
     const size_t need = (size_t)cap * (5 * sizeof(double) + sizeof(float4) + 3 * real) +
                         (size_t)49 * threads * sizeof(unsigned short);
     if (optin > 0 && need + 1024 > (size_t)optin)
         return simp_fail(c, SIMP_ERR_BADARG, "tile shape exceeds the shared memory of a block");
-    c->pass_impl = impl;   // (one implementation serves every form)
+    c->pass_impl = impl;
     c->tile_threads = threads;
     c->tile_cap = cap;
+    const int halo_cap = impl == SIMP_PASSES_TILED ? std::min(cap, kMostHaloCap) : 0;
+    if (halo_cap == c->halo_cap) return SIMP_OK;
+    c->halo_cap = halo_cap;
+    if (c->have_state) launch_recut(c);
+    invalidate_graph(c);
+    SIMP_CUDA(c, cudaGetLastError());
     return SIMP_OK;
 }
 
@@ -1852,9 +1860,9 @@ int32_t simp_gpu_autotune(simp_ctx *c, int32_t reps, double *ms_best) {
     if (!c || reps < 1) return SIMP_ERR_BADARG;
     if (!c->have_state || c->n == 0) return simp_fail(c, SIMP_ERR_STATE, "autotune needs particles");
     TRY(flush_batch(c, true));
+    TRY(simp_gpu_set_passes(c, SIMP_PASSES_GATHER_ONE, 256, 1024));
     double t = 0.0;
     TRY(time_rhs(c, reps, &t));
-    TRY(simp_gpu_set_passes(c, SIMP_PASSES_GATHER_ONE, 256, 1024));
     c->err.clear();
     if (ms_best) *ms_best = t;
     return SIMP_OK;

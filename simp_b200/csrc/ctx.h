@@ -116,10 +116,12 @@ struct simp_ctx {
     // cell lists
     int *cell_start = nullptr;
     size_t cell_cap = 0;
-    // what simp_gpu_set_passes named (every form runs the same passes)
+    // what simp_gpu_set_passes named; SIMP_PASSES_TILED sets the tiles' halo
+    // capacity, the others leave it to the passes (0)
     int pass_impl = SIMP_PASSES_GATHER;
     int tile_threads = 256;
     int tile_cap = 1024;
+    int halo_cap = 0;
     // rebuild scratch
     int *cnt = nullptr;            // per-cell counters (cell_cap)
     int *perm = nullptr;           // maxn
@@ -147,12 +149,12 @@ struct simp_ctx {
     // captured once and replayed while what they capture stays the same
     cudaGraphExec_t sort_graph = nullptr;
     struct SortKey {
-        int n = -1, total_cells = -1, nchunks = -1;
+        int n = -1, total_cells = -1, nchunks = -1, halo_cap = -1;
         bool uniform = false;
         const void *cell_start = nullptr, *scan_tmp = nullptr;
         bool operator==(const SortKey &o) const {
-            return n == o.n && total_cells == o.total_cells && nchunks == o.nchunks && uniform == o.uniform &&
-                   cell_start == o.cell_start && scan_tmp == o.scan_tmp;
+            return n == o.n && total_cells == o.total_cells && nchunks == o.nchunks &&
+                   halo_cap == o.halo_cap && uniform == o.uniform && cell_start == o.cell_start && scan_tmp == o.scan_tmp;
         }
     } sort_key;
     long long sort_kernels = 0;    // kernels per re-sort replay
@@ -223,6 +225,11 @@ inline size_t chunk_capacity(int maxn, int max_inst) {
 }
 void launch_chunks(simp_ctx *c);
 void launch_split(simp_ctx *c, const DueMask &due);   // after a sort
+// Another halo capacity for the tiles of a resident state: cuts them anew and
+// marks the lists stale.
+void launch_recut(simp_ctx *c);
+constexpr int kMostHaloCap = 1344;   // (what the auxiliary passes' 64 bytes per slot leave of kMostTileSmem)
+constexpr size_t kMostTileSmem = 96 * 1024;
 int passes_configure(simp_ctx *c);
 
 // abi.cu: device bytes per particle of capacity

@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         if (Walls::kKeep) pair_sums();
         Walls wl;
         if (have_walls && h.walls) {
-            int bytes = (int)tile_smem_bytes(a.cap, arrays, UNIFORM);
+            int bytes = (int)stress_smem_bytes(a.cap, arrays, UNIFORM);
             __syncthreads();
             double *keep = reinterpret_cast<double *>(smem + bytes) - 4 * kTile + t;
             if (Walls::kKeep) {
@@ -636,9 +636,10 @@ __device__ __forceinline__ void tile_fill(const Halo &h, F &&fill) {
     }
 }
 constexpr int kAuxArrays = 3;
-size_t aux_smem_bytes(int cap) {
+constexpr size_t aux_smem_bytes(int cap) {
     return tile_smem_bytes(cap, 2, false) + (size_t)kAuxArrays * cap * sizeof(double);
 }
+static_assert(aux_smem_bytes(kMostHaloCap) <= kMostTileSmem, "ctx.h: kMostHaloCap");
 
 // Copies a tile part's halo record, records and lists to shared memory and
 // fills the other values.  Called by the whole block; false, for all of it,
@@ -1163,6 +1164,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps)
 // us per step); a larger one is faster with what shared memory then leaves to
 // the L1 cache (1,048,576 particles FP64: 598 us against 632 with room for 832).
 int tile_cap(const simp_ctx *c) {
+    if (c->halo_cap > 0) return c->halo_cap;
     if (c->nchunks <= kResidentTiles) return 832;
     return c->uniform ? 528 : 704;
 }
@@ -1209,7 +1211,7 @@ void each_kernel(F &&f) {
 template <class T, int SKF>
 cudaError_t allow_smem() {
     cudaError_t e = cudaSuccess;
-    const int most = 96 * 1024;   // (a tile takes 40 to 64 KB)
+    const int most = (int)kMostTileSmem;   // (a tile takes 40 to 64 KB)
     each_kernel<T, SKF>([&](auto *k) {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     });
@@ -1240,7 +1242,7 @@ void launch_tiles(simp_ctx *c, const A &a) {
     if constexpr (std::is_same<A, KinArgs>::value)
         launch_pass(c, k_kinematic<T, SKF, HS, BLOCKS>, g, kTile, tile_smem_bytes(a.cap, 3, c->uniform), a);
     else
-        launch_pass(c, k_stress<T, SKF, HS, BLOCKS>, g, kTile, tile_smem_bytes(a.cap, Rec<T>::stress_arrays, c->uniform), a);
+        launch_pass(c, k_stress<T, SKF, HS, BLOCKS>, g, kTile, stress_smem_bytes(a.cap, Rec<T>::stress_arrays, c->uniform), a);
 }
 template <class T, int SKF, int BLOCKS, class A>
 void launch_hsml_form(simp_ctx *c, const A &a) {
@@ -1275,6 +1277,23 @@ void launch_split(simp_ctx *c, const DueMask &due) {
     k_split<<<nblk(c->nchunks, kSplitWarps), 32 * kSplitWarps, 0, c->stream>>>(
         c->nchunks, c->nsrc, c->chunk_src, kTile, c->chunks, due, c->inst_dev, c->cell_start, c->cell, tile_cap(c));
     c->launches += 1;
+}
+
+namespace {
+__global__ void k_uncut(Inst *inst, int ninst) {
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= ninst) return;
+    inst[q].list_ok = 0;
+    inst[q].spares = 0;
+}
+}  // namespace
+void launch_recut(simp_ctx *c) {
+    k_uncut<<<nblk(c->ninst, 128), 128, 0, c->stream>>>(c->inst_dev, c->ninst);
+    c->launches += 1;
+    launch_chunks(c);
+    DueMask all;
+    for (unsigned long long &w : all.w) w = ~0ull;
+    launch_split(c, all);
 }
 
 int passes_configure(simp_ctx *c) {

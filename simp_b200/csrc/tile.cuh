@@ -125,7 +125,7 @@ struct TileMem {
     __device__ __forceinline__ float *hf() const { return reinterpret_cast<float *>(rec[1]); }
 };
 
-__host__ __device__ inline size_t tile_smem_bytes(int cap, int arrays, bool uniform) {
+__host__ __device__ constexpr size_t tile_smem_bytes(int cap, int arrays, bool uniform) {
     return (size_t)cap * (16 * arrays + (uniform ? 0 : 8)) + (size_t)kListRows * kTile * sizeof(unsigned short);
 }
 

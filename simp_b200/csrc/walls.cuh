@@ -32,6 +32,12 @@ struct WallTile {
     int cnt[kTile];
 };
 static_assert(kTile <= 128 && kWallCap <= 128, "WallTile::pair");
+// Shared memory of the stress pass: its tile's, and at least what the wall sums
+// put in its place (the pair sums behind them).
+__host__ __device__ constexpr size_t stress_smem_bytes(int cap, int arrays, bool uniform) {
+    const size_t tile = tile_smem_bytes(cap, arrays, uniform), walls = sizeof(WallTile) + 4 * kTile * sizeof(double);
+    return tile > walls ? tile : walls;
+}
 
 __device__ __forceinline__ int warp_scan(int v, int lane) {   // inclusive
 #pragma unroll
