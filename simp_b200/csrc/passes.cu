@@ -303,16 +303,11 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
         if (!build) {
             if (t < kHaloWords)
                 reinterpret_cast<int *>(&h)[t] = p0 == ch.p0 ? first : halo_word(&halos[(p0 - ch.p0) >> shift], t);
-        } else if (t == 0) {
-            // the largest part of the tile whose halo fits
-            for (int S = kTile;; S >>= 1) {
-                make_halo(I, a.cell_start, a.bstart, a.cell, p0, min(p0 + S, ch.p1), a.cap,
-                          sqrt((double)__uint_as_float(moved2)) * (1.0 + 1e-6), h,
-                          reinterpret_cast<HaloWalls *>(a.halo_walls) + (size_t)blockIdx.x * kParts +
-                              ((p0 - ch.p0) >> shift));
-                if (h.kind == HALO_TILE || S <= (1 << shift) || h.nseg > kMaxSeg) break;
-            }
-            rows_max = 0;
+        } else if (t < 32) {
+            make_halo(I, a.cell_start, a.bstart, a.cell, p0, ch.p1, shift, a.cap,
+                      sqrt((double)__uint_as_float(moved2)) * (1.0 + 1e-6), h,
+                      reinterpret_cast<HaloWalls *>(a.halo_walls)[(size_t)blockIdx.x * kParts + ((p0 - ch.p0) >> shift)]);
+            if (t == 0) rows_max = 0;
         }
         __syncthreads();
         if (failed < 2 * p0) return;
@@ -1159,14 +1154,17 @@ __global__ void __launch_bounds__(32 * kSplitWarps)
 // Halo slots of a tile in shared memory.  Three rows of cells around 128
 // particles take up to 520 slots at hsml = 2.4 spacings and 650 at the
 // reference's 3 spacings; five rows (after more motion), or a sparse row's tile
-// among full ones, about 850.  A context whose tiles are resident all at once
-// has room for the latter (40,401 particles with the density passes: 158 -> 137
-// us per step); a larger one is faster with what shared memory then leaves to
-// the L1 cache (1,048,576 particles FP64: 598 us against 632 with room for 832).
+// among full ones, about 850.  A context of up to kResidentTiles has room for the
+// latter (40,401 particles with the density passes: 158 -> 137 us per step); a
+// larger one is faster with what shared memory then leaves to the L1 cache
+// (1,048,576 particles, us per step with room for 528, 576, 640, 832: FP64 541,
+// 542, 547, 563, mixed 528, 531, 560, 579), but not with less than 576 where
+// particles move: a fifth of hsml between sorts, FP64 1066, 908, 916, 936, mixed
+// 1046, 892, 935, 973; or at 2.6 spacings, FP64 596, 544, 548, 564.
 int tile_cap(const simp_ctx *c) {
     if (c->halo_cap > 0) return c->halo_cap;
     if (c->nchunks <= kResidentTiles) return 832;
-    return c->uniform ? 528 : 704;
+    return c->uniform ? 576 : 704;
 }
 
 // Whether a pass fetches its epilogue's values ahead of its pairs: where they

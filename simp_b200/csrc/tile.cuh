@@ -171,45 +171,68 @@ constexpr int kParts = kTile / kPartMin;
 __device__ __forceinline__ int part_shift(const Chunk &ch) { return ch.p1 - ch.p0 <= kParts ? 0 : 3; }
 static_assert(kPartMin == 1 << 3, "part_shift");
 
-// The halo of particles [p0, p1) of instance I, and its walls, if it has any
-// and they are asked for.  `moved`: how far any of the particles is from where
-// it was sorted.  Called by one thread.
+// The halo of the longest part of a tile from p0 on that fits (up to p1, parts in
+// steps of 1 << shift), and its walls, if it has any.  `moved`: how far any of the
+// tile's particles is from where it was sorted.  Called by a warp: a lane per
+// size, and a lane per row of walls (262,144 particles that move a fifth of hsml
+// between sorts, so that lists are built in every step, FP64, at 528 slots: 288 us
+// per step; 343 with one thread that halved the size until it fitted).
 __device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, const int *bstart, const int *cell, int p0,
-                                       int p1, int cap, double moved, Halo &h, HaloWalls *hw) {
+                                       int p1, int shift, int cap, double moved, Halo &h, HaloWalls &hw) {
+    const int lane = threadIdx.x & 31;
     const Grid g = inst_grid(I, cell_start);
     // The farthest of a basin's particles are few: with the tile's own distance
     // for one side of a pair, the tiles of the others keep a radius of 1 (one
     // step of 262,144 particles of which some race along a wall: 260 -> 237 us).
     const double disp = inst_disp(I);
     const int R = stencil_radius(I.hmax, 0.5 * (fmin(moved, disp) + disp), g, I.hmax + I.delta);
-    h.size = p1 - p0;
-    h.nseg = 2 * R + 1;
-    h.rows = 0;
-    h.kind = R <= kMaxRadius ? HALO_TILE : HALO_GLOBAL;
-    const int ka = cell[p0], kb = cell[p1 - 1], end = I.base + I.ncx * I.ncy;
-    // walls within b_length of any place its particles take while the lists
-    // stay valid (they move less than delta)
-    h.walls = 0;
-    const int Rb = wall_radius(inst_disp(I), g, I.b_length + I.delta);
-    for (int d = -Rb; d <= Rb && !h.walls; ++d)
-        if (bstart[clampi(kb + d * I.ncx + Rb + 1, I.base, end)] > bstart[clampi(ka + d * I.ncx - Rb, I.base, end)])
-            h.walls = Rb;
-    if (h.walls && hw) {
-        const int rows = 2 * Rb + 1, b_first = bstart[I.base];
-        int past = 0;
-        for (int d = 0; d < kMaxWallRows; ++d) {
-            int b0 = past, b1 = past;
-            if (d < rows) {
-                const int sh = (d - Rb) * I.ncx;
-                b0 = max(bstart[clampi(ka + sh - Rb, I.base, end)], past);
-                b1 = bstart[clampi(kb + sh + Rb + 1, I.base, end)];
+    const int e = min(p0 + max((kParts - lane) << shift, 1), p1);
+    const int ka = cell[p0], ke = cell[e - 1], end = I.base + I.ncx * I.ncy;
+    int lo[kMaxSeg], off[kMaxSeg + 1];
+    const bool fits = lane < kParts && R <= kMaxRadius && halo_ranges(I, cell_start, ka, ke, R, lo, off) <= cap;
+    const unsigned ok = __ballot_sync(0xffffffffu, fits);
+    // (the longest; if none fits the shortest, or all where the radius is too wide)
+    const int w = ok ? __ffs(ok) - 1 : R <= kMaxRadius ? kParts - 1 : 0;
+    if (lane == w) {
+        h.kind = fits ? HALO_TILE : HALO_GLOBAL;
+        h.nseg = 2 * R + 1;
+        h.rows = 0;
+        h.size = e - p0;
+        if (fits) {
+#pragma unroll
+            for (int d = 0; d < kMaxSeg; ++d) {
+                if (d >= 2 * R + 1) break;
+                h.lo[d] = lo[d];
+                h.off[d + 1] = off[d + 1];
             }
-            hw->lo[d] = b0 - b_first;
-            hw->n[d] = d == 0 && rows > kMaxWallRows ? -1 : max(b1 - b0, 0);
-            past = max(past, b1);
+            h.off[0] = 0;
         }
     }
-    if (h.kind == HALO_TILE && halo_ranges(I, cell_start, ka, kb, R, h.lo, h.off) > cap) h.kind = HALO_GLOBAL;
+    // walls within b_length of any place its particles take while the lists
+    // stay valid (they move less than delta)
+    const int kb = __shfl_sync(0xffffffffu, ke, w);
+    const int Rb = wall_radius(disp, g, I.b_length + I.delta), rows = 2 * Rb + 1;
+    auto first = [&](int d) { return bstart[clampi(ka + (d - Rb) * I.ncx - Rb, I.base, end)]; };
+    auto past = [&](int d) { return bstart[clampi(kb + (d - Rb) * I.ncx + Rb + 1, I.base, end)]; };
+    bool any = false;
+    for (int d = lane; d < rows; d += 32) any = any || past(d) > first(d);
+    any = __any_sync(0xffffffffu, any);
+    if (lane == 0) h.walls = any ? Rb : 0;
+    if (!any) return;
+    // each row's, from where the rows before it end
+    const int b0 = lane < rows ? first(lane) : 0, b1 = lane < rows ? past(lane) : 0, b_first = bstart[I.base];
+    int upto = b1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto = max(upto, u);
+    }
+    const int before = max(__shfl_up_sync(0xffffffffu, upto, 1), 0);
+    if (lane < kMaxWallRows) {
+        const int b = lane > 0 ? max(b0, before) : b0;
+        hw.lo[lane] = b - b_first;
+        hw.n[lane] = lane == 0 && rows > kMaxWallRows ? -1 : max(b1 - b, 0);
+    }
 }
 
 // Slot of particle j, which the halo holds.

@@ -159,3 +159,19 @@ def test_sparse_rows_stay_cut_as_others_join(gpu_lib, tiles):
         want = alone.get_state()
     for k in ("x", "vx", "h", "A"):
         assert np.array_equal(got[k], want[k]), k
+
+
+def test_parts_after_motion(gpu_lib, tiles):
+    """Five rows of cells of a large basin, whose tiles hold a halo of 576: 13
+    lattice rows of 43 columns, 13 of which lie beside the part.  A part then has
+    30 columns of the cell row's two or three lattice rows, 60 to 90 particles,
+    so that a tile takes two or three parts."""
+    b = basins.make_basin(384, 2000.0, 5, walls="", dt=1.0)
+    b.vx = smooth_velocity(b.x, b.L, amp=0.3, seed=4) + np.array([60.0, 30.0])
+    b.params.wind_force = b.params.water_force = 0
+    with Simp.from_basin(b) as g:
+        g.time_integration(14)          # (of 16 between sorts)
+        kinds, _ = tiles(g)
+    whole = -(-b.n // 128)
+    assert kinds[0] == kinds[2] == 0, kinds
+    assert 1.5 < kinds[1] / whole < 2.6, kinds[1] / whole
