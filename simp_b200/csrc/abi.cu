@@ -965,6 +965,7 @@ int create(const simp_params *params, int32_t maxn, int32_t maxnb, int32_t max_i
     c->id_stride = (max_inst > 1) ? (1 << kIdShift) : 0;
     c->insts.assign(max_inst, InstHost{});
     cudaGetDevice(&c->device);
+    cudaDeviceGetAttribute(&c->l2_bytes, cudaDevAttrL2CacheSize, c->device);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess)
         return simp_fail(c, SIMP_ERR_CUDA, "cudaStreamCreate failed (no usable CUDA device?)");
     const size_t M = (size_t)maxn, MB = (size_t)c->maxnb, MX = std::max(M, MB);

@@ -122,6 +122,7 @@ struct simp_ctx {
     int tile_threads = 256;
     int tile_cap = 1024;
     int halo_cap = 0;
+    int l2_bytes = 0;
     // rebuild scratch
     int *cnt = nullptr;            // per-cell counters (cell_cap)
     int *perm = nullptr;           // maxn

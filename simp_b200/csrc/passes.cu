@@ -14,12 +14,15 @@ using namespace pass;
 
 constexpr int kBlock = kTile;
 // Resident blocks per SM the register allocation aims at.  4 (128 registers)
-// holds the pair math of two candidates without spills: FP64 always (5 and 6
+// holds the pair math of two candidates: FP64 always (5 and 6
 // blocks per step at 262,144 particles: 160 -> 168 and 234 us; the reference's
-// switches at 90,007: 131 -> 154 and 197), and the mixed form where all tiles
-// are resident at once anyway (24,649 particles: 54 -> 49 us).  Above that the
-// mixed form takes 5 (1,048,576: 597 against 617 and 609 us at 4 and 6).
-constexpr int kResidentTiles = 1024;
+// switches at 90,007: 131 -> 154 and 197).  The mixed form takes 5 above
+// kSmallTiles tiles, where more of them at a time begin to pay; up to 4,000 or so
+// it depends on how full the last wave is (592 tiles a wave with 4, 740 with 5).
+// us per step with 4 and 5: 57,600 particles 56 and 66, 102,400 88 and 98, 131,044
+// 92 and 106, 160,000 116 and 111, 200,704 127 and 143, 262,144 162 and 163,
+// 640,000 366 and 364, 1,048,576 560 and 548.
+constexpr int kSmallTiles = 1024;
 
 // hsml of the halo's particles, where it varies.
 __device__ __forceinline__ void tile_hsml(const Halo &h, const TileMem &m, const State &s) {
@@ -1154,7 +1157,7 @@ __global__ void __launch_bounds__(32 * kSplitWarps)
 // Halo slots of a tile in shared memory.  Three rows of cells around 128
 // particles take up to 520 slots at hsml = 2.4 spacings and 650 at the
 // reference's 3 spacings; five rows (after more motion), or a sparse row's tile
-// among full ones, about 850.  A context of up to kResidentTiles has room for the
+// among full ones, about 850.  A context of up to kSmallTiles has room for the
 // latter (40,401 particles with the density passes: 158 -> 137 us per step); a
 // larger one is faster with what shared memory then leaves to the L1 cache
 // (1,048,576 particles, us per step with room for 528, 576, 640, 832: FP64 541,
@@ -1163,14 +1166,17 @@ __global__ void __launch_bounds__(32 * kSplitWarps)
 // 1046, 892, 935, 973; or at 2.6 spacings, FP64 596, 544, 548, 564.
 int tile_cap(const simp_ctx *c) {
     if (c->halo_cap > 0) return c->halo_cap;
-    if (c->nchunks <= kResidentTiles) return 832;
+    if (c->nchunks <= kSmallTiles) return 832;
     return c->uniform ? 576 : 704;
 }
 
 // Whether a pass fetches its epilogue's values ahead of its pairs: where they
-// come from DRAM (1,048,576 particles: 597 -> 588 us FP64, 583 -> 570 mixed;
-// 600,011: 376 -> 370), not where L2 holds the state (262,144: 158 -> 161).
-bool prefetch_own(const simp_ctx *c) { return c->n > 400000; }
+// come from DRAM, which is where the arrays of a step (about 280 bytes per
+// particle) outgrow two thirds of L2.  us per step without and with it, FP64 and
+// mixed: 176,400 particles 122.3 and 122.9, 114.9 and 116.5; 262,144 158.6 and
+// 159.8, 162.2 and 164.0; 313,600 189.4 and 188.7, 201.5 and 200.8; 399,424 237.9
+// and 234.1, 250.6 and 249.2; 1,048,576 558 and 548, 560 and 546.
+bool prefetch_own(const simp_ctx *c) { return 280.0 * c->n > 2.0 / 3.0 * c->l2_bytes; }
 
 TauRec tau_rec(simp_ctx *c) {
     TauRec r;
@@ -1251,7 +1257,7 @@ void launch_hsml_form(simp_ctx *c, const A &a) {
 template <int SKF, class A>
 void launch_kernel_form(simp_ctx *c, const A &a) {
     if (c->prm.precision != SIMP_PREC_MIXED) launch_hsml_form<double, SKF, 4>(c, a);
-    else if (c->nchunks <= kResidentTiles) launch_hsml_form<float, SKF, 4>(c, a);
+    else if (c->nchunks <= kSmallTiles) launch_hsml_form<float, SKF, 4>(c, a);
     else launch_hsml_form<float, SKF, 5>(c, a);
 }
 template <class A>
