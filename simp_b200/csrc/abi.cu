@@ -938,7 +938,7 @@ int maybe_regrid(simp_ctx *c, bool *done) {
 int check_after(simp_ctx *c) {
     if (const unsigned f = take_bounds_flags())
         return simp_fail(c, SIMP_ERR_BOUNDS, "device index check failed (sites " + std::to_string(f) +
-                                                 ": 1 neighbour, 2 cell, 4 sort slot, 8 tile slot)");
+                                                 ": 2 cell, 4 sort slot, 8 tile slot)");
     const Scalars &s = *c->sc_host;
     if (s.flags & FLAG_TIMEOUT) return simp_fail(c, SIMP_ERR_TIMEOUT, "a tile's copies did not arrive");
     if ((s.flags & FLAG_NONFINITE) && c->max_inst == 1)   // batches flag the basin instead

@@ -13,11 +13,10 @@
 // Sort: counting sort on cell keys (one radix digit of width log2(ncells)):
 // key histogram, exclusive prefix scan, scatter, then a per-cell sort by
 // original particle index so the order is deterministic.
-#include <cstring>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 
 #include "ctx.h"

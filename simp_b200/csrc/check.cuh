@@ -17,7 +17,6 @@
 namespace simp {
 
 enum : unsigned {
-    SITE_NEIGHBOUR = 1u,   // a neighbour index from a Verlet or pair list
     SITE_CELL = 2u,        // a cell key of the stencil walk
     SITE_SORT = 4u,        // a slot of the counting sort
     SITE_TILE = 8u,        // a shared-memory slot of the tiled passes

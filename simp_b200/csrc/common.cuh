@@ -47,7 +47,6 @@ constexpr int kListRows = 44;   // (even)
 struct PairList {
     unsigned short *slot;
     int *count;
-    int n = 0;   // particles in the context (the debug build's index checks)
 };
 
 // Uniform cell grid of one basin.  cell = clamp(floor((x - x0) * inv_cs));
@@ -166,12 +165,6 @@ struct Phys {
     // 1 / e^2, 1 / (1 + k_t), 1 / rho_ice, 1 / b_length
     double em2, inv_1kt, inv_rho_ice, inv_b_length;
 };
-
-// Interaction-count bookkeeping for nnps.f90:613-670.
-__device__ __forceinline__ void note_interactions(Scalars *sc, int cnt) {
-    atomicMax(&sc->maxip, cnt);
-    atomicMin(&sc->minip, cnt);
-}
 
 // ---------------------------------------------------------------------------
 // Bit-exact pair criterion of nnps.f90:277-281:

@@ -98,24 +98,15 @@ __device__ __forceinline__ int for_each_wall(const double *__restrict__ BX, cons
     return count;
 }
 
-// FP32 prefilter of the pair criterion.  The float copies of x, y, hsml are
+// Margin of the FP32 search that builds the lists.  The float copies of x, y, hsml are
 // within X 2^-24 (X = max |coordinate|) and hsml 2^-24 of the doubles; the
 // float subtraction of two nearby coordinates is exact.  So the float
 // squared distance and squared mhsml differ from the exact ones by at most
 // (5.7 X / hmin + 12) 2^-24 relative near the decision boundary (where
-// mhsml >= hmin).  The returned margin doubles that bound; a candidate is
-// decided in FP32 only outside the margin, otherwise by the exact FP64 test.
+// mhsml >= hmin).  The returned margin doubles that bound; only a candidate
+// beyond it is left out.
 __device__ __forceinline__ float prefilter_margin(double xabs, double hmin) {
     return (float)((12.0 * xabs / hmin + 40.0) * 0x1p-24);
-}
-
-// 0: not a pair, 1: a pair, 2: undecided (use the FP64 test)
-__device__ __forceinline__ int prefilter(float dxf, float dyf, float mf, float margin) {
-    const float sf = dxf * dxf + dyf * dyf;
-    const float tf = mf * mf;
-    if (sf > tf * (1.0f + margin)) return 0;
-    if (sf < tf * (1.0f - margin)) return 1;
-    return 2;
 }
 
 // Stencil radius for wall pairs: walls are static, the particle moved at

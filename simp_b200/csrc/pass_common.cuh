@@ -2,10 +2,8 @@
 // and the predictor-corrector update fused into the second pass's epilogue.
 //
 // Kinematic pass (single_step.f90:50-84 + internal_stress.f90:20-42), per
-// particle i, in two phases:
-//   1. candidate scan of the cell stencil with an FP32 prefilter
-//      (neighbors.cuh), one bit per candidate;
-//   2. the exact FP64 criterion and the pair math over the set bits:
+// particle i: the exact criterion and the pair math over its candidates (a
+// Verlet list, built first where the basin's are stale):
 //        wdvx = (v_i - v_j) (x) grad W_ij            (kernel.f90:515-518)
 //        div_i  -= m_j (wdvx1 + wdvx4)               (vector_divergence.f90:27)
 //        grad_i -= m_j wdvx / rho_j                  (vector_gradient.f90:56-69)
@@ -264,7 +262,6 @@ struct KinArgs {
     const double2 *xyr;    // sort positions
     const int *cell_start, *bstart;
     const Inst *inst;
-    const int *pinst;      // instance of each particle
     const int *cell;
     Phys P;
     Scalars *sc;
@@ -272,7 +269,7 @@ struct KinArgs {
     TauRec rec;            // the stress pass's records (written here)
     double *diag;
     PairList pl;
-    int n, maxn;
+    int maxn;
     const Chunk *chunks;   // tile of each block
     unsigned char *halos;  // their halos (written here)
     unsigned char *halo_walls;
@@ -367,7 +364,6 @@ struct StressArgs {
     State out;     // state written by the epilogue
     const int *cell_start;
     Inst *inst;
-    const int *pinst;
     const int *cell;
     const double *bx, *by, *bm;
     const double *bnx, *bny;   // wall normals (bfa = 2)
@@ -384,7 +380,7 @@ struct StressArgs {
     // which a rates epilogue replaces by dx/dt; null when both are off
     double *reg;
     double *hs_next;
-    int n, maxn, mode, single, prefetch;
+    int maxn, mode, single, prefetch;
     const Chunk *chunks;
     const unsigned char *halos, *halo_walls;
     int cap;
@@ -398,31 +394,21 @@ __device__ __forceinline__ unsigned long long warp_top(unsigned long long v) {
 }
 __device__ __forceinline__ unsigned long long warp_least(unsigned long long v) { return ~warp_top(~v); }
 
-// Block-wide max / min folded into one device atomic per block (the
+// Block-wide max folded into one device atomic per block (the
 // same-address atomics of every warp would serialise in L2).  Called by all
 // threads of the block at the same point.
-template <bool MAX>
-__device__ __forceinline__ void block_reduce_u64(unsigned long long *dst, unsigned long long v) {
+__device__ __forceinline__ void block_max_u64(unsigned long long *dst, unsigned long long v) {
     __shared__ unsigned long long part[32];
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xffffffffu, v, o);
-        v = MAX ? (t > v ? t : v) : (t < v ? t : v);
-    }
+    v = warp_top(v);
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
     __syncthreads();
     if (threadIdx.x == 0) {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = MAX ? (part[w] > v ? part[w] : v) : (part[w] < v ? part[w] : v);
-        if (MAX) atomicMax(dst, v); else atomicMin(dst, v);
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = part[w] > v ? part[w] : v;
+        atomicMax(dst, v);
     }
     __syncthreads();
 }
-__device__ __forceinline__ void warp_max_u64(unsigned long long *dst, unsigned long long v) {
-    block_reduce_u64<true>(dst, v);
-}
-__device__ __forceinline__ void warp_min_u64(unsigned long long *dst, unsigned long long v) {
-    block_reduce_u64<false>(dst, v);
-}
-__device__ __forceinline__ void warp_max_i32(int *dst, int v) {
+__device__ __forceinline__ void block_max_i32(int *dst, int v) {
     __shared__ int part[32];
     for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
     if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
@@ -573,7 +559,7 @@ __device__ __forceinline__ void stress_finish(const StressArgs &a, int i, bool l
     const double dhdt = -hh * dv * irho;
     const double dAdt = -AA * dv * irho;
     if (a.mode == EPI_RATES) {
-        warp_max_i32(&a.sc->maxip, live ? cnt : 0);
+        block_max_i32(&a.sc->maxip, live ? cnt : 0);
         if (live) {
             const size_t M = (size_t)a.maxn;
             a.rates[i] = ax;

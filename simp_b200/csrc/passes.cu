@@ -609,7 +609,7 @@ struct RegArgs {
     Scalars *sc;
     Phys P;
     double *reg;
-    int n, maxn;
+    int maxn;
 };
 
 // lv / rho^2 of the Hernquist-Katz viscosity of particle k
@@ -806,7 +806,7 @@ struct DensArgs {
     const Inst *inst;
     Scalars *sc;
     Phys P;
-    int n, rho_upd, tail;
+    int rho_upd, tail;
     int dt_div;          // the Monaghan time step's divergence (artificial viscosity)
     // summation density (den_alg = 1, density.f90:41-100): rho_out =
     // (k0 m_i + sum_j m_j W_ij) / (k0 m_i / rho_i + sum_j m_j W_ij / rho_j)
@@ -997,7 +997,7 @@ __global__ void __launch_bounds__(256) k_commit_hsml(int n, const double *__rest
     // how far any hsml grew, for the Verlet lists' bound (NaN: as infinity)
     double grown = i < n ? hs_next[i] - s0.hs[i] : 0.0;
     if (!(grown <= 1e300)) grown = INFINITY;
-    warp_max_u64(&sc->acc_dh, dbits(fmax(grown, 0.0)));
+    block_max_u64(&sc->acc_dh, dbits(fmax(grown, 0.0)));
     if (i >= n) return;
     const double v = hs_next[i];
     const float vf = (float)v;
@@ -1190,7 +1190,6 @@ PairList pair_list(simp_ctx *c) {
     PairList pl;
     pl.slot = c->pair_slot;
     pl.count = c->pair_count;
-    pl.n = c->n;
     return pl;
 }
 
@@ -1322,7 +1321,6 @@ void launch_kinematic(simp_ctx *c, const State &s, bool diag, bool second) {
     a.cell_start = c->cell_start;
     a.bstart = c->bcell_start;
     a.inst = c->inst_dev;
-    a.pinst = c->pinst;
     a.cell = c->cell;
     a.P = c->phys;
     a.sc = c->sc;
@@ -1330,7 +1328,6 @@ void launch_kinematic(simp_ctx *c, const State &s, bool diag, bool second) {
     a.rec = tau_rec(c);
     a.diag = diag ? c->diag : nullptr;
     a.pl = pair_list(c);
-    a.n = c->n;
     a.maxn = c->maxn;
     a.single = c->max_inst == 1;
     a.prefetch = prefetch_own(c);
@@ -1353,7 +1350,6 @@ void launch_stress(simp_ctx *c, const State &rhs, const State &base, EpiMode mod
     a.out = (mode == EPI_PREDICT || mode == EPI_EULER) ? c->s1 : c->s0;
     a.cell_start = c->cell_start;
     a.inst = c->inst_dev;
-    a.pinst = c->pinst;
     a.cell = c->cell;
     a.bx = c->bx;
     a.by = c->by;
@@ -1370,7 +1366,6 @@ void launch_stress(simp_ctx *c, const State &rhs, const State &base, EpiMode mod
     a.rates = c->rates;
     a.reg = c->reg;
     a.hs_next = c->tmp;   // hsml of the next step (committed by launch_step_finish)
-    a.n = c->n;
     a.maxn = c->maxn;
     a.mode = mode;
     a.single = c->max_inst == 1;
@@ -1399,7 +1394,6 @@ void launch_regularize(simp_ctx *c, const State &s) {
     a.sc = c->sc;
     a.P = c->phys;
     a.reg = c->reg;
-    a.n = c->n;
     a.maxn = c->maxn;
     k_regularize<<<c->nchunks, kTile, aux_smem_bytes(a.cap), c->stream>>>(a);
     c->launches += 1;
@@ -1424,7 +1418,6 @@ void launch_density_rate(simp_ctx *c, const State &g, const State &v, int rho_up
     a.inst = c->inst_dev;
     a.sc = c->sc;
     a.P = c->phys;
-    a.n = c->n;
     a.rho_upd = rho_upd;
     a.tail = tail ? 1 : 0;
     a.dt_div = (tail && c->prm.tse == 1 && c->prm.artificial_visc) ? 1 : 0;
@@ -1452,7 +1445,6 @@ void launch_sum_density(simp_ctx *c, const State &g, const State &v, const doubl
     a.inst = c->inst_dev;
     a.sc = c->sc;
     a.P = c->phys;
-    a.n = c->n;
     a.rho_upd = 0;
     a.tail = tail ? 1 : 0;
     a.dt_div = (tail && c->prm.tse == 1 && c->prm.artificial_visc) ? 1 : 0;
