@@ -481,6 +481,7 @@ int layout(simp_ctx *c) {
         SIMP_CUDA(c, cudaMemcpyAsync(c->chunk_src, src.data(), sizeof(int4) * src.size(), cudaMemcpyHostToDevice, s));
         launch_chunks(c);
         c->chunks_new = true;
+        TRY(passes_configure(c));
     }
     std::vector<Inst> table(c->max_inst);
     for (int q = 0; q < c->max_inst; ++q) table[q] = c->insts[q].active ? c->insts[q].I : Inst{};
@@ -1044,7 +1045,6 @@ int create(const simp_params *params, int32_t maxn, int32_t maxnb, int32_t max_i
     std::memcpy(&sc.acc_dt, &inf, sizeof(double));
     sc.minip = 0x7fffffff;
     SIMP_CUDA(c, cudaMemcpyAsync(c->sc, c->sc_host, sizeof(Scalars), cudaMemcpyHostToDevice, c->stream));
-    TRY(passes_configure(c));
     TRY(layout(c));
     return SIMP_OK;
 }

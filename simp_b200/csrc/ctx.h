@@ -123,6 +123,7 @@ struct simp_ctx {
     int tile_cap = 1024;
     int halo_cap = 0;
     int l2_bytes = 0;
+    int pass_form = -1;            // form whose kernels passes_configure last prepared
     // rebuild scratch
     int *cnt = nullptr;            // per-cell counters (cell_cap)
     int *perm = nullptr;           // maxn

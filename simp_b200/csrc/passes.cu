@@ -1193,34 +1193,6 @@ PairList pair_list(simp_ctx *c) {
     return pl;
 }
 
-// (calls f with every kernel of a form)
-template <class T, int SKF, int HS, class F>
-void each_pass(F &&f) {
-    f(k_kinematic<T, SKF, HS, 4>);
-    f(k_stress<T, SKF, HS, 4>);
-    if (sizeof(T) == sizeof(float)) {
-        f(k_kinematic<float, SKF, HS, 5>);
-        f(k_stress<float, SKF, HS, 5>);
-    }
-}
-template <class T, int SKF, class F>
-void each_kernel(F &&f) {
-    each_pass<T, SKF, HSML_ONE>(f);
-    each_pass<T, SKF, HSML_VARIED>(f);
-    if (SKF != 0) each_pass<T, SKF, SKF ? HSML_EITHER : HSML_VARIED>(f);   // (the generic kernels' arithmetic is one)
-    f(k_regularize);
-    f(k_density_rate);
-}
-template <class T, int SKF>
-cudaError_t allow_smem() {
-    cudaError_t e = cudaSuccess;
-    const int most = (int)kMostTileSmem;   // (a tile takes 40 to 64 KB)
-    each_kernel<T, SKF>([&](auto *k) {
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    });
-    return e;
-}
-
 // Launches a kernel that calls pass_begin, overlapping the one before it where
 // the context says so (within a step graph: after the kernel before it, which
 // may be any).
@@ -1239,32 +1211,30 @@ void launch_pass(simp_ctx *c, void (*k)(P...), int grid, int block, size_t smem,
     cudaLaunchKernelEx(&cfg, k, args...);   // (an error is found by the caller's next check)
 }
 
-template <class T, int SKF, int HS, int BLOCKS, class A>
-void launch_tiles(simp_ctx *c, const A &a) {
-    const int g = c->nchunks;
-    if constexpr (std::is_same<A, KinArgs>::value)
-        launch_pass(c, k_kinematic<T, SKF, HS, BLOCKS>, g, kTile, tile_smem_bytes(a.cap, 3, c->uniform), a);
-    else
-        launch_pass(c, k_stress<T, SKF, HS, BLOCKS>, g, kTile, stress_smem_bytes(a.cap, Rec<T>::stress_arrays, c->uniform), a);
+// The passes' form of a context's current layout, for f.
+template <class T_, int SKF, int HS, int BLOCKS>
+struct Form {
+    using T = T_;
+    static constexpr int skf = SKF, hs = HS, blocks = BLOCKS;
+};
+template <class T, int SKF, int BLOCKS, class F>
+void with_hsml_form(const simp_ctx *c, F &&f) {
+    if (c->uniform) f(Form<T, SKF, HSML_ONE, BLOCKS>());
+    else if (c->max_inst == 1 || SKF == 0) f(Form<T, SKF, HSML_VARIED, BLOCKS>());   // (the generic kernels' arithmetic is one)
+    else f(Form<T, SKF, SKF ? HSML_EITHER : HSML_VARIED, BLOCKS>());
 }
-template <class T, int SKF, int BLOCKS, class A>
-void launch_hsml_form(simp_ctx *c, const A &a) {
-    if (c->uniform) launch_tiles<T, SKF, HSML_ONE, BLOCKS>(c, a);
-    else if (c->max_inst == 1 || SKF == 0) launch_tiles<T, SKF, HSML_VARIED, BLOCKS>(c, a);
-    else launch_tiles<T, SKF, SKF ? HSML_EITHER : HSML_VARIED, BLOCKS>(c, a);
+template <int SKF, class F>
+void with_kernel_form(const simp_ctx *c, F &&f) {
+    if (c->prm.precision != SIMP_PREC_MIXED) with_hsml_form<double, SKF, 4>(c, f);
+    else if (c->nchunks <= kSmallTiles) with_hsml_form<float, SKF, 4>(c, f);
+    else with_hsml_form<float, SKF, 5>(c, f);
 }
-template <int SKF, class A>
-void launch_kernel_form(simp_ctx *c, const A &a) {
-    if (c->prm.precision != SIMP_PREC_MIXED) launch_hsml_form<double, SKF, 4>(c, a);
-    else if (c->nchunks <= kSmallTiles) launch_hsml_form<float, SKF, 4>(c, a);
-    else launch_hsml_form<float, SKF, 5>(c, a);
-}
-template <class A>
-void launch_form(simp_ctx *c, const A &a) {
+template <class F>
+void with_form(const simp_ctx *c, F &&f) {
     switch (skf_compiled(c->prm.skf)) {
-        case SIMP_SKF_CUBIC: launch_kernel_form<SIMP_SKF_CUBIC>(c, a); break;
-        case SIMP_SKF_WENDLAND_C6: launch_kernel_form<SIMP_SKF_WENDLAND_C6>(c, a); break;
-        default: launch_kernel_form<0>(c, a);
+        case SIMP_SKF_CUBIC: with_kernel_form<SIMP_SKF_CUBIC>(c, f); break;
+        case SIMP_SKF_WENDLAND_C6: with_kernel_form<SIMP_SKF_WENDLAND_C6>(c, f); break;
+        default: with_kernel_form<0>(c, f);
     }
 }
 
@@ -1299,17 +1269,28 @@ void launch_recut(simp_ctx *c) {
     launch_split(c, all);
 }
 
+// Lets the kernels of the current layout's form take their shared memory.  Only
+// those: asking loads a kernel, and loading every form with the first context of
+// a process took 28 to 39 ms instead of 12.
 int passes_configure(simp_ctx *c) {
-    const bool mixed = c->prm.precision == SIMP_PREC_MIXED;
-    cudaError_t e;
-    switch (skf_compiled(c->prm.skf)) {
-        case SIMP_SKF_CUBIC: e = mixed ? allow_smem<float, SIMP_SKF_CUBIC>() : allow_smem<double, SIMP_SKF_CUBIC>(); break;
-        case SIMP_SKF_WENDLAND_C6:
-            e = mixed ? allow_smem<float, SIMP_SKF_WENDLAND_C6>() : allow_smem<double, SIMP_SKF_WENDLAND_C6>();
-            break;
-        default: e = mixed ? allow_smem<float, 0>() : allow_smem<double, 0>();
-    }
+    const int form = (c->uniform ? 1 : 0) | (c->nchunks <= kSmallTiles ? 2 : 0);
+    if (c->pass_form == form) return SIMP_OK;
+    cudaError_t e = cudaSuccess;
+    auto allow = [&](auto *k) {
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostTileSmem);
+    };
+    with_form(c, [&](auto w) {
+        using W = decltype(w);
+        allow(k_kinematic<typename W::T, W::skf, W::hs, W::blocks>);
+        allow(k_stress<typename W::T, W::skf, W::hs, W::blocks>);
+    });
+    // (the passes that enqueue_step and simp_gpu_single_step may add)
+    const simp_params &p = c->prm;
+    if (c->reg) allow(k_regularize);
+    if (p.den_alg == 1 || p.den_alg == 2 || p.sle == 1 || (p.tse == 1 && p.artificial_visc)) allow(k_density_rate);
     if (e != cudaSuccess) return simp_cuda_check(c, e, "cudaFuncSetAttribute (tile shared memory)");
+    c->pass_form = form;
     return SIMP_OK;
 }
 
@@ -1337,7 +1318,11 @@ void launch_kinematic(simp_ctx *c, const State &s, bool diag, bool second) {
     a.halo_walls = c->halo_walls;
     a.cap = tile_cap(c);
     a.second = second ? 1 : 0;
-    launch_form(c, a);
+    with_form(c, [&](auto w) {
+        using W = decltype(w);
+        launch_pass(c, k_kinematic<typename W::T, W::skf, W::hs, W::blocks>, c->nchunks, kTile,
+                    tile_smem_bytes(a.cap, 3, c->uniform), a);
+    });
     c->launches += 1;
 }
 
@@ -1374,7 +1359,11 @@ void launch_stress(simp_ctx *c, const State &rhs, const State &base, EpiMode mod
     a.halos = c->halos;
     a.halo_walls = c->halo_walls;
     a.cap = tile_cap(c);
-    launch_form(c, a);
+    with_form(c, [&](auto w) {
+        using W = decltype(w);
+        launch_pass(c, k_stress<typename W::T, W::skf, W::hs, W::blocks>, c->nchunks, kTile,
+                    stress_smem_bytes(a.cap, Rec<typename W::T>::stress_arrays, c->uniform), a);
+    });
     c->launches += 1;
 }
 
