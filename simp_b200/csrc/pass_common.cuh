@@ -386,6 +386,19 @@ struct StressArgs {
     int cap;
 };
 
+// The two passes' kernels, compiled by kernel function and precision
+// (pass_kernels.cuh), for an hsml form (Hsml) and resident blocks per SM.
+struct PassForm {
+    void (*kin)(KinArgs);
+    void (*stress)(StressArgs);
+};
+PassForm passes_cubic_fp64(int hs, int blocks);
+PassForm passes_cubic_mixed(int hs, int blocks);
+PassForm passes_wendland_fp64(int hs, int blocks);
+PassForm passes_wendland_mixed(int hs, int blocks);
+PassForm passes_generic_fp64(int hs, int blocks);
+PassForm passes_generic_mixed(int hs, int blocks);
+
 // Max / min of 64-bit values over a warp, word by word.
 __device__ __forceinline__ unsigned long long warp_top(unsigned long long v) {
     const unsigned hi = (unsigned)(v >> 32), H = __reduce_max_sync(0xffffffffu, hi);

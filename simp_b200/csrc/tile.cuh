@@ -97,7 +97,7 @@ __device__ __forceinline__ bool bar_wait(unsigned long long *bar, unsigned parit
 // `at` of a wait that failed, so that a thread that looks late does not see one
 // of a wait that others have reached since.
 constexpr int kNoneFailed = 0x7fffffff;
-__device__ __noinline__ void copies_failed(unsigned long long *bar, unsigned parity, int at, int *failed, int *flags) {
+inline __device__ __noinline__ void copies_failed(unsigned long long *bar, unsigned parity, int at, int *failed, int *flags) {
     atomicOr(flags, FLAG_TIMEOUT);
     bar_wait(bar, parity);
     atomicMin(failed, at);
@@ -177,7 +177,7 @@ static_assert(kPartMin == 1 << 3, "part_shift");
 // size, and a lane per row of walls (262,144 particles that move a fifth of hsml
 // between sorts, so that lists are built in every step, FP64, at 528 slots: 288 us
 // per step; 343 with one thread that halved the size until it fitted).
-__device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, const int *bstart, const int *cell, int p0,
+inline __device__ __noinline__ void make_halo(const Inst &I, const int *cell_start, const int *bstart, const int *cell, int p0,
                                        int p1, int shift, int cap, double moved, Halo &h, HaloWalls &hw) {
     const int lane = threadIdx.x & 31;
     const Grid g = inst_grid(I, cell_start);
@@ -292,7 +292,7 @@ __device__ __forceinline__ void tile_fetch(const Halo &h, const TileMem &m, cons
 constexpr double kBand = 0x1p-40;
 
 // The exact reference criterion (nnps.f90:277-281 and the bucket rule).
-__device__ __noinline__ bool exact_pair(const State &s, const Inst &I, bool rule, int i, int j) {
+inline __device__ __noinline__ bool exact_pair(const State &s, const Inst &I, bool rule, int i, int j) {
     const double2 p = s.xy[i], q = s.xy[j];
     double r;
     const double mh = __dmul_rn(__dadd_rn(s.hs[i], s.hs[j]), 0.5);
@@ -301,7 +301,7 @@ __device__ __noinline__ bool exact_pair(const State &s, const Inst &I, bool rule
 }
 // The same for two candidates at slots q0 and q1, as classified: bit 0 and bit 1
 // set where they are pairs.
-__device__ __noinline__ int exact_two(const State &s, const Inst &I, bool rule, int i, const Halo &h, int q0, int q1,
+inline __device__ __noinline__ int exact_two(const State &s, const Inst &I, bool rule, int i, const Halo &h, int q0, int q1,
                                       int in0, int in1) {
     if (in0) in0 = in0 == 1 && !rule ? 1 : exact_pair(s, I, rule, i, particle_of(h, q0));
     if (in1) in1 = in1 == 1 && !rule ? 1 : exact_pair(s, I, rule, i, particle_of(h, q1));
