@@ -657,6 +657,11 @@ int add_instance(simp_ctx *c, int slot, const simp_forcing &f, const Extents &e,
     I.hmin = hmin;
     I.hmax = hmax;
     I.bs = 2.0 * hmin;
+    // (qscale and factor of the compiled kernels, pass_common.cuh: Grad)
+    const bool c6 = c->prm.skf == SIMP_SKF_WENDLAND_C6;
+    const long double H2 = (long double)hmax * hmax;
+    I.grad_k = (double)((c6 ? 1.0L : 4.0L) / H2);
+    I.grad_c = (double)((c6 ? 78.0L : 240.0L) / (7.0L * kPi) / (H2 * H2));
     I.disp = 0.0;
     std::memcpy(&I.xabs_bits, &pxa, sizeof(double));
     I.delta = 0.4 * list_skin(c, hmax);

@@ -76,6 +76,9 @@ struct Inst {
     int list_ok, spares;
     double delta, list_d;
     unsigned long long half2_bits, step2_bits;   // this step's max squared moves, S0 -> S1 and S0 -> S0'
+    // where hsml is one value, of the pair gradients (Grad): (qscale / hsml)^2 and
+    // factor / hsml^4, each rounded once
+    double grad_k, grad_c;
     unsigned long long xabs_bits;   // bound on any particle's |coordinate|, at the step's start: the largest at
                                     // the last sort and the farthest moves since
 };

@@ -176,17 +176,13 @@ struct PairGrad {
         if (SKF == 0) {
             inv_hi = T(1) / h;
         } else if (HS != HSML_VARIED) {
-            const T r = (T)Grad<T, SKF ? SKF : SIMP_SKF_CUBIC>::qscale / h;
-            k = r * r;
+            k = (T)I.grad_k;
         }
     }
     // factor common to all pairs of the particle
-    __device__ __forceinline__ double common() const {
+    __device__ __forceinline__ double common(const Inst &I) const {
         if (SKF == 0) return 1.0;
-        const double f = Grad<T, SKF ? SKF : SIMP_SKF_CUBIC>::factor;
-        if (HS == HSML_VARIED || !one) return f;
-        const double ih = 1.0 / (double)hi;
-        return f * ((ih * ih) * (ih * ih));
+        return HS == HSML_VARIED || !one ? Grad<T, SKF ? SKF : SIMP_SKF_CUBIC>::factor : I.grad_c;
     }
     __device__ __forceinline__ T operator()(const Phys &P, T s, T hj) const {
         if constexpr (SKF == 0) {

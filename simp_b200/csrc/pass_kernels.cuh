@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_const
             ks = sizeof(T) == sizeof(double) ? kin_stencil_call<T, SKF, HS>(a, I, h, i) : kin_stencil<T, SKF, HS>(a, I, h, i);
         }
         if (live) {
-            const double c = -grad.common();
+            const double c = -grad.common(I);
             kin_rheology(a, i, c * ks.dv.get(), c * ks.g1.get(), c * ks.g23.get(), c * ks.g4.get());
         }
         p0 += h.size;
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant
         // stays as it was until the batch's next compaction drops them)
         double S[4];
         auto pair_sums = [&] {
-            const double c = grad.common();
+            const double c = grad.common(I);
             S[0] = c * ss.sx.get();
             S[1] = c * ss.sy.get();
             S[2] = c * ss.tx.get();
