@@ -250,10 +250,10 @@ __device__ __noinline__ KinSums<T> kin_stencil_call(const KinArgs &a, const Inst
 
 // Kinematic pass over tiles.  Bound by shared memory and latency: a block waits
 // for its tile's copies, then reads three 16-byte records per pair at slots that
-// have no order, so that their banks collide (L1 55% busy in FP64, 70% mixed;
-// issue slots 31% and 51%).  Two candidates at a time put six such reads in
-// flight.  262,144 particles, FP64: 79 -> 40 us per pass against gathers from
-// global memory; mixed at 1,048,576: 237 -> 132 us.
+// have no order, so that their banks collide (L1 57% busy in FP64, 73% mixed;
+// issue slots 32% and 54%).  Two candidates at a time put six such reads in
+// flight.  262,144 particles, FP64: 79 -> 38 us per pass against gathers from
+// global memory; mixed at 1,048,576: 237 -> 124 us.
 template <class T, int SKF, int HS, int BLOCKS>
 __global__ void __launch_bounds__(kBlock, BLOCKS) k_kinematic(const __grid_constant__ KinArgs a) {
     constexpr bool UNIFORM = HS == HSML_ONE;
@@ -429,9 +429,9 @@ __device__ __noinline__ StressSums<T> stress_stencil_call(const StressArgs &a, c
 // Stress pass over the same tiles, then the epilogue, whose twenty own values
 // are loaded together ahead of the walls and the update (68 -> 50 us against
 // loading each where it is used).  Half of a block's time is the latency of its
-// copies and of that epilogue (issue slots 29%, L1 50%).  262,144 particles,
-// FP64: 71 -> 44 us per pass against gathers from global memory; mixed at
-// 1,048,576: 192 -> 147 us.
+// copies and of that epilogue (issue slots 30%, L1 52%).  262,144 particles,
+// FP64: 71 -> 45 us per pass against gathers from global memory; mixed at
+// 1,048,576: 192 -> 149 us.
 template <class T, int SKF, int HS, int BLOCKS>
 __global__ void __launch_bounds__(kBlock, BLOCKS) k_stress(const __grid_constant__ StressArgs a) {
     constexpr bool UNIFORM = HS == HSML_ONE;

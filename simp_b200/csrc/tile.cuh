@@ -182,8 +182,9 @@ inline __device__ __noinline__ void make_halo(const Inst &I, const int *cell_sta
     const int lane = threadIdx.x & 31;
     const Grid g = inst_grid(I, cell_start);
     // The farthest of a basin's particles are few: with the tile's own distance
-    // for one side of a pair, the tiles of the others keep a radius of 1 (one
-    // step of 262,144 particles of which some race along a wall: 260 -> 237 us).
+    // for one side of a pair, the tiles of the others keep a smaller radius (one
+    // particle in a thousand moves a fifth of hsml between sorts, FP64: 262,144
+    // particles 243 -> 208 us per step, 1,048,576 875 -> 692).
     const double disp = inst_disp(I);
     const int R = stencil_radius(I.hmax, 0.5 * (fmin(moved, disp) + disp), g, I.hmax + I.delta);
     const int e = min(p0 + max((kParts - lane) << shift, 1), p1);

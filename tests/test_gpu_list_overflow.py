@@ -162,10 +162,10 @@ def test_sparse_rows_stay_cut_as_others_join(gpu_lib, tiles):
 
 
 def test_parts_after_motion(gpu_lib, tiles):
-    """Five rows of cells of a large basin, whose tiles hold a halo of 576: 13
-    lattice rows of 43 columns, 13 of which lie beside the part.  A part then has
-    30 columns of the cell row's two or three lattice rows, 60 to 90 particles,
-    so that a tile takes two or three parts."""
+    """Five rows of cells of a large basin, whose tiles hold a halo of 576.  A cell
+    is three lattice spacings wide: 15 lattice rows of 38 columns, some 14 of
+    which lie beside the part.  A part then has 24 columns of the cell row's three
+    lattice rows, 72 particles, so that a tile takes two parts, three at times."""
     b = basins.make_basin(384, 2000.0, 5, walls="", dt=1.0)
     b.vx = smooth_velocity(b.x, b.L, amp=0.3, seed=4) + np.array([60.0, 30.0])
     b.params.wind_force = b.params.water_force = 0
