@@ -248,13 +248,15 @@ int32_t simp_server_create(const simp_params *params, const simp_server_config *
         budget -= spot_n * (simp::bytes_per_particle(p64, single) + kBytesPerWall / kWallsPerParticleDiv);
     }
     // a budget that would hold the largest request but not the tiles of so many
-    // basins holds fewer of them at once
+    // basins holds fewer of them at once, and is not refused for the fewest's
+    // (0.2 MB)
+    const double least = std::floor(budget / per) >= cfg->max_request_particles ? cfg->max_request_particles : 0.0;
     const double slot = simp::bytes_per_basin();
     const double room = std::floor((budget - per * cfg->max_request_particles) / slot);
     const double share = std::min(1.0, std::max(0.0, room / (s->slots_main + s->slots_spot)));
     for (int *k : {&s->slots_main, &s->slots_spot}) *k = std::max((int)(*k * share), std::min(*k, 2));
     budget -= slot * (s->slots_main + s->slots_spot);
-    const double cap = std::floor(budget / per);
+    const double cap = std::max(std::floor(budget / per), least);
     if (cap < cfg->max_request_particles)
         return fail(s, SIMP_ERR_NOMEM, "the budget does not hold the largest request");
     s->maxn_main = (int)std::min(cap, 2.0e9);

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from simp_b200 import basins, serve
-from simp_b200.simp import Batch
+from simp_b200.simp import Batch, SimpError
 
 pytestmark = pytest.mark.gpu
 
@@ -40,3 +40,15 @@ def test_a_tight_budget_holds_fewer_basins(gpu_lib, spot):
                 slot = alone.add(r.basin)
                 alone.step(r.nsteps)
                 assert np.array_equal(s.outputs[i]["vx"], alone.get_state(slot)["vx"])
+
+
+@pytest.mark.parametrize("instances", [2, 1024])
+def test_a_budget_of_just_the_largest_request_is_accepted(gpu_lib, instances):
+    """The tiles of the fewest basins a batch may hold refuse no budget that holds the largest request itself."""
+    prm = basins.instance(0, 1000).params
+    per = 3.0e8 / (_capacity(prm, 6.0e8, 2) - _capacity(prm, 3.0e8, 2))   # bytes per particle, to 1e-5
+    n = 100_000
+    with serve.Server(prm, per * n * (1.0 + 1e-4), max_instances=instances, max_request_particles=n) as s:
+        assert s.stats()["capacity_particles"] == n
+    with pytest.raises(SimpError):
+        serve.Server(prm, per * n * (1.0 - 1e-4), max_instances=instances, max_request_particles=n)
