@@ -278,10 +278,8 @@ Phys make_phys(const simp_params &p, double max_hsml) {
     P.delta_min = p.delta_min;
     P.k_t = p.k_t;
     P.rho_ice = p.rho_ice;
-    P.rho_air = p.rho_air;
-    P.rho_water = p.rho_water;
-    P.c_wind = p.c_wind;
-    P.c_water = p.c_water;
+    P.k_wind = (double)((long double)p.c_wind * p.rho_air / p.rho_ice);
+    P.k_water = (double)((long double)p.c_water * p.rho_water / p.rho_ice);
     P.b_length = p.b_length;
     P.kappa_n = p.kappa_n;
     P.alpha = p.alpha;

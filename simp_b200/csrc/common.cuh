@@ -151,7 +151,7 @@ struct Phys {
     int max_ind_int;
     int nnps;       // 1 direct search, 2 bucket search (the pair orientation)
     double P_star, c_eos, e, delta_min, k_t;
-    double rho_ice, rho_air, rho_water, c_wind, c_water;
+    double rho_ice, k_wind, k_water;   // k: c_wind rho_air / rho_ice and c_water rho_water / rho_ice, rounded once
     double b_length, kappa_n, alpha;
     double wind_u, wind_v, current_u, current_v;
     double vortex_x, vortex_y, vortex_umax, vortex_radius;

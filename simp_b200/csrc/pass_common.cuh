@@ -539,13 +539,13 @@ __device__ __forceinline__ void stress_finish(const StressArgs &a, int i, bool l
         double wu, wv;
         wind_at(I, xi, yi, &wu, &wv);
         const double ru = wu - vxi, rv = wv - vyi;
-        const double k = P.c_wind * P.rho_air * P.inv_rho_ice * ih;
+        const double k = P.k_wind * ih;
         ax += k * ru * fabs(ru);
         ay += k * rv * fabs(rv);
     }
     if (P.water_force && tnow > 0.0) {
         const double ru = P.current_u - vxi, rv = P.current_v - vyi;
-        const double k = P.c_water * P.rho_water * P.inv_rho_ice * ih;
+        const double k = P.k_water * ih;
         ax += k * ru * fabs(ru);
         ay += k * rv * fabs(rv);
     }
