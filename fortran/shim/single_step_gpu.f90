@@ -5,7 +5,7 @@
 !   state to the library and reads the rates dxdt, dvxdt, dhdt, dAdt      !
 !   back.  While the state continues the one of the previous call (same   !
 !   particles, walls and hsml, moved less than a cell) the library keeps  !
-!   its sort and neighbour lists, so a call costs the two copies and one  !
+!   its sort and cell lists, so a call costs the two copies and one       !
 !   right-hand side.  Link with -lsimp_gpu; compile simp_gpu_mod.f90 and  !
 !   simp_host_params.f90 first, and leave the reference's single_step.f90 out of the build.    !
 !!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!!
